@@ -613,7 +613,7 @@ int32_t yule_cuda_prepare_weights(yule_cuda_ctx *ctx, yule_buffer weights, uint3
         return fail(YULE_ERR_INVALID_ARGUMENT, "n_cols %u is not a multiple of the block size", n_cols);
     FIND(ctx, weights, W);
     NEED_BYTES(W, tensor_bytes(gguf_type, n_rows, n_cols), "prepare_weights");
-    if (gguf_type != YULE_DTYPE_Q6_K || !q6k_mma_supported(n_cols) || n_rows == 0) return YULE_OK;
+    if (gguf_type != YULE_DTYPE_Q6_K || n_rows == 0) return YULE_OK;
     const uint64_t n_blocks = (uint64_t)n_rows * (n_cols / 256);
     if (W.planar && W.planar_blocks == n_blocks && W.planar_cols == n_cols) return YULE_OK;
     if (W.planar) {

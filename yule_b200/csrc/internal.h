@@ -21,24 +21,6 @@
 // Both are no-ops for a normal launch.
 __device__ __forceinline__ void yule_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void yule_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Asks L2 to fetch [p, p + bytes) from HBM without waiting for it (p 16-byte aligned, bytes a
-// multiple of 16).  Used by a matvec to pull in the weights of the kernel that runs after it,
-// so HBM keeps streaming across the dependency between the two.
-__device__ __forceinline__ void yule_prefetch_l2(const void *p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-// Each CTA takes an equal 16-byte-granular slice of [base, base + bytes) and prefetches it in
-// pieces of at most 32 KB from one thread.
-__device__ __forceinline__ void yule_prefetch_l2_slice(const void *base, uint64_t bytes) {
-    if (!base || threadIdx.x != 0) return;
-    const uint64_t per = ((bytes / gridDim.x) + 15) & ~(uint64_t)15;
-    uint64_t lo = (uint64_t)blockIdx.x * per;
-    uint64_t hi = lo + per < bytes ? lo + per : (bytes & ~(uint64_t)15);
-    for (; lo < hi; lo += 32768) {
-        const uint64_t n = hi - lo < 32768 ? hi - lo : 32768;
-        yule_prefetch_l2(reinterpret_cast<const char *>(base) + lo, (uint32_t)n);
-    }
-}
 #endif
 
 namespace yule {
@@ -214,24 +196,42 @@ struct QmvArgs {
     const float *residual = nullptr;  // out[row] = residual[row] + dot   (o-proj / down-proj)
     bool pdl = false;                 // programmatic dependent launch
     // With pdl: none of this call's inputs (x, residual) is written by the previous kernel of the stream, so
-    // only this kernel's stores have to wait for it (Q4_K / Q6_K tensor-pipe kernels; ignored elsewhere).
+    // only this kernel's stores have to wait for it (one-vector and Q8_0 / Q4_0 batch kernels; ignored elsewhere).
     bool late_wait = false;
     const uint8_t *planar = nullptr;  // Q6_K: planar copy of the same tensor, when one was prepared
-    const float *norm_w = nullptr;    // RMSNorm prologue (planar Q6_K and Q4_K paths only)
+    const float *norm_w = nullptr;    // RMSNorm prologue (one-vector kernel and kquant_batch_can_share only)
     float eps = 0.f;
-    const void *next_w[2] = {nullptr, nullptr};  // tensor-pipe paths: weights to prefetch into L2
-    uint64_t next_bytes[2] = {0, 0};
-    TpFuse tp;                        // Q4_K tensor-pipe path only
+    TpFuse tp;                        // one vector of Q4_K only
     int *status = nullptr;            // device status word for bounded waits inside the kernels, or null
     long long wait_cycles = kDefaultWaitCycles;
 };
 cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t *launches);
-// Q8_0 / Q4_0 on the tensor pipe from a shared-memory ring (qmv_q8q4_ring.cu): n_cols a multiple of 256, weights and
-// activations 16-byte aligned, one activation vector.
-bool q8q4_ring_supported(const QmvArgs &a);
-cudaError_t launch_q8q4_ring(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t *launches);
-// The same kernels over two to four activation vectors per pass: the number of vectors one pass can take for this
-// call (0: not supported), and one pass over the first `nb` vectors of `a`.
+// One activation vector against one to three matrices of one format (qmv_digits.cu).
+struct QmvDigits {
+    uint32_t type = 0;
+    const uint8_t *w[3] = {nullptr, nullptr, nullptr};  // raw blocks, 16-byte aligned; Q6_K: the row-planar copies
+    float *out[3] = {nullptr, nullptr, nullptr};
+    uint32_t rows[3] = {0, 0, 0};
+    uint32_t n_seg = 1;
+    const float *x = nullptr;
+    uint32_t n_cols = 0;              // a multiple of 256
+    const float *norm_w = nullptr;    // RMSNorm prologue on x when set
+    float eps = 0.f;
+    const float *residual = nullptr;  // out[0] += residual when set
+    bool swiglu_pair = false;         // w[0], w[1] = gate, up → out[0] = SiLU(gate)·up (qmv_digits_can_pair)
+    bool pdl = false;                 // programmatic dependent launch
+    bool late_wait = false;           // with pdl: inputs do not come from the previous kernel; only the stores wait for it
+    TpFuse tp;                        // Q4_K: pushes out[0] to the peers / waits for a gathered x
+    int *status = nullptr;            // device status word for the kernel's bounded waits, or null
+    long long wait_cycles = kDefaultWaitCycles;
+};
+bool qmv_digits_supported(uint32_t type, const void *w, uint32_t n_cols);
+bool qmv_digits_can_pair(uint32_t n_cols);
+cudaError_t launch_qmv_digits(const QmvDigits &f, int sm_count, cudaStream_t s, uint64_t *launches);
+
+// Q8_0 / Q4_0 over two to four activation vectors per pass (qmv_q8q4_ring.cu: n_cols a multiple of 256, weights and
+// activations 16-byte aligned): the number of vectors one pass can take for this call (0: not supported), and one pass
+// over the first `nb` vectors of `a`.
 uint32_t q8q4_ring_batch_width(const QmvArgs &a);
 cudaError_t launch_q8q4_ring_batch(const QmvArgs &a, uint32_t nb, int sm_count, cudaStream_t s, uint64_t *launches);
 
@@ -282,61 +282,24 @@ cudaError_t launch_qgemm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t 
 cudaError_t launch_qgemm_xprep(const QGemm &g, cudaStream_t s, uint64_t *launches);
 cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
 
-// Q4_K tensor-pipe matvec with the neighbouring ops folded in (qmv_q4k_mma.cu).
-struct Q4kFused {
-    const uint8_t *w[3] = {nullptr, nullptr, nullptr};  // up to three matrices sharing x
-    float *out[3] = {nullptr, nullptr, nullptr};
-    uint32_t rows[3] = {0, 0, 0};
-    uint32_t out_stride[3] = {0, 0, 0};
-    uint32_t n_seg = 1;
-    const float *x = nullptr;  // [batch][x_stride]
-    uint32_t x_stride = 0, n_cols = 0, batch = 1;
-    const float *norm_w = nullptr;    // RMSNorm prologue on x when set
-    float eps = 0.f;
-    const float *residual = nullptr;  // out[0] += residual when set
-    bool swiglu_pair = false;         // w[0], w[1] = gate, up → out[0] = SiLU(gate)·up
-    bool q5 = false;                  // the matrices are Q5_K (176-byte super-blocks), 16-byte aligned
+// Q4_K / Q5_K over two to four activation vectors per pass on fp16 fragments (qmv_q4k_mma.cu).
+struct Q4kBatch {
+    const uint8_t *w = nullptr;       // 16-byte aligned
+    float *out = nullptr;             // [batch][out_stride]
+    uint32_t rows = 0, out_stride = 0;
+    const float *x = nullptr;         // [batch][x_stride]
+    uint32_t x_stride = 0, n_cols = 0, batch = 2;
+    const float *residual = nullptr;  // added to out when set (same layout)
+    bool q5 = false;                  // Q5_K (176-byte super-blocks)
     bool pdl = false;                 // programmatic dependent launch
-    bool late_wait = false;           // with pdl: inputs do not come from the previous kernel; only the stores wait for it
-    const void *next_w[2] = {nullptr, nullptr};  // weights of the kernel(s) that follow: prefetched into L2
-    uint64_t next_bytes[2] = {0, 0};
-    TpFuse tp;                        // pushes out[0] to the peers / waits for a gathered x
-    int *status = nullptr;            // device status word for the kernel's own bounded waits, or null
-    long long wait_cycles = kDefaultWaitCycles;
 };
 bool q4k_mma_supported(uint32_t n_cols, uint32_t batch);
-// Routes to the shared-memory-ring kernel (qmv_q4k_ring.cu) when it takes the case, else to the
-// register-streaming kernel of qmv_q4k_mma.cu.
-cudaError_t launch_q4k_mma(const Q4kFused &f, int sm_count, cudaStream_t s, uint64_t *launches);
-bool q4k_ring_supported(const Q4kFused &f);
-cudaError_t launch_q4k_ring(const Q4kFused &f, int sm_count, cudaStream_t s, uint64_t *launches);
+cudaError_t launch_q4k_mma(const Q4kBatch &f, int sm_count, cudaStream_t s, uint64_t *launches);
 
-// Q6_K tensor-pipe matvec over the row-planar device copy of a tensor (qmv_q6k_ring.cu).
-struct Q6kPlanar {
-    const uint8_t *planar = nullptr;  // per row: ql | qh | scales | d of all its blocks, built by launch_q6k_repack
-    float *out = nullptr;
-    uint32_t n_rows = 0, n_cols = 0;
-    const float *x = nullptr;
-    const float *norm_w = nullptr;    // RMSNorm prologue on x when set
-    float eps = 0.f;
-    const float *residual = nullptr;  // out += residual when set
-    bool pdl = false;
-    bool late_wait = false;           // with pdl: inputs do not come from the previous kernel; only the stores wait for it
-    const void *next_w[2] = {nullptr, nullptr};  // unused by the ring kernel (its successor fetches its own weights early)
-    uint64_t next_bytes[2] = {0, 0};
-    int *status = nullptr;            // device status word for the kernel's bounded waits, or null
-    long long wait_cycles = kDefaultWaitCycles;
-};
+// Row-planar device copy of a Q6_K tensor (q6k_planar.cu): n_cols a multiple of 256.
 size_t q6k_planar_bytes(uint64_t n_rows, uint32_t n_cols);
 cudaError_t launch_q6k_repack(const uint8_t *raw, uint8_t *planar, uint64_t n_rows, uint32_t n_cols, cudaStream_t s,
                               uint64_t *launches);
-bool q6k_mma_supported(uint32_t n_cols);
-// Shared-memory-ring kernel (qmv_q6k_ring.cu): the kernel of calls whose inputs do not depend on the previous
-// kernel (late wait), which overlap with it on the same SMs.
-cudaError_t launch_q6k_mma(const Q6kPlanar &f, int sm_count, cudaStream_t s, uint64_t *launches);
-// Register-streaming kernel (qmv_q6k_mma.cu): the kernel of dependent chains.
-bool q6k_stream_supported(uint32_t n_cols);
-cudaError_t launch_q6k_stream(const Q6kPlanar &f, int sm_count, cudaStream_t s, uint64_t *launches);
 
 // Tensor parallelism (tp.cu).
 struct NcclId {

@@ -191,47 +191,7 @@ size_t smem_bytes(uint32_t n_cols, uint32_t nb) {
 
 constexpr int kThreadsCta = kGroups * kWarps * 32;  // 512
 
-// Kept out of line: the tensor-parallel path must not cost the single-GPU kernels registers.
-__device__ __noinline__ void tp_push_value(const TpFuse &tp, size_t o, float v) {
-    const uint2 pair = make_uint2(__float_as_uint(v), *tp.tick * tp.epochs_per_tick + tp.push_index + 1u);
-    for (uint32_t pp = 0; pp < tp.world; pp++)  // one 8-byte store each
-        asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(tp.pair_out[pp] + o), "r"(pair.x), "r"(pair.y) : "memory");
-}
-// Eight consecutive elements of a gathered vector from its (value, epoch) pairs: polls until all eight
-// carry `epoch`.  Bounded, and bounded once per failure: the first wait that runs out of `budget` cycles
-// writes the status word, and every wait that starts (or polls) after that returns at once, so a lost peer
-// costs one budget per kernel in flight, not one per wait.  The values returned after a give-up are
-// whatever the buffer held; the host reads the status word and discards the step.
-__device__ __forceinline__ void tp_load8(const uint2 *pairs, uint32_t epoch, int *status, long long budget, float (&a)[8]) {
-    long long t0 = 0;
-    for (uint32_t it = 0;; it++) {
-        uint4 q[4];
-        // one 16-byte load per two pairs: value and epoch of a pair must come from the same access
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(q[i].x), "=r"(q[i].y), "=r"(q[i].z), "=r"(q[i].w)
-                         : "l"(pairs + 2 * i)
-                         : "memory");
-        bool ok = true;
-#pragma unroll
-        for (int i = 0; i < 4; i++) ok = ok && q[i].y == epoch && q[i].w == epoch;
-        if (!ok) {
-            if (it == 0) t0 = clock64();
-            if (it != 0 && (it & 63u) != 63u) continue;
-            if (*reinterpret_cast<volatile int *>(status) == 0) {
-                if (clock64() - t0 < budget) continue;
-                atomicCAS(status, 0, kStatusPeerTimeout);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            a[2 * i] = __uint_as_float(q[i].x);
-            a[2 * i + 1] = __uint_as_float(q[i].z);
-        }
-        return;
-    }
-}
+#include "tp_pairs.cuh"
 
 // Stage NB activation vectors: optional RMSNorm, power-of-two normalisation, hi/lo split,
 // fragment order, per-32-column sums.  Each thread owns groups of 8 consecutive columns; the first
@@ -452,58 +412,4 @@ __device__ __forceinline__ RowScalesF unpack_scales_f(const uint4 &hdr, int u, b
     r.mn[2] = (__uint_as_float(__byte_perm(mn4, 0x4B000000u, 0x7442)) - k23) * dmin;
     r.mn[3] = (__uint_as_float(__byte_perm(mn4, 0x4B000000u, 0x7443)) - k23) * dmin;
     return r;
-}
-
-template <int NR, bool Q5>
-__device__ __forceinline__ void consume_block_subcol(const BlockLoads (&ld)[NR], const uint4 *bp, const float *sfp, int u,
-                                                     int t, bool charge_mins, float (&acc)[NR][2]) {
-    float dl[4] = {0.f, 0.f, 0.f, 0.f}, dh[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int wp = 0; wp < 4; wp++) {
-        const uint4 bl = bp[wp * 8], bh = bp[32 + wp * 8];
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int wi = 2 * wp + e;
-            uint32_t lo02[2], lo13[2], hi02[2], hi13[2];
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                const uint32_t w = word_of(ld[r], wi), w8 = w >> 8;
-                if (Q5) {
-                    // four 5-bit values per register first (nibble | fifth bit << 4), then one byte
-                    // permute per operand: both halves of the word are q·2^-24 (no factor 16 on the
-                    // high nibbles, see unpack_scales_f)
-                    const uint32_t f = fifth_word<Q5>(ld[r], wi) >> (2 * t);
-                    const uint32_t cl = (w & 0x0F0F0F0Fu) | ((f << 4) & 0x10101010u);
-                    const uint32_t ch = ((w >> 4) & 0x0F0F0F0Fu) | ((f << 3) & 0x10101010u);
-                    lo02[r] = __byte_perm(cl, 0u, 0x4240);
-                    lo13[r] = __byte_perm(cl, 0u, 0x4341);
-                    hi02[r] = __byte_perm(ch, 0u, 0x4240);
-                    hi13[r] = __byte_perm(ch, 0u, 0x4341);
-                } else {
-                    lo02[r] = w & 0x000F000Fu;
-                    lo13[r] = w8 & 0x000F000Fu;
-                    hi02[r] = w & 0x00F000F0u;
-                    hi13[r] = w8 & 0x00F000F0u;
-                }
-            }
-            if (NR == 1) lo02[1] = lo13[1] = hi02[1] = hi13[1] = 0u;
-            mma_16816(dl, lo02[0], lo02[1], lo13[0], lo13[1], e ? bl.z : bl.x, e ? bl.w : bl.y);
-            mma_16816(dh, hi02[0], hi02[1], hi13[0], hi13[1], e ? bh.z : bh.x, e ? bh.w : bh.y);
-        }
-    }
-    const float4 sx = *reinterpret_cast<const float4 *>(sfp);  // Σx of sub-blocks 4u..4u+3
-#pragma unroll
-    for (int r = 0; r < NR; r++) {
-        const RowScalesF rs = unpack_scales_f<Q5>(ld[r].hdr, u, charge_mins);
-        float a = acc[r][0];
-        a = fmaf(rs.sc[0], dl[2 * r + 0], a);
-        a = fmaf(rs.sc[1], dh[2 * r + 0], a);
-        a = fmaf(rs.sc[2], dl[2 * r + 1], a);
-        a = fmaf(rs.sc[3], dh[2 * r + 1], a);
-        float m = rs.mn[0] * sx.x;
-        m = fmaf(rs.mn[1], sx.y, m);
-        m = fmaf(rs.mn[2], sx.z, m);
-        m = fmaf(rs.mn[3], sx.w, m);
-        acc[r][0] = a - m;
-    }
 }

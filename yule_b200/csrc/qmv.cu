@@ -566,43 +566,60 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
         }
         return cudaSuccess;
     }
-    const bool q5_mma = a.type == YULE_DTYPE_Q5_K && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0 && !a.tp.push && !a.tp.wait;
-    if ((a.type == YULE_DTYPE_Q4_K || q5_mma) && q4k_mma_supported(a.n_cols, 1)) {
-        // tensor-pipe path, up to four activation vectors per pass over the weights
-        uint32_t done = 0;
-        while (done < a.batch) {
-            uint32_t nb = a.batch - done < 4 ? a.batch - done : 4;
-            while (!q4k_mma_supported(a.n_cols, nb)) nb--;
-            Q4kFused f;
-            f.w[0] = a.w;
-            f.out[0] = a.out + (size_t)done * a.out_stride;
+    // one vector, tuned block format (Q6_K: prepared): the fp8-digit kernel
+    if (a.batch == 1) {
+        const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
+        if (qmv_digits_supported(a.type, w, a.n_cols) && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0) {
+            QmvDigits f;
+            f.type = a.type;
+            f.w[0] = w;
+            f.out[0] = a.out;
             f.rows[0] = a.n_rows;
-            f.out_stride[0] = a.out_stride;
-            f.n_seg = 1;
-            f.q5 = q5_mma;
-            f.x = a.x + (size_t)done * a.x_stride;
-            f.x_stride = a.x_stride;
+            f.x = a.x;
             f.n_cols = a.n_cols;
-            f.batch = nb;
-            f.residual = a.residual ? a.residual + (size_t)done * a.out_stride : nullptr;
             f.norm_w = a.norm_w;
             f.eps = a.eps;
+            f.residual = a.residual;
             f.pdl = a.pdl;
             f.late_wait = a.late_wait;
             f.tp = a.tp;
             f.status = a.status;
             f.wait_cycles = a.wait_cycles;
-            for (int i = 0; i < 2; i++) {
-                f.next_w[i] = a.next_w[i];
-                f.next_bytes[i] = a.next_bytes[i];
-            }
+            return launch_qmv_digits(f, sm_count, s, launches);
+        }
+    }
+    const bool q5_mma = a.type == YULE_DTYPE_Q5_K && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
+    if (a.batch > 1 && (a.type == YULE_DTYPE_Q4_K || q5_mma) && q4k_mma_supported(a.n_cols, 2)) {
+        // up to four activation vectors per pass over the weights
+        uint32_t done = 0;
+        while (done < a.batch) {
+            QmvArgs part = a;
+            part.x = a.x + (size_t)done * a.x_stride;
+            part.out = a.out + (size_t)done * a.out_stride;
+            part.residual = a.residual ? a.residual + (size_t)done * a.out_stride : nullptr;
+            part.batch = a.batch - done;
+            if (part.batch == 1) return launch_qmv(part, sm_count, s, launches);
+            uint32_t nb = part.batch < 4 ? part.batch : 4;
+            while (!q4k_mma_supported(a.n_cols, nb)) nb--;
+            Q4kBatch f;
+            f.w = a.w;
+            f.out = part.out;
+            f.rows = a.n_rows;
+            f.out_stride = a.out_stride;
+            f.q5 = q5_mma;
+            f.x = part.x;
+            f.x_stride = a.x_stride;
+            f.n_cols = a.n_cols;
+            f.batch = nb;
+            f.residual = part.residual;
+            f.pdl = a.pdl;
             cudaError_t e = launch_q4k_mma(f, sm_count, s, launches);
             if (e != cudaSuccess) return e;
             done += nb;
         }
         return cudaSuccess;
     }
-    if (a.type == YULE_DTYPE_Q6_K && a.planar && a.batch > 1 && a.batch <= 8 && q6k_mma_supported(a.n_cols) && q6k_stream_supported(a.n_cols)) {
+    if (a.type == YULE_DTYPE_Q6_K && a.planar && a.batch > 1 && a.batch <= 8) {
         // rows too long for the batched kernel's activation image: one pass of the one-vector kernel per vector
         for (uint32_t b = 0; b < a.batch; b++) {
             QmvArgs one = a;
@@ -615,29 +632,6 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
         }
         return cudaSuccess;
     }
-    if (a.type == YULE_DTYPE_Q6_K && a.planar && a.batch == 1 && q6k_mma_supported(a.n_cols) && q6k_stream_supported(a.n_cols)) {
-        Q6kPlanar f;
-        f.planar = a.planar;
-        f.out = a.out;
-        f.n_rows = a.n_rows;
-        f.n_cols = a.n_cols;
-        f.x = a.x;
-        f.norm_w = a.norm_w;
-        f.eps = a.eps;
-        f.residual = a.residual;
-        f.pdl = a.pdl;
-        f.late_wait = a.late_wait;
-        f.status = a.status;
-        f.wait_cycles = a.wait_cycles;
-        // independent call → ring kernel (overlaps with its predecessor; measured against the streaming kernel: 5.1 / 6.7 µs at
-        // 4096x4096, 12.7 / 14.5 at 14336x4096, 93 / 91 at 128256x4096); dependent chain or very long matrix → streaming kernel
-        bool ring = a.pdl && a.late_wait && (a.n_rows + 15) / 16 <= 8u * (uint32_t)sm_count;
-        if (const char *k = knob("YULE_QMV_RING")) ring = atoi(k) != 0;
-        return ring ? launch_q6k_mma(f, sm_count, s, launches) : launch_q6k_stream(f, sm_count, s, launches);
-    }
-    // Q8_0 / Q4_0, one vector, 256-column multiples: the tensor-pipe ring kernel (YULE_QMV_Q8Q4_RING=0: the SIMT kernel)
-    if (q8q4_ring_supported(a) && !(knob("YULE_QMV_Q8Q4_RING") && atoi(knob("YULE_QMV_Q8Q4_RING")) == 0))
-        return launch_q8q4_ring(a, sm_count, s, launches);
     // Q8_0 / Q4_0, several vectors: two to four per pass of the batched ring kernel, a single left-over vector on the
     // one-vector kernel
     if (q8q4_ring_batch_width(a) >= 2 && !(knob("YULE_QMV_Q8Q4_RING") && atoi(knob("YULE_QMV_Q8Q4_RING")) == 0)) {
@@ -655,19 +649,12 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
                 done += nb;
             } else {
                 part.batch = 1;
-                if (!q8q4_ring_supported(part)) break;  // the SIMT kernels below take the rest
-                e = launch_q8q4_ring(part, sm_count, s, launches);
+                e = launch_qmv(part, sm_count, s, launches);
                 done += 1;
             }
             if (e != cudaSuccess) return e;
         }
-        if (done == a.batch) return cudaSuccess;
-        QmvArgs rest = a;
-        rest.x = a.x + (size_t)done * a.x_stride;
-        rest.out = a.out + (size_t)done * a.out_stride;
-        rest.residual = a.residual ? a.residual + (size_t)done * a.out_stride : nullptr;
-        rest.batch = a.batch - done;
-        return launch_qmv(rest, sm_count, s, launches);
+        return cudaSuccess;
     }
     if (qmv_smem_bytes(a.type, a.n_cols, 1) > kMaxSmem) return cudaErrorInvalidValue;
     uint32_t done = 0;

@@ -247,24 +247,6 @@ struct Step {
     void ok(cudaError_t e) {
         if (err == cudaSuccess && e != cudaSuccess) err = e;
     }
-    // Weights of the kernel(s) that will run next; the tensor-pipe matvecs prefetch them into L2.
-    const void *next_w[2] = {nullptr, nullptr};
-    uint64_t next_bytes[2] = {0, 0};
-    void then(const Tensor *a, const Tensor *b = nullptr) {
-        const Tensor *ts[2] = {a, b};
-        // measured neutral-to-slightly-negative on the TinyLlama-size step, so off unless asked for
-        static const bool enabled = knob("YULE_CUDA_PREFETCH") && atoi(knob("YULE_CUDA_PREFETCH")) != 0;
-        if (!enabled) ts[0] = ts[1] = nullptr;
-        for (int i = 0; i < 2; i++) {
-            const Tensor *t = ts[i];
-            next_w[i] = nullptr;
-            next_bytes[i] = 0;
-            if (!t || !t->set) continue;
-            // the bytes the next kernel will actually read: the planar copy when there is one
-            next_w[i] = t->buf.planar ? (const void *)t->buf.planar : t->buf.ptr;
-            next_bytes[i] = t->buf.planar ? q6k_planar_bytes(t->buf.planar_blocks / (t->buf.planar_cols / 256), t->buf.planar_cols) - 256 : t->buf.size;
-        }
-    }
     // norm_w set: RMSNorm of x folded into the matvec (only valid when fusable(w, cols) holds)
     void qmv(const Tensor &w, const float *x, float *out, uint32_t rows, uint32_t cols, const float *residual = nullptr,
              const float *norm_w = nullptr, const TpFuse *tp = nullptr) {
@@ -286,10 +268,6 @@ struct Step {
         a.eps = r->cfg.norm_eps;
         a.status = r->ctx->device_status;
         a.wait_cycles = r->ctx->wait_cycles;
-        for (int i = 0; i < 2; i++) {
-            a.next_w[i] = next_w[i];
-            a.next_bytes[i] = next_bytes[i];
-        }
         ok(launch_qmv(a, r->ctx->prop.multiProcessorCount, r->ctx->stream, &n));
     }
 };
@@ -450,18 +428,19 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
     // Timing aid: YULE_CUDA_SKIP is a bit mask of kernel classes to leave out of the graph (results
     // are then meaningless); the time that disappears is that class's cost inside the real step.
     const unsigned skip = knob("YULE_CUDA_SKIP") ? (unsigned)strtoul(knob("YULE_CUDA_SKIP"), nullptr, 0) : 0u;
-    auto all_q4k = [&](std::initializer_list<const Tensor *> ts, uint32_t cols) {
-        for (const Tensor *t : ts)
-            if (t->type != YULE_DTYPE_Q4_K) return false;
-        return q4k_mma_supported(cols, 1);
+    // the bytes the one-vector kernel reads of a tensor (null: it does not take it)
+    auto digits_w = [&](const Tensor &t, uint32_t cols) -> const uint8_t * {
+        const uint8_t *w = t.type == YULE_DTYPE_Q6_K ? (t.buf.planar_cols == cols ? t.buf.planar : nullptr) : (const uint8_t *)t.buf.ptr;
+        return qmv_digits_supported(t.type, w, cols) ? w : nullptr;
     };
-    // Matrices that can share one launch of the tensor-pipe kernel: all Q4_K, or (single GPU) all Q5_K.
-    auto all_mma = [&](std::initializer_list<const Tensor *> ts, uint32_t cols) {
-        if (all_q4k(ts, cols)) return true;
-        if (N > 1) return false;
+    // matrices that can share one launch of that kernel: one format
+    auto can_share = [&](std::initializer_list<const Tensor *> ts, uint32_t cols) {
         for (const Tensor *t : ts)
-            if (t->type != YULE_DTYPE_Q5_K || (reinterpret_cast<uintptr_t>(t->buf.ptr) & 15)) return false;
-        return q4k_mma_supported(cols, 1);
+            if (t->type != (*ts.begin())->type || !digits_w(*t, cols)) return false;
+        return true;
+    };
+    auto all_q4k = [&](std::initializer_list<const Tensor *> ts, uint32_t cols) {
+        return (*ts.begin())->type == YULE_DTYPE_Q4_K && can_share(ts, cols);
     };
     // Tensor parallelism folded into the Q4_K matvecs: when both the kernel that produces a gathered vector
     // and the one that consumes it are the Q4_K tensor-pipe kernel, the producer stores (value, epoch) pairs
@@ -469,7 +448,7 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
     // stages x: no exchange launch, no fence, no flag.  YULE_TP_FUSE=0 keeps the exchange kernel everywhere.
     // (the folded exchange assumes the Llama op sequence: a variant model takes the exchange kernel everywhere)
     const bool tp_fuse = N > 1 && r->xchg && !skip_gather && !is_variant(r) && !(knob("YULE_TP_FUSE") && atoi(knob("YULE_TP_FUSE")) == 0);
-    auto is_q4k_mma = [&](const Tensor &t, uint32_t cols) { return t.type == YULE_DTYPE_Q4_K && q4k_mma_supported(cols, 1); };
+    auto is_q4k_mma = [&](const Tensor &t, uint32_t cols) { return all_q4k({&t}, cols); };
     auto epoch_index = [&](uint32_t layer, uint32_t k) { return k == 4 ? 4 * c.n_layers : 4 * layer + k; };
     auto push_of = [&](size_t pair_off, uint32_t per_rank, uint32_t layer, uint32_t k) {
         TpFuse f;
@@ -487,8 +466,8 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
         const Layer &L = r->layers[layer];
         const Tensor &ow = r->output.set ? r->output : r->token_embd;
         if (k == 0) return r->attn_gqa && attn_decode_supported(hd) && is_q4k_mma(L.attn_output, qdim);
-        if (k == 1) return is_q4k_mma(L.attn_output, qdim) && all_q4k({&L.ffn_gate, &L.ffn_up}, dim);
-        if (k == 2) return all_q4k({&L.ffn_gate, &L.ffn_up}, dim) && is_q4k_mma(L.ffn_down, ff);
+        if (k == 1) return is_q4k_mma(L.attn_output, qdim) && all_q4k({&L.ffn_gate, &L.ffn_up}, dim) && qmv_digits_can_pair(dim);
+        if (k == 2) return all_q4k({&L.ffn_gate, &L.ffn_up}, dim) && qmv_digits_can_pair(dim) && is_q4k_mma(L.ffn_down, ff);
         if (k == 3) {
             if (!is_q4k_mma(L.ffn_down, ff)) return false;
             if (layer + 1 < c.n_layers) {
@@ -499,37 +478,29 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
         }
         return false;
     };
-    // x → (optional RMSNorm) → up to three Q4_K matrices in one launch
+    // x → (optional RMSNorm) → up to three matrices of one format in one launch
     auto fused = [&](std::initializer_list<std::pair<const Tensor *, std::pair<float *, uint32_t>>> segs, const float *x,
-                     uint32_t cols, const float *norm_w, const float *residual, bool pair, const TpFuse *tp = nullptr) {
-        Q4kFused f;
+                     uint32_t cols, const float *norm_w, bool pair, const TpFuse *tp = nullptr) {
+        QmvDigits f;
         if (tp) f.tp = *tp;
         uint32_t i = 0;
-        f.q5 = segs.begin()->first->type == YULE_DTYPE_Q5_K;
+        f.type = segs.begin()->first->type;
         for (auto &sg : segs) {
-            f.w[i] = (const uint8_t *)sg.first->buf.ptr;
+            f.w[i] = digits_w(*sg.first, cols);
             f.out[i] = sg.second.first;
             f.rows[i] = sg.second.second;
-            f.out_stride[i] = sg.second.second;
             i++;
         }
         f.n_seg = i;
         f.x = x;
-        f.x_stride = cols;
         f.n_cols = cols;
-        f.batch = 1;
         f.norm_w = norm_w;
         f.eps = c.norm_eps;
-        f.residual = residual;
         f.swiglu_pair = pair;
         f.pdl = pdl;
         f.status = r->ctx->device_status;
         f.wait_cycles = r->ctx->wait_cycles;
-        for (int k = 0; k < 2; k++) {
-            f.next_w[k] = st.next_w[k];
-            f.next_bytes[k] = st.next_bytes[k];
-        }
-        st.ok(launch_q4k_mma(f, sms, s, &st.n));
+        st.ok(launch_qmv_digits(f, sms, s, &st.n));
     };
 
     if (!(skip & 256))
@@ -540,14 +511,16 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
         st.ok(launch_elementwise(kElemScale, r->hidden, nullptr, r->hidden, dim, sqrtf((float)dim), s, &st.n, pdl));
     for (uint32_t l = 0; l < c.n_layers; l++) {
         Layer &L = r->layers[l];
-        const Tensor &out_w_ = r->output.set ? r->output : r->token_embd;
-        st.then(&L.attn_output);  // while Q/K/V and attention run, o-proj's weights come in
         if (skip & 1) {
-        } else if (all_mma({&L.attn_q, &L.attn_k, &L.attn_v}, dim)) {
+        } else if (can_share({&L.attn_q, &L.attn_k, &L.attn_v}, dim)) {
             TpFuse tq;
             if (l > 0 && folded(l - 1, 3)) add_wait(tq, r->x_pair_hidden, l - 1, 3);
             fused({{&L.attn_q, {r->q, qdim_l}}, {&L.attn_k, {r->k_tmp, kvdim_l}}, {&L.attn_v, {r->v_tmp, kvdim_l}}},
-                  r->hidden, dim, L.attn_norm_f32, nullptr, false, &tq);
+                  r->hidden, dim, L.attn_norm_f32, false, &tq);
+        } else if (can_share({&L.attn_q, &L.attn_k}, dim) && digits_w(L.attn_v, dim)) {
+            // files that keep V in a wider format than Q and K
+            fused({{&L.attn_q, {r->q, qdim_l}}, {&L.attn_k, {r->k_tmp, kvdim_l}}}, r->hidden, dim, L.attn_norm_f32, false);
+            fused({{&L.attn_v, {r->v_tmp, kvdim_l}}}, r->hidden, dim, L.attn_norm_f32, false);
         } else {
             st.ok(launch_rms_norm(r->hidden, L.attn_norm_f32, r->normed, dim, c.norm_eps, s, &st.n, pdl));
             st.qmv(L.attn_q, r->normed, r->q, qdim_l, dim);
@@ -597,7 +570,6 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
         if (!folded(l, 0)) gather(r->attn_out, r->x_attn_out, qdim_l, l, 0);
         float *hidden_l = r->hidden + (size_t)R * dim_l;
         // hidden = hidden + W_o · attn_out (the Add dispatch folded into the matvec epilogue)
-        st.then(&L.ffn_gate, &L.ffn_up);
         {
             TpFuse to;
             if (folded(l, 1)) to = push_of(r->x_pair_hidden, dim_l, l, 1);
@@ -612,14 +584,13 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
             }
         }
         if (!folded(l, 1)) gather(r->hidden, r->x_hidden, dim_l, l, 1);
-        st.then(&L.ffn_down);
         if (skip & 16) {
-        } else if (!c.geglu && all_mma({&L.ffn_gate, &L.ffn_up}, dim)) {
+        } else if (!c.geglu && can_share({&L.ffn_gate, &L.ffn_up}, dim) && qmv_digits_can_pair(dim)) {
             TpFuse tg;
             if (folded(l, 2)) tg = push_of(r->x_pair_gate, ff_l, l, 2);
             if (folded(l, 1)) add_wait(tg, r->x_pair_hidden, l, 1);
             fused({{&L.ffn_gate, {r->gate + (size_t)R * ff_l, ff_l}}, {&L.ffn_up, {r->up, ff_l}}}, r->hidden, dim,
-                  L.ffn_norm_f32, nullptr, true, &tg);
+                  L.ffn_norm_f32, true, &tg);
         } else {
             st.ok(launch_rms_norm(r->hidden, L.ffn_norm_f32, r->normed, dim, c.norm_eps, s, &st.n, pdl));
             st.qmv(L.ffn_gate, r->normed, r->gate + (size_t)R * ff_l, ff_l, dim);
@@ -630,11 +601,6 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
                 st.ok(launch_silu_mul(r->gate + (size_t)R * ff_l, r->up, r->gate + (size_t)R * ff_l, ff_l, s, &st.n, pdl));
         }
         if (!folded(l, 2)) gather(r->gate, r->x_gate, ff_l, l, 2);
-        // during down-proj: the next layer's Q and K/V (or the output matrix after the last layer)
-        if (l + 1 < c.n_layers)
-            st.then(&r->layers[l + 1].attn_q, &r->layers[l + 1].attn_k);
-        else
-            st.then(&out_w_);
         {
             TpFuse td;
             if (folded(l, 3)) td = push_of(r->x_pair_hidden, dim_l, l, 3);
@@ -650,15 +616,12 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
         }
         if (!folded(l, 3)) gather(r->hidden, r->x_hidden, dim_l, l, 3);
     }
-    st.then(nullptr);
     const Tensor &out_w = r->output.set ? r->output : r->token_embd;
     if (skip & 64) {
-    } else if (all_mma({&out_w}, dim)) {
+    } else if (can_share({&out_w}, dim)) {
         TpFuse tw;
         if (c.n_layers && folded(c.n_layers - 1, 3)) add_wait(tw, r->x_pair_hidden, c.n_layers - 1, 3);
-        fused({{&out_w, {r->logits + (size_t)R * vocab_l, vocab_l}}}, r->hidden, dim, r->output_norm_f32, nullptr, false, &tw);
-    } else if (out_w.type == YULE_DTYPE_Q6_K && out_w.buf.planar && q6k_mma_supported(dim)) {
-        st.qmv(out_w, r->hidden, r->logits + (size_t)R * vocab_l, vocab_l, dim, nullptr, r->output_norm_f32);
+        fused({{&out_w, {r->logits + (size_t)R * vocab_l, vocab_l}}}, r->hidden, dim, r->output_norm_f32, false, &tw);
     } else {
         st.ok(launch_rms_norm(r->hidden, r->output_norm_f32, r->normed, dim, c.norm_eps, s, &st.n, pdl));
         st.qmv(out_w, r->normed, r->logits + (size_t)R * vocab_l, vocab_l, dim);

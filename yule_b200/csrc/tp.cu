@@ -347,13 +347,12 @@ int32_t yule_cuda_selftest_bounded_wait(yule_cuda_ctx *ctx, uint32_t which, uint
     const long long budget = budget_cycles ? (long long)budget_cycles : ctx->wait_cycles;
     uint64_t launches = 0;
     if (e == cudaSuccess && which == 0) {
-        Q4kFused f;
+        QmvDigits f;
+        f.type = YULE_DTYPE_Q4_K;
         f.w[0] = w;
         f.out[0] = out;
         f.rows[0] = n_rows;
-        f.out_stride[0] = n_rows;
         f.x = x;
-        f.x_stride = n_cols;
         f.n_cols = n_cols;
         f.status = ctx->device_status;
         f.wait_cycles = budget;
@@ -365,7 +364,7 @@ int32_t yule_cuda_selftest_bounded_wait(yule_cuda_ctx *ctx, uint32_t which, uint
         f.tp.wait = true;
         f.tp.wait_index = 0;
         f.tp.pair_in = reinterpret_cast<const uint2 *>(region_a);
-        e = launch_q4k_mma(f, ctx->prop.multiProcessorCount, ctx->stream, &launches);
+        e = launch_qmv_digits(f, ctx->prop.multiProcessorCount, ctx->stream, &launches);
     } else if (e == cudaSuccess) {
         const long long saved_budget = ctx->wait_cycles;
         ctx->tp_peer_base[0] = region_a;
