@@ -827,11 +827,11 @@ int32_t yule_cuda_sample(yule_cuda_ctx *ctx, yule_buffer logits, uint32_t n, con
     SampleArgs a;
     a.logits = (const float *)L.ptr;
     a.n = n;
-    a.temperature = params->temperature;
-    a.top_p = params->top_p;
-    a.top_k = params->top_k;
-    a.min_p = params->min_p;
-    a.repetition_penalty = params->repetition_penalty;
+    a.set.temperature = params->temperature;
+    a.set.top_p = params->top_p;
+    a.set.top_k = params->top_k;
+    a.set.min_p = params->min_p;
+    a.set.repetition_penalty = params->repetition_penalty;
     a.previous = prev;
     a.n_previous = n_previous;
     a.r = random_value;

@@ -7,11 +7,16 @@
 
 #include <cfloat>
 
+#include <cooperative_groups.h>
+
 #include "internal.h"
 
 namespace yule {
 
 namespace {
+
+namespace cg = cooperative_groups;
+
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -193,12 +198,11 @@ __global__ void rope_kv_write_batch_kernel(float *__restrict__ q, const float *_
                                            float *__restrict__ k_cache, float *__restrict__ v_cache,
                                            const float *__restrict__ cos_table, const float *__restrict__ sin_table,
                                            uint32_t pos0, uint32_t head_dim, uint32_t n_heads, uint32_t n_kv_heads,
-                                           const uint32_t *__restrict__ row_pos, size_t cache_stride) {
-    const uint32_t z = blockIdx.y, pos = row_pos ? row_pos[z] : pos0 + z;
-    if (row_pos) {
-        k_cache += (size_t)z * cache_stride;
-        v_cache += (size_t)z * cache_stride;
-    }
+                                           const uint32_t *__restrict__ row_pos, size_t cache_stride, uint32_t seq_tokens) {
+    // row z: sequence z at row_pos[z]; or token z % seq_tokens, counted from pos0, of sequence z / seq_tokens
+    const uint32_t z = blockIdx.y, seq = row_pos ? z : z / seq_tokens, pos = row_pos ? row_pos[z] : pos0 + z % seq_tokens;
+    k_cache += (size_t)seq * cache_stride;
+    v_cache += (size_t)seq * cache_stride;
     const uint32_t half = head_dim / 2;
     const uint32_t kv_stride = n_kv_heads * head_dim, q_stride = n_heads * head_dim;
     const uint32_t total_q = n_heads * half, total_k = n_kv_heads * half;
@@ -373,27 +377,42 @@ multihead_attention_kernel(const float *__restrict__ q, const float *__restrict_
 // Greedy pick with ties to the highest index (yule-infer/src/sampler.rs:150-163) into state[0];
 // with `history` the pick is also logged at history[position] and the position (state[1]) is
 // advanced, so the next graph replay continues the sequence without the host.
-__global__ void argmax_kernel(const float *__restrict__ v, uint32_t n, uint32_t *__restrict__ state,
-                              uint32_t *__restrict__ history) {
-    yule_pdl_launch_dependents();
-    yule_pdl_wait();
-    __shared__ float bv[32];
-    __shared__ uint32_t bi[32];
+//
+// One cluster of kArgmaxCtas CTAs per row: 128256 logits are 512 KB, which one CTA takes 20 us (40 on a busy chip) to fetch
+// from L2; the partial picks meet in the first CTA's shared memory.
+constexpr uint32_t kArgmaxCtas = 8;
+struct ArgmaxShared {
+    float v[32];
+    uint32_t i[32];
+    float best;     // of the CTA, read by the first CTA of the cluster
+    uint32_t at;
+};
+__device__ __forceinline__ void better(float &v, uint32_t &i, float ov, uint32_t oi) {
+    if (ov > v || (ov == v && oi > i)) {
+        v = ov;
+        i = oi;
+    }
+}
+// The pick of row v[0..n), valid in thread 0 of the cluster's first CTA; called by 1024 threads of every CTA.
+__device__ __forceinline__ uint32_t cluster_argmax(const float *__restrict__ v, uint32_t n, ArgmaxShared &sh) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), slice = (n + kArgmaxCtas - 1) / kArgmaxCtas;
+    const uint32_t lo = rank * slice < n ? rank * slice : n, hi = lo + slice < n ? lo + slice : n;
     float best = -FLT_MAX;
-    uint32_t idx = 0;
+    uint32_t idx = lo;
     bool any = false;
     // eight loads in flight per thread (the logits sit in L2; one load at a time is all latency)
-    for (uint32_t base = threadIdx.x; base < n; base += blockDim.x * 8) {
+    for (uint32_t base = lo + threadIdx.x; base < hi; base += blockDim.x * 8) {
         float x[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const uint32_t i = base + k * blockDim.x;
-            x[k] = i < n ? v[i] : 0.f;
+            x[k] = i < hi ? v[i] : 0.f;
         }
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const uint32_t i = base + k * blockDim.x;
-            if (i < n && (!any || x[k] >= best)) {
+            if (i < hi && (!any || x[k] >= best)) {
                 best = x[k];
                 idx = i;
                 any = true;
@@ -401,95 +420,65 @@ __global__ void argmax_kernel(const float *__restrict__ v, uint32_t n, uint32_t 
         }
     }
     if (!any) best = -FLT_MAX;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (ob > best || (ob == best && oi > idx)) {
-            best = ob;
-            idx = oi;
-        }
-    }
+    for (int o = 16; o > 0; o >>= 1) better(best, idx, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, idx, o));
     if (lane == 0) {
-        bv[wid] = best;
-        bi[wid] = idx;
+        sh.v[wid] = best;
+        sh.i[wid] = idx;
     }
     __syncthreads();
     if (wid == 0) {
-        best = lane < nw ? bv[lane] : -FLT_MAX;
-        idx = lane < nw ? bi[lane] : 0;
+        best = sh.v[lane];
+        idx = sh.i[lane];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (ob > best || (ob == best && oi > idx)) {
-                best = ob;
-                idx = oi;
-            }
-        }
+        for (int o = 16; o > 0; o >>= 1) better(best, idx, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, idx, o));
         if (lane == 0) {
-            state[0] = idx;
-            if (history) {
-                const uint32_t pos = state[1];
-                history[pos] = idx;
-                state[1] = pos + 1;
-                state[2] += 1;  // token counter that reset() never rewinds (epochs of the peer exchange)
-            }
+            sh.best = best;
+            sh.at = idx;
+        }
+    }
+    cluster.sync();
+    if (rank == 0 && wid == 0) {
+        const uint32_t c = lane < (int)kArgmaxCtas && lane * slice < n ? lane : 0;
+        const ArgmaxShared *o = cluster.map_shared_rank(&sh, c);
+        best = o->best;
+        idx = o->at;
+#pragma unroll
+        for (int q = kArgmaxCtas / 2; q > 0; q >>= 1) better(best, idx, __shfl_xor_sync(0xffffffffu, best, q), __shfl_xor_sync(0xffffffffu, idx, q));
+    }
+    cluster.sync();  // nobody leaves while its words may still be read
+    return idx;
+}
+__global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(1024)
+argmax_kernel(const float *__restrict__ v, uint32_t n, uint32_t *__restrict__ state, uint32_t *__restrict__ history) {
+    __shared__ ArgmaxShared sh;
+    yule_pdl_launch_dependents();
+    yule_pdl_wait();
+    const uint32_t idx = cluster_argmax(v, n, sh);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        state[0] = idx;
+        if (history) {
+            const uint32_t pos = state[1];
+            history[pos] = idx;
+            state[1] = pos + 1;
+            state[2] += 1;  // token counter that reset() never rewinds (epochs of the peer exchange)
         }
     }
 }
 
 // Batched decode: row b = blockIdx.x of [batch][n] logits → tokens[b] (ties to the highest index, as above),
 // logged at history[b * history_stride + step[0]]; block 0 advances every sequence's position and the step.
-__global__ void argmax_rows_kernel(const float *__restrict__ v, uint32_t n, uint32_t *__restrict__ tokens, uint32_t *__restrict__ pos,
-                                   uint32_t *__restrict__ step, uint32_t *__restrict__ history, uint32_t history_stride) {
-    __shared__ float bv[32];
-    __shared__ uint32_t bi[32];
-    const float *row = v + (size_t)blockIdx.x * n;
-    float best = -FLT_MAX;
-    uint32_t idx = 0;
-    bool any = false;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const float x = row[i];
-        if (!any || x >= best) {
-            best = x;
-            idx = i;
-            any = true;
-        }
-    }
-    if (!any) best = -FLT_MAX;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (ob > best || (ob == best && oi > idx)) {
-            best = ob;
-            idx = oi;
-        }
-    }
-    if (lane == 0) {
-        bv[wid] = best;
-        bi[wid] = idx;
-    }
-    __syncthreads();
-    if (wid == 0) {
-        best = lane < nw ? bv[lane] : -FLT_MAX;
-        idx = lane < nw ? bi[lane] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (ob > best || (ob == best && oi > idx)) {
-                best = ob;
-                idx = oi;
-            }
-        }
-        if (lane == 0) {
-            tokens[blockIdx.x] = idx;
-            if (history) history[(size_t)blockIdx.x * history_stride + step[0]] = idx;
-        }
+__global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(1024)
+argmax_rows_kernel(const float *__restrict__ v, uint32_t n, uint32_t *__restrict__ tokens, uint32_t *__restrict__ step,
+                   uint32_t *__restrict__ history, uint32_t history_stride) {
+    __shared__ ArgmaxShared sh;
+    yule_pdl_launch_dependents();
+    yule_pdl_wait();
+    const uint32_t row = blockIdx.y, idx = cluster_argmax(v + (size_t)row * n, n, sh);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        tokens[row] = idx;
+        if (history) history[(size_t)row * history_stride + step[0]] = idx;
     }
 }
 // After the picks of a step: every sequence moves one position on.
@@ -559,12 +548,12 @@ cudaError_t launch_rope_kv_write(float *q, const float *k_tmp, const float *v_tm
 cudaError_t launch_rope_kv_write_batch(float *q, const float *k, const float *v, float *k_cache, float *v_cache,
                                        const float *cos_table, const float *sin_table, uint32_t pos0, uint32_t n_tokens,
                                        uint32_t head_dim, uint32_t n_heads, uint32_t n_kv_heads, cudaStream_t s,
-                                       uint64_t *launches, const uint32_t *row_pos, size_t cache_stride) {
+                                       uint64_t *launches, const uint32_t *row_pos, size_t cache_stride, uint32_t seq_tokens) {
     uint32_t total = (n_heads + n_kv_heads) * (head_dim / 2);
     *launches += 1;
     rope_kv_write_batch_kernel<<<dim3((total + 255) / 256, n_tokens), 256, 0, s>>>(q, k, v, k_cache, v_cache, cos_table, sin_table,
                                                                                   pos0, head_dim, n_heads, n_kv_heads, row_pos,
-                                                                                  cache_stride);
+                                                                                  cache_stride, seq_tokens ? seq_tokens : n_tokens);
     return cudaGetLastError();
 }
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint32_t n, cudaStream_t s,
@@ -624,11 +613,11 @@ cudaError_t launch_elementwise(int op, const float *a, const float *b, float *ou
 cudaError_t launch_argmax(const float *v, uint32_t n, uint32_t *state, uint32_t *history, cudaStream_t s,
                           uint64_t *launches, bool pdl) {
     *launches += 1;
-    return launch_kernel(argmax_kernel, dim3(1), dim3(1024), 0, s, pdl, v, n, state, history);
+    return launch_kernel(argmax_kernel, dim3(kArgmaxCtas), dim3(1024), 0, s, pdl, v, n, state, history);
 }
-cudaError_t launch_argmax_rows(const float *v, uint32_t n, uint32_t batch, uint32_t *tokens, uint32_t *pos, uint32_t *step,
+cudaError_t launch_argmax_rows(const float *v, uint32_t n, uint32_t batch, uint32_t *tokens, uint32_t *step,
                                uint32_t *history, uint32_t history_stride, cudaStream_t s, uint64_t *launches) {
-    argmax_rows_kernel<<<batch, 1024, 0, s>>>(v, n, tokens, pos, step, history, history_stride);
+    argmax_rows_kernel<<<dim3(kArgmaxCtas, batch), 1024, 0, s>>>(v, n, tokens, step, history, history_stride);
     *launches += 1;
     return cudaGetLastError();
 }

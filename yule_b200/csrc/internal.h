@@ -352,10 +352,11 @@ cudaError_t launch_embed_gather_batch(const uint8_t *table, uint32_t type, uint3
 cudaError_t launch_rope_kv_write_batch(float *q, const float *k, const float *v, float *k_cache, float *v_cache,
                                        const float *cos_table, const float *sin_table, uint32_t pos0, uint32_t n_tokens,
                                        uint32_t head_dim, uint32_t n_heads, uint32_t n_kv_heads, cudaStream_t s,
-                                       uint64_t *launches, const uint32_t *row_pos = nullptr, size_t cache_stride = 0);
+                                       uint64_t *launches, const uint32_t *row_pos = nullptr, size_t cache_stride = 0,
+                                       uint32_t seq_tokens = 0);  // seq_tokens: tokens per sequence (0: one sequence)
 // Batched decode: greedy pick per row of [batch][n] logits (ties to the highest index) into tokens[b] and
 // history[b * history_stride + step[0]]; then every position and the step counter move on by one.
-cudaError_t launch_argmax_rows(const float *v, uint32_t n, uint32_t batch, uint32_t *tokens, uint32_t *pos, uint32_t *step,
+cudaError_t launch_argmax_rows(const float *v, uint32_t n, uint32_t batch, uint32_t *tokens, uint32_t *step,
                                uint32_t *history, uint32_t history_stride, cudaStream_t s, uint64_t *launches);
 cudaError_t launch_advance_rows(uint32_t *pos, uint32_t *step, uint32_t batch, cudaStream_t s, uint64_t *launches);
 
@@ -427,6 +428,17 @@ struct AttnDecode {
     float softcap = 0.f;     // attention logit softcap (:716-721): score = cap · tanh(score / cap); 0 = none
     bool gqa = false;        // grouped-query kernel: one CTA per (KV head, split); n_splits from attn_gqa_pick_splits
 };
+// Causal attention of n_seq sequences x n_tokens queries (attn_prefill.cu): row b·n_tokens + i of q / out is the query at
+// position pos0 + i of sequence b, whose caches lie b · kv_batch_stride floats on and hold positions [0, pos0 + n_tokens).
+struct AttnPrefill {
+    const float *q = nullptr, *k_cache = nullptr, *v_cache = nullptr;
+    float *out = nullptr;
+    uint32_t n_tokens = 0, n_seq = 1, pos0 = 0, hd = 0, n_heads = 0, n_kv_heads = 0, kv_stride = 0, q_stride = 0, out_stride = 0;
+    size_t kv_batch_stride = 0;
+    bool pdl = false;
+};
+bool attn_prefill_preferred(uint32_t hd, uint32_t n_heads, uint32_t n_kv_heads, uint32_t n_tokens, uint32_t n_seq, uint32_t pos0, int sm_count);
+cudaError_t launch_attn_prefill(const AttnPrefill &a, cudaStream_t s, uint64_t *launches);
 bool attn_gqa_supported(uint32_t hd, uint32_t n_heads, uint32_t n_kv_heads);
 uint32_t attn_gqa_pick_splits(uint32_t n_kv_heads, uint32_t max_seq_len, int sm_count);
 size_t attn_scratch_floats(uint32_t n_heads, uint32_t n_splits, uint32_t hd);
@@ -446,18 +458,28 @@ cudaError_t launch_argmax(const float *v, uint32_t n, uint32_t *state, uint32_t 
 cudaError_t launch_fill_bytes(void *p, size_t n, int value, cudaStream_t s, uint64_t *launches);
 
 // Token sampler on the device (sampler.cu; yule-infer/src/sampler.rs:17-136).
+struct SampleSettings {
+    float temperature = 0.7f, top_p = 0.9f, min_p = 0.05f, repetition_penalty = 1.1f;  // SamplingParams::default
+    uint32_t top_k = 40;
+};
 struct SampleArgs {
     const float *logits = nullptr;
     uint32_t n = 0;
-    float temperature = 0.7f, top_p = 0.9f, min_p = 0.05f, repetition_penalty = 1.1f;  // SamplingParams::default
-    uint32_t top_k = 40;
+    SampleSettings set;
     const uint32_t *previous = nullptr;  // tokens seen so far, device memory
     uint32_t n_previous = 0;
     float r = 0.f;                       // uniform random value in [0, 1)
+    // Replayed from a graph: settings, random values and counters come from device memory.  loop[0] counts the picks (value
+    // loop[0] of r_values is used, and it moves on), loop[1] is the number of tokens before the first pick;
+    // feed_state[1] receives the position of the token just picked.
+    const SampleSettings *device_set = nullptr;
+    const float *r_values = nullptr;
+    uint32_t *loop = nullptr;
     float *scratch = nullptr;            // 2 * n floats
     uint32_t *out_token = nullptr;       // device word that receives the pick
     uint32_t *append_to = nullptr;       // optional: the pick also goes to append_to[n_previous]
     uint32_t *feed_state = nullptr;      // optional: the pick also goes to feed_state[0]
+    bool pdl = false;
 };
 cudaError_t launch_sample(const SampleArgs &a, cudaStream_t s, uint64_t *launches);
 int32_t ensure_sampler_scratch(yule_cuda_ctx *ctx, size_t n_floats);

@@ -101,6 +101,11 @@ struct yule_cuda_runner {
     uint32_t xb_rows = 0, xb_logit_rows = 0;  // rows those regions were sized for
     uint32_t *d_btick = nullptr;
     uint32_t *d_seq = nullptr;  // sampled generation: every token of the sequence so far (prompt and picks)
+    SampleSettings *d_sample_set = nullptr;  // and what the replayed sampler reads: settings, random values, counters
+    float *d_sample_r = nullptr;
+    uint32_t *d_sample_loop = nullptr;
+    cudaGraphExec_t sample_graph = nullptr;  // sampler, then the token step without its greedy pick
+    uint32_t sample_graph_kernels = 0;
 
     uint32_t pos = 0;
     bool fused = false;
@@ -398,7 +403,8 @@ cudaError_t enqueue_forward_by_value(yule_cuda_runner *r, uint32_t token, uint32
 //         → [RMSNorm + output] → [argmax + history + position advance]
 // Brackets are single kernels when the matrices involved are Q4_K; other formats fall back to a
 // separate RMSNorm / SiLU·mul kernel around the per-matrix matvec.
-cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
+// `pick`: with the greedy pick (and the advance of token, position and history that goes with it).
+cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches, bool pick = true) {
     const yule_runner_config &c = r->cfg;
     cudaStream_t s = r->ctx->stream;
     const int sms = r->ctx->prop.multiProcessorCount;
@@ -630,7 +636,7 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches) {
     // final logit softcap (Gemma2, model_runner.rs:1027-1032)
     if (c.logit_softcap != 0.f)
         st.ok(launch_elementwise(kElemSoftcap, r->logits, nullptr, r->logits, c.vocab_size, c.logit_softcap, s, &st.n, pdl));
-    if (!(skip & 128)) st.ok(launch_argmax(r->logits, c.vocab_size, r->d_state, r->d_history, s, &st.n, pdl));
+    if (pick && !(skip & 128)) st.ok(launch_argmax(r->logits, c.vocab_size, r->d_state, r->d_history, s, &st.n, pdl));
     *launches += st.n;
     return st.err;
 }
@@ -1135,7 +1141,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         lin(out_w, vocab_l, dim, r->bd_logits + (size_t)R * vocab_l, c.vocab_size, nullptr);
         exchange(r->xb_logits, vocab_l, c.vocab_size);
         flush();
-        ok(launch_argmax_rows(r->bd_logits, c.vocab_size, ps.n_live, r->bd_tokens, r->bd_pos, r->bd_step, r->bd_history, c.max_seq_len + 1, s, launches));
+        ok(launch_argmax_rows(r->bd_logits, c.vocab_size, ps.n_live, r->bd_tokens, r->bd_step, r->bd_history, c.max_seq_len + 1, s, launches));
         ok(launch_advance_rows(r->bd_pos, r->bd_step, ps.n_live, s, launches));
     }
     flush();
@@ -1483,6 +1489,7 @@ int32_t yule_cuda_runner_destroy(yule_cuda_runner *r) {
     cudaStreamSynchronize(r->ctx->stream);
     if (r->graph_exec) cudaGraphExecDestroy(r->graph_exec);
     if (r->bd_graph) cudaGraphExecDestroy(r->bd_graph);
+    if (r->sample_graph) cudaGraphExecDestroy(r->sample_graph);
     if (r->mega) mega_destroy(r->mega);
     if (r->h_logits) cudaFreeHost(r->h_logits);
     if (r->h_moe_sel) cudaFreeHost(r->h_moe_sel);
@@ -1510,6 +1517,10 @@ int32_t yule_cuda_runner_set_tensor(yule_cuda_runner *r, const char *name, yule_
     if (r->graph_exec) {  // pointers are baked into the graph
         cudaGraphExecDestroy(r->graph_exec);
         r->graph_exec = nullptr;
+    }
+    if (r->sample_graph) {
+        cudaGraphExecDestroy(r->sample_graph);
+        r->sample_graph = nullptr;
     }
     if (r->mega) {
         mega_destroy(r->mega);
@@ -1676,37 +1687,80 @@ int32_t yule_cuda_runner_generate_sampled(yule_cuda_runner *r, const uint32_t *p
     if ((uint64_t)n_prompt + n_generate > c.max_seq_len) return fail(YULE_ERR_CONTEXT_LENGTH, "context length exceeded");
     if ((rc = ensure_sampler_scratch(r->ctx, 2 * (size_t)c.vocab_size + 4))) return rc;
     if (!r->d_seq) {
-        float *p = nullptr;
-        if ((rc = alloc_f32(r, (size_t)c.max_seq_len + 1, &p))) return rc;
-        r->d_seq = (uint32_t *)p;
+        float *seq = nullptr, *set = nullptr, *rv = nullptr, *loop = nullptr;
+        if ((rc = alloc_f32(r, (size_t)c.max_seq_len + 1, &seq)) || (rc = alloc_f32(r, (sizeof(SampleSettings) + 3) / 4, &set)) ||
+            (rc = alloc_f32(r, (size_t)c.max_seq_len + 1, &rv)) || (rc = alloc_f32(r, 4, &loop)))
+            return rc;
+        r->d_sample_set = (SampleSettings *)set;
+        r->d_sample_r = rv;
+        r->d_sample_loop = (uint32_t *)loop;
+        r->d_seq = (uint32_t *)seq;
     }
     cudaStream_t s = r->ctx->stream;
     // the prompt: KV caches and the logits after its last token, exactly as generate_greedy feeds it
     uint32_t dummy = 0;
     if ((rc = yule_cuda_runner_generate_greedy(r, prompt, n_prompt, 0, &dummy))) return rc;
     YULE_CUDA_TRY(cudaMemcpyAsync(r->d_seq, prompt, (size_t)n_prompt * 4, cudaMemcpyHostToDevice, s));
+    SampleArgs a;
+    a.logits = r->logits;
+    a.n = c.vocab_size;
+    a.set.temperature = params->temperature;
+    a.set.top_p = params->top_p;
+    a.set.top_k = params->top_k;
+    a.set.min_p = params->min_p;
+    a.set.repetition_penalty = params->repetition_penalty;
+    a.previous = r->d_seq;
+    a.scratch = r->ctx->sampler_scratch;
+    a.out_token = reinterpret_cast<uint32_t *>(r->ctx->sampler_scratch + 2 * (size_t)c.vocab_size);
+    a.append_to = r->d_seq;
+    a.feed_state = r->d_state;  // the token step reads its input token here
     uint64_t launches = 0;
     cudaError_t e = cudaSuccess;
-    for (uint32_t g = 0; g < n_generate && e == cudaSuccess; g++) {
-        SampleArgs a;
-        a.logits = r->logits;
-        a.n = c.vocab_size;
-        a.temperature = params->temperature;
-        a.top_p = params->top_p;
-        a.top_k = params->top_k;
-        a.min_p = params->min_p;
-        a.repetition_penalty = params->repetition_penalty;
-        a.previous = r->d_seq;
-        a.n_previous = n_prompt + g;
-        a.r = yule_cuda_sampling_random_value(seed, g);
-        a.scratch = r->ctx->sampler_scratch;
-        a.out_token = reinterpret_cast<uint32_t *>(r->ctx->sampler_scratch + 2 * (size_t)c.vocab_size);
-        a.append_to = r->d_seq;
-        a.feed_state = r->d_state;  // the token step reads its input token here
-        e = launch_sample(a, s, &launches);
-        if (e == cudaSuccess) e = cudaGraphLaunch(r->graph_exec, s);
+    if (r->mega || r->xchg) {
+        // the persistent kernel's step ends with its own pick, and under tensor parallelism every step moves the epoch
+        // counter on: the sampler goes out between whole steps
+        for (uint32_t g = 0; g < n_generate && e == cudaSuccess; g++) {
+            a.n_previous = n_prompt + g;
+            a.r = yule_cuda_sampling_random_value(seed, g);
+            e = launch_sample(a, s, &launches);
+            if (e == cudaSuccess) e = cudaGraphLaunch(r->graph_exec, s);
+        }
+        launches += (uint64_t)graph_kernels(r) * n_generate;
+    } else if (n_generate) {
+        // one graph per token: sampler, token step without the greedy pick
+        a.device_set = r->d_sample_set;
+        a.r_values = r->d_sample_r;
+        a.loop = r->d_sample_loop;
+        if (!r->sample_graph) {
+            cudaGraph_t graph = nullptr;
+            YULE_CUDA_TRY(cudaStreamSynchronize(s));
+            YULE_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+            uint64_t n = 0;
+            e = launch_sample(a, s, &n);
+            if (e == cudaSuccess) e = enqueue_forward_graph(r, &n, false);
+            const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
+            if (e == cudaSuccess) e = e2;
+            if (e == cudaSuccess) e = cudaGraphInstantiate(&r->sample_graph, graph, 0);
+            if (graph) cudaGraphDestroy(graph);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                r->sample_graph = nullptr;
+                return fail_cuda(e, "graph capture of the sampled token step");
+            }
+            r->sample_graph_kernels = (uint32_t)n;
+        }
+        std::vector<float> rv(n_generate);
+        for (uint32_t g = 0; g < n_generate; g++) rv[g] = yule_cuda_sampling_random_value(seed, g);
+        const uint32_t loop[2] = {0, n_prompt};
+        YULE_CUDA_TRY(cudaMemcpyAsync(r->d_sample_set, &a.set, sizeof(a.set), cudaMemcpyHostToDevice, s));
+        YULE_CUDA_TRY(cudaMemcpyAsync(r->d_sample_r, rv.data(), (size_t)n_generate * 4, cudaMemcpyHostToDevice, s));
+        YULE_CUDA_TRY(cudaMemcpyAsync(r->d_sample_loop, loop, sizeof(loop), cudaMemcpyHostToDevice, s));
+        for (uint32_t g = 0; g < n_generate && e == cudaSuccess; g++) e = cudaGraphLaunch(r->sample_graph, s);
+        launches += (uint64_t)r->sample_graph_kernels * n_generate;
+        // the greedy continuation after the last token, as every other way of feeding tokens leaves it
+        if (e == cudaSuccess) e = launch_argmax(r->logits, c.vocab_size, r->d_state, r->d_history, s, &launches);
     }
-    r->ctx->launches.fetch_add(launches + (uint64_t)graph_kernels(r) * n_generate);
+    r->ctx->launches.fetch_add(launches);
     if (e != cudaSuccess) return fail_cuda(e, "sampled generation");
     r->pos += n_generate;
     if (n_generate)
