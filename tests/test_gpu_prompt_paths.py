@@ -1,0 +1,67 @@
+"""Prompts that share their passes over the weights: the tiled causal attention (128 query rows per CTA against 64-position
+tiles of the fp32 cache) and prompts of a whole batch.  Oracle: the CPU runner restated (yule-infer/src/model_runner.rs:533-1036), which feeds one token at a time."""
+
+import numpy as np
+import pytest
+
+from conftest import REL_TOL
+from test_gpu_runner import guarded_rel_err, make_oracle_model
+from yule_b200 import CudaTransformerRunner, DType, ModelConfig, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (8, 4, 64), (4, 4, 64), (8, 1, 128), (8, 2, 128), (4, 4, 128)])
+@pytest.mark.parametrize("n", [17, 65, 129, 200])
+def test_tiled_prompt_attention(backend, oracle, heads, kv_heads, head_dim, n):
+    """One query tile and several, one K / V tile, its edge and several, then a second prompt that starts inside a tile."""
+    cfg = ModelConfig(dim=512, n_layers=1, n_heads=heads, n_kv_heads=kv_heads, head_dim=head_dim, vocab_size=300, ff_dim=512,
+                      max_seq_len=320)
+    weights = synth.synthetic_model(cfg, seed=60 + n, std=0.06, linear=DType.Q4_K)
+    ref = make_oracle_model(oracle, cfg, weights)
+    run = CudaTransformerRunner(backend, cfg, weights, fused=1)
+    for part, m in enumerate((n, 70)):
+        prompt = synth.tokens(5 + part, m, cfg.vocab_size)
+        assert guarded_rel_err(run.prefill(prompt), ref.prefill(prompt)) <= REL_TOL
+    assert guarded_rel_err(run.decode_step(7), ref.decode_step(7)) <= REL_TOL
+    run.close()
+
+
+def test_tiled_prompt_attention_large_and_small_values(backend, oracle):
+    """Values far outside fp16's range and far below its normal numbers: every K / V tile has its own power of two."""
+    cfg = ModelConfig(dim=256, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, vocab_size=300, ff_dim=512, max_seq_len=160)
+    for factor in (3e4, 2e-3):
+        weights = synth.synthetic_model(cfg, seed=70, std=0.06, linear=DType.Q4_K)
+        data, dt = weights["blk.0.attn_v.weight"]
+        blocks = np.array(data).reshape(-1, 144).copy()
+        d = blocks[:, :4].copy().view(np.float16).astype(np.float32) * np.float32(factor)  # d and dmin
+        blocks[:, :4] = d.astype(np.float16).view(np.uint8)
+        weights["blk.0.attn_v.weight"] = (blocks.reshape(-1), dt)
+        ref = make_oracle_model(oracle, cfg, weights)
+        run = CudaTransformerRunner(backend, cfg, weights, fused=1)
+        prompt = synth.tokens(8, 130, cfg.vocab_size)
+        assert guarded_rel_err(run.prefill(prompt), ref.prefill(prompt)) <= REL_TOL
+        run.close()
+
+
+@pytest.mark.parametrize("batch,n_prompt", [(3, 5), (2, 70), (9, 33), (33, 65)])
+def test_batch_prompts_in_passes(backend, batch, n_prompt):
+    """Prompts of all sequences in shared passes (more rows than one pass takes in the last case) against the same
+    sequences one by one."""
+    cfg = ModelConfig(dim=512, n_layers=2, n_heads=8, n_kv_heads=2, head_dim=64, vocab_size=700, ff_dim=768, max_seq_len=128)
+    weights = synth.synthetic_model(cfg, seed=81, std=0.05, linear=DType.Q4_K, ffn_down=DType.Q6_K, output=DType.Q6_K)
+    prompts = synth.tokens(82, batch * n_prompt, cfg.vocab_size).reshape(batch, n_prompt)
+    run = CudaTransformerRunner(backend, cfg, weights, fused=1)
+    got = run.generate_greedy_batch(prompts, 6)
+    again = run.generate_greedy_batch(prompts, 6)
+    assert np.array_equal(got, again)
+    single = CudaTransformerRunner(backend, cfg, weights, fused=1)
+    for b in {0, batch // 2, batch - 1}:
+        single.reset()
+        assert np.array_equal(got[b], single.generate_greedy(prompts[b], 6)), f"sequence {b}"
+    # a larger pass replaces the row buffers of the runner: the captured step must follow
+    longer = synth.tokens(83, batch * 100, cfg.vocab_size).reshape(batch, 100)
+    run.generate_greedy_batch(longer, 2)
+    assert np.array_equal(run.generate_greedy_batch(prompts, 6), got)
+    single.close()
+    run.close()

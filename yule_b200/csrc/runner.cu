@@ -82,6 +82,7 @@ struct yule_cuda_runner {
     float *pf_x = nullptr, *pf_q = nullptr, *pf_k = nullptr, *pf_v = nullptr, *pf_att = nullptr, *pf_gate = nullptr,
           *pf_up = nullptr, *pf_attn_scratch = nullptr, *pf_norm = nullptr;
     uint32_t *pf_tokens = nullptr, *pf_tickets = nullptr;
+    std::vector<yule_buffer> pf_owned;  // the row buffers, replaced when a pass needs more rows
 
     // Batched decode: `bd_batch` independent sequences advancing one token per step, each with its own KV
     // caches and position; every linear is one GEMM over the batch (the chunk buffers above hold the rows).
@@ -861,6 +862,10 @@ int32_t ensure_pinned(yule_cuda_runner *r, size_t n_words) {
 // wait has given up (the waits themselves return at once after the first failure).
 constexpr uint32_t kStatusCheckTokens = 32;
 constexpr uint32_t kPrefillChunk = 512, kPrefillMinTokens = 16, kPrefillMinChunk = 256;
+// One GPU: passes of up to this many rows.  A launch's fixed part (about 10 us per GEMM) and the last, partly filled wave of
+// tiles count once per pass.
+constexpr uint32_t kPrefillMaxRows = 2048;
+uint32_t prefill_max_rows() { return knob("YULE_CUDA_PREFILL_CHUNK") ? 0u : kPrefillMaxRows; }  // the knob fixes the chunk size
 // Up to this many live rows a pass over the layers runs its linears on the batched matvec kernels (two to four rows
 // per pass over the weights, about the time of one) instead of the GEMM, whose fixed cost per launch is several
 // matvec passes.
@@ -892,45 +897,67 @@ bool prefill_batched_ok(const yule_cuda_runner *r) {
     return score_bytes <= 96 * 1024;
 }
 
-// Row buffers of the GEMM-driven paths (chunked prefill, batched decode), allocated on first use.  Under tensor
-// parallelism the matrices that are gathered (x, attention output, gate, up) live in the exchange region, which
-// every peer maps; q / k / v hold this rank's heads only.
-int32_t ensure_chunk_buffers(yule_cuda_runner *r) {
+// Row buffers of the GEMM-driven paths (chunked prefill, batched decode) for passes of up to `rows` rows, allocated on first
+// use and replaced when a pass needs more.  Under tensor parallelism the matrices that are gathered (x, attention output,
+// gate, up) live in the exchange region, which every peer maps (its size is fixed); q / k / v hold this rank's heads only.
+int32_t ensure_chunk_buffers(yule_cuda_runner *r, uint32_t rows) {
     const yule_runner_config &c = r->cfg;
     const uint32_t N = r->ctx->tp_world > 1 ? r->ctx->tp_world : 1;
     const uint32_t dim = c.dim, hd = c.head_dim, qdim = c.n_heads * hd, kvdim = c.n_kv_heads * hd, ff = c.ff_dim;
     int32_t rc;
-    if (!r->pf_chunk) {
-        uint32_t C = prefill_chunk_size(r);
-        if (N > 1 && C > r->xb_rows) C = r->xb_rows;
+    uint32_t C = prefill_chunk_size(r);
+    if (N > 1)
+        C = C > r->xb_rows ? r->xb_rows : C;
+    else
+        C = rows > C ? (rows + 127) / 128 * 128 : C;
+    if (r->pf_chunk < C) {
+        if (r->pf_chunk) {
+            // nothing that is still running may hold the old buffers, and the captured step must not
+            YULE_CUDA_TRY(cudaStreamSynchronize(r->ctx->stream));
+            if (r->bd_graph) cudaGraphExecDestroy(r->bd_graph);
+            r->bd_graph = nullptr;
+            for (yule_buffer h : r->pf_owned) yule_cuda_free(r->ctx, h);
+            r->pf_owned.clear();
+            r->pf_chunk = 0;
+        }
+        auto alloc = [&](size_t n, float **out) {
+            yule_buffer h;
+            const int32_t e = alloc_f32(r, n, out, &h);
+            if (e == YULE_OK) {
+                r->owned.pop_back();
+                r->pf_owned.push_back(h);
+            }
+            return e;
+        };
         r->pf_splits = c.max_seq_len / 1024 < 1 ? 1 : (c.max_seq_len / 1024 > 8 ? 8 : c.max_seq_len / 1024);
         float *tok_f = nullptr, *tick_f = nullptr, *bt = nullptr;
+        // rows that may go through the one-query-per-CTA attention kernel
+        const uint32_t A = C < kPrefillChunk ? C : kPrefillChunk;
         if (N > 1) {
             float *base = r->ctx->tp_peer_base[r->ctx->tp_rank];
             r->pf_x = base + r->xb_x;
             r->pf_att = base + r->xb_att;
             r->pf_gate = base + r->xb_gate;
             r->pf_up = base + r->xb_up;
-            if ((rc = alloc_f32(r, 4, &bt))) return rc;
+            if ((rc = alloc(4, &bt))) return rc;
             r->d_btick = (uint32_t *)bt;
-        } else if ((rc = alloc_f32(r, (size_t)C * dim, &r->pf_x)) || (rc = alloc_f32(r, (size_t)C * qdim, &r->pf_att)) ||
-                   (rc = alloc_f32(r, (size_t)C * ff, &r->pf_gate)) || (rc = alloc_f32(r, (size_t)C * ff, &r->pf_up))) {
+        } else if ((rc = alloc((size_t)C * dim, &r->pf_x)) || (rc = alloc((size_t)C * qdim, &r->pf_att)) ||
+                   (rc = alloc((size_t)C * ff, &r->pf_gate)) || (rc = alloc((size_t)C * ff, &r->pf_up))) {
             return rc;
         }
-        if ((rc = alloc_f32(r, (size_t)C * (qdim / N), &r->pf_q)) || (rc = alloc_f32(r, (size_t)C * (kvdim / N), &r->pf_k)) ||
-            (rc = alloc_f32(r, (size_t)C * (kvdim / N), &r->pf_v)) || (rc = alloc_f32(r, C, &tok_f)) ||
-            (rc = alloc_f32(r, (size_t)C * c.n_heads, &tick_f)) ||
-            (rc = alloc_f32(r, (size_t)C * attn_scratch_floats(c.n_heads / N, r->pf_splits, hd) + 4, &r->pf_attn_scratch)) ||
-            (rc = alloc_f32(r, (size_t)kRowsMatvecMax * dim, &r->pf_norm)))
+        if ((rc = alloc((size_t)C * (qdim / N), &r->pf_q)) || (rc = alloc((size_t)C * (kvdim / N), &r->pf_k)) ||
+            (rc = alloc((size_t)C * (kvdim / N), &r->pf_v)) || (rc = alloc(C > c.max_seq_len ? C : c.max_seq_len, &tok_f)) ||
+            (rc = alloc((size_t)A * c.n_heads, &tick_f)) ||
+            (rc = alloc((size_t)A * attn_scratch_floats(c.n_heads / N, r->pf_splits, hd) + 4, &r->pf_attn_scratch)) ||
+            (rc = alloc((size_t)kRowsMatvecMax * dim, &r->pf_norm)))
             return rc;
         r->pf_tokens = (uint32_t *)tok_f;
         r->pf_tickets = (uint32_t *)tick_f;  // zero-filled by the allocator; the kernel leaves them at zero
         r->pf_chunk = C;
     }
-    const uint32_t C = r->pf_chunk;
     const uint32_t widest = ff > qdim ? (ff > dim ? ff : dim) : (qdim > dim ? qdim : dim);
-    if ((rc = ensure_gemm_scratch(r->ctx, qgemm_scratch_bytes(C, widest)))) return rc;
-    return ensure_pinned(r, C);
+    if ((rc = ensure_gemm_scratch(r->ctx, qgemm_scratch_bytes(r->pf_chunk, widest)))) return rc;
+    return ensure_pinned(r, r->pf_chunk);
 }
 
 // One pass of `m` rows through every layer with one GEMM per linear: the body shared by the chunked prefill
@@ -942,8 +969,10 @@ struct RowsPass {
     uint32_t m = 0;            // rows the GEMMs run over
     uint32_t n_live = 0;       // rows that carry a token (RoPE, KV write and attention touch only these)
     const uint32_t *tokens = nullptr;
-    bool batch = false;        // false: prefill at positions pos0 .. pos0 + n_live − 1 of the runner's caches
-    uint32_t pos0 = 0;
+    bool batch = false;        // one row per sequence of the decode batch, each at its own position
+    // otherwise: prompt tokens at positions pos0, pos0 + 1, … of the runner's caches, or (n_seq > 0) of the caches of n_seq
+    // sequences of the decode batch, n_live / n_seq rows each
+    uint32_t pos0 = 0, n_seq = 0;
 };
 
 cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t *launches) {
@@ -1090,6 +1119,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         lin(L.attn_v, kvdim_l, dim, r->pf_v, kvdim_l, nullptr);
         flush();
         AttnDecode a;
+        bool tiled = false;  // the queries share K / V tiles
         if (ps.batch) {
             ok(launch_rope_kv_write_batch(r->pf_q, r->pf_k, r->pf_v, r->bd_k[l], r->bd_v[l], r->rope_cos, r->rope_sin, 0, ps.n_live, hd,
                                           c.n_heads / N, c.n_kv_heads / N, s, launches, r->bd_pos, cache_stride));
@@ -1099,8 +1129,30 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
             a.pos_per_query = true;
             a.kv_batch_stride = cache_stride;
         } else {
-            ok(launch_rope_kv_write_batch(r->pf_q, r->pf_k, r->pf_v, L.k_cache, L.v_cache, r->rope_cos, r->rope_sin, ps.pos0, ps.n_live, hd,
-                                          c.n_heads / N, c.n_kv_heads / N, s, launches));
+            float *kc = ps.n_seq ? r->bd_k[l] : L.k_cache, *vc = ps.n_seq ? r->bd_v[l] : L.v_cache;
+            const uint32_t n_seq = ps.n_seq ? ps.n_seq : 1, n_tok = ps.n_live / n_seq;
+            ok(launch_rope_kv_write_batch(r->pf_q, r->pf_k, r->pf_v, kc, vc, r->rope_cos, r->rope_sin, ps.pos0, ps.n_live, hd,
+                                          c.n_heads / N, c.n_kv_heads / N, s, launches, nullptr, cache_stride, n_tok));
+            if (ps.n_seq || ps.n_live > kPrefillChunk || attn_prefill_preferred(hd, c.n_heads / N, c.n_kv_heads / N, n_tok, n_seq, ps.pos0, sms)) {
+                AttnPrefill ap;
+                ap.q = r->pf_q;
+                ap.k_cache = kc;
+                ap.v_cache = vc;
+                ap.out = r->pf_att + (size_t)R * qdim_l;
+                ap.n_tokens = n_tok;
+                ap.n_seq = n_seq;
+                ap.pos0 = ps.pos0;
+                ap.hd = hd;
+                ap.n_heads = c.n_heads / N;
+                ap.n_kv_heads = c.n_kv_heads / N;
+                ap.kv_stride = kvdim_l;
+                ap.q_stride = qdim_l;
+                ap.out_stride = qdim;
+                ap.kv_batch_stride = cache_stride;
+                ap.pdl = true;
+                ok(launch_attn_prefill(ap, s, launches));
+                tiled = true;
+            }
             a.k_cache = L.k_cache;
             a.v_cache = L.v_cache;
             a.seq_len = ps.pos0 + 1;  // query z attends to positions [0, pos0 + z]
@@ -1120,7 +1172,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         a.n_tokens = ps.n_live;
         a.q_stride = qdim_l;
         a.out_stride = qdim;
-        ok(launch_attn_decode(a, s, launches));
+        if (!tiled) ok(launch_attn_decode(a, s, launches));
         exchange(r->xb_att, qdim_l, qdim);
         prep(r->pf_att, qdim, nullptr, nullptr);
         lin(L.attn_output, dim_l, qdim, r->pf_x + (size_t)R * dim_l, dim, r->pf_x + (size_t)R * dim_l);  // x += Wo · attention
@@ -1152,7 +1204,9 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
     yule_cuda_ctx *ctx = r->ctx;
     cudaStream_t s = ctx->stream;
     int32_t rc;
-    if ((rc = ensure_chunk_buffers(r))) return rc;
+    if ((rc = ensure_chunk_buffers(r, n < prefill_max_rows() ? n : prefill_max_rows()))) return rc;
+    YULE_CUDA_TRY(cudaStreamSynchronize(s));  // staging words may still be in flight
+    if ((rc = ensure_pinned(r, n))) return rc;
     const uint32_t C = r->pf_chunk;
     uint64_t launches = 0;
     struct Guard {
@@ -1160,15 +1214,14 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
         uint64_t *n;
         ~Guard() { ctx->launches.fetch_add(*n); }
     } guard{ctx, &launches};
+    memcpy(r->h_pinned, tokens, (size_t)n * 4);
+    YULE_CUDA_TRY(cudaMemcpyAsync(r->pf_tokens, r->h_pinned, (size_t)n * 4, cudaMemcpyHostToDevice, s));
     for (uint32_t c0 = 0; c0 < n; c0 += C) {
         const uint32_t m = n - c0 < C ? n - c0 : C;
-        YULE_CUDA_TRY(cudaStreamSynchronize(s));  // the staging words of the previous chunk may still be in flight
-        for (uint32_t i = 0; i < m; i++) r->h_pinned[i] = tokens[c0 + i];
-        YULE_CUDA_TRY(cudaMemcpyAsync(r->pf_tokens, r->h_pinned, (size_t)m * 4, cudaMemcpyHostToDevice, s));
         RowsPass ps;
         ps.m = m;
         ps.n_live = m;
-        ps.tokens = r->pf_tokens;
+        ps.tokens = r->pf_tokens + c0;
         ps.pos0 = r->pos + c0;
         cudaError_t e = enqueue_rows_pass(r, ps, &launches);
         if (e != cudaSuccess) return fail_cuda(e, "batched prefill");
@@ -1205,9 +1258,10 @@ int32_t ensure_batch_state(yule_cuda_runner *r, uint32_t batch) {
         return fail(YULE_ERR_INVALID_ARGUMENT, "batched decode needs a runner created with fused = 1 (under tensor parallelism: with "
                                                "the peer exchange), block-quantised linears with column counts in multiples of 256 "
                                                "and the Llama op sequence");
-    int32_t rc = ensure_chunk_buffers(r);
+    int32_t rc = ensure_chunk_buffers(r, 0);
     if (rc) return rc;
-    if (batch == 0 || batch > r->pf_chunk) return fail(YULE_ERR_INVALID_ARGUMENT, "batch %u outside 1..%u", batch, r->pf_chunk);
+    const uint32_t most = r->pf_chunk < prefill_chunk_size(r) ? r->pf_chunk : prefill_chunk_size(r);
+    if (batch == 0 || batch > most) return fail(YULE_ERR_INVALID_ARGUMENT, "batch %u outside 1..%u", batch, most);
     if (r->bd_batch == batch) return YULE_OK;
     if (r->bd_batch) return fail(YULE_ERR_INVALID_ARGUMENT, "this runner decodes batches of %u sequences; %u asked for", r->bd_batch, batch);
     const uint32_t tpw = r->ctx->tp_world > 1 ? r->ctx->tp_world : 1;
@@ -1495,6 +1549,7 @@ int32_t yule_cuda_runner_destroy(yule_cuda_runner *r) {
     if (r->h_moe_sel) cudaFreeHost(r->h_moe_sel);
     if (r->h_pinned) cudaFreeHost(r->h_pinned);
     for (yule_buffer h : r->owned) yule_cuda_free(r->ctx, h);
+    for (yule_buffer h : r->pf_owned) yule_cuda_free(r->ctx, h);
     // collective: every rank destroys its runner at the same point (a runner whose creation failed half-way leaves
     // the region to the context, which frees it without a rendezvous)
     if (r->xchg && r->created) tp_release_exchange(r->ctx);
@@ -1822,9 +1877,15 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
     if ((uint64_t)n_prompt + n_generate > c.max_seq_len) return fail(YULE_ERR_CONTEXT_LENGTH, "context length exceeded");
     for (size_t i = 0; i < (size_t)batch * n_prompt; i++)
         if (prompts[i] >= c.vocab_size) return fail(YULE_ERR_INVALID_ARGUMENT, "token %u outside the vocabulary", prompts[i]);
-    if ((rc = ensure_batch_graph(r))) return rc;
     cudaStream_t s = r->ctx->stream;
-    // prompts to the device, position-major, so that step i takes its tokens with one small device copy
+    // All prompt tokens but the last are known in advance: they go through the layers in passes of many rows (KV caches
+    // only); the last one is the first step of the batch.
+    const uint32_t fed = n_prompt - 1;
+    uint32_t per_seq = (r->xchg || !prefill_max_rows() ? r->pf_chunk : prefill_max_rows()) / batch;  // prompt tokens of each sequence per pass
+    per_seq = per_seq < 1 ? 1 : (per_seq > fed ? fed : per_seq);
+    if (fed && (rc = ensure_chunk_buffers(r, per_seq * batch))) return rc;
+    if ((rc = ensure_batch_graph(r))) return rc;
+    // prompts to the device, pass by pass, the rows of a pass in the order of the sequences
     const size_t n_words = (size_t)batch * n_prompt;
     if (r->bd_prompts_cap < n_words) {
         float *pw = nullptr;
@@ -1834,19 +1895,34 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
     }
     if ((rc = ensure_pinned(r, n_words + batch + 1))) return rc;
     YULE_CUDA_TRY(cudaStreamSynchronize(s));
-    for (uint32_t i = 0; i < n_prompt; i++)
-        for (uint32_t b = 0; b < batch; b++) r->h_pinned[(size_t)i * batch + b] = prompts[(size_t)b * n_prompt + i];
-    for (uint32_t b = 0; b <= batch; b++) r->h_pinned[n_words + b] = 0;  // positions and step start at zero
+    for (uint32_t p0 = 0; p0 < n_prompt;) {
+        const uint32_t n = p0 < fed ? (fed - p0 < per_seq ? fed - p0 : per_seq) : 1;
+        for (uint32_t b = 0; b < batch; b++)
+            for (uint32_t i = 0; i < n; i++) r->h_pinned[(size_t)p0 * batch + (size_t)b * n + i] = prompts[(size_t)b * n_prompt + p0 + i];
+        p0 += n;
+    }
+    for (uint32_t b = 0; b <= batch; b++) r->h_pinned[n_words + b] = fed;  // positions and step of the first batch step
     YULE_CUDA_TRY(cudaMemcpyAsync(r->bd_prompts, r->h_pinned, n_words * 4, cudaMemcpyHostToDevice, s));
     YULE_CUDA_TRY(cudaMemcpyAsync(r->bd_pos, r->h_pinned + n_words, (size_t)batch * 4, cudaMemcpyHostToDevice, s));
     YULE_CUDA_TRY(cudaMemcpyAsync(r->bd_step, r->h_pinned + n_words + batch, 4, cudaMemcpyHostToDevice, s));
-    for (uint32_t i = 0; i < n_prompt + n_generate; i++) {
-        // prompt steps take their tokens from the prompt; afterwards each step consumes the previous step's picks
-        if (i < n_prompt)
-            YULE_CUDA_TRY(cudaMemcpyAsync(r->bd_tokens, r->bd_prompts + (size_t)i * batch, (size_t)batch * 4, cudaMemcpyDeviceToDevice, s));
-        YULE_CUDA_TRY(cudaGraphLaunch(r->bd_graph, s));
+    uint64_t launches = 0;
+    for (uint32_t p0 = 0; p0 < fed; p0 += per_seq) {
+        RowsPass ps;
+        ps.n_seq = batch;
+        ps.n_live = ps.m = (fed - p0 < per_seq ? fed - p0 : per_seq) * batch;
+        ps.tokens = r->bd_prompts + (size_t)p0 * batch;
+        ps.pos0 = p0;
+        if (ps.m < 8) ps.m = 8;  // the GEMM works on at least eight rows; the extra ones stay unused
+        const cudaError_t e = enqueue_rows_pass(r, ps, &launches);
+        if (e != cudaSuccess) {
+            r->ctx->launches.fetch_add(launches);
+            return fail_cuda(e, "batched prefill");
+        }
     }
-    r->ctx->launches.fetch_add((uint64_t)r->bd_graph_kernels * (n_prompt + n_generate));
+    YULE_CUDA_TRY(cudaMemcpyAsync(r->bd_tokens, r->bd_prompts + (size_t)fed * batch, (size_t)batch * 4, cudaMemcpyDeviceToDevice, s));
+    for (uint32_t i = fed; i < n_prompt + n_generate; i++)  // each step after the first consumes the picks of the one before
+        YULE_CUDA_TRY(cudaGraphLaunch(r->bd_graph, s));
+    r->ctx->launches.fetch_add(launches + (uint64_t)r->bd_graph_kernels * (1 + n_generate));
     // token g of sequence b is the pick made after position n_prompt − 1 + g
     const size_t hist_stride = (size_t)c.max_seq_len + 1;
     for (uint32_t b = 0; b < batch && n_generate; b++)
