@@ -492,6 +492,9 @@ static uint32_t gemm_min_batch(const QmvArgs &a) {
         const int v = atoi(e);
         return v < 8 ? 8u : (uint32_t)v;
     }
+    // the matvec over sixteen vectors a pass wins up to the line that qmv_rows_preferred draws
+    const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
+    if (a.batch >= 8 && qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) return qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) ? ~0u : 8u;
     const bool tuned = a.type == YULE_DTYPE_Q4_K || a.type == YULE_DTYPE_Q6_K || a.type == YULE_DTYPE_Q8_0 || a.type == YULE_DTYPE_Q4_0;
     if (tuned && a.batch >= 8 && kquant_batch_width(a) < 2 && q8q4_ring_batch_width(a) < 2) return 8u;
     if (a.type == YULE_DTYPE_Q4_K) return (uint64_t)a.n_rows * a.n_cols <= (8ull << 20) ? 32u : 16u;

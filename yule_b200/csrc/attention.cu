@@ -222,6 +222,8 @@ __global__ void __launch_bounds__(kThreads) attn_decode_gqa_kernel(const __grid_
     au.k_cache = p.k_cache + (size_t)z * p.kv_batch_stride;
     au.v_cache = p.v_cache + (size_t)z * p.kv_batch_stride;
     au.q_in = p.q + (size_t)z * p.q_stride;
+    au.k_new = p.k_new ? p.k_new + (size_t)z * p.kv_stride : nullptr;
+    au.v_new = p.v_new ? p.v_new + (size_t)z * p.kv_stride : nullptr;
     au.scratch = p.scratch + (size_t)z * p.n_heads * p.n_splits * (HD + 2);
     au.tickets = p.tickets + (size_t)z * p.n_heads;
     au.q_pairs = au.k_pairs = au.v_pairs = nullptr;
@@ -317,8 +319,10 @@ cudaError_t launch_attn_decode(const AttnDecode &a, cudaStream_t s, uint64_t *la
         p.q_stride = a.q_stride;
         p.out_stride = a.out_stride;
         p.tp = a.tp;
-        // several queries per launch read the caches only; a device position is one per query then (batched decode)
-        if (a.n_tokens > 1 && (a.k_new || (a.pos_ptr && !a.pos_per_query))) return cudaErrorInvalidValue;
+        // several queries per launch: consecutive positions of one cache, which they only read, or (batched decode) each with a
+        // device position, a cache and new rows of its own
+        if (a.n_tokens > 1 && (a.k_new || a.pos_ptr) && !a.pos_per_query) return cudaErrorInvalidValue;
+        if (a.n_tokens > 1 && a.k_new && !a.kv_batch_stride) return cudaErrorInvalidValue;
 #define YULE_GQA_CASE(G, H) if (g == G && a.hd == H) return launch_gqa_variant<G, H>(p, smem, a.pdl, s, a.n_tokens)
         YULE_GQA_CASE(1, 64); YULE_GQA_CASE(2, 64); YULE_GQA_CASE(4, 64); YULE_GQA_CASE(8, 64);
         YULE_GQA_CASE(1, 128); YULE_GQA_CASE(2, 128); YULE_GQA_CASE(4, 128); YULE_GQA_CASE(8, 128);

@@ -21,8 +21,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 struct AttnParams {
     // inputs
     const float *q;        // [n_heads][hd]; rotated here when cos_table is set
-    const float *k_new;    // [n_kv][hd] un-rotated K row of the current token (fused mode) or null
-    const float *v_new;    // [n_kv][hd] V row of the current token (fused mode) or null
+    const float *k_new;    // [n_kv][hd] un-rotated K row of the current token (fused mode; of each query, kv_stride apart) or null
+    const float *v_new;    // [n_kv][hd] V row of the current token (fused mode; likewise) or null
     float *k_cache;        // [max_seq][kv_stride]
     float *v_cache;
     const float *cos_table, *sin_table;  // [max_seq][hd/2] or null
@@ -49,6 +49,7 @@ struct AttnUnit {
     uint32_t *tickets;   // [n_kv_heads] of this query, zero between uses
     float *scratch;      // split partials of this query
     const float *q_in;   // [n_heads][HD], or null when the inputs are pairs
+    const float *k_new, *v_new;  // this query's new rows (fused mode without pairs), else null
     const uint2 *q_pairs, *k_pairs, *v_pairs;
     uint32_t in_epoch;
     uint32_t pos;
@@ -217,7 +218,7 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
     float *scratch_z = au.scratch;
     uint32_t *tickets_z = au.tickets;
     const uint32_t seq = pos + 1;
-    const bool fused = PAIRS || p.k_new != nullptr;
+    const bool fused = PAIRS || au.k_new != nullptr;
     // Sliding window: the reference masks positions t < pos − window to −inf once pos >= window; they then carry
     // no weight, so the splits simply cover [begin, seq) instead of [0, seq).  With an attention softcap as well
     // the reference caps after masking (model_runner.rs:688-721), and cap·tanh(−inf / cap) is −cap, a finite
@@ -286,11 +287,11 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
         if (tid < HD) pv = pair_peek(au.v_pairs + (size_t)kvh * HD + tid);
     }
     auto k_at = [&](size_t i) {
-        if (!PAIRS) return p.k_new[i];
+        if (!PAIRS) return au.k_new[i];
         return pair_settle(pk[i & 1], au.k_pairs + i, au.in_epoch, p.status, p.wait_cycles);  // i = kvh·HD + 2·tid + {0, 1}
     };
     auto v_at = [&](size_t i) {
-        if (!PAIRS) return p.v_new[i];
+        if (!PAIRS) return au.v_new[i];
         return pair_settle(pv, au.v_pairs + i, au.in_epoch, p.status, p.wait_cycles);  // i = kvh·HD + tid
     };
 #pragma unroll

@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_token_kernel(const __g
                 au.v_cache = reinterpret_cast<float *>(hot[ph].ptr[1]);
                 au.tickets = reinterpret_cast<uint32_t *>(hot[ph].ptr[2]);
                 au.scratch = p.attn.scratch;
-                au.q_in = nullptr;
+                au.q_in = au.k_new = au.v_new = nullptr;
                 au.q_pairs = p.vec[kVecQ];
                 au.k_pairs = p.vec[kVecK];
                 au.v_pairs = p.vec[kVecV];

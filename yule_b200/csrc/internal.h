@@ -199,7 +199,7 @@ struct QmvArgs {
     // only this kernel's stores have to wait for it (one-vector and Q8_0 / Q4_0 batch kernels; ignored elsewhere).
     bool late_wait = false;
     const uint8_t *planar = nullptr;  // Q6_K: planar copy of the same tensor, when one was prepared
-    const float *norm_w = nullptr;    // RMSNorm prologue (one-vector kernel and kquant_batch_can_share only)
+    const float *norm_w = nullptr;    // RMSNorm prologue (one-vector kernel and qmv_rows only)
     float eps = 0.f;
     TpFuse tp;                        // one vector of Q4_K only
     int *status = nullptr;            // device status word for bounded waits inside the kernels, or null
@@ -229,6 +229,29 @@ bool qmv_digits_supported(uint32_t type, const void *w, uint32_t n_cols);
 bool qmv_digits_can_pair(uint32_t n_cols);
 cudaError_t launch_qmv_digits(const QmvDigits &f, int sm_count, cudaStream_t s, uint64_t *launches);
 
+// Several activation vectors against one to three matrices of one format, up to sixteen vectors per pass (qmv_rows.cu).
+struct QmvRows {
+    uint32_t type = 0;
+    const uint8_t *w[3] = {nullptr, nullptr, nullptr};  // raw blocks, 16-byte aligned; Q6_K: the row-planar copies
+    float *out[3] = {nullptr, nullptr, nullptr};        // [batch][out_stride]
+    uint32_t rows[3] = {0, 0, 0}, out_stride[3] = {0, 0, 0};
+    uint32_t n_seg = 1;
+    const float *x = nullptr;         // [batch][x_stride], 16-byte aligned, x_stride a multiple of 4
+    uint32_t n_cols = 0, x_stride = 0, batch = 0;
+    const float *norm_w = nullptr;    // RMSNorm prologue on every vector when set
+    float eps = 0.f;
+    const float *residual = nullptr;  // added to out[0] when set (same layout)
+    bool swiglu_pair = false;         // w[0], w[1] = gate, up of equal size → out[0] = SiLU(gate)·up
+    bool pdl = false, late_wait = false;  // as in QmvDigits
+    int *status = nullptr;            // device status word for the kernel's bounded waits, or null
+    long long wait_cycles = kDefaultWaitCycles;
+};
+// Whether `batch` vectors (two or more) against a matrix of this format belong to qmv_rows rather than to the kernels for two to four
+// vectors per pass or to the GEMM (the pointers and strides have to be qmv_rows_supported besides).
+bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch);
+bool qmv_rows_supported(uint32_t type, const void *w, const float *x, uint32_t n_cols, uint32_t x_stride);
+cudaError_t launch_qmv_rows(const QmvRows &f, cudaStream_t s, uint64_t *launches);
+
 // Q8_0 / Q4_0 over two to four activation vectors per pass (qmv_q8q4_ring.cu: n_cols a multiple of 256, weights and
 // activations 16-byte aligned): the number of vectors one pass can take for this call (0: not supported), and one pass
 // over the first `nb` vectors of `a`.
@@ -239,11 +262,6 @@ cudaError_t launch_q8q4_ring_batch(const QmvArgs &a, uint32_t nb, int sm_count, 
 // vectors one pass can take for this call (0: not supported), and one pass over the first `nb` vectors of `a`.
 uint32_t kquant_batch_width(const QmvArgs &a);
 cudaError_t launch_kquant_batch(const QmvArgs &a, uint32_t nb, int sm_count, cudaStream_t s, uint64_t *launches);
-// Up to three matrices that read the same activation rows (Q/K/V; gate/up) as ONE launch per pass of four vectors, with
-// the optional RMSNorm prologue (norm_w / eps of the arguments): whether the arguments allow it, and the launch.
-bool kquant_batch_can_share(const QmvArgs *segs, uint32_t n_seg);
-cudaError_t launch_kquant_batch_shared(const QmvArgs *segs, uint32_t n_seg, int sm_count, cudaStream_t s, uint64_t *launches);
-
 // Quantised GEMM on tcgen05 for eight or more activation rows (qgemm_tc.cu): an activation
 // re-layout kernel followed by the persistent GEMM.  `scratch` holds qgemm_scratch_bytes().
 struct QGemm {
@@ -486,10 +504,10 @@ int32_t ensure_sampler_scratch(yule_cuda_ctx *ctx, size_t n_floats);
 
 // Tiled 2-D tensor map (qgemm_tc.cu); `out` points to a CUtensorMap (128 bytes, 64-byte aligned).
 cudaError_t encode_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t inner, uint64_t n_rows, uint64_t row_stride_bytes,
-                                 uint32_t box_inner, uint32_t box_rows, void *out);
+                                 uint32_t box_inner, uint32_t box_rows, void *out, uint32_t swizzle = 0);  // swizzle: 0, 64 or 128 bytes
 
 cudaError_t cached_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t inner, uint64_t n_rows, uint64_t row_stride_bytes,
-                                 uint32_t box_inner, uint32_t box_rows, void *out);
+                                 uint32_t box_inner, uint32_t box_rows, void *out, uint32_t swizzle = 0);
 
 // Persistent decode kernel (decode_mega.cu): the whole token step of a dense Llama-family model in one cooperative
 // launch.  Covers: one GPU, no architecture variant, Q4_K attn_q/k/v and ffn_gate/up, Q4_K or Q6_K (row-planar copy)

@@ -1194,32 +1194,32 @@ uint32_t pick_bn(uint32_t n_tokens) { return n_tokens <= 32 ? 32 : (n_tokens <= 
 // The same through a per-process cache: a map depends on the address and the shape only, and encoding one costs a
 // driver call, which the matvec entry points would otherwise pay on every launch.
 cudaError_t cached_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t inner, uint64_t n_rows, uint64_t row_stride_bytes,
-                                 uint32_t box_inner, uint32_t box_rows, void *out) {
+                                 uint32_t box_inner, uint32_t box_rows, void *out, uint32_t swizzle) {
     struct Key {
         const void *base;
         uint64_t inner, n_rows, stride;
-        uint32_t elem, box_inner, box_rows;
+        uint32_t elem, box_inner, box_rows, swizzle;
         bool operator==(const Key &o) const {
             return base == o.base && inner == o.inner && n_rows == o.n_rows && stride == o.stride && elem == o.elem &&
-                   box_inner == o.box_inner && box_rows == o.box_rows;
+                   box_inner == o.box_inner && box_rows == o.box_rows && swizzle == o.swizzle;
         }
     };
     struct Hash {
         size_t operator()(const Key &k) const {
             size_t h = std::hash<const void *>()(k.base);
-            for (uint64_t v : {k.inner, k.n_rows, k.stride, (uint64_t)k.elem, (uint64_t)k.box_inner, (uint64_t)k.box_rows})
+            for (uint64_t v : {k.inner, k.n_rows, k.stride, (uint64_t)k.elem, (uint64_t)k.box_inner, (uint64_t)k.box_rows, (uint64_t)k.swizzle})
                 h = h * 0x9E3779B97F4A7C15ull + std::hash<uint64_t>()(v);
             return h;
         }
     };
     static std::unordered_map<Key, CUtensorMap, Hash> cache;
     static std::mutex mu;
-    const Key key{base, inner, n_rows, row_stride_bytes, elem_bytes, box_inner, box_rows};
+    const Key key{base, inner, n_rows, row_stride_bytes, elem_bytes, box_inner, box_rows, swizzle};
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it == cache.end()) {
         CUtensorMap m;
-        cudaError_t e = encode_tensor_map_2d(base, elem_bytes, inner, n_rows, row_stride_bytes, box_inner, box_rows, &m);
+        cudaError_t e = encode_tensor_map_2d(base, elem_bytes, inner, n_rows, row_stride_bytes, box_inner, box_rows, &m, swizzle);
         if (e != cudaSuccess) return e;
         if (cache.size() >= 16384) cache.clear();
         it = cache.emplace(key, m).first;
@@ -1229,10 +1229,10 @@ cudaError_t cached_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t
 }
 
 // Tiled 2-D tensor map over rows of `elem_bytes`-sized elements (1 or 8): `inner` elements per row, `n_rows` rows
-// `row_stride_bytes` apart (a multiple of 16; base 16-byte aligned), box of box_inner x box_rows elements, no
-// swizzle, out-of-range elements read as zeros.  `out` is a CUtensorMap.
+// `row_stride_bytes` apart (a multiple of 16; base 16-byte aligned), box of box_inner x box_rows elements, swizzled
+// within 0 (not at all), 64 or 128 bytes, out-of-range elements read as zeros.  `out` is a CUtensorMap.
 cudaError_t encode_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t inner, uint64_t n_rows, uint64_t row_stride_bytes,
-                                 uint32_t box_inner, uint32_t box_rows, void *out) {
+                                 uint32_t box_inner, uint32_t box_rows, void *out, uint32_t swizzle) {
     typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1255,7 +1255,8 @@ cudaError_t encode_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t
     const cuuint32_t box[2] = {box_inner, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(static_cast<CUtensorMap *>(out), elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT64, 2,
-                        const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }

@@ -548,6 +548,31 @@ constexpr size_t kMaxSmem = 200 * 1024;
 }  // namespace
 
 cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t *launches) {
+    // several vectors, up to sixteen per pass (YULE_QMV_ROWS=0 / 1: never / wherever it can)
+    if (a.batch >= 2) {
+        const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
+        const bool wanted = knob("YULE_QMV_ROWS") ? atoi(knob("YULE_QMV_ROWS")) != 0 : qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch);
+        if (wanted && qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) {
+            QmvRows f;
+            f.type = a.type;
+            f.w[0] = w;
+            f.out[0] = a.out;
+            f.rows[0] = a.n_rows;
+            f.out_stride[0] = a.out_stride;
+            f.x = a.x;
+            f.n_cols = a.n_cols;
+            f.x_stride = a.x_stride;
+            f.batch = a.batch;
+            f.norm_w = a.norm_w;
+            f.eps = a.eps;
+            f.residual = a.residual;
+            f.pdl = a.pdl;
+            f.late_wait = a.late_wait;
+            f.status = a.status;
+            f.wait_cycles = a.wait_cycles;
+            return launch_qmv_rows(f, s, launches);
+        }
+    }
     // Q4_K / Q6_K, several vectors: two to four per pass of the batched ring kernel (YULE_QMV_KBATCH=0: the older paths);
     // a single left-over vector goes through the one-vector routing below
     if (a.batch >= 2 && kquant_batch_width(a) >= 2 && !(knob("YULE_QMV_KBATCH") && atoi(knob("YULE_QMV_KBATCH")) == 0)) {
@@ -566,7 +591,7 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
         }
         return cudaSuccess;
     }
-    // one vector, tuned block format (Q6_K: prepared): the fp8-digit kernel
+    // one vector, tuned block format (Q6_K: prepared): the integer-digit kernel
     if (a.batch == 1) {
         const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
         if (qmv_digits_supported(a.type, w, a.n_cols) && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0) {

@@ -635,55 +635,6 @@ uint32_t kquant_batch_width(const QmvArgs &a) {
     return 0;
 }
 
-// Matrices that share their activations (Q/K/V, gate/up) as one launch: same format, columns, vectors, prologue.
-bool kquant_batch_can_share(const QmvArgs *segs, uint32_t n_seg) {
-    if (n_seg < 1 || n_seg > (uint32_t)kMaxSegs) return false;
-    const QmvArgs &a = segs[0];
-    const uint32_t nb = kquant_batch_width(a);
-    if (nb < 2) return false;
-    if (part_cols_for(a.type == YULE_DTYPE_Q6_K, a.n_cols, nb) != a.n_cols) return false;  // rows that need several launches: one matrix at a time
-    for (uint32_t i = 1; i < n_seg; i++) {
-        const QmvArgs &g = segs[i];
-        if (g.type != a.type || g.n_cols != a.n_cols || g.x != a.x || g.batch != a.batch || g.x_stride != a.x_stride || g.norm_w != a.norm_w ||
-            g.residual || a.residual || kquant_batch_width(g) != nb)
-            return false;
-    }
-    return true;
-}
-
-cudaError_t launch_kquant_batch_shared(const QmvArgs *segs, uint32_t n_seg, int sm_count, cudaStream_t s, uint64_t *launches) {
-    if (!kquant_batch_can_share(segs, n_seg)) return cudaErrorInvalidValue;
-    // passes of up to four vectors over all the matrices
-    const QmvArgs &a = segs[0];
-    const bool q6 = a.type == YULE_DTYPE_Q6_K;
-    uint32_t done = 0;
-    while (done < a.batch) {
-        QmvArgs part[kMaxSegs];
-        for (uint32_t i = 0; i < n_seg; i++) {
-            part[i] = segs[i];
-            part[i].x = segs[i].x + (size_t)done * segs[i].x_stride;
-            part[i].out = segs[i].out + (size_t)done * segs[i].out_stride;
-            part[i].residual = segs[i].residual ? segs[i].residual + (size_t)done * segs[i].out_stride : nullptr;
-            part[i].batch = a.batch - done;
-        }
-        const uint32_t nb = kquant_batch_width(part[0]);
-        if (nb < 2) {  // one vector left: the one-vector kernels, matrix by matrix
-            for (uint32_t i = 0; i < n_seg; i++) {
-                cudaError_t e = launch_qmv(part[i], sm_count, s, launches);
-                if (e != cudaSuccess) return e;
-            }
-            return cudaSuccess;
-        }
-        const uint32_t stages = batch_stages(q6, a.n_cols, nb);
-        cudaError_t e = q6 ? launch_variant<true>(part, n_seg, nb, stages, 0, a.n_cols, part[0].residual, sm_count, s)
-                           : launch_variant<false>(part, n_seg, nb, stages, 0, a.n_cols, part[0].residual, sm_count, s);
-        if (e != cudaSuccess) return e;
-        *launches += 1;
-        done += nb;
-    }
-    return cudaSuccess;
-}
-
 cudaError_t launch_kquant_batch(const QmvArgs &a, uint32_t nb, int sm_count, cudaStream_t s, uint64_t *launches) {
     const bool q6 = a.type == YULE_DTYPE_Q6_K;
     if (nb < 2 || nb > 4) return cudaErrorInvalidValue;

@@ -866,9 +866,8 @@ constexpr uint32_t kPrefillChunk = 512, kPrefillMinTokens = 16, kPrefillMinChunk
 // tiles count once per pass.
 constexpr uint32_t kPrefillMaxRows = 2048;
 uint32_t prefill_max_rows() { return knob("YULE_CUDA_PREFILL_CHUNK") ? 0u : kPrefillMaxRows; }  // the knob fixes the chunk size
-// Up to this many live rows a pass over the layers runs its linears on the batched matvec kernels (two to four rows
-// per pass over the weights, about the time of one) instead of the GEMM, whose fixed cost per launch is several
-// matvec passes.
+// Up to this many live rows the linears in formats that qmv_rows does not take run on the element-wise matvec instead of the
+// GEMM, whose fixed cost per launch is several matvec passes.
 constexpr uint32_t kRowsMatvecMax = 12;
 
 uint32_t prefill_chunk_size(const yule_cuda_runner *r) {
@@ -1040,50 +1039,102 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         gq_open = true;
         if (residual) mm_flush();
     };
-    // Few live rows: the same sequence of linears on the matvec kernels.  `prep` leaves the rows the next linears read
-    // in `act`: normed rows in a buffer of their own, SwiGLU in place, anything else where it is.
-    bool mv = ps.n_live <= kRowsMatvecMax;
-    if (const char *k = knob("YULE_ROWS_MATVEC")) mv = mv && atoi(k) != 0;
-    // The matrices that read the same rows (Q/K/V; gate/up) are collected and launched together by `flush`: as one
-    // launch with the RMSNorm folded into its staging where the batched kernel allows it, else one by one behind a
-    // separate RMSNorm kernel.
-    const float *act = nullptr, *act_norm = nullptr;
-    QmvArgs pending[3];
+    // Few live rows: the same sequence of linears on the matvec kernels, decided matrix by matrix (`on_matvec`).  `prep` says what the
+    // next linears read: rows, normed rows, or (gate set) SwiGLU of two; each kernel family takes it from there — the GEMMs
+    // through one re-layout, the matvec kernels with the norm folded in where they can and SwiGLU done in place.
+    float *act = nullptr;
+    const float *act_norm = nullptr, *act_gate = nullptr;
+    uint32_t act_cols = 0;
+    bool act_laid_out = false;
+    const bool few = ps.n_live <= kRowsMatvecMax;
+    bool mv = true;
+    if (const char *k = knob("YULE_ROWS_MATVEC")) mv = atoi(k) != 0;
+    auto bytes_of = [&](const Tensor &t, uint32_t cols) -> const uint8_t * {  // what the tuned matvec kernels read
+        if (t.type == YULE_DTYPE_Q6_K) return t.buf.planar_cols == cols ? t.buf.planar : nullptr;
+        return (const uint8_t *)t.buf.ptr;
+    };
+    // (in a chain of dependent launches qmv_rows is no slower with two to four vectors either, and it folds more in)
+    auto on_rows = [&](const Tensor &t, uint64_t rows, uint32_t cols) {
+        return ps.n_live >= 2 && qmv_rows_supported(t.type, bytes_of(t, cols), act, cols, cols) &&
+               (ps.n_live <= 4 || qmv_rows_preferred(t.type, rows, cols, ps.n_live));
+    };
+    auto on_matvec = [&](const Tensor &t, uint32_t rows, uint32_t cols) {
+        if (!mv) return false;
+        if (ps.n_live >= 2 && qmv_rows_supported(t.type, bytes_of(t, cols), act, cols, cols)) return on_rows(t, rows, cols);
+        return few;
+    };
+    // The matrices that read the same rows (Q/K/V; gate/up) are collected and launched together by `flush`: neighbours of one
+    // tuned format as one launch with the RMSNorm folded in, others one by one behind a separate RMSNorm kernel.
+    struct Pending {
+        QmvArgs a;
+        bool rows;  // on qmv_rows
+    } pending[3];
     uint32_t n_pending = 0;
     auto flush = [&]() {
         mm_flush();
-        if (n_pending == 0) return;
-        for (uint32_t i = 0; i < n_pending; i++) pending[i].norm_w = act_norm;
-        if (act_norm && !kquant_batch_can_share(pending, n_pending)) {
-            ok(launch_rms_norm_rows(act, act_norm, r->pf_norm, pending[0].n_cols, ps.n_live, c.norm_eps, s, launches));
-            for (uint32_t i = 0; i < n_pending; i++) {
-                pending[i].x = r->pf_norm;
-                pending[i].norm_w = nullptr;
+        bool normed = false;
+        for (uint32_t i = 0; i < n_pending;) {
+            uint32_t n = 1;
+            while (i + n < n_pending && pending[i + n].a.type == pending[i].a.type && pending[i + n].rows == pending[i].rows) n++;
+            if (pending[i].rows) {
+                QmvRows f;
+                const QmvArgs &a0 = pending[i].a;
+                f.type = a0.type;
+                f.n_seg = n;
+                for (uint32_t k = 0; k < n; k++) {
+                    const QmvArgs &ak = pending[i + k].a;
+                    f.w[k] = ak.type == YULE_DTYPE_Q6_K ? ak.planar : ak.w;
+                    f.out[k] = ak.out;
+                    f.rows[k] = ak.n_rows;
+                    f.out_stride[k] = ak.out_stride;
+                }
+                f.x = a0.x;
+                f.x_stride = a0.x_stride;
+                f.n_cols = a0.n_cols;
+                f.batch = a0.batch;
+                f.norm_w = act_norm;
+                f.eps = a0.eps;
+                f.residual = a0.residual;
+                f.pdl = true;
+                f.status = a0.status;
+                f.wait_cycles = a0.wait_cycles;
+                ok(launch_qmv_rows(f, s, launches));
+            } else {
+                if (act_norm && !normed) {
+                    ok(launch_rms_norm_rows(act, act_norm, r->pf_norm, act_cols, ps.n_live, c.norm_eps, s, launches));
+                    normed = true;
+                }
+                for (uint32_t k = 0; k < n; k++) {
+                    QmvArgs &ak = pending[i + k].a;
+                    if (normed) ak.x = r->pf_norm;
+                    ok(launch_qmv(ak, sms, s, launches));
+                }
             }
+            i += n;
         }
-        if (kquant_batch_can_share(pending, n_pending))
-            ok(launch_kquant_batch_shared(pending, n_pending, sms, s, launches));
-        else
-            for (uint32_t i = 0; i < n_pending; i++) ok(launch_qmv(pending[i], sms, s, launches));
         n_pending = 0;
     };
     auto prep = [&](float *x, uint32_t cols, const float *norm_w, const float *gate) {
         flush();
-        if (!mv) {
-            xprep(x, cols, norm_w, gate);
-            return;
-        }
-        if (gate) ok(launch_silu_mul(gate, x, x, ps.n_live * cols, s, launches, true));  // SwiGLU in place
         act = x;
+        act_cols = cols;
         act_norm = norm_w;
+        act_gate = gate;
+        act_laid_out = false;
     };
     auto lin = [&](const Tensor &t, uint32_t rows, uint32_t cols, float *out, uint32_t stride, const float *residual) {
-        if (!mv) {
+        if (!on_matvec(t, rows, cols)) {
+            if (!act_laid_out) xprep(act, act_cols, act_norm, act_gate);
+            act_laid_out = true;
             mm(t, rows, cols, out, stride, residual);
             return;
         }
-        if (n_pending == 3) flush();
-        QmvArgs a = {};
+        if (act_gate) ok(launch_silu_mul(act_gate, act, act, ps.n_live * cols, s, launches, true));  // SwiGLU in place
+        act_gate = nullptr;
+        if (n_pending == 3 || (residual && n_pending)) flush();
+        Pending &pd = pending[n_pending++];
+        pd.rows = on_rows(t, rows, cols);
+        QmvArgs &a = pd.a = QmvArgs{};
         a.w = (const uint8_t *)t.buf.ptr;
         a.x = act;
         a.out = out;
@@ -1099,7 +1150,30 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         a.status = ctx->device_status;
         a.wait_cycles = ctx->wait_cycles;
         a.pdl = true;  // set-up and the first weight copies run under the tail of the kernel before; the rows are read after the wait
-        pending[n_pending++] = a;
+        if (residual) flush();
+    };
+    // gate and up as one launch that leaves SiLU(gate)·up in `out`
+    auto swiglu = [&](const Tensor &tg, const Tensor &tu, uint32_t rows, uint32_t cols, float *out, uint32_t stride) {
+        QmvRows f;
+        f.type = tg.type;
+        f.n_seg = 2;
+        f.w[0] = bytes_of(tg, cols);
+        f.w[1] = bytes_of(tu, cols);
+        for (uint32_t k = 0; k < 2; k++) {
+            f.out[k] = out;
+            f.rows[k] = rows;
+            f.out_stride[k] = stride;
+        }
+        f.x = act;
+        f.x_stride = f.n_cols = cols;
+        f.batch = ps.n_live;
+        f.norm_w = act_norm;
+        f.eps = c.norm_eps;
+        f.swiglu_pair = true;
+        f.pdl = true;
+        f.status = ctx->device_status;
+        f.wait_cycles = ctx->wait_cycles;
+        ok(launch_qmv_rows(f, s, launches));
     };
     const uint32_t epochs_per_tick = 5 * c.n_layers + 1;
     uint32_t xchg_index = 0;
@@ -1121,8 +1195,12 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         AttnDecode a;
         bool tiled = false;  // the queries share K / V tiles
         if (ps.batch) {
-            ok(launch_rope_kv_write_batch(r->pf_q, r->pf_k, r->pf_v, r->bd_k[l], r->bd_v[l], r->rope_cos, r->rope_sin, 0, ps.n_live, hd,
-                                          c.n_heads / N, c.n_kv_heads / N, s, launches, r->bd_pos, cache_stride));
+            // rotation, KV append and attention in one launch, each sequence at its own position
+            a.k_new = r->pf_k;
+            a.v_new = r->pf_v;
+            a.cos_table = r->rope_cos;
+            a.sin_table = r->rope_sin;
+            a.pdl = true;
             a.k_cache = r->bd_k[l];
             a.v_cache = r->bd_v[l];
             a.pos_ptr = r->bd_pos;
@@ -1179,11 +1257,16 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         exchange(r->xb_x, dim_l, dim);
         // feed-forward block: RMSNorm folded in, gate/up share the re-layout, SwiGLU folded into the next one
         prep(r->pf_x, dim, L.ffn_norm_f32, nullptr);
-        lin(L.ffn_gate, ff_l, dim, r->pf_gate + (size_t)R * ff_l, ff, nullptr);
-        lin(L.ffn_up, ff_l, dim, r->pf_up + (size_t)R * ff_l, ff, nullptr);
-        exchange(r->xb_gate, ff_l, ff);
-        exchange(r->xb_up, ff_l, ff);
-        prep(r->pf_up, ff, nullptr, r->pf_gate);
+        if (N == 1 && mv && L.ffn_gate.type == L.ffn_up.type && on_rows(L.ffn_gate, 2 * (uint64_t)ff, dim) && on_rows(L.ffn_up, 2 * (uint64_t)ff, dim)) {
+            swiglu(L.ffn_gate, L.ffn_up, ff, dim, r->pf_up, ff);
+            prep(r->pf_up, ff, nullptr, nullptr);
+        } else {
+            lin(L.ffn_gate, ff_l, dim, r->pf_gate + (size_t)R * ff_l, ff, nullptr);
+            lin(L.ffn_up, ff_l, dim, r->pf_up + (size_t)R * ff_l, ff, nullptr);
+            exchange(r->xb_gate, ff_l, ff);
+            exchange(r->xb_up, ff_l, ff);
+            prep(r->pf_up, ff, nullptr, r->pf_gate);
+        }
         lin(L.ffn_down, dim_l, ff, r->pf_x + (size_t)R * dim_l, dim, r->pf_x + (size_t)R * dim_l);  // x += Wdown · (silu(gate) · up)
         exchange(r->xb_x, dim_l, dim);
     }
