@@ -141,3 +141,43 @@ def test_column_split(backend, oracle, monkeypatch, dtype, n_rows, n_cols, batch
     for b in (0, batch // 2, batch - 1):
         ref = oracle.qmv(int(dtype), w, x[b * n_cols:(b + 1) * n_cols], n_rows, n_cols)
         assert guarded_rel_err(y[b], ref) <= REL_TOL
+
+
+@pytest.mark.parametrize("dtype", [DType.Q8_0, DType.Q4_0, DType.Q6_K, DType.Q5_K])
+def test_extreme_block_scales(backend, oracle, dtype):
+    """The unpacking of the generic kernel in half precision: scales from the smallest subnormal to just below 64, where d·2^10 is
+    still a half (above it the product with a quant is outside the operands' range), and quants at both ends."""
+    n_rows, n_cols, batch = 130, 512, 70
+    size, per_row = dtype.size_of_block, n_cols // dtype.block_size
+    w = np.array(synth.random_blocks(dtype, 31, n_rows * per_row)).reshape(-1, size).copy()
+    at = 208 if dtype == DType.Q6_K else 0
+    exps = np.arange(n_rows) % 28
+    d = np.repeat((2.0 ** -24 * 2.0 ** exps * 1.37).astype(np.float16), per_row)  # 2^-24 … 2^3
+    w[:, at:at + 2] = d.view(np.uint8).reshape(-1, 2)
+    if dtype == DType.Q5_K:
+        w[:, 2:4] = d.view(np.uint8).reshape(-1, 2)
+    if dtype in (DType.Q6_K, DType.Q5_K):  # d times a scale times a quant stays below 64
+        big = np.repeat(exps, per_row) > 15
+        w[big, at:at + 2] = 0
+        if dtype == DType.Q5_K:
+            w[big, 2:4] = 0
+    # a weight of 64 or more is outside the operands' range: 127 d, 8 d below it, or quants of 1
+    if dtype == DType.Q8_0:
+        w[np.repeat(exps, per_row) > 22, 2:] = 1
+    if dtype == DType.Q4_0:
+        w[np.repeat(exps, per_row) > 26, 2:] = 0x99
+    w[0, at + 2 if at == 0 else 0] = 0xFF
+    w[1, at + 2 if at == 0 else 0] = 0x80
+    w = w.reshape(-1)
+    x = synth.normal(32, batch * n_cols).reshape(batch, n_cols)
+    deq = oracle.dequant(int(dtype), w).reshape(n_rows, n_cols).astype(np.float64)
+    ref = x.astype(np.float64) @ deq.T
+    wh, xh, oh = backend.upload(w), backend.upload(x.reshape(-1)), backend.allocate(batch * n_rows * 4)
+    backend.quantized_matmul_batched(wh, xh, oh, n_rows, n_cols, dtype, batch)
+    y = backend.download(oh, batch * n_rows).reshape(batch, n_rows)
+    for h in (wh, xh, oh):
+        backend.free(h)
+    # row by row: 22 bits of x and of each weight (weights below 2^-24 in the lo term lose theirs: 2^-25 each, after the scaling
+    # by 2^10), fp32 sums
+    bound = 16 * 2.0 ** -22 * np.abs(x).astype(np.float64) @ np.abs(deq).T + 2.0 ** -35 * np.abs(x).sum(1)[:, None]
+    assert np.all(np.abs(y - ref) <= bound)

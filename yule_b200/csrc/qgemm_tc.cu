@@ -366,6 +366,145 @@ __device__ __forceinline__ void dequant8_unit(const unsigned char *unit, uint32_
     }
 }
 
+// Words of four bytes from a 2-byte-aligned shared-memory address (one word more is read than returned).
+template <int N>
+__device__ __forceinline__ void words_at(const unsigned char *p, uint32_t (&w)[N]) {
+    const uint32_t mis = smem_u32(p) & 2u;
+    const uint32_t *a = reinterpret_cast<const uint32_t *>(p - mis);
+    uint32_t prev = a[0];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint32_t next = a[k + 1];
+        w[k] = __funnelshift_r(prev, next, 8 * mis);
+        prev = next;
+    }
+}
+// 32 consecutive weights (columns col0 .. col0 + 31 of a 256-column unit) times 2^10 as fp16 hi + lo, eight columns at a time to
+// put(i, hi, lo) in the order 0,2,1,3,4,6,5,7.  The same values as dequant8_unit and its split give, without conversion
+// instructions: a quant is a half after one OR and one subtraction, 2^10·d is a half (fp16 d below 64, subnormals included),
+// hi = rn(d·q) and lo = fma(d, q, -hi), which is exact.  Q6_K: d·sc is a pair of halves itself.  False: not this
+// format, or a scale that is not finite or too large; nothing was written.  Q6_K 2048x5632 against 777 rows: 275 us with dequant8_unit, 185 with this.
+template <class Put>
+__device__ __forceinline__ bool unpack32(const unsigned char *unit, uint32_t type, uint32_t col0, bool live, Put put) {
+    const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
+    auto finite = [](__half2 d) { return __hle(__habs(__low2half(d)), __ushort_as_half(0x7BFF)); };  // false for infinities and NaN
+    auto u16_at = [&](uint32_t off) { return *reinterpret_cast<const unsigned short *>(unit + off); };
+    if (type == YULE_DTYPE_Q8_0 || type == YULE_DTYPE_Q4_0) {
+        const bool q8 = type == YULE_DTYPE_Q8_0;
+        const uint32_t b = (col0 >> 5) * (q8 ? 34u : 18u);
+        const __half2 d = live ? __hmul2(__half2half2(__ushort_as_half(u16_at(b))), k1024) : __half2half2(__ushort_as_half(0));
+        if (!finite(d)) return false;
+        auto split = [&](uint32_t biased, uint32_t bias, uint32_t &hi, uint32_t &lo) {
+            const __half2 q = __hsub2(as_half2(biased), as_half2(bias)), h = __hmul2(d, q);
+            hi = as_u32(h);
+            lo = as_u32(__hfma2(d, q, __hneg2(h)));
+        };
+        if (q8) {
+            uint32_t w[8];
+            words_at(unit + b + 2, w);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                uint4 h, l;
+                split((w[2 * i] & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.x, l.x);  // byte ^ 128 = byte + 128
+                split(((w[2 * i] >> 8) & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.y, l.y);
+                split((w[2 * i + 1] & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.z, l.z);
+                split(((w[2 * i + 1] >> 8) & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.w, l.w);
+                put(i, h, l);
+            }
+        } else {
+            uint32_t w[4];
+            words_at(unit + b + 2, w);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {  // byte k: columns 2k (low nibble) and 2k + 1
+                const uint32_t v = w[i] & 0x0F0F0F0Fu, u = (w[i] >> 4) & 0x0F0F0F0Fu;
+                uint4 h, l;
+                split(biased_pair(v, 0x4140u), 0x64086408u, h.x, l.x);
+                split(biased_pair(u, 0x4140u), 0x64086408u, h.y, l.y);
+                split(biased_pair(v, 0x4342u), 0x64086408u, h.z, l.z);
+                split(biased_pair(u, 0x4342u), 0x64086408u, h.w, l.w);
+                put(i, h, l);
+            }
+        }
+        return true;
+    }
+    if (type == YULE_DTYPE_Q6_K) {
+        const uint32_t h = col0 >> 7, g = (col0 >> 5) & 3u;
+        const float d = live ? f16_bits_to_f32(u16_at(208)) * kGenericWScale : 0.f;
+        const uint32_t scw = u16_at(192 + 8 * h + 2 * g);  // the scales of the first and the last sixteen columns
+        __half2 dh[2], dl[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const float ds = d * (float)(int)(signed char)(scw >> (8 * k));
+            dh[k] = __float2half2_rn(ds);
+            dl[k] = __float2half2_rn(ds - __low2float(dh[k]));
+        }
+        if (!finite(dh[0]) || !finite(dh[1])) return false;
+        uint32_t ql[8], qh[8];
+        words_at(unit + 64 * h + 32 * (g & 1u), ql);
+        words_at(unit + 128 + 32 * h, qh);
+        const uint32_t sl = 4 * (g >> 1), sh = 2 * g;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            auto split = [&](uint32_t q6, uint32_t &hi, uint32_t &lo) {
+                const __half2 q = __hsub2(as_half2((q6 & 0x00FF00FFu) | 0x64006400u), as_half2(0x64206420u));  // 1056
+                const __half2 a = dh[i >> 1], b = dl[i >> 1], x = __hfma2(a, q, __hmul2(b, q));
+                hi = as_u32(x);
+                lo = as_u32(__hfma2(b, q, __hfma2(a, q, __hneg2(x))));
+            };
+            const uint32_t v = ((ql[2 * i] >> sl) & 0x0F0F0F0Fu) | (((qh[2 * i] >> sh) & 0x03030303u) << 4);
+            const uint32_t u = ((ql[2 * i + 1] >> sl) & 0x0F0F0F0Fu) | (((qh[2 * i + 1] >> sh) & 0x03030303u) << 4);
+            uint4 hv, lv;
+            split(v, hv.x, lv.x);
+            split(v >> 8, hv.y, lv.y);
+            split(u, hv.z, lv.z);
+            split(u >> 8, hv.w, lv.w);
+            put(i, hv, lv);
+        }
+        return true;
+    }
+    if (type == YULE_DTYPE_Q5_K) {  // the minimum is subtracted in fp32, as the CPU does
+        const uint32_t sb = col0 >> 5;
+        uint32_t sc, mn;
+        if (sb < 4) {
+            sc = unit[4 + sb] & 63u;
+            mn = unit[8 + sb] & 63u;
+        } else {
+            sc = (unit[8 + sb] & 0xFu) | ((unit[sb] >> 6) << 4);
+            mn = (unit[8 + sb] >> 4) | ((unit[4 + sb] >> 6) << 4);
+        }
+        // (scaling by 2^10 commutes with the roundings)
+        const float ds = __fmul_rn(f16_bits_to_f32(u16_at(0)), (float)sc) * kGenericWScale;
+        const float dm = __fmul_rn(f16_bits_to_f32(u16_at(2)), (float)mn) * kGenericWScale;
+        uint32_t ql[8], qh[8];
+        words_at(unit + 48 + 32 * (sb >> 1), ql);
+        words_at(unit + 16, qh);
+        const uint32_t sl = 4 * (sb & 1u);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            auto five = [&](int k) { return ((ql[k] >> sl) & 0x0F0F0F0Fu) | (((qh[k] >> sb) & 0x01010101u) << 4); };
+            auto value = [&](uint32_t q, uint32_t byte) {
+                const float f = __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7440u + byte)) - 8388608.f;
+                return live ? __fsub_rn(__fmul_rn(f, ds), dm) : 0.f;
+            };
+            auto split = [&](float x, float y, uint32_t &hi, uint32_t &lo) {
+                const __half2 hh = __floats2half2_rn(x, y);
+                const float2 back = __half22float2(hh);
+                hi = as_u32(hh);
+                lo = as_u32(__floats2half2_rn(x - back.x, y - back.y));
+            };
+            const uint32_t v = five(2 * i), u = five(2 * i + 1);
+            uint4 h, l;
+            split(value(v, 0), value(v, 2), h.x, l.x);
+            split(value(v, 1), value(v, 3), h.y, l.y);
+            split(value(u, 0), value(u, 2), h.z, l.z);
+            split(value(u, 1), value(u, 3), h.w, l.w);
+            put(i, h, l);
+        }
+        return true;
+    }
+    return false;
+}
+
 // Position in the stage ring without a runtime division (an integer division runs on the same
 // slow pipe as the half conversions): slot and phase parity, advanced once per stage.
 struct RingPos {
@@ -727,8 +866,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                         break;
                     }
                     unsigned char *a_hi = smem + (size_t)ring.s * kStageBytes, *a_lo = a_hi + kABytes;
+                    const bool done = unpack32(rawrow, p.type, g * kBK + hf * 32, live, [&](uint32_t c8, const uint4 &h, const uint4 &l) {
+                        const uint32_t kc = hf * 4 + c8;
+                        *reinterpret_cast<uint4 *>(a_hi + kc * 2048 + in_core) = h;
+                        *reinterpret_cast<uint4 *>(a_lo + kc * 2048 + in_core) = l;
+                    });
 #pragma unroll 1
-                    for (uint32_t c8 = 0; c8 < 4; c8++) {
+                    for (uint32_t c8 = 0; c8 < 4 && !done; c8++) {
                         const uint32_t col0 = g * kBK + hf * 32 + c8 * 8;  // column inside the unit
                         float v[8];
                         dequant8_unit(rawrow, p.type, col0, v);
@@ -967,27 +1111,38 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                         for (uint32_t j = 0; j < CW; j++) acc[j] += v[q][j];
                 }
 #pragma unroll
-                for (uint32_t j = 0; j < CW; j++) {
-                    const uint32_t n = n0 + j;
-                    if (row < p.n_rows[wi.seg] && n < p.n_tokens) {
-                        const size_t o = (size_t)n * p.out_stride[wi.seg] + row;
-                        p.out[wi.seg][o] = p.residual ? acc[j] + p.residual[o] : acc[j];
+                for (uint32_t c0 = 0; c0 < CW; c0 += 4) {
+                    const size_t o0 = (size_t)(n0 + c0) * p.out_stride[wi.seg] + row;
+                    const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 < p.n_tokens ? p.n_tokens - (n0 + c0) : 0u;
+                    float res[4];
+                    if (p.residual) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
                     }
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; j++)
+                        if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? acc[c0 + j] + res[j] : acc[c0 + j];
                 }
                 continue;
             }
 #pragma unroll
             for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
                 const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;  // padded to whole tiles
+                // Four residuals are asked for before the first of their stores (which may be to the same matrix, so nothing but
+                // this order lets them overlap): one by one they took 24 us per tile, so they take 7.
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const float sc = __shfl_sync(0xffffffffu, osc, j);
-                    const uint32_t n = n0 + c0 + j;
-                    if (row < p.n_rows[wi.seg] && n < p.n_tokens) {
-                        float val = acc[c0 + j] * sc * p.out_scale;
-                        const size_t o = (size_t)n * p.out_stride[wi.seg] + row;
-                        if (p.residual) val += p.residual[o];
-                        p.out[wi.seg][o] = val;
+                for (int j0 = 0; j0 < 16; j0 += 4) {
+                    const size_t o0 = (size_t)(n0 + c0 + j0) * p.out_stride[wi.seg] + row;
+                    const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 + j0 < p.n_tokens ? p.n_tokens - (n0 + c0 + j0) : 0u;
+                    float res[4];
+                    if (p.residual) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
+                    }
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; j++) {
+                        const float val = acc[c0 + j0 + j] * __shfl_sync(0xffffffffu, osc, j0 + j) * p.out_scale;
+                        if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? val + res[j] : val;
                     }
                 }
             }
@@ -1032,9 +1187,10 @@ struct XprepParams {
     float *oscale;
 };
 
-// One CTA of 1024 threads per row; a thread keeps its 8·CHUNKS columns in registers from the single read of the row
-// to the stores, so a row of up to 8192·CHUNKS columns costs one round trip to memory and two block reductions
-// whatever its length.
+// One CTA per row, as many threads (up to 1024) as have columns to work on; a thread keeps its 8·CHUNKS columns in registers from
+// the single read of the row to the stores, so a row of up to 8192·CHUNKS columns costs one round trip to memory and two block
+// reductions whatever its length.  (With 1024 threads whatever the row length 2048 rows of 4096 columns took 42 us, now 31: half of the
+// threads of an SM held no data.)
 constexpr int kXprepThreads = 1024;
 template <int CHUNKS>
 __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepParams p) {
@@ -1058,7 +1214,7 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
                                           term * (p.bn * 16) + core) + s;
     };
     if (n >= p.n_tokens) {  // padding row of the last tile
-        for (uint32_t k0 = threadIdx.x * 8; k0 < p.n_cols; k0 += kXprepThreads * 8) {
+        for (uint32_t k0 = threadIdx.x * 8; k0 < p.n_cols; k0 += blockDim.x * 8) {
             *reinterpret_cast<uint4 *>(slab16(k0, 0)) = make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4 *>(slab16(k0, 1)) = make_uint4(0, 0, 0, 0);
             if ((k0 & 31u) == 0) {
@@ -1079,8 +1235,12 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         __syncthreads();
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
         __syncthreads();
-        v = red[0];
-        for (int i = 1; i < kXprepThreads / 32; i++) v = is_max ? fmaxf(v, red[i]) : v + red[i];
+        const uint32_t lane = threadIdx.x & 31u, n_warps = blockDim.x >> 5;
+        v = lane < n_warps ? red[lane] : 0.f;  // (sums of squares, magnitudes: nothing is below zero)
+        for (int o = 16; o > 0; o >>= 1) {
+            const float other = __shfl_xor_sync(0xffffffffu, v, o);
+            v = is_max ? fmaxf(v, other) : v + other;
+        }
         return v;
     };
     // rows start on a 16-byte boundary when the stride is a multiple of four floats; otherwise scalar loads
@@ -1088,7 +1248,7 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
     float v[CHUNKS][8];
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
-        const uint32_t k0 = ((uint32_t)c * kXprepThreads + threadIdx.x) * 8;
+        const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
         if (k0 < p.n_cols) {
             if (vec) {
                 const float4 a = *reinterpret_cast<const float4 *>(x + k0), b = *reinterpret_cast<const float4 *>(x + k0 + 4);
@@ -1112,7 +1272,7 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         const float inv = 1.0f / sqrtf(ss / (float)p.n_cols + p.eps);
 #pragma unroll
         for (int c = 0; c < CHUNKS; c++) {
-            const uint32_t k0 = ((uint32_t)c * kXprepThreads + threadIdx.x) * 8;
+            const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
             if (k0 < p.n_cols) {
 #pragma unroll
                 for (int i = 0; i < 8; i++) v[c][i] = v[c][i] * inv * p.norm_w[k0 + i];
@@ -1122,7 +1282,7 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
     if (gate) {
 #pragma unroll
         for (int c = 0; c < CHUNKS; c++) {
-            const uint32_t k0 = ((uint32_t)c * kXprepThreads + threadIdx.x) * 8;
+            const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
             if (k0 < p.n_cols) {
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
@@ -1148,7 +1308,7 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
     if (threadIdx.x == 0) p.oscale[n] = 1.0f / scale;
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
-        const uint32_t k0 = ((uint32_t)c * kXprepThreads + threadIdx.x) * 8;
+        const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
         if (k0 >= p.n_cols) break;  // whole groups of four threads (32 columns) leave together
         float sum = 0.f;
 #pragma unroll
@@ -1293,14 +1453,15 @@ cudaError_t launch_qgemm_xprep(const QGemm &g, cudaStream_t s, uint64_t *launche
     xp.xb = xb;
     xp.oscale = oscale;
     cudaError_t e;
+    auto threads = [&](uint32_t chunks) { return dim3(((g.n_cols / 8 + chunks - 1) / chunks + 31) / 32 * 32); };
     if (g.n_cols <= 8192)
-        e = launch_kernel(gemm_xprep_kernel<1>, dim3(padded), dim3(kXprepThreads), 0, s, g.pdl, xp);
+        e = launch_kernel(gemm_xprep_kernel<1>, dim3(padded), threads(1), 0, s, g.pdl, xp);
     else if (g.n_cols <= 16384)
-        e = launch_kernel(gemm_xprep_kernel<2>, dim3(padded), dim3(kXprepThreads), 0, s, g.pdl, xp);
+        e = launch_kernel(gemm_xprep_kernel<2>, dim3(padded), threads(2), 0, s, g.pdl, xp);
     else if (g.n_cols <= 32768)
-        e = launch_kernel(gemm_xprep_kernel<4>, dim3(padded), dim3(kXprepThreads), 0, s, g.pdl, xp);
+        e = launch_kernel(gemm_xprep_kernel<4>, dim3(padded), threads(4), 0, s, g.pdl, xp);
     else if (g.n_cols <= 65536)
-        e = launch_kernel(gemm_xprep_kernel<8>, dim3(padded), dim3(kXprepThreads), 0, s, g.pdl, xp);
+        e = launch_kernel(gemm_xprep_kernel<8>, dim3(padded), threads(8), 0, s, g.pdl, xp);
     else
         return cudaErrorInvalidValue;
     if (e != cudaSuccess) return e;
