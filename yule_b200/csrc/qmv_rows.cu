@@ -9,9 +9,10 @@
 // cheapest way to make them, they cost seven bits of every product; relative error 1e-6 instead of 1e-7), the eight B columns
 // are the hi and lo fp16 terms of four vectors (column 2v: hi of vector v, 2v + 1: lo; 22 bits of each x, every 256 columns
 // of a vector with a power-of-two scale of their own).  A lane owns four consecutive quant bytes per MMA, receives hi and lo
-// of one vector for two rows, adds the two and applies the group's scale in fp32.  Mins (Q4_K, Q5_K): one more MMA per 256
-// columns, mins times the sums of x over the sub-blocks, which enter as three fp16 terms (k slots 0-7: hi | lo, 8-15: the
-// rest).  Formats with a constant offset subtract it from the fp16 quants, exactly.
+// of one vector for two rows, adds the two and applies the group's scale in fp32.  Formats with a constant offset subtract it
+// from the fp16 quants, exactly.  Q4_K and Q5_K: the middle of the quants is subtracted likewise, so that what the minimum takes
+// away is not in the sums in the first place (error 2.6e-7 without that); two more MMAs per 256 columns, the mins and the scales
+// times the sums of x over the sub-blocks, which enter as three fp16 terms (k slots 0-7: hi | lo, 8-15: the rest).
 //
 // What bounds it.  Per 512 weights and four vectors two MMAs of eight clocks per SM sub-partition, and about as many issue
 // slots for unpacking and scaling: from eight vectors on the issue slots, below that HBM on the large matrices and the
@@ -177,14 +178,14 @@ __device__ __forceinline__ void consume_q4k(const unsigned char *u, int g, int t
                         if (Q5) {
                             // fifth bits: bit sb of byte l belongs to column l of the sub-block
                             const uint32_t e = q5[h][rr][c], q = ((nib ? v >> 4 : v) & 0x0F0F0F0Fu) | ((sb <= 4 ? e << (4 - sb) : e >> (sb - 4)) & 0x10101010u);
-                            a[c][rr] = minus((q & 0x00FF00FFu) | k1024, k1024);
-                            a[c][2 + rr] = minus(((q >> 8) & 0x00FF00FFu) | k1024, k1024);
+                            a[c][rr] = minus((q & 0x00FF00FFu) | k1024, 0x64106410u);  // 1040
+                            a[c][2 + rr] = minus(((q >> 8) & 0x00FF00FFu) | k1024, 0x64106410u);
                         } else {
-                            // 1024 + byte, 1024 + 16·(high nibble): the high ones are used as 16·q
+                            // 1024 + byte, and 1024 + 16·(high nibble) + 8: low − 8 is the difference, 16·(high − 8) the second minus 1160
                             const uint32_t b02 = __byte_perm(v, 0x64646464u, 0x4240u), b13 = __byte_perm(v, 0x64646464u, 0x4341u);
-                            const uint32_t h02 = b02 & 0xFFF0FFF0u, h13 = b13 & 0xFFF0FFF0u;
-                            a[c][rr] = nib ? minus(h02, k1024) : minus(b02, h02);
-                            a[c][2 + rr] = nib ? minus(h13, k1024) : minus(b13, h13);
+                            const uint32_t h02 = (b02 & 0xFFF0FFF0u) | 0x00080008u, h13 = (b13 & 0xFFF0FFF0u) | 0x00080008u;
+                            a[c][rr] = nib ? minus(h02, 0x64886488u) : minus(b02, h02);
+                            a[c][2 + rr] = nib ? minus(h13, 0x64886488u) : minus(b13, h13);
                         }
                     }
                 const float up = nib && !Q5 ? 0.0625f : 1.f;
@@ -205,15 +206,21 @@ __device__ __forceinline__ void consume_q4k(const unsigned char *u, int g, int t
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const float d0 = half_bits(dd[h][0]), d1 = half_bits(dd[h][1]);
-        const float m0 = half_bits(dd[h][0] >> 16) * -32.f, m1 = half_bits(dd[h][1] >> 16) * -32.f;  // the sums of x went in with a factor 2^-5
+        // The sums of x went in with a factor 2^-5; with the scales they make up for the subtracted middle of the quants.
+        const float m0 = half_bits(dd[h][0] >> 16) * -32.f, m1 = half_bits(dd[h][1] >> 16) * -32.f;
+        const float c0 = d0 * (Q5 ? 512.f : 256.f), c1 = d1 * (Q5 ? 512.f : 256.f);
+        uint32_t as[2];  // scales 2t, 2t + 1 as halves
+#pragma unroll
+        for (int rr = 0; rr < 2; rr++) as[rr] = minus(__byte_perm(t < 2 ? sc[h][rr][0] : sc[h][rr][1], 0x64u, (t & 1) ? 0x4342u : 0x4140u), k1024);
 #pragma unroll
         for (int n = 0; n < NT; n++) {
             const uint2 b = *reinterpret_cast<const uint2 *>(im.mins + n * 256);
             const float f = im.f[4 * n];
-            float d[4];
+            float d[4], e[4];
             mma16816_z(d, am[h][0], am[h][1], am[h][0], am[h][1], b.x, b.y);
-            acc[h][n][0] = fmaf(f, fmaf(d0, s[h][n][0], m0 * (d[0] + d[1])), acc[h][n][0]);
-            acc[h][n][1] = fmaf(f, fmaf(d1, s[h][n][1], m1 * (d[2] + d[3])), acc[h][n][1]);
+            mma16816_z(e, as[0], as[1], as[0], as[1], b.x, b.y);
+            acc[h][n][0] = fmaf(f, fmaf(d0, s[h][n][0], fmaf(c0, e[0] + e[1], m0 * (d[0] + d[1]))), acc[h][n][0]);
+            acc[h][n][1] = fmaf(f, fmaf(d1, s[h][n][1], fmaf(c1, e[2] + e[3], m1 * (d[2] + d[3]))), acc[h][n][1]);
         }
     }
 }
@@ -844,13 +851,13 @@ cudaError_t launch_format(const QmvRows &f, cudaStream_t s, uint64_t *launches) 
 // Measured per launch, this kernel against the others.  Two to four vectors: the kernels for so few read rows of up to 4096 columns
 // whole and overlap independent calls (Q4_K 2048x2048, 4 vectors: 2.8 against 4.0 us), longer ones take several launches there (8192x8192
 // 29 against 17 us).  Q4_K GEMM: 16 vectors 4096x4096 14.7 against 12.2 us, 4096x14336 28.4 against 33, 12 vectors 28672x8192
-// 86 against 81.  The other formats' GEMM unpacks at a third of that rate: Q8_0 14336x4096, 48 vectors 153 against 81, 4096x4096 48
-// against 45, with 64 vectors 48 against 60.
+// 86 against 81.  The other formats' GEMM is half as fast: Q8_0 32 vectors 4096x4096 33 against 30, 14336x4096
+// 107 against 54; 48 vectors 4096x4096 37 against 44 (Q4_0 34 against 32), 14336x4096 116 against 80.
 bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch) {
     if (batch < 2) return false;
     if (batch <= 4 && type != YULE_DTYPE_Q5_K) return n_cols > 4096;
     if (type == YULE_DTYPE_Q4_K) return batch <= 12 || (batch <= 16 && n_rows * n_cols <= (17ull << 20));
-    return batch <= 48;
+    return batch <= 32 || (batch <= 48 && (n_rows * n_cols > (17ull << 20) || type == YULE_DTYPE_Q4_0 || type == YULE_DTYPE_Q5_K));
 }
 
 bool qmv_rows_supported(uint32_t type, const void *w, const float *x, uint32_t n_cols, uint32_t x_stride) {
