@@ -327,3 +327,29 @@ def test_independent_calls_share_inputs(backend, oracle):
     assert guarded_rel_err(backend.download(outs[3], n), oracle.qmv(int(DType.Q6_K), w6, refs[1], n, n)) <= REL_TOL
     for h in whs + [w6h, xh] + outs:
         backend.free(h)
+
+
+def test_calls_of_a_chain_that_share_an_output(backend, oracle):
+    """Matvecs that overlap: the second and the third read what the first one writes, the second through a grid so small that
+    the third starts while the first is still running; and a chain with more outputs than are tracked."""
+    n = 2048
+    big, small = synth.random_quantized(DType.Q4_K, 71, 14336 * n), synth.random_quantized(DType.Q4_K, 72, 16 * n)
+    bh, sh = backend.upload(big), backend.upload(small)
+    xs = [synth.normal(73 + i, n) for i in range(24)]
+    first = [oracle.qmv(int(DType.Q4_K), big, x, 14336, n) for x in xs[:2]]
+    ah, outs = backend.allocate(14336 * 4), [backend.allocate(16 * 4) for _ in range(24)]
+    handles = [backend.upload(x) for x in xs]
+    for turn in range(20):
+        k = turn & 1
+        backend.quantized_matmul(bh, handles[k], ah, 14336, n, DType.Q4_K)
+        backend.quantized_matmul(sh, ah, outs[0], 16, n, DType.Q4_K)
+        backend.quantized_matmul(sh, ah, outs[1], 16, n, DType.Q4_K)
+        want = oracle.qmv(int(DType.Q4_K), small, first[k][:n].astype(np.float32), 16, n)
+        for o in outs[:2]:
+            assert guarded_rel_err(backend.download(o, 16), want) <= REL_TOL
+    for h, o in zip(handles, outs):
+        backend.quantized_matmul(sh, h, o, 16, n, DType.Q4_K)
+    for x, o in zip(xs, outs):
+        assert guarded_rel_err(backend.download(o, 16), oracle.qmv(int(DType.Q4_K), small, x, 16, n)) <= REL_TOL
+    for h in [bh, sh, ah] + handles + outs:
+        backend.free(h)

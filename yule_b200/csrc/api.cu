@@ -563,6 +563,9 @@ static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight
     // too and no call that may still be running writes what this one reads as weights.  When its activations
     // are not such an output either (Q, K and V from one normed vector; gate and up), nothing this kernel reads
     // depends on its predecessors: only its stores are ordered behind them (late wait).
+    // Any call since the chain began may still be running when this kernel starts, whatever the ones between wait for: a
+    // kernel lets its successor start before its own wait.  So the outputs stay listed until a call without the attribute
+    // has waited for everything; a chain with more outputs than the list holds is ended by one.
     const char *w_lo = (const char *)a.w, *w_hi = w_lo + wbytes;
     const char *x_lo = (const char *)X.ptr, *x_hi = x_lo + ((size_t)(batch - 1) * x_stride + n_cols) * 4;
     const char *o_lo = (const char *)O.ptr, *o_hi = o_lo + ((size_t)(batch - 1) * out_stride + n_rows) * 4;
@@ -572,15 +575,18 @@ static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight
         w_hazard = w_hazard || (w_lo < ctx->chain_hi[i] && ctx->chain_lo[i] < w_hi);
         x_hazard = x_hazard || (x_lo < ctx->chain_hi[i] && ctx->chain_lo[i] < x_hi);
     }
-    a.pdl = _pdl_chain && !w_hazard;
-    a.late_wait = a.pdl && !x_hazard && ctx->chain_n < yule_cuda_ctx::kChainRanges;
+    bool listed = false;
+    for (int i = 0; i < ctx->chain_n; i++) listed = listed || (ctx->chain_lo[i] <= o_lo && o_hi <= ctx->chain_hi[i]);
+    a.pdl = _pdl_chain && !w_hazard && (listed || ctx->chain_n < yule_cuda_ctx::kChainRanges);
+    a.late_wait = a.pdl && !x_hazard;
     a.status = ctx->device_status;
     a.wait_cycles = ctx->wait_cycles;
     LAUNCHED(ctx, launch_qmv(a, ctx->prop.multiProcessorCount, ctx->stream, &_n));
     ctx->pdl_chain = true;
-    if (!a.late_wait) ctx->chain_n = 0;  // this kernel waits for all its predecessors before it reads or writes
-    bool listed = false;
-    for (int i = 0; i < ctx->chain_n; i++) listed = listed || (ctx->chain_lo[i] <= o_lo && o_hi <= ctx->chain_hi[i]);
+    if (!a.pdl) {
+        ctx->chain_n = 0;
+        listed = false;
+    }
     if (!listed) {
         ctx->chain_lo[ctx->chain_n] = o_lo;
         ctx->chain_hi[ctx->chain_n] = o_hi;

@@ -105,9 +105,8 @@ struct yule_cuda_ctx {
     // previous operation enqueued on the stream was one of this library's kernels, and its output does not
     // overlap the weights of the call being launched (weights are read before the dependency wait).
     bool pdl_chain = false;
-    // Outputs of the matvec calls of the current chain that may still be running when the next one starts:
-    // a kernel that waits for its predecessor before reading anything settles everything before it, a kernel
-    // whose stores alone wait (late wait) does not.
+    // Outputs of the matvec calls of the current chain, any of which may still be running when the next one starts (a kernel
+    // lets its successor start before it waits itself).
     static constexpr int kChainRanges = 8;
     const char *chain_lo[kChainRanges] = {}, *chain_hi[kChainRanges] = {};
     int chain_n = 0;
