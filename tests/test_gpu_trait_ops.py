@@ -183,3 +183,17 @@ def test_allocations_are_zeroed_and_handles_checked(backend):
         backend.copy_to_device(b"abcd", BufferHandle(123456789))
     info = backend.device_info()
     assert backend.name() == "cuda" and info.compute_units > 0 and info.memory_bytes > 0
+
+
+@pytest.mark.parametrize("hd,seqs", [(64, (199, 200, 201, 511, 512)), (128, (99, 100, 101, 511))])
+def test_attention_around_the_lines_between_its_kernels(backend, oracle, hd, seqs):
+    """A query head per CTA below 12800 values of a KV head, the queries of a KV head together from there on."""
+    n_heads, n_kv = 8, 2
+    for seq in seqs:
+        q, K, V = synth.normal(1, n_heads * hd), synth.normal(2, seq * n_kv * hd), synth.normal(3, seq * n_kv * hd)
+        qh, kh, vh, oh = backend.upload(q), backend.upload(K), backend.upload(V), backend.allocate(n_heads * hd * 4)
+        backend.multihead_attention(qh, kh, vh, oh, hd, seq, n_heads, n_kv, n_kv * hd)
+        ref = oracle.attention(q, K.reshape(seq, -1), V.reshape(seq, -1), n_heads, n_kv, hd, seq)
+        assert guarded_rel_err(backend.download(oh, n_heads * hd), ref) <= REL_TOL
+        for h in (qh, kh, vh, oh):
+            backend.free(h)

@@ -692,7 +692,9 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
     if (attn_decode_supported(head_dim) && kv_stride % 4 == 0) {
         // split over positions; the partial results live in a context-owned scratch grown on demand
         AttnDecode a;
-        a.gqa = attn_gqa_supported(head_dim, n_heads, n_kv_heads) && seq_len >= 512;
+        // One KV head's queries together from 100 rows of 128 or 200 of 64 values: 8 KV heads of 128, 101 positions 7.5 -> 6.4 us,
+        // 400 13.7 -> 7.6; 4 of 64, 200 positions 7.2 -> 6.9, but 101 5.2 -> 6.1 (splits of 32 positions that have to be merged).
+        a.gqa = attn_gqa_supported(head_dim, n_heads, n_kv_heads) && (uint64_t)seq_len * head_dim >= 12800;
         a.n_splits = a.gqa ? attn_gqa_pick_splits(n_kv_heads, seq_len, ctx->prop.multiProcessorCount)
                            : attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount);
         const size_t need = attn_scratch_floats(n_heads, a.n_splits, head_dim);

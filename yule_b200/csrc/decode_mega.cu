@@ -22,7 +22,7 @@
 //     take the gate and the up tile of the same rows), down + residual (the groups split the column chunks of a
 //     tile) } → RMSNorm + output matrix with a running arg-max → pick (ties to the highest index,
 //     yule-infer/src/sampler.rs:150-163), history and position advance.
-//   * Arithmetic is that of the tensor-pipe matvec kernels (qmv_q4k_ring.cu, qmv_q6k_ring.cu) and of the
+//   * Arithmetic is that of fp16 tensor-pipe matvecs (q4k_mma_common.cuh, q6k_ring_common.cuh) and of the
 //     grouped-query attention kernel (attention.cu), whose device code this file includes.
 //   * Registers and L1.  With 224 KB of the SM given to shared memory L1 is tiny: a register spill, or a descriptor
 //     read from global memory, is an L2 round trip.  The kernel compiles without spills (128 registers per thread)

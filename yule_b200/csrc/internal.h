@@ -299,20 +299,6 @@ cudaError_t launch_qgemm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t 
 cudaError_t launch_qgemm_xprep(const QGemm &g, cudaStream_t s, uint64_t *launches);
 cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
 
-// Q4_K / Q5_K over two to four activation vectors per pass on fp16 fragments (qmv_q4k_mma.cu).
-struct Q4kBatch {
-    const uint8_t *w = nullptr;       // 16-byte aligned
-    float *out = nullptr;             // [batch][out_stride]
-    uint32_t rows = 0, out_stride = 0;
-    const float *x = nullptr;         // [batch][x_stride]
-    uint32_t x_stride = 0, n_cols = 0, batch = 2;
-    const float *residual = nullptr;  // added to out when set (same layout)
-    bool q5 = false;                  // Q5_K (176-byte super-blocks)
-    bool pdl = false;                 // programmatic dependent launch
-};
-bool q4k_mma_supported(uint32_t n_cols, uint32_t batch);
-cudaError_t launch_q4k_mma(const Q4kBatch &f, int sm_count, cudaStream_t s, uint64_t *launches);
-
 // Row-planar device copy of a Q6_K tensor (q6k_planar.cu): n_cols a multiple of 256.
 size_t q6k_planar_bytes(uint64_t n_rows, uint32_t n_cols);
 cudaError_t launch_q6k_repack(const uint8_t *raw, uint8_t *planar, uint64_t n_rows, uint32_t n_cols, cudaStream_t s,

@@ -1,5 +1,4 @@
-// q4k_mma_common.cuh — device code shared by the Q4_K / Q5_K tensor-pipe matvec kernels
-// (qmv_q4k_mma.cu: weights streamed through registers; qmv_q4k_ring.cu: weights staged in shared memory):
+// q4k_mma_common.cuh — Q4_K device code of the persistent decode kernel (decode_mega.cu, weights staged in shared memory):
 // fragment construction from packed nibbles, the 6-bit scale unpack, the shared-memory image of the
 // activations and the tensor-parallel (value, epoch) pair helpers.  Include inside namespace yule { namespace { … } }.
 #pragma once

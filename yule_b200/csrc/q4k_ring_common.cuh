@@ -1,5 +1,5 @@
 // q4k_ring_common.cuh — the Q4_K stage layout in shared memory and the multiplication of one staged super-block,
-// shared by qmv_q4k_ring.cu and decode_mega.cu.  Include after q4k_mma_common.cuh, inside the same namespace.
+// of decode_mega.cu.  Include after q4k_mma_common.cuh, inside the same namespace.
 #pragma once
 
 constexpr int kStageRows = 16;

@@ -1,5 +1,5 @@
 // q6k_ring_common.cuh — the Q6_K stage layout in shared memory, the activation image and the multiplication of one
-// staged super-block, shared by qmv_q6k_ring.cu and decode_mega.cu.  Include inside namespace yule { namespace { … } }
+// staged super-block, of decode_mega.cu.  Include inside namespace yule { namespace { … } }
 // (decode_mega.cu wraps it in a namespace of its own: the names mirror those of the Q4_K headers).
 #pragma once
 

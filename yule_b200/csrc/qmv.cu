@@ -613,37 +613,6 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
             return launch_qmv_digits(f, sm_count, s, launches);
         }
     }
-    const bool q5_mma = a.type == YULE_DTYPE_Q5_K && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
-    if (a.batch > 1 && (a.type == YULE_DTYPE_Q4_K || q5_mma) && q4k_mma_supported(a.n_cols, 2)) {
-        // up to four activation vectors per pass over the weights
-        uint32_t done = 0;
-        while (done < a.batch) {
-            QmvArgs part = a;
-            part.x = a.x + (size_t)done * a.x_stride;
-            part.out = a.out + (size_t)done * a.out_stride;
-            part.residual = a.residual ? a.residual + (size_t)done * a.out_stride : nullptr;
-            part.batch = a.batch - done;
-            if (part.batch == 1) return launch_qmv(part, sm_count, s, launches);
-            uint32_t nb = part.batch < 4 ? part.batch : 4;
-            while (!q4k_mma_supported(a.n_cols, nb)) nb--;
-            Q4kBatch f;
-            f.w = a.w;
-            f.out = part.out;
-            f.rows = a.n_rows;
-            f.out_stride = a.out_stride;
-            f.q5 = q5_mma;
-            f.x = part.x;
-            f.x_stride = a.x_stride;
-            f.n_cols = a.n_cols;
-            f.batch = nb;
-            f.residual = part.residual;
-            f.pdl = a.pdl;
-            cudaError_t e = launch_q4k_mma(f, sm_count, s, launches);
-            if (e != cudaSuccess) return e;
-            done += nb;
-        }
-        return cudaSuccess;
-    }
     if (a.type == YULE_DTYPE_Q6_K && a.planar && a.batch > 1 && a.batch <= 8) {
         // rows too long for the batched kernel's activation image: one pass of the one-vector kernel per vector
         for (uint32_t b = 0; b < a.batch; b++) {

@@ -14,7 +14,7 @@
 // offset term (Q6_K: −32·Σx of the group; Q4_K: −dmin·m·Σx of the sub-block) and multiplies by d·sc in fp32.
 // Only the order of the fp32 additions differs from the CPU.
 //
-// Schedule: the one of the one-vector ring kernels (qmv_q4k_ring.cu, qmv_q6k_ring.cu) — one CTA of two 8-warp
+// Schedule: one CTA of two 8-warp
 // groups per SM, 16-row tiles dealt round-robin over the groups, a stage = 16 rows × 8 super-blocks (one per warp),
 // slots refilled by the warp that releases them last, every wait bounded.  The activation image (all vectors) is
 // built once per CTA.

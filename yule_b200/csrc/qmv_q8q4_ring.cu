@@ -10,7 +10,7 @@
 // copy (cp.async.bulk.tensor.2d + mbarrier, issued before `griddepcontrol.wait`), and the odd alignment is dealt
 // with there — aligned 32-bit shared-memory loads and a funnel shift by 0 or 16 bits.
 //
-// Tensor-core formulation (the same ideas as qmv_q4k_mma.cu):
+// Tensor-core formulation (hi and lo terms of fp16, as in qmv_rows.cu):
 //   A  the quant as an fp16 subnormal, exact: the byte + 128 (Q8_0: one XOR, two PRMT per four weights) or the
 //      nibble in place (Q4_0: one AND per pair of weights; high nibbles carry a factor 16);
 //   B  x·2^e split into fp16 hi / lo, two columns per vector (see below);

@@ -1,5 +1,5 @@
 // ring_common.cuh — mbarrier and bulk-copy helpers of the kernels that stage weights through a shared-memory
-// ring (qmv_q4k_ring.cu, qmv_q6k_ring.cu, decode_mega.cu).  Include inside namespace yule { namespace { … } }.
+// ring (qmv_digits.cu, qmv_rows.cu, decode_mega.cu and others).  Include inside namespace yule { namespace { … } }.
 #pragma once
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -731,10 +731,18 @@ int32_t finalize(yule_cuda_runner *r) {
 
 // fused = 2: describes the model to the persistent decode kernel.  A model it does not cover keeps the
 // multi-kernel graph (the reason is kept for yule_cuda_runner_token_step_kind).
+constexpr uint32_t kMegaMaxLayers = 3;
 int32_t setup_mega(yule_cuda_runner *r) {
     const yule_runner_config &c = r->cfg;
     if (is_variant(r)) {
         r->mega_why = "architecture variant";
+        return YULE_OK;
+    }
+    // The graph's one-vector kernels hand over faster than the phases of the persistent kernel once there are a few layers: per token,
+    // persistent against graph, 1.1B shape 22 layers 589 against 530 us, 4 layers 134 against 118; dim 1024, 16 layers 352 against
+    // 335; dim 512, 12 layers 230 against 218, 3 layers 60 against 61.
+    if (c.n_layers > kMegaMaxLayers && !knob("YULE_CUDA_MEGA")) {
+        r->mega_why = "the graph is faster on a model of this depth";
         return YULE_OK;
     }
     MegaModel m;
