@@ -740,7 +740,8 @@ int32_t setup_mega(yule_cuda_runner *r) {
     }
     // The graph's one-vector kernels hand over faster than the phases of the persistent kernel once there are a few layers: per token,
     // persistent against graph, 1.1B shape 22 layers 589 against 530 us, 4 layers 134 against 118; dim 1024, 16 layers 352 against
-    // 335; dim 512, 12 layers 230 against 218, 3 layers 60 against 61.
+    // 335; dim 512, 12 layers 230 against 218, 3 layers 60 against 61.  Models of up to three layers keep what fused = 2 asks for: the
+    // very small ones lose nothing, others some (1.1B shape, 2 layers 76 against 67).
     if (c.n_layers > kMegaMaxLayers && !knob("YULE_CUDA_MEGA")) {
         r->mega_why = "the graph is faster on a model of this depth";
         return YULE_OK;
