@@ -23,7 +23,7 @@
 // rows x 2048 columns, one 256-column block per warp: two neighbouring column ranges of one 16-row tile, or the same
 // columns of two tiles (of gate and up for a pair), whichever leaves fewer warps idle.  Units of one or two tiles are
 // dealt round-robin.  Row sums meet in shared memory; the warps take turns finishing units (one named barrier per unit in
-// flight, only the finishing warp waits on it).  Rows longer than the image of x may be are several launches over a
+// flight, only the finishing warp waits on it, and a warp whose copy never came).  Rows longer than the image of x may be are several launches over a
 // part of the columns each, every one adding to the result of the one before.
 //   Two launches side by side on an SM (half the shared memory each) were tried: the hardware puts two CTAs of one launch
 // on an SM as soon as there is room, 148 CTAs landed on 74 to 97 SMs, and a chain of launches took 1.3 times as long.
@@ -95,7 +95,7 @@ struct Smem {
     unsigned char *img;   // digits of x: 4 bytes per column
     float *f, *sx;        // 2^-e per 128 columns; (offset constant ·) Σx per scale group
     float *red;           // sums of squares per warp
-    float *inv;           // 1/rms
+    float *inv;           // 1/rms; behind it a word that a warp sets when it gives up waiting for a copy
     float *part;          // [finish][matrix of a pair whose tiles go one by one][warp][row]
     uint64_t *bars;       // full[kMaxSlots], empty[kMaxSlots]
 };
@@ -402,6 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
     const uint32_t slots = p.slots;
     const Smem sm = carve<F>(smem_raw, p.n_cols, slots, p.finish, nq);
     const uint32_t bar_full = smem_u32(sm.bars), bar_empty = bar_full + 8 * kMaxSlots;
+    volatile uint32_t *gave_up = reinterpret_cast<volatile uint32_t *>(sm.inv + 1);
 
     // Tile `half` of unit k (q: matrix of a pair whose tiles go one by one): its matrix and its number there.
     auto locate = [&](uint32_t k, uint32_t q, uint32_t half, uint32_t &seg) {
@@ -427,6 +428,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
     if (warp == kWarpsCta) {
         // ── the copying warp (one thread) ──
         if (lane == 0) {
+            *gave_up = 0;
             for (uint32_t i = 0; i < slots; i++) {
                 mbar_init(bar_full + 8 * i, 1);
                 mbar_init(bar_empty + 8 * i, kWarpsCta);
@@ -483,6 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
         if (lane == 0)
             while (n < total) {
                 if (!ring_wait(bar_empty + 8 * slot, phase ^ 1u, p.status, p.wait_cycles)) break;
+                if (*gave_up) break;  // the slot was released by a warp that did not wait for it: its copy may still be on its way
                 issue();
             }
         return;
@@ -552,7 +555,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
     else if (F != kQ6K) r_base += g * S::kPitch + local * S::kBlockBytes;
     BRegs b;
     bool dead = false;
-    uint32_t slot = 0, phase = 0, buf = 0;
+    uint32_t slot = 0, phase = 0, buf = 0, bar_id = 1;
     for (uint32_t k = 0; k < my_units; k++) {
         float *part = sm.part + (size_t)(buf * nq) * (kWarpsCta * kTileRows);
         const bool mine = !two || box_live(k, 0, box);
@@ -560,9 +563,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
             Acc acc;
             uint32_t blk = two ? local : warp;
             for (uint32_t c = 0; c < chunks; c++, blk += chunk_blocks) {
-                // A copy that never arrives: the warp stops multiplying but keeps its place at the barriers, so that nobody hangs.
-                if (!dead) dead = !ring_wait(bar_full + 8 * slot, phase, p.status, p.wait_cycles);
-                if (blk < bpr && mine && !dead) {
+                // A copy that never arrives: the lane waits for no other one, what the warp multiplies from here on means nothing.
+                if (!dead && !ring_wait(bar_full + 8 * slot, phase, p.status, p.wait_cycles)) {
+                    dead = true;
+                    *gave_up = 1;
+                }
+                if (blk < bpr && mine) {
                     const unsigned char *r0 = r_base + slot * S::kStageBytes;
                     if constexpr (F == kQ6K)
                         consume_q6k(r0, local, blk, g, t, lv, sm, b, acc);
@@ -590,9 +596,17 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
             }
         }
         // the sums of unit k are parked; its finishing warp adds them up and stores
-        const uint32_t bar_id = 1 + buf;
-        if ((k & (kWarpsCta - 1)) == warp) {
+        const bool finishes = (k & (kWarpsCta - 1)) == warp;
+        // A warp that has given up keeps its place at the barriers, but the ring no longer holds it back: it waits for the others at
+        // every unit, or it could arrive a second time at a barrier that a slower warp has yet to reach, whose phase would then be
+        // over without that warp, and its wait never.  (For the same reason there is one barrier more than there are buffers: the
+        // unit at which it gives up is one further on than the ring would have let it come.)
+        dead = __any_sync(0xffffffffu, dead);
+        if (finishes || dead)
             asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kMulThreads) : "memory");
+        else
+            asm volatile("bar.arrive %0, %1;" ::"r"(bar_id), "n"(kMulThreads) : "memory");
+        if (finishes) {
             const uint32_t rr = lane & 15, half = lane >> 4;  // half: the warps of box 0 or 1
             auto collect = [&](uint32_t q) {
                 const float *src = part + q * (kWarpsCta * kTileRows) + half * (8 * kTileRows) + rr;
@@ -622,10 +636,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
                 p.out[seg][row] = v;
                 if (TP && p.tp.push && seg == 0) tp_push_value(p.tp, row, v);
             }
-        } else {
-            asm volatile("bar.arrive %0, %1;" ::"r"(bar_id), "n"(kMulThreads) : "memory");
         }
         if (++buf == p.finish) buf = 0;
+        if (++bar_id == p.finish + 2) bar_id = 1;
     }
     if (dead)  // copies of this CTA that are still on their way get time to land before its shared memory goes
         for (const long long t0 = clock64(); clock64() - t0 < 2000000LL;) {

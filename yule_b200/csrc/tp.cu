@@ -333,7 +333,8 @@ int32_t yule_cuda_selftest_bounded_wait(yule_cuda_ctx *ctx, uint32_t which, uint
     if (ctx->tp_world > 1) return fail(YULE_ERR_INVALID_ARGUMENT, "the self-test runs on a context without tensor parallelism");
     YULE_CUDA_TRY(cudaSetDevice(ctx->device));
     YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    const uint32_t n_rows = 16, n_cols = 256, per_rank = 128;
+    // (rows: more units per CTA than its sums have buffers, so that a warp which gives up early would run into their reuse)
+    const uint32_t n_rows = 65536, n_cols = 256, per_rank = 128;
     const size_t payload = 1024;  // floats: pairs of the 256-element vector, or the two 128-float slices
     const size_t region_bytes = payload * sizeof(float) + (kFlagSlots * kMaxRanks + 64) * sizeof(uint32_t);
     char *mem = nullptr;
