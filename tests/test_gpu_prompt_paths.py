@@ -44,6 +44,38 @@ def test_tiled_prompt_attention_large_and_small_values(backend, oracle):
         run.close()
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (8, 2, 128)])
+@pytest.mark.parametrize("size", ["infinite", "huge"])
+def test_later_tokens_do_not_reach_earlier_ones(backend, oracle, heads, kv_heads, head_dim, size):
+    """A token whose K and V rows are not finite, or 10^24 times as large as the others', shares a K / V tile with tokens before
+    it: what those compute (the K rows of the second layer) is what they compute without it."""
+    n, at, odd = 600, 550, 299  # more than 512 tokens always go through the tiled kernel
+    cfg = ModelConfig(dim=512, n_layers=2, n_heads=heads, n_kv_heads=kv_heads, head_dim=head_dim, vocab_size=300, ff_dim=512,
+                      max_seq_len=640)
+    weights = synth.synthetic_model(cfg, seed=90, std=0.06, linear=DType.Q4_K, token_embd=DType.Q8_0)
+    embd = np.array(weights["token_embd.weight"][0]).reshape(cfg.vocab_size, cfg.dim // 32, 34).copy()
+    if size == "infinite":
+        embd[odd, :, :2] = np.full(1, np.inf, np.float16).view(np.uint8)
+    else:  # one element of the hidden state that only this token has, and a large weight for it in the first norm
+        embd[:, 0, 2] = 0
+        embd[odd, 0, 2] = 100
+        norm = np.ones(cfg.dim, np.float32)
+        norm[0] = 1e25
+        weights["blk.0.attn_norm.weight"] = (norm.view(np.uint8), DType.F32)
+    weights["token_embd.weight"] = (embd.reshape(-1), DType.Q8_0)
+    prompt = synth.tokens(91, n, odd)
+    prompt[at] = odd
+    ref = make_oracle_model(oracle, cfg, weights)
+    ref.prefill(prompt[:at])
+    run = CudaTransformerRunner(backend, cfg, weights, fused=1)
+    run.prefill(prompt)
+    kv = cfg.n_kv_heads * cfg.head_dim
+    rows = backend.download(run.buffer("k_cache", 1), n * kv).reshape(n, kv)
+    assert guarded_rel_err(rows[:at].reshape(-1), np.asarray(ref.k_cache(1, at)).reshape(-1)) <= REL_TOL
+    assert size == "huge" or np.isnan(rows[at:]).all()
+    run.close()
+
+
 @pytest.mark.parametrize("batch,n_prompt", [(3, 5), (2, 70), (9, 33), (33, 65)])
 def test_batch_prompts_in_passes(backend, batch, n_prompt):
     """Prompts of all sequences in shared passes (more rows than one pass takes in the last case) against the same
