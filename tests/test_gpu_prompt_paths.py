@@ -12,11 +12,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (8, 4, 64), (4, 4, 64), (8, 1, 128), (8, 2, 128), (4, 4, 128)])
-@pytest.mark.parametrize("n", [17, 65, 129, 200])
+@pytest.mark.parametrize("n", [17, 65, 129, 200, 577])
 def test_tiled_prompt_attention(backend, oracle, heads, kv_heads, head_dim, n):
-    """One query tile and several, one K / V tile, its edge and several, then a second prompt that starts inside a tile."""
+    """One query tile and several, one K / V tile, its edge and several, then a second prompt that starts inside a tile.  (With so few
+    heads only more than 512 tokens go through the tiled kernel; the others stay below its line.)"""
     cfg = ModelConfig(dim=512, n_layers=1, n_heads=heads, n_kv_heads=kv_heads, head_dim=head_dim, vocab_size=300, ff_dim=512,
-                      max_seq_len=320)
+                      max_seq_len=700)
     weights = synth.synthetic_model(cfg, seed=60 + n, std=0.06, linear=DType.Q4_K)
     ref = make_oracle_model(oracle, cfg, weights)
     run = CudaTransformerRunner(backend, cfg, weights, fused=1)
@@ -42,6 +43,55 @@ def test_tiled_prompt_attention_large_and_small_values(backend, oracle):
         prompt = synth.tokens(8, 130, cfg.vocab_size)
         assert guarded_rel_err(run.prefill(prompt), ref.prefill(prompt)) <= REL_TOL
         run.close()
+
+
+def unit_rows(columns, dim, factor=1.0):
+    """Q8_0 matrix whose row r is `factor` times the unit vector `columns[r]`."""
+    blocks = np.zeros((len(columns), dim // 32, 34), np.uint8)
+    for r, c in enumerate(columns):
+        blocks[r, c // 32, :2] = np.array([factor], np.float16).view(np.uint8)
+        blocks[r, c // 32, 2 + c % 32] = 1
+    return blocks.reshape(-1), DType.Q8_0
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (4, 1, 128)])
+def test_prompt_attention_error(backend, heads, kv_heads, head_dim):
+    """The tiled attention against 64 bits.  Matrices of unit vectors make its operands known: the first layer's caches hold them
+    (a query is -4 times the K row of its position), and the second layer's V rows are its normalised output, 32 times as large as the
+    hidden state it is added to.  The bound: the scores are about N(0, 4^2), and rounding one of 8 to 16 to 24 bits alone moves its
+    probability by up to 8 units of 2^-24.  (This kernel 3.4 and 3.7 units; with all MMAs of a sum on one accumulator, which
+    truncates, 11 and 18.)"""
+    n, dim, kv = 700, 512, kv_heads * head_dim
+    cfg = ModelConfig(dim=dim, n_layers=2, n_heads=heads, n_kv_heads=kv_heads, head_dim=head_dim, vocab_size=800, ff_dim=512, max_seq_len=768)
+    weights = synth.synthetic_model(cfg, seed=92, std=0.06, linear=DType.Q8_0, token_embd=DType.Q8_0)
+    group = heads // kv_heads
+    for layer in range(2):
+        name = f"blk.{layer}."
+        weights[name + "attn_q.weight"] = unit_rows([r // (group * head_dim) * head_dim + r % head_dim for r in range(dim)], dim, -4.0)
+        weights[name + "attn_k.weight"] = unit_rows(range(kv), dim)
+        weights[name + "attn_v.weight"] = unit_rows(range(dim - kv, dim) if layer == 0 else [r // head_dim * group * head_dim + r % head_dim for r in range(kv)], dim)
+        weights[name + "attn_output.weight"] = unit_rows(range(dim), dim, 32.0)
+        weights[name + "ffn_down.weight"] = (np.zeros(dim * cfg.ff_dim // 32 * 34, np.uint8), DType.Q8_0)
+        for norm in ("attn_norm", "ffn_norm"):
+            weights[name + norm + ".weight"] = (np.ones(dim, np.float32).view(np.uint8), DType.F32)
+    run = CudaTransformerRunner(backend, cfg, weights, fused=1)
+    prompt = synth.tokens(93, n, cfg.vocab_size)
+    run.prefill(prompt)
+    m = n - 1  # the last token goes through the token step
+    k, v, out = (backend.download(run.buffer(which, layer), n * kv).astype(np.float64).reshape(n, kv_heads, head_dim)[:m]
+                 for which, layer in (("k_cache", 0), ("v_cache", 0), ("v_cache", 1)))
+    run.close()
+    embd = np.array(weights["token_embd.weight"][0]).reshape(cfg.vocab_size, dim // 32, 34)
+    x = (embd[:, :, :2].copy().view(np.float16).astype(np.float64) * embd[:, :, 2:].copy().view(np.int8)).reshape(cfg.vocab_size, dim)[prompt[:m]]
+    s = np.einsum("ihd,jhd->hij", -4 * k, k) / np.sqrt(head_dim)
+    s[:, np.arange(m)[:, None] < np.arange(m)] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    att = np.einsum("hij,jhd->ihd", p / p.sum(-1, keepdims=True), v)
+    hidden = x + 32 * np.repeat(att, group, axis=1).reshape(m, dim)
+    normed = hidden / np.sqrt((hidden ** 2).mean(-1, keepdims=True) + cfg.norm_eps)
+    want = normed.reshape(m, kv_heads, group, head_dim)[:, :, 0]
+    error = np.linalg.norm(out - want) / np.linalg.norm(want)
+    assert error <= 8 * 2.0 ** -24, error
 
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (8, 2, 128)])

@@ -6,24 +6,30 @@
 // for a 2048-token prompt of the 8B shape.  Here 128 query rows share each K / V tile and the products run on mma.sync.
 //
 // Precision.  The cache and the queries are fp32; every operand is scaled by a power of two (per query row; per tile of K
-// and of V) and split into fp16 hi + lo (22 significant bits), and a product is three MMAs, lo·hi + hi·lo + hi·hi in that
-// order.  Probabilities are split the same way.  A K/V tile's P·V sums start from zero and are added to the running output
-// in fp32, so that no tensor-core accumulation chain is longer than 24 MMAs.  Soft-max is fp32 with a running maximum.
+// and of V) and split into fp16 hi + lo (22 significant bits); a product is four MMAs.  Probabilities are split the same way.
+// The tensor core truncates what it adds to, so every hi·hi MMA starts from zero and its result is added in fp32, and what
+// truncation takes on average (kTruncation) is given back; the three smaller products have an accumulator of their own, whose
+// truncation nobody sees.  For the scores it also collects what the fp32 additions and the scaling round off, and
+// multiplies the probability as 1 + rest.  Soft-max is fp32 with a running maximum.  Error against 64 bits (2-norm, N(0, 1) K and V)
+// as a multiple of that of one query per CTA on the FMA pipe: 40 tokens 0.98 to 1.08, 200 to 2048 tokens 0.85 to 0.98, with queries
+// four times as large 0.60 to 0.84, with a few channels of K and V 20 times as large 0.55 to 0.85.  (All MMAs of a sum on one
+// accumulator: 2.3 to 4.6, 532 us where this takes 718; without lo·lo up to 1.11, 636 us.)
 //
 // What a query does not see.  One scale for a tile's rows is a loss to the small ones, and a masked position's probability of
 // zero makes NaN of an infinite V row.  Either would let a token change what tokens before it get.  So a CTA that
 // meets rows of K or V whose largest elements lie more than kRange binary orders apart (the small ones would lose bits), or
 // a value that is not finite, computes its rows over again on the FMA pipe (exact_rows), where a query touches the
-// positions that it attends to and no others.  With rows of one model's layer neither happens; looking takes 3 to 4 % (2048
-// tokens of the 8B shape 517 -> 532 us, of the 1.1B shape 277 -> 288).  Powers of two of their own for the rows of K and V, the
-// latter's in the probabilities, would keep wide ranges on the tensor pipe, at 542 us.
+// positions that it attends to and no others.  With rows of one model's layer neither happens; looking takes 3 to 4 %.  Powers
+// of two of their own for the rows of K and V, the latter's in the probabilities, would keep wide ranges on the tensor pipe, at 2 % more.
 //
 // Work split.  CTA (query tile, KV head, sequence): 128 rows = GROUP query heads x 128/GROUP tokens, so that all rows share
 // the K / V tiles of one KV head and the causal edge cuts few tiles; warp w has rows 16w .. 16w + 15.  K / V come in tiles of
 // 64 positions: asynchronous copies of the next tile's fp32 rows run under the MMAs of the current one; every thread then
-// converts the pieces it copied itself.
+// converts the pieces it copied itself.  The split queries stay in shared memory (in registers they left too few for the scores
+// and their rest).  Per layer, 2048 tokens of the 8B shape 718 us, of the 1.1B shape 378.
 
 #include <cfloat>
+#include <mutex>
 
 #include <cuda_fp16.h>
 
@@ -36,6 +42,9 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kRows = 128;  // query rows per CTA
 constexpr int kKeys = 64;   // positions per K / V tile
+// Mean of the part that truncation to 24 bits takes of a sum: half a unit of the last place, over mantissas of equal density in the
+// logarithm, 2^-24 / (2 ln 2).
+constexpr float kTruncation = 4.3e-8f;
 constexpr uint32_t kRange = 14;  // scaled, a tile's largest element is 2^13 to 2^14 and lo ends at 2^-24: 2^-1 keeps its 22 bits
 constexpr float kProbScale = 4096.f;  // keeps small probabilities clear of fp16's subnormals; cancels in the division by the sum
 
@@ -52,6 +61,12 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16_z(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -84,7 +99,8 @@ struct Layout {
     static constexpr uint32_t kPitch = HD * 2 + 16;               // bytes of an fp16 row: rows 16 bytes apart in bank terms
     static constexpr uint32_t kPlane = kKeys * kPitch;            // one of K hi, K lo, V hi, V lo
     static constexpr uint32_t kRaw = kKeys * HD * 4;              // fp32 tile of K or V
-    static constexpr uint32_t kSmem = 4 * kPlane + 2 * kRaw + 128;
+    static constexpr uint32_t kQPlane = kRows * kPitch;           // Q hi or lo
+    static constexpr uint32_t kSmem = 4 * kPlane + 2 * kQPlane + 2 * kRaw + 128;
 };
 
 // The 16 rows of a warp, position by position in fp32.
@@ -126,7 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
     constexpr int NT = HD / 8;       // n8 tiles of the output
     constexpr int CH = HD / 4;       // 16-byte pieces per row
     constexpr int PER = kKeys * CH / kThreads;  // pieces of K (and of V) per thread and tile
-    unsigned char *planes = smem, *raw = smem + 4 * L::kPlane;
+    unsigned char *planes = smem, *q_planes = smem + 4 * L::kPlane, *raw = q_planes + 2 * L::kQPlane;
     uint4 *red = reinterpret_cast<uint4 *>(raw + 2 * L::kRaw);  // per warp: largest |K|, |V|, and the smallest of its rows' largest
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const uint32_t kvh = blockIdx.y, seq = blockIdx.z;
@@ -155,8 +171,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
     };
     copy_tile(0);
 
-    // this lane's two query rows as A fragments, and the factor of their scores
-    uint32_t qh[KS][4], ql[KS][4];
+    // this lane's two query rows to shared memory, and the factor of their scores
     float row_scale[2];
     uint32_t qpos[2];
     {
@@ -177,11 +192,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
             mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
             float sc;
             pow2_scale(mx[r], sc, row_scale[r]);
+            unsigned char *to = q_planes + (warp * 16 + g + 8 * r) * L::kPitch + 4 * t;
 #pragma unroll
-            for (int k = 0; k < KS; k++) {
-                const float2 v0 = *reinterpret_cast<const float2 *>(qp[r] + 16 * k), v1 = *reinterpret_cast<const float2 *>(qp[r] + 16 * k + 8);
-                split2(v0.x * sc, v0.y * sc, qh[k][r], ql[k][r]);
-                split2(v1.x * sc, v1.y * sc, qh[k][2 + r], ql[k][2 + r]);
+            for (int k = 0; k < 2 * KS; k++) {
+                const float2 v = *reinterpret_cast<const float2 *>(qp[r] + 8 * k);
+                uint32_t hi, lo;
+                split2(v.x * sc, v.y * sc, hi, lo);
+                *reinterpret_cast<uint32_t *>(to + 16 * k) = hi;
+                *reinterpret_cast<uint32_t *>(to + L::kQPlane + 16 * k) = lo;
             }
             row_scale[r] *= 1.0f / sqrtf((float)HD);
         }
@@ -242,24 +260,40 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
         if (j + 1 < n_tiles) copy_tile(j + 1);  // the raw pieces have been read by the threads that own them
 
         // scores of 16 rows x 64 keys
-        float s[kKeys / 8][4];
-#pragma unroll
-        for (int n = 0; n < kKeys / 8; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+        float s[kKeys / 8][4], c[kKeys / 8][4];  // sums of hi·hi; everything smaller
         // ldmatrix: lanes 0-7 rows of (n, k low), 8-15 (n, k high), 16-23 (n + 1, k low), 24-31 (n + 1, k high)
         const uint32_t k_addr = planes_u32 + ((lane & 7) + ((lane >> 4) & 1) * 8) * L::kPitch + ((lane >> 3) & 1) * 16;
+        // A fragments: lanes 0-7 rows 0-7, 8-15 rows 8-15 of the k low half, 16-31 the same of the k high half
+        const uint32_t q_addr = planes_u32 + 4 * L::kPlane + (warp * 16 + (lane & 15)) * L::kPitch + (lane >> 4) * 16;
 #pragma unroll
         for (int k = 0; k < KS; k++) {
+            uint32_t qh[4], ql[4];
+            ldsm4(qh, q_addr + k * 32);
+            ldsm4(ql, q_addr + L::kQPlane + k * 32);
 #pragma unroll
             for (int n = 0; n < kKeys / 8; n += 2) {
                 uint32_t bh[4], bl[4];
                 ldsm4(bh, k_addr + n * 8 * L::kPitch + k * 32);
                 ldsm4(bl, k_addr + L::kPlane + n * 8 * L::kPitch + k * 32);
-                mma_f16(s[n], ql[k], bh[0], bh[1]);
-                mma_f16(s[n + 1], ql[k], bh[2], bh[3]);
-                mma_f16(s[n], qh[k], bl[0], bl[1]);
-                mma_f16(s[n + 1], qh[k], bl[2], bl[3]);
-                mma_f16(s[n], qh[k], bh[0], bh[1]);
-                mma_f16(s[n + 1], qh[k], bh[2], bh[3]);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    float d[4];
+                    mma_f16_z(d, qh, bh[2 * i], bh[2 * i + 1]);
+                    if (k == 0) mma_f16_z(c[n + i], ql, bl[2 * i], bl[2 * i + 1]);
+                    else mma_f16(c[n + i], ql, bl[2 * i], bl[2 * i + 1]);
+                    mma_f16(c[n + i], ql, bh[2 * i], bh[2 * i + 1]);
+                    mma_f16(c[n + i], qh, bl[2 * i], bl[2 * i + 1]);
+#pragma unroll
+                    for (int x = 0; x < 4; x++) {
+                        if (k == 0) {
+                            s[n + i][x] = d[x];
+                        } else {  // what the addition rounds off goes to the small terms
+                            const float sum = s[n + i][x] + d[x];
+                            c[n + i][x] += d[x] - (sum - s[n + i][x]);
+                            s[n + i][x] = sum;
+                        }
+                    }
+                }
             }
         }
         // scale, mask, running soft-max
@@ -273,10 +307,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
 #pragma unroll
             for (int n = 0; n < kKeys / 8; n++)
 #pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    float v = s[n][2 * r + c] * f;
-                    if (edge && key0 + 8 * n + c > qpos[r]) v = -FLT_MAX;
-                    s[n][2 * r + c] = v;
+                for (int x = 2 * r; x < 2 * r + 2; x++) {
+                    c[n][x] = fmaf(s[n][x], kTruncation, c[n][x]);
+                    const float sum = s[n][x] + c[n][x];
+                    float v = sum * f;
+                    c[n][x] = fmaf(c[n][x] - (sum - s[n][x]), f, fmaf(sum, f, -v));  // what sum and product round off
+                    if (edge && key0 + 8 * n + (x & 1) > qpos[r]) v = -FLT_MAX;
+                    s[n][x] = v;
                     mx = fmaxf(mx, v);
                 }
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -288,10 +325,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
 #pragma unroll
             for (int n = 0; n < kKeys / 8; n++)
 #pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    const float v = s[n][2 * r + c];
-                    const float e = v == -FLT_MAX ? 0.f : expf(v - mn) * kProbScale;
-                    s[n][2 * r + c] = e;
+                for (int x = 2 * r; x < 2 * r + 2; x++) {
+                    // e^(v + c - mn), what the subtraction rounds off included: it is the first power that the small terms enter by
+                    const float v = s[n][x], d = v - mn, w = expf(d), small = c[n][x] + (v - (d + mn));
+                    const float e = v == -FLT_MAX ? 0.f : fmaf(w, small, w) * kProbScale;
+                    s[n][x] = e;
                     sum += e;
                 }
             l[r] = fmaf(l[r], alpha[r], sum);
@@ -308,29 +346,29 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
         // ldmatrix.trans: lanes 0-7 keys (k low, n), 8-15 (k high, n), 16-23 (k low, n + 1), 24-31 (k high, n + 1)
         const uint32_t v_addr = planes_u32 + 2 * L::kPlane + ((lane & 7) + ((lane >> 3) & 1) * 8) * L::kPitch + ((lane >> 4) & 1) * 16;
 #pragma unroll
-        for (int n = 0; n < NT; n += 4) {
-            float d[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
+        for (int n = 0; n < NT; n += 2) {
+            float small[2][4], sum[2][4];
 #pragma unroll
             for (int k = 0; k < kKeys / 16; k++) {
+                uint32_t bh[4], bl[4];
+                ldsm4t(bh, v_addr + k * 16 * L::kPitch + n * 16);
+                ldsm4t(bl, v_addr + L::kPlane + k * 16 * L::kPitch + n * 16);
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    uint32_t bh[4], bl[4];
-                    ldsm4t(bh, v_addr + k * 16 * L::kPitch + (n + 2 * q) * 16);
-                    ldsm4t(bl, v_addr + L::kPlane + k * 16 * L::kPitch + (n + 2 * q) * 16);
-                    mma_f16(d[2 * q], pl[k], bh[0], bh[1]);
-                    mma_f16(d[2 * q + 1], pl[k], bh[2], bh[3]);
-                    mma_f16(d[2 * q], ph[k], bl[0], bl[1]);
-                    mma_f16(d[2 * q + 1], ph[k], bl[2], bl[3]);
-                    mma_f16(d[2 * q], ph[k], bh[0], bh[1]);
-                    mma_f16(d[2 * q + 1], ph[k], bh[2], bh[3]);
+                for (int i = 0; i < 2; i++) {
+                    float d[4];
+                    mma_f16_z(d, ph[k], bh[2 * i], bh[2 * i + 1]);
+                    if (k == 0) mma_f16_z(small[i], pl[k], bl[2 * i], bl[2 * i + 1]);
+                    else mma_f16(small[i], pl[k], bl[2 * i], bl[2 * i + 1]);
+                    mma_f16(small[i], pl[k], bh[2 * i], bh[2 * i + 1]);
+                    mma_f16(small[i], ph[k], bl[2 * i], bl[2 * i + 1]);
+#pragma unroll
+                    for (int x = 0; x < 4; x++) sum[i][x] = k == 0 ? d[x] : sum[i][x] + d[x];
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 2; i++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) o[n + i][c] = fmaf(o[n + i][c], alpha[c >> 1], d[i][c] * vi);
+                for (int x = 0; x < 4; x++) o[n + i][x] = fmaf(o[n + i][x], alpha[x >> 1], (sum[i][x] + fmaf(sum[i][x], kTruncation, small[i][x])) * vi);
         }
     }
 #pragma unroll
@@ -350,8 +388,19 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
 template <int HD, int GROUP>
 cudaError_t launch_variant(const PrefillParams &p, uint32_t n_seq, bool pdl, cudaStream_t s) {
     auto kern = attn_prefill_kernel<HD, GROUP>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Layout<HD>::kSmem);
+    static bool attr_done[64] = {};  // the opt-in for large dynamic shared memory belongs to the device
+    static std::mutex mu;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Layout<HD>::kSmem);
+            if (e != cudaSuccess) return e;
+            if (dev >= 0 && dev < 64) attr_done[dev] = true;
+        }
+    }
     const uint32_t tiles = (p.n_tokens * GROUP + kRows - 1) / kRows;
     return launch_kernel(kern, dim3(tiles, p.n_kv_heads, n_seq), dim3(kThreads), Layout<HD>::kSmem, s, pdl, p);
 }
@@ -359,7 +408,7 @@ cudaError_t launch_variant(const PrefillParams &p, uint32_t n_seq, bool pdl, cud
 }  // namespace
 
 // Whether the tiled kernel is the faster one: its time goes with (waves of CTAs) x (K / V tiles of the longest CTA), about
-// 5 us each at head_dim 128; one query per CTA (attn_decode_gqa_kernel) takes about 1.1 ns per query and key of eight KV
+// 7 us each at head_dim 128; one query per CTA (attn_decode_gqa_kernel) takes about 1.1 ns per query and key of eight KV
 // heads of 512 output columns, and spreads a few queries over all SMs.
 bool attn_prefill_preferred(uint32_t hd, uint32_t n_heads, uint32_t n_kv_heads, uint32_t n_tokens, uint32_t n_seq, uint32_t pos0, int sm_count) {
     if (!attn_gqa_supported(hd, n_heads, n_kv_heads)) return false;
@@ -367,7 +416,7 @@ bool attn_prefill_preferred(uint32_t hd, uint32_t n_heads, uint32_t n_kv_heads, 
     const uint64_t ctas = (uint64_t)((n_tokens * group + kRows - 1) / kRows) * n_kv_heads * n_seq;
     const uint64_t waves = (ctas + sm_count - 1) / sm_count;
     const double keys = pos0 + 0.5 * n_tokens;
-    const double tiled = (double)waves * ((pos0 + n_tokens + kKeys - 1) / kKeys) * 5.0 * hd / 128;
+    const double tiled = (double)waves * ((pos0 + n_tokens + kKeys - 1) / kKeys) * 7.0 * hd / 128;
     const double single = 1.1e-3 * n_seq * n_tokens * keys * ((double)n_heads * hd / 4096);
     return tiled < single;
 }
