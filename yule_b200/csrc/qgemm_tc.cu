@@ -16,9 +16,11 @@
 // its largest element in [2¹³, 2¹⁴) and split into fp16 hi + lo (22 significant bits); two MMAs per
 // 16 columns, W·x_hi and W·x_lo (up to 64 activation rows one MMA against both terms side by side as
 // one operand of twice the rows).  The tensor core adds into its fp32 accumulator with truncation, a
-// bias that grows with the chain length; draining after every stage keeps a chain at 8 MMAs and
-// leaves the long sum to ordinary round-to-nearest fp32.  The result matches the fp32 matvec to
-// fp32 rounding.
+// bias that grows with the chain length; draining after every stage, and the small products before the
+// large ones, keep a chain of large ones at 4 MMAs (8 at 32 rows) and leave the long sum to ordinary
+// round-to-nearest fp32; the mean of the bias is given back at the end.  Error against 64 bits (2-norm) at
+// 200 rows: Q8_0 and Q6_K 1.2e-7 to 1.4e-7, Q4_K 2.4e-7 to 2.7e-7; with large and small
+// products in turn, 3.2e-7 and 3.9e-7, in the same time.
 //
 // Work items: (row tile, activation tile) pairs; when these are few (small matrices, tensor-parallel
 // shards, few activation rows) the super-blocks of a row are split into up to 16 parts, one item each,
@@ -101,6 +103,9 @@ __host__ __device__ constexpr uint32_t groups_per_stage(uint32_t bn, bool generi
 constexpr uint32_t kRawBytes = kBM * 144;          // one super-block of 128 rows: 18 KB
 constexpr uint32_t kABytes = kBM * kBK * 2;  // the W slab of a stage: 16 KB
 constexpr float kSumScale = 1.0f / 32.0f;     // the sub-block sums of x are stored divided by 32
+// 1 + 2^-23: what truncation takes of a stage's sum on average (measured 0.9e-7 of the result, exact kernel 0.7e-7, at 32 rows
+// 1.2e-7) is given back.
+constexpr float kTruncation = 1.00000012f;
 constexpr float kGenericWScale = 1024.f;      // generic kernel: weights are scaled by 2^10 before the fp16 hi/lo split
 constexpr uint32_t kAmBytes = kBM * 16 * 2;  // the m slab of a super-block: 128 rows × 16 columns, 4 KB
 constexpr long long kWaitCycles = 2000000000LL;  // ~1 s: far beyond any real stall
@@ -139,7 +144,7 @@ struct GemmParams {
     uint32_t raw_stride;   // generic kernel: shared-memory row stride of the raw copy (an odd multiple of 16 bytes)
     uint32_t raw_chunks;   // generic kernel: 16-byte chunks copied per row and unit
     uint32_t raw_ring_bytes;  // generic kernel: two slots of 128 rows
-    float out_scale;       // generic kernel: 1 / kGenericWScale; exact kernel: 1
+    float out_scale;       // kTruncation; generic kernel: / kGenericWScale
     uint32_t prof;         // timing aid: record cycle counters of CTA 0
     uint32_t skip;         // timing aid (YULE_GEMM_SKIP, bits): 1 no unpacking, 2 no MMAs, 4 no draining, 8 no activation copies,
                            // 64 no weight copies, 256 the MMA threads wait for their own commits; results meaningless
@@ -740,33 +745,44 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                     // issuing thread's own instruction stream, not the tensor pipe, bounded the MMA rate).
                     const uint64_t da0 = smem_desc(a, 2048, 128);
                     const uint64_t db0 = T::MERGED ? smem_desc(x_hi, 2 * x_lbo, 128) : smem_desc(x_hi, x_lbo, 128);
-                    auto step = [&](auto k16c) {
-                        constexpr uint32_t k16 = decltype(k16c)::value;
-                        const uint64_t da = da0 + (uint64_t)((k16 * 4096u) >> 4);
-                        if constexpr (T::MERGED) {
-                            // rows [0, BN) of an 8-column step are the hi terms, rows [BN, 2·BN) the lo terms
-                            const uint64_t db = db0 + (uint64_t)((k16 * 4u * x_lbo) >> 4);
-                            umma_f16_c<(k16 != 0)>(d_main, da, db, idesc2);  // every stage starts a fresh accumulator
-                            if (GENERIC)  // the lo term of the weights against the hi term of the activations: the first BN rows
-                                umma_f16_c<1>(d_main, da + (uint64_t)(kABytes >> 4), db, idesc);
-                        } else {
-                            const uint64_t dbh = db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4);
-                            umma_f16_c<(k16 != 0)>(d_main, da, dbh, idesc);  // every stage starts a fresh accumulator
-                            umma_f16_c<1>(d_main, da, dbh + (uint64_t)(kXHalfBytes >> 4), idesc);
-                            if (GENERIC)  // the lo term of the weights against the hi term of the activations
-                                umma_f16_c<1>(d_main, da + (uint64_t)(kABytes >> 4), dbh, idesc);
+                    // The tensor core truncates when it adds to an accumulator, which costs a part of what the accumulator holds.  So
+                    // the products with lo terms go first, or to the columns of their own: the hi·hi sums see four additions (eight at two
+                    // column groups per stage), not eight or twelve.
+                    auto steps = [&](auto f) {
+                        f(std::integral_constant<uint32_t, 0>{});
+                        f(std::integral_constant<uint32_t, 1>{});
+                        f(std::integral_constant<uint32_t, 2>{});
+                        f(std::integral_constant<uint32_t, 3>{});
+                        if constexpr (T::KG == 2) {  // the second group's slabs follow the first's in both operands
+                            f(std::integral_constant<uint32_t, 4>{});
+                            f(std::integral_constant<uint32_t, 5>{});
+                            f(std::integral_constant<uint32_t, 6>{});
+                            f(std::integral_constant<uint32_t, 7>{});
                         }
                     };
                     if (!(skip & 2u)) {
-                        step(std::integral_constant<uint32_t, 0>{});
-                        step(std::integral_constant<uint32_t, 1>{});
-                        step(std::integral_constant<uint32_t, 2>{});
-                        step(std::integral_constant<uint32_t, 3>{});
-                        if constexpr (T::KG == 2) {  // the second group's slabs follow the first's in both operands
-                            step(std::integral_constant<uint32_t, 4>{});
-                            step(std::integral_constant<uint32_t, 5>{});
-                            step(std::integral_constant<uint32_t, 6>{});
-                            step(std::integral_constant<uint32_t, 7>{});
+                        if constexpr (T::MERGED) {
+                            steps([&](auto k16c) {
+                                constexpr uint32_t k16 = decltype(k16c)::value;
+                                const uint64_t da = da0 + (uint64_t)((k16 * 4096u) >> 4);
+                                // rows [0, BN) of an 8-column step are the hi terms, rows [BN, 2·BN) the lo terms
+                                const uint64_t db = db0 + (uint64_t)((k16 * 4u * x_lbo) >> 4);
+                                umma_f16_c<(k16 != 0)>(d_main, da, db, idesc2);  // every stage starts a fresh accumulator
+                                if (GENERIC)  // the lo term of the weights against the hi term of the activations: beside the other small products
+                                    umma_f16_c<1>(d_main + BN, da + (uint64_t)(kABytes >> 4), db, idesc);
+                            });
+                        } else {
+                            steps([&](auto k16c) {
+                                constexpr uint32_t k16 = decltype(k16c)::value;
+                                const uint64_t da = da0 + (uint64_t)((k16 * 4096u) >> 4), dbh = db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4);
+                                umma_f16_c<(k16 != 0)>(d_main, da, dbh + (uint64_t)(kXHalfBytes >> 4), idesc);  // every stage starts a fresh accumulator
+                                if (GENERIC)  // the lo term of the weights against the hi term of the activations
+                                    umma_f16_c<1>(d_main, da + (uint64_t)(kABytes >> 4), dbh, idesc);
+                            });
+                            steps([&](auto k16c) {
+                                constexpr uint32_t k16 = decltype(k16c)::value;
+                                umma_f16_c<1>(d_main, da0 + (uint64_t)((k16 * 4096u) >> 4), db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4), idesc);
+                            });
                         }
                     }
                     if (!GENERIC && kb % T::SPB == T::SPB - 1)  // Σ_s m_s · (sum of x over sub-block s), hi and lo sums side by side
@@ -1532,7 +1548,7 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     p.stages = stages > (uint32_t)kMaxStages ? (uint32_t)kMaxStages : stages;
     p.type = g.type;
     p.w_row_bytes = (uint64_t)(g.n_cols / block_size(g.type)) * block_bytes(g.type);
-    p.out_scale = generic ? 1.0f / kGenericWScale : 1.0f;
+    p.out_scale = (generic ? 1.0f / kGenericWScale : 1.0f) * kTruncation;
     p.status = g.status;
     p.prof = (kProfile && knob("YULE_GEMM_PROF")) ? 1u : 0u;
     p.skip = (kProfile && knob("YULE_GEMM_SKIP")) ? (uint32_t)atoi(knob("YULE_GEMM_SKIP")) : 0u;
