@@ -37,6 +37,24 @@ def test_sampler_over_a_cut_vocabulary(backend, oracle, n):
     backend.free(lh)
 
 
+def test_filtered_tokens_are_never_picked(backend):
+    """Random values at and around the mass that lies before each run of 32 tokens (what a warp adds up): runs begin and end with
+    tokens that min-p removes, so a pick must be one of the tokens between."""
+    n = 8192
+    logits = synth.normal(310, n).reshape(-1, 32)
+    logits[:, :8] = logits[:, 24:] = -30.0
+    lh = backend.upload(logits.astype(np.float32).reshape(-1))
+    kept = np.exp(logits.astype(np.float64))
+    kept[:, :8] = kept[:, 24:] = 0
+    edges = np.cumsum(kept.sum(1) / kept.sum())[:-1:3].astype(np.float32)
+    kw = dict(temperature=1.0, top_p=1.0, top_k=0, repetition_penalty=1.0, min_p=1e-6)
+    for edge in edges:
+        for step in range(-4, 5):
+            r = np.uint32(int(edge.view(np.uint32)) + step).view(np.float32)
+            assert 8 <= backend.sample(lh, n, float(r), **kw) % 32 < 24, (float(r), step)
+    backend.free(lh)
+
+
 def test_sampled_stream_continues_greedily(backend):
     """A sampled run leaves the runner where feeding its tokens would have left it."""
     cfg = ModelConfig(dim=512, n_layers=2, n_heads=8, n_kv_heads=2, head_dim=64, vocab_size=700, ff_dim=768, max_seq_len=128)

@@ -405,19 +405,22 @@ __global__ void __cluster_dims__(kSampCtas, 1, 1) __launch_bounds__(kSampThreads
             }
         }
     } else {
-        // inverse CDF in index order (sampler.rs:166-183): the first token whose running sum reaches r, else the last
+        // inverse CDF in index order (sampler.rs:166-183): the first token whose running sum reaches r, else the last.  A token
+        // without mass does not move the reference's sum, so it is never the one (but for r = 0, which the first token reaches):
+        // here the sums of a warp's start and of the end of the warp before may differ by a rounding, and r may fall between.
         const float inv_total = 1.0f / total;
         float carry = (earlier + before) * inv_total;
         if (carry + wsum * inv_total * 1.001f >= rnd) {  // (warps that cannot hold the crossing do not look)
             for (uint32_t base = s0; base < s1; base += 32) {
                 const uint32_t i = base + lane;
-                float q = i < s1 ? probs[i] * inv_total : 0.f;
+                const float own = i < s1 ? probs[i] : 0.f;
+                float q = own * inv_total;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const float v = __shfl_up_sync(0xffffffffu, q, o);
                     if (lane >= (uint32_t)o) q += v;
                 }
-                const uint32_t hit = __ballot_sync(0xffffffffu, i < s1 && carry + q >= rnd);
+                const uint32_t hit = __ballot_sync(0xffffffffu, i < s1 && carry + q >= rnd && (own > 0.f || rnd <= 0.f));
                 if (hit) {
                     if (lane == 0) atomicMin(&s_first, base + __ffs(hit) - 1);
                     break;
