@@ -45,18 +45,27 @@ int32_t ensure_gemm_scratch(yule_cuda_ctx *ctx, size_t bytes) {
     if (ctx->capturing)
         return fail(YULE_ERR_INVALID_ARGUMENT, "the GEMM scratch (%zu bytes) cannot grow during graph capture", bytes);
     YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (ctx->gemm_scratch) ctx->retired_scratch.push_back(ctx->gemm_scratch);  // graphs captured earlier may still use it
-    ctx->gemm_scratch = nullptr;
-    ctx->gemm_scratch_bytes = 0;
-    cudaError_t e = cudaMalloc(&ctx->gemm_scratch, bytes);
+    // At least twice the block before, so that all the outgrown ones together are no larger than this one.
+    void *block = nullptr;
+    size_t got = bytes < 2 * ctx->gemm_scratch_bytes ? 2 * ctx->gemm_scratch_bytes : bytes;
+    cudaError_t e = cudaMalloc(&block, got);
+    if (e != cudaSuccess && got > bytes) {
+        cudaGetLastError();
+        e = cudaMalloc(&block, got = bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(YULE_ERR_OUT_OF_MEMORY, "cuda allocation of %zu bytes of GEMM scratch failed", bytes);
     }
     // the scratch opens with the split-column tickets of the GEMM, which the kernels expect (and leave) at zero
-    e = cudaMemset(ctx->gemm_scratch, 0, bytes < kGemmTicketBytes ? bytes : kGemmTicketBytes);
-    if (e != cudaSuccess) return fail_cuda(e, "cudaMemset of the GEMM tickets");
-    ctx->gemm_scratch_bytes = bytes;
+    e = cudaMemset(block, 0, got < kGemmTicketBytes ? got : kGemmTicketBytes);
+    if (e != cudaSuccess) {
+        cudaFree(block);
+        return fail_cuda(e, "cudaMemset of the GEMM tickets");
+    }
+    if (ctx->gemm_scratch) ctx->retired_scratch.push_back(ctx->gemm_scratch);  // graphs captured earlier may still use it
+    ctx->gemm_scratch = block;
+    ctx->gemm_scratch_bytes = got;
     return YULE_OK;
 }
 

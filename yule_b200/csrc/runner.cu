@@ -83,6 +83,8 @@ struct yule_cuda_runner {
           *pf_up = nullptr, *pf_attn_scratch = nullptr, *pf_norm = nullptr;
     uint32_t *pf_tokens = nullptr, *pf_tickets = nullptr;
     std::vector<yule_buffer> pf_owned;  // the row buffers, replaced when a pass needs more rows
+    uint32_t pf_refused = 0;  // rows for which there was no memory, and how much was free then
+    size_t pf_refused_free = 0;
 
     // Batched decode: `bd_batch` independent sequences advancing one token per step, each with its own KV
     // caches and position; every linear is one GEMM over the batch (the chunk buffers above hold the rows).
@@ -905,67 +907,96 @@ bool prefill_batched_ok(const yule_cuda_runner *r) {
     return score_bytes <= 96 * 1024;
 }
 
-// Row buffers of the GEMM-driven paths (chunked prefill, batched decode) for passes of up to `rows` rows, allocated on first
-// use and replaced when a pass needs more.  Under tensor parallelism the matrices that are gathered (x, attention output,
-// gate, up) live in the exchange region, which every peer maps (its size is fixed); q / k / v hold this rank's heads only.
-int32_t ensure_chunk_buffers(yule_cuda_runner *r, uint32_t rows) {
+// Gives the row buffers back.  Nothing that is still running may hold them, and the captured step must not.
+int32_t drop_chunk_buffers(yule_cuda_runner *r) {
+    if (r->pf_owned.empty()) return YULE_OK;
+    YULE_CUDA_TRY(cudaStreamSynchronize(r->ctx->stream));
+    if (r->bd_graph) cudaGraphExecDestroy(r->bd_graph);
+    r->bd_graph = nullptr;
+    for (yule_buffer h : r->pf_owned) yule_cuda_free(r->ctx, h);
+    r->pf_owned.clear();
+    r->pf_chunk = 0;
+    return YULE_OK;
+}
+
+// What passes of up to C rows need besides the buffers of this function's callers: GEMM scratch and pinned words.
+int32_t ensure_pass_scratch(yule_cuda_runner *r, uint32_t C) {
+    const yule_runner_config &c = r->cfg;
+    const uint32_t qdim = c.n_heads * c.head_dim, widest = c.ff_dim > qdim ? (c.ff_dim > c.dim ? c.ff_dim : c.dim) : (qdim > c.dim ? qdim : c.dim);
+    const int32_t rc = ensure_gemm_scratch(r->ctx, qgemm_scratch_bytes(C, widest));
+    return rc ? rc : ensure_pinned(r, C);
+}
+
+int32_t alloc_chunk_buffers(yule_cuda_runner *r, uint32_t C) {
     const yule_runner_config &c = r->cfg;
     const uint32_t N = r->ctx->tp_world > 1 ? r->ctx->tp_world : 1;
     const uint32_t dim = c.dim, hd = c.head_dim, qdim = c.n_heads * hd, kvdim = c.n_kv_heads * hd, ff = c.ff_dim;
     int32_t rc;
-    uint32_t C = prefill_chunk_size(r);
-    if (N > 1)
-        C = C > r->xb_rows ? r->xb_rows : C;
-    else
-        C = rows > C ? (rows + 127) / 128 * 128 : C;
-    if (r->pf_chunk < C) {
-        if (r->pf_chunk) {
-            // nothing that is still running may hold the old buffers, and the captured step must not
-            YULE_CUDA_TRY(cudaStreamSynchronize(r->ctx->stream));
-            if (r->bd_graph) cudaGraphExecDestroy(r->bd_graph);
-            r->bd_graph = nullptr;
-            for (yule_buffer h : r->pf_owned) yule_cuda_free(r->ctx, h);
-            r->pf_owned.clear();
-            r->pf_chunk = 0;
+    auto alloc = [&](size_t n, float **out) {
+        yule_buffer h;
+        const int32_t e = alloc_f32(r, n, out, &h);
+        if (e == YULE_OK) {
+            r->owned.pop_back();
+            r->pf_owned.push_back(h);
         }
-        auto alloc = [&](size_t n, float **out) {
-            yule_buffer h;
-            const int32_t e = alloc_f32(r, n, out, &h);
-            if (e == YULE_OK) {
-                r->owned.pop_back();
-                r->pf_owned.push_back(h);
-            }
-            return e;
-        };
-        r->pf_splits = c.max_seq_len / 1024 < 1 ? 1 : (c.max_seq_len / 1024 > 8 ? 8 : c.max_seq_len / 1024);
-        float *tok_f = nullptr, *tick_f = nullptr, *bt = nullptr;
-        // rows that may go through the one-query-per-CTA attention kernel
-        const uint32_t A = C < kPrefillChunk ? C : kPrefillChunk;
-        if (N > 1) {
-            float *base = r->ctx->tp_peer_base[r->ctx->tp_rank];
-            r->pf_x = base + r->xb_x;
-            r->pf_att = base + r->xb_att;
-            r->pf_gate = base + r->xb_gate;
-            r->pf_up = base + r->xb_up;
-            if ((rc = alloc(4, &bt))) return rc;
-            r->d_btick = (uint32_t *)bt;
-        } else if ((rc = alloc((size_t)C * dim, &r->pf_x)) || (rc = alloc((size_t)C * qdim, &r->pf_att)) ||
-                   (rc = alloc((size_t)C * ff, &r->pf_gate)) || (rc = alloc((size_t)C * ff, &r->pf_up))) {
-            return rc;
-        }
-        if ((rc = alloc((size_t)C * (qdim / N), &r->pf_q)) || (rc = alloc((size_t)C * (kvdim / N), &r->pf_k)) ||
-            (rc = alloc((size_t)C * (kvdim / N), &r->pf_v)) || (rc = alloc(C > c.max_seq_len ? C : c.max_seq_len, &tok_f)) ||
-            (rc = alloc((size_t)A * c.n_heads, &tick_f)) ||
-            (rc = alloc((size_t)A * attn_scratch_floats(c.n_heads / N, r->pf_splits, hd) + 4, &r->pf_attn_scratch)) ||
-            (rc = alloc((size_t)kRowsMatvecMax * dim, &r->pf_norm)))
-            return rc;
-        r->pf_tokens = (uint32_t *)tok_f;
-        r->pf_tickets = (uint32_t *)tick_f;  // zero-filled by the allocator; the kernel leaves them at zero
-        r->pf_chunk = C;
+        return e;
+    };
+    r->pf_splits = c.max_seq_len / 1024 < 1 ? 1 : (c.max_seq_len / 1024 > 8 ? 8 : c.max_seq_len / 1024);
+    float *tok_f = nullptr, *tick_f = nullptr, *bt = nullptr;
+    // rows that may go through the one-query-per-CTA attention kernel
+    const uint32_t A = C < kPrefillChunk ? C : kPrefillChunk;
+    if (N > 1) {
+        float *base = r->ctx->tp_peer_base[r->ctx->tp_rank];
+        r->pf_x = base + r->xb_x;
+        r->pf_att = base + r->xb_att;
+        r->pf_gate = base + r->xb_gate;
+        r->pf_up = base + r->xb_up;
+        if ((rc = alloc(4, &bt))) return rc;
+        r->d_btick = (uint32_t *)bt;
+    } else if ((rc = alloc((size_t)C * dim, &r->pf_x)) || (rc = alloc((size_t)C * qdim, &r->pf_att)) ||
+               (rc = alloc((size_t)C * ff, &r->pf_gate)) || (rc = alloc((size_t)C * ff, &r->pf_up))) {
+        return rc;
     }
-    const uint32_t widest = ff > qdim ? (ff > dim ? ff : dim) : (qdim > dim ? qdim : dim);
-    if ((rc = ensure_gemm_scratch(r->ctx, qgemm_scratch_bytes(r->pf_chunk, widest)))) return rc;
-    return ensure_pinned(r, r->pf_chunk);
+    if ((rc = alloc((size_t)C * (qdim / N), &r->pf_q)) || (rc = alloc((size_t)C * (kvdim / N), &r->pf_k)) ||
+        (rc = alloc((size_t)C * (kvdim / N), &r->pf_v)) || (rc = alloc(C > c.max_seq_len ? C : c.max_seq_len, &tok_f)) ||
+        (rc = alloc((size_t)A * c.n_heads, &tick_f)) ||
+        (rc = alloc((size_t)A * attn_scratch_floats(c.n_heads / N, r->pf_splits, hd) + 4, &r->pf_attn_scratch)) ||
+        (rc = alloc((size_t)kRowsMatvecMax * dim, &r->pf_norm)) || (rc = ensure_pass_scratch(r, C)))
+        return rc;
+    r->pf_tokens = (uint32_t *)tok_f;
+    r->pf_tickets = (uint32_t *)tick_f;  // zero-filled by the allocator; the kernel leaves them at zero
+    r->pf_chunk = C;
+    return YULE_OK;
+}
+
+// Row buffers of the GEMM-driven paths (chunked prefill, batched decode), allocated on first use: of the basic chunk size, and
+// on one GPU replaced by ones of twice as many rows, and so on, when a pass of `rows` rows would fill them.  Where there is no
+// memory for those, passes stay at the chunk size (pf_chunk says what a pass may have).  Under tensor parallelism the
+// matrices that are gathered (x, attention output, gate, up) live in the exchange region, which every peer maps (its size is
+// fixed); q / k / v hold this rank's heads only.
+int32_t ensure_chunk_buffers(yule_cuda_runner *r, uint32_t rows) {
+    const uint32_t basic = r->ctx->tp_world > 1 && prefill_chunk_size(r) > r->xb_rows ? r->xb_rows : prefill_chunk_size(r);
+    uint32_t C = basic;
+    if (r->ctx->tp_world <= 1)
+        while (C < rows) C *= 2;
+    size_t free_bytes = 0, total_bytes = 0;
+    if (C > r->pf_chunk && r->pf_chunk && r->pf_refused && C >= r->pf_refused) {
+        YULE_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+        if (free_bytes <= r->pf_refused_free) C = r->pf_chunk;  // no more memory than when it was refused
+    }
+    if (r->pf_chunk >= C) return ensure_pass_scratch(r, r->pf_chunk);
+    int32_t rc = drop_chunk_buffers(r);
+    if (rc == YULE_OK) rc = alloc_chunk_buffers(r, C);
+    if (rc == YULE_ERR_OUT_OF_MEMORY && C > basic) {
+        if ((rc = drop_chunk_buffers(r)) || (rc = alloc_chunk_buffers(r, basic))) {
+            drop_chunk_buffers(r);
+            return rc;
+        }
+        r->pf_refused = C;
+        YULE_CUDA_TRY(cudaMemGetInfo(&r->pf_refused_free, &total_bytes));
+    }
+    if (rc) drop_chunk_buffers(r);
+    return rc;
 }
 
 // One pass of `m` rows through every layer with one GEMM per linear: the body shared by the chunked prefill
@@ -1976,6 +2007,7 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
     uint32_t per_seq = (r->xchg || !prefill_max_rows() ? r->pf_chunk : prefill_max_rows()) / batch;  // prompt tokens of each sequence per pass
     per_seq = per_seq < 1 ? 1 : (per_seq > fed ? fed : per_seq);
     if (fed && (rc = ensure_chunk_buffers(r, per_seq * batch))) return rc;
+    if (fed && per_seq * batch > r->pf_chunk) per_seq = r->pf_chunk / batch;  // (a batch is no larger than the basic chunk)
     if ((rc = ensure_batch_graph(r))) return rc;
     // prompts to the device, pass by pass, the rows of a pass in the order of the sequences
     const size_t n_words = (size_t)batch * n_prompt;
