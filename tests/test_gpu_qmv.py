@@ -285,21 +285,26 @@ def test_dependent_chain_of_matvecs(backend, oracle):
         backend.free(h)
 
 
-@pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q6_K])
-@pytest.mark.parametrize("kernel", ["ring", "stream"])
-@pytest.mark.parametrize("n_rows,blocks_per_row", [(1, 1), (7, 2), (129, 22), (5632, 8), (2048, 22), (300, 56), (40000, 16)])
-def test_both_q4k_q6k_kernels(backend, oracle, monkeypatch, dtype, kernel, n_rows, blocks_per_row):
-    """The shared-memory-ring kernel (independent calls) and the register-streaming kernel (dependent chains)
-    are picked by what a call depends on; here each is forced in turn on the same inputs, prepared weights."""
-    monkeypatch.setenv("YULE_QMV_RING", "1" if kernel == "ring" else "0")
+@pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q5_K, DType.Q6_K, DType.Q8_0, DType.Q4_0])
+@pytest.mark.parametrize("chain", ["first", "dependent", "independent"])
+@pytest.mark.parametrize("n_rows,blocks_per_row", [(1, 1), (7, 2), (129, 22), (5632, 8), (2048, 22), (300, 56), (40000, 16), (600, 130), (7, 33)])
+def test_one_vector_schedules(backend, oracle, dtype, chain, n_rows, blocks_per_row):
+    """The one-vector kernel splits a call by what it depends on (independent calls overlap in half-size CTAs, three or two to an
+    SM, as long as their rows fit), by the number of tiles (one or two at a time) and by the length of the rows (several launches
+    over a part of the columns each, 130 blocks): a call by itself, one whose vector the call before it wrote, and
+    calls that nothing before them writes for."""
     n_cols = blocks_per_row * 256
     w, x = case(dtype, n_rows, n_cols, seed=300 + n_rows)
     wh, xh, oh = backend.upload(w), backend.upload(x), backend.allocate(n_rows * 4)
     backend.prepare_weights(wh, dtype, n_rows, n_cols)
-    for _ in range(3):  # the second and third calls are chained to their predecessor (late wait)
+    if chain == "dependent":
+        first, v = synth.random_quantized(DType.Q4_K, 77, n_cols * 256), synth.normal(78, 256)
+        fh, vh = backend.upload(first), backend.upload(v)
+        backend.quantized_matmul(fh, vh, xh, n_cols, 256, DType.Q4_K)
+    for _ in range(4 if chain == "independent" else 1):
         backend.quantized_matmul(wh, xh, oh, n_rows, n_cols, dtype)
-    y = backend.download(oh, n_rows)
-    for h in (wh, xh, oh):
+    y, x = backend.download(oh, n_rows), backend.download(xh, n_cols)
+    for h in (wh, xh, oh) + ((fh, vh) if chain == "dependent" else ()):
         backend.free(h)
     ref = oracle.qmv(int(dtype), w, x, n_rows, n_cols, simd=oracle.SCALAR)
     assert guarded_rel_err(y, ref) <= REL_TOL

@@ -18,15 +18,15 @@
 //   fewer MMAs (8 instead of 32 per 4096 Q4_K weights) and fewer unpacking ops (3 instead of 5 per word) both count:
 //   the fp16 formulation this replaced was bound by the two at 0.64 of the copy bandwidth on a 128256x4096 matrix.
 //
-// Schedule.  16 warps that multiply and one that copies; one CTA per SM, whose shared memory holds the digits of x and a ring
+// Schedule.  16 warps that multiply and one that copies (8 and one for independent calls, see launch_sized); one CTA per SM, whose shared memory holds the digits of x and a ring
 // of weight stages (tiled TMA copies, the first ones issued before `griddepcontrol.wait`).  A stage is two boxes of 16
 // rows x 2048 columns, one 256-column block per warp: two neighbouring column ranges of one 16-row tile, or the same
 // columns of two tiles (of gate and up for a pair), whichever leaves fewer warps idle.  Units of one or two tiles are
 // dealt round-robin.  Row sums meet in shared memory; the warps take turns finishing units (one named barrier per unit in
 // flight, only the finishing warp waits on it, and a warp whose copy never came).  Rows longer than the image of x may be are several launches over a
 // part of the columns each, every one adding to the result of the one before.
-//   Two launches side by side on an SM (half the shared memory each) were tried: the hardware puts two CTAs of one launch
-// on an SM as soon as there is room, 148 CTAs landed on 74 to 97 SMs, and a chain of launches took 1.3 times as long.
+//   In a chain of dependent launches two CTAs of 16 warps to an SM (half the shared memory each) were tried: the hardware puts two
+// CTAs of one launch on an SM as soon as there is room, 148 CTAs landed on 74 to 97 SMs, and the chain took 1.3 times as long.
 //
 // Folded in: RMSNorm of x (the 1/rms factor multiplies the finished rows), up to three matrices that share x, SiLU(gate)·up
 // of a pair, the residual, and under tensor parallelism the (value, epoch) pairs of the exchange.
@@ -45,13 +45,16 @@ namespace {
 #include "ring_common.cuh"
 #include "tp_pairs.cuh"
 
-constexpr int kWarpsCta = 16;                  // warps that multiply
-constexpr int kMulThreads = kWarpsCta * 32;
-constexpr int kThreads = kMulThreads + 32;     // and the one that issues the copies
+// Warps that multiply, W: 16, or 8 in CTAs of half the size; and one that issues the copies.
+__host__ __device__ constexpr int mul_threads(int w) { return w * 32; }
+__host__ __device__ constexpr int cta_threads(int w) { return w * 32 + 32; }
+// CTAs that registers leave room for on an SM
+__host__ __device__ constexpr int ctas_per_sm(int w) { return w == 8 ? 3 : 1; }
 constexpr int kTileRows = 16;
 constexpr uint32_t kMaxSlots = 8;        // ring slots
 constexpr uint32_t kMaxFinish = 8;       // tiles whose sums may be waiting for their finishing warp
-constexpr size_t kMaxSmem = 200 * 1024;   // leaves room for a CTA of the small kernels of a chain beside this one
+// Shared memory of a CTA where `share` of them are to fit on an SM (one: leaves room for a CTA of the small kernels of a chain)
+__host__ __device__ constexpr size_t max_smem(uint32_t share) { return (share == 3 ? 72 : share == 2 ? 110 : 200) * (size_t)1024; }
 
 enum : int { kQ4K, kQ5K, kQ6K, kQ8, kQ4 };
 
@@ -69,7 +72,6 @@ struct Fmt {
     static constexpr uint32_t kQhOff = kTileRows * kQlPitch, kScOff = kQhOff + kTileRows * kQhPitch, kDOff = kScOff + kTileRows * kScPitch;
     static constexpr uint32_t kBoxBytes = F == kQ6K ? kDOff + kTileRows * kDPitch : kCopies * kTileRows * kPitch;
     static_assert(kBoxBytes % 128 == 0, "boxes stay 128-byte aligned");
-    static constexpr uint32_t kStageBytes = 2 * kBoxBytes;
     static constexpr uint32_t kGroupCols = F == kQ6K ? 16 : 32;           // columns that share a scale
 };
 
@@ -100,16 +102,18 @@ struct Smem {
     uint64_t *bars;       // full[kMaxSlots], empty[kMaxSlots]
 };
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
-template <int F>
+template <int F, int W>
+constexpr uint32_t kStageBytes = W / 8 * Fmt<F>::kBoxBytes;
+template <int F, int W>
 __host__ __device__ inline size_t fixed_bytes(uint32_t n_cols, uint32_t finish, uint32_t nq) {
     return (size_t)n_cols * 4 + align16((size_t)(n_cols / 128) * 4) + align16((size_t)(n_cols / Fmt<F>::kGroupCols) * 4) + 64 + 16 +
-           (size_t)finish * nq * kWarpsCta * kTileRows * 4 + 2 * kMaxSlots * 8;
+           (size_t)finish * nq * W * kTileRows * 4 + 2 * kMaxSlots * 8;
 }
-template <int F>
+template <int F, int W>
 __device__ __forceinline__ Smem carve(unsigned char *base, uint32_t n_cols, uint32_t slots, uint32_t finish, uint32_t nq) {
     Smem s;
     s.ring = base;
-    size_t off = (size_t)slots * Fmt<F>::kStageBytes;
+    size_t off = (size_t)slots * kStageBytes<F, W>;
     s.img = base + off;
     off += (size_t)n_cols * 4;
     s.f = reinterpret_cast<float *>(base + off);
@@ -121,7 +125,7 @@ __device__ __forceinline__ Smem carve(unsigned char *base, uint32_t n_cols, uint
     s.inv = reinterpret_cast<float *>(base + off);
     off += 16;
     s.part = reinterpret_cast<float *>(base + off);
-    off += (size_t)finish * nq * kWarpsCta * kTileRows * 4;
+    off += (size_t)finish * nq * W * kTileRows * 4;
     s.bars = reinterpret_cast<uint64_t *>(base + off);
     return s;
 }
@@ -387,20 +391,22 @@ __device__ __forceinline__ void put8(const Smem &sm, uint32_t c, const float (&a
     if ((threadIdx.x & 15) == 0) sm.f[c >> 7] = eb == 0xFF ? __uint_as_float(0x7FC00000u) : __uint_as_float((el - 29u) << 23);  // 2^(E − 29)
 }
 
-template <int F, bool TP>
-__global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_constant__ DigitsParams<F> p) {
+template <int F, bool TP, int W>
+__global__ void __launch_bounds__(cta_threads(W), ctas_per_sm(W)) qmv_digits_kernel(const __grid_constant__ DigitsParams<F> p) {
     using S = Fmt<F>;
+    constexpr int kBoxes = W / 8;  // boxes per stage
+    constexpr uint32_t kStage = kStageBytes<F, W>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     yule_pdl_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const bool two = p.two_tiles != 0;
-    const uint32_t bpr = p.n_cols / 256, chunk_blocks = two ? S::kBoxBlocks : 2 * S::kBoxBlocks, chunks = (bpr + chunk_blocks - 1) / chunk_blocks;
+    const bool two = kBoxes == 2 && p.two_tiles != 0;
+    const uint32_t bpr = p.n_cols / 256, chunk_blocks = two ? S::kBoxBlocks : kBoxes * S::kBoxBlocks, chunks = (bpr + chunk_blocks - 1) / chunk_blocks;
     const uint32_t nq = p.pair && !two ? 2 : 1;
     const uint32_t first = blockIdx.x, stride = gridDim.x;
     const uint32_t my_units = (p.n_units - first + stride - 1) / stride;  // the grid never exceeds the units
     const uint32_t slots = p.slots;
-    const Smem sm = carve<F>(smem_raw, p.n_cols, slots, p.finish, nq);
+    const Smem sm = carve<F, W>(smem_raw, p.n_cols, slots, p.finish, nq);
     const uint32_t bar_full = smem_u32(sm.bars), bar_empty = bar_full + 8 * kMaxSlots;
     volatile uint32_t *gave_up = reinterpret_cast<volatile uint32_t *>(sm.inv + 1);
 
@@ -425,13 +431,13 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
         return two ? (p.pair || 2 * (first + k * stride) + 1 < p.n_tiles) : c * chunk_blocks + S::kBoxBlocks < bpr;
     };
 
-    if (warp == kWarpsCta) {
+    if (warp == W) {
         // ── the copying warp (one thread) ──
         if (lane == 0) {
             *gave_up = 0;
             for (uint32_t i = 0; i < slots; i++) {
                 mbar_init(bar_full + 8 * i, 1);
-                mbar_init(bar_empty + 8 * i, kWarpsCta);
+                mbar_init(bar_empty + 8 * i, W);
             }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -444,12 +450,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
                 if (two && box_live(k, 0, 1)) row[1] = locate(k, q, 1, seg[1]) * kTileRows;
             }
             const uint32_t bar = bar_full + 8 * slot;
-            const bool both = box_live(k, c, 1);
-            mbar_arrive_expect_tx(bar, both ? S::kStageBytes : S::kBoxBytes);
+            const bool both = kBoxes == 2 && box_live(k, c, 1);
+            mbar_arrive_expect_tx(bar, both ? kStage : S::kBoxBytes);
 #pragma unroll
-            for (int box = 0; box < 2; box++) {
+            for (int box = 0; box < kBoxes; box++) {
                 if (box == 1 && !both) break;
-                const uint32_t dst = ring_u32 + slot * S::kStageBytes + box * S::kBoxBytes;
+                const uint32_t dst = ring_u32 + slot * kStage + box * S::kBoxBytes;
                 const uint32_t blk = p.col0 / 256 + c * chunk_blocks + (two ? 0 : box * S::kBoxBlocks);
                 auto copy = [&](int plane, uint32_t to, uint32_t x) {
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(to),
@@ -505,7 +511,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
             *reinterpret_cast<float4 *>(a) = *reinterpret_cast<const float4 *>(p.x + c);
             *reinterpret_cast<float4 *>(a + 4) = *reinterpret_cast<const float4 *>(p.x + c + 4);
         };
-        for (uint32_t c = threadIdx.x * 8; c < p.n_cols; c += kMulThreads * 8) {  // n_cols is a multiple of 256: whole warps are in or out
+        for (uint32_t c = threadIdx.x * 8; c < p.n_cols; c += mul_threads(W) * 8) {  // n_cols is a multiple of 256: whole warps are in or out
             float a[8];
             load8(p.col0 + c, a);
             if (p.norm_w) {
@@ -522,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
         }
         if (p.norm_w) {
             if (p.n_cols < p.full_cols)  // the columns of other launches count for the norm too
-                for (uint32_t c = threadIdx.x * 8; c < p.full_cols; c += kMulThreads * 8)
+                for (uint32_t c = threadIdx.x * 8; c < p.full_cols; c += mul_threads(W) * 8)
                     if (c < p.col0 || c >= p.col0 + p.n_cols) {
                         float a[8];
                         load8(c, a);
@@ -540,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
         if (p.norm_w) {
             float ss = 0.f;
 #pragma unroll
-            for (int i = 0; i < kWarpsCta; i++) ss += sm.red[i];
+            for (int i = 0; i < W; i++) ss += sm.red[i];
             inv = 1.0f / sqrtf(ss / (float)p.full_cols + p.eps);  // as the CPU runner forms it (model_runner.rs:254-258)
         }
         *sm.inv = inv;  // read by finishing warps, behind a barrier that this warp passes first
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
     bool dead = false;
     uint32_t slot = 0, phase = 0, buf = 0, bar_id = 1;
     for (uint32_t k = 0; k < my_units; k++) {
-        float *part = sm.part + (size_t)(buf * nq) * (kWarpsCta * kTileRows);
+        float *part = sm.part + (size_t)(buf * nq) * (W * kTileRows);
         const bool mine = !two || box_live(k, 0, box);
         for (uint32_t q = 0; q < nq; q++) {
             Acc acc;
@@ -569,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
                     *gave_up = 1;
                 }
                 if (blk < bpr && mine) {
-                    const unsigned char *r0 = r_base + slot * S::kStageBytes;
+                    const unsigned char *r0 = r_base + slot * kStage;
                     if constexpr (F == kQ6K)
                         consume_q6k(r0, local, blk, g, t, lv, sm, b, acc);
                     else if constexpr (F == kQ4K || F == kQ5K)
@@ -590,29 +596,29 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
             v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
             v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
             if (t == 0) {
-                float *to = part + q * (kWarpsCta * kTileRows) + warp * kTileRows + g;
+                float *to = part + q * (W * kTileRows) + warp * kTileRows + g;
                 to[0] = v0;
                 to[8] = v1;
             }
         }
         // the sums of unit k are parked; its finishing warp adds them up and stores
-        const bool finishes = (k & (kWarpsCta - 1)) == warp;
+        const bool finishes = (k & (W - 1)) == warp;
         // A warp that has given up keeps its place at the barriers, but the ring no longer holds it back: it waits for the others at
         // every unit, or it could arrive a second time at a barrier that a slower warp has yet to reach, whose phase would then be
         // over without that warp, and its wait never.  (For the same reason there is one barrier more than there are buffers: the
         // unit at which it gives up is one further on than the ring would have let it come.)
         dead = __any_sync(0xffffffffu, dead);
         if (finishes || dead)
-            asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kMulThreads) : "memory");
+            asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(mul_threads(W)) : "memory");
         else
-            asm volatile("bar.arrive %0, %1;" ::"r"(bar_id), "n"(kMulThreads) : "memory");
+            asm volatile("bar.arrive %0, %1;" ::"r"(bar_id), "n"(mul_threads(W)) : "memory");
         if (finishes) {
-            const uint32_t rr = lane & 15, half = lane >> 4;  // half: the warps of box 0 or 1
+            const uint32_t rr = lane & 15, half = lane >> 4;  // half: of the warps (two tiles: those of box 0 or 1)
             auto collect = [&](uint32_t q) {
-                const float *src = part + q * (kWarpsCta * kTileRows) + half * (8 * kTileRows) + rr;
+                const float *src = part + q * (W * kTileRows) + half * (W / 2 * kTileRows) + rr;
                 float s = 0.f;  // fixed order over the warps: deterministic
 #pragma unroll
-                for (int w = 0; w < 8; w++) s += src[w * kTileRows];
+                for (int w = 0; w < W / 2; w++) s += src[w * kTileRows];
                 return s * *sm.inv;
             };
             float v = collect(0), other = __shfl_xor_sync(0xffffffffu, v, 16);
@@ -645,9 +651,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_digits_kernel(const __grid_co
         }
 }
 
-template <int F, bool TP>
+template <int F, bool TP, int W>
 cudaError_t launch_variant(const DigitsParams<F> &p, uint32_t grid, size_t smem, bool pdl, cudaStream_t s) {
-    auto kern = qmv_digits_kernel<F, TP>;
+    auto kern = qmv_digits_kernel<F, TP, W>;
     static bool attr_done[64] = {};  // the opt-in for large dynamic shared memory belongs to the device
     static std::mutex mu;
     int dev = 0;
@@ -656,16 +662,16 @@ cudaError_t launch_variant(const DigitsParams<F> &p, uint32_t grid, size_t smem,
     {
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem(W == 8 ? 2 : 1));
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 64) attr_done[dev] = true;
         }
     }
-    return launch_kernel(kern, dim3(grid), dim3(kThreads), smem, s, pdl, p);
+    return launch_kernel(kern, dim3(grid), dim3(cta_threads(W)), smem, s, pdl, p);
 }
 
-template <int F>
-cudaError_t launch_format(const QmvDigits &f, int sm_count, cudaStream_t s, uint64_t *launches) {
+template <int F, int W>
+cudaError_t launch_format(const QmvDigits &f, int sm_count, uint32_t share, cudaStream_t s, uint64_t *launches) {
     using S = Fmt<F>;
     DigitsParams<F> p = {};
     const uint32_t full_bpr = f.n_cols / 256;
@@ -700,10 +706,10 @@ cudaError_t launch_format(const QmvDigits &f, int sm_count, cudaStream_t s, uint
     p.status = f.status;
     p.wait_cycles = f.wait_cycles;
     p.tp = f.tp;
-    // Parts of the columns, in whole boxes of eight blocks: as few as leave room for two ring slots, of equal size.
+    // Parts of the columns, in whole boxes of eight blocks: as few as leave room for two ring slots, of equal size (half-size CTAs: one part).
     const uint32_t units8 = (full_bpr + 7) / 8;
     uint32_t n_parts = 1;
-    while (n_parts < units8 && 2 * (size_t)S::kStageBytes + fixed_bytes<F>((units8 + n_parts - 1) / n_parts * 2048, 3, 2) > kMaxSmem) n_parts++;
+    while (W == 16 && n_parts < units8 && 2 * (size_t)kStageBytes<F, W> + fixed_bytes<F, W>((units8 + n_parts - 1) / n_parts * 2048, 3, 2) > max_smem(share)) n_parts++;
     if (f.swiglu_pair && n_parts > 1) return cudaErrorInvalidValue;
     for (uint32_t part = 0, unit0 = 0; part < n_parts; part++) {
         const uint32_t unit1 = (uint32_t)((uint64_t)units8 * (part + 1) / n_parts);
@@ -713,17 +719,17 @@ cudaError_t launch_format(const QmvDigits &f, int sm_count, cudaStream_t s, uint
         p.n_cols = bpr * 256;
         // One tile per unit (sixteen blocks of a row per stage) or two (eight of each)?  The time of a CTA goes with its
         // number of stages; with few tiles two per unit would leave SMs without work.
-        const uint32_t chunks1 = (bpr + 15) / 16, chunks2 = (bpr + 7) / 8;
+        const uint32_t chunks1 = (bpr + W - 1) / W, chunks2 = (bpr + 7) / 8;
         const uint32_t units1 = n_tiles * (f.swiglu_pair ? 2 : 1), units2 = f.swiglu_pair ? n_tiles : (n_tiles + 1) / 2;
-        auto rounds = [&](uint32_t units) { return (units + sm_count - 1) / sm_count; };
+        const uint32_t ctas = (uint32_t)sm_count * share;
+        auto rounds = [&](uint32_t units) { return (units + ctas - 1) / ctas; };
         const uint32_t rounds1 = f.swiglu_pair ? 2 * rounds(n_tiles) : rounds(units1);
-        p.two_tiles = rounds(units2) * chunks2 < rounds1 * chunks1 ? 1u : 0u;
+        p.two_tiles = W == 16 && rounds(units2) * chunks2 < rounds1 * chunks1 ? 1u : 0u;
         p.n_units = p.two_tiles ? units2 : n_tiles;
         const uint32_t nq = f.swiglu_pair && !p.two_tiles ? 2 : 1, chunks = p.two_tiles ? chunks2 : chunks1;
-        const uint32_t grid = p.n_units < (uint32_t)sm_count ? p.n_units : (uint32_t)sm_count;
+        const uint32_t grid = p.n_units < ctas ? p.n_units : ctas;
         const uint32_t need = (p.n_units + grid - 1) / grid * nq * chunks;
-        // A part after the first waits for the whole of the one before, whose result it adds to.
-        p.late_wait = f.pdl && f.late_wait && n_parts == 1 ? 1u : 0u;
+        p.late_wait = f.pdl && f.late_wait ? 1u : 0u;  // (a part after the first reads the result of the one before, behind the wait)
         p.accumulate = part > 0 ? 1u : 0u;
         p.residual = part == 0 ? f.residual : nullptr;
         // Ring slots: what fits beside the image, no more than will be used.
@@ -731,24 +737,47 @@ cudaError_t launch_format(const QmvDigits &f, int sm_count, cudaStream_t s, uint
         size_t smem;
         for (;; slots--) {
             finish = 2 + (slots - 1 + nq * chunks - 1) / (nq * chunks);  // the finishing warp of a unit may lag behind a warp a whole ring ahead
-            smem = (size_t)slots * S::kStageBytes + fixed_bytes<F>(p.n_cols, finish, nq);
-            if (slots == 1 || (finish <= kMaxFinish && slots <= need && smem <= kMaxSmem)) break;
+            smem = (size_t)slots * kStageBytes<F, W> + fixed_bytes<F, W>(p.n_cols, finish, nq);
+            if (slots == 1 || (finish <= kMaxFinish && slots <= need && smem <= max_smem(share))) break;
         }
-        if (smem > kMaxSmem) return cudaErrorInvalidValue;
+        if (smem > max_smem(share)) return cudaErrorInvalidValue;
         p.slots = slots;
         p.finish = finish;
         p.tp.push = f.tp.push && part + 1 == n_parts;
         const bool tp = p.tp.push || f.tp.wait;
         const bool pdl = f.pdl || part > 0;  // a part reads its weights early, everything else after its wait
         cudaError_t e;
-        if constexpr (F == kQ4K)
-            e = tp ? launch_variant<F, true>(p, grid, smem, pdl, s) : launch_variant<F, false>(p, grid, smem, pdl, s);
+        if constexpr (F == kQ4K && W == 16)
+            e = tp ? launch_variant<F, true, W>(p, grid, smem, pdl, s) : launch_variant<F, false, W>(p, grid, smem, pdl, s);
         else
-            e = tp ? cudaErrorInvalidValue : launch_variant<F, false>(p, grid, smem, pdl, s);  // the exchange is built for Q4_K only
+            e = tp ? cudaErrorInvalidValue : launch_variant<F, false, W>(p, grid, smem, pdl, s);  // the exchange is built for Q4_K only
         if (e != cudaSuccess) return e;
         *launches += 1;
     }
     return cudaSuccess;
+}
+
+// A call whose inputs nothing before it writes overlaps with the calls before it, if an SM has room for CTAs of several: then the
+// start of one, its image of x and its last sums run under the multiplying of the others.  So such calls take half-size CTAs, three
+// to an SM where image and two ring slots fit a third of its shared memory, else two.  Not for rows of more than 8192 columns, whose
+// image costs more than the overlap gives, and two to an SM not where a CTA has more than eight stages, which two slots do
+// not keep fed.  us per independent call, 16-warp CTAs against these: Q4_K 2048x2048 2.26, 0.95, 5632x2048 3.29, 2.30, 14336x4096
+// 9.1, 6.7, 28672x8192 23.3, 22.7; Q8_0 2048x2048 2.45, 1.14; two to an SM Q6_K 14336x4096 11.3, 9.5, Q8_0 4096x4096 4.5, 3.4;
+// beyond the lines Q4_K 4096x14336 7.2, 8.6, Q5_K 28672x8192 27.7, 29.7.
+template <int F>
+cudaError_t launch_sized(const QmvDigits &f, int sm_count, cudaStream_t s, uint64_t *launches) {
+    if (f.pdl && f.late_wait && f.n_cols <= 8192 && !f.tp.push && !f.tp.wait) {
+        uint32_t n_tiles = 0;
+        for (uint32_t i = 0; i < (f.swiglu_pair ? 1 : f.n_seg); i++) n_tiles += (f.rows[i] + kTileRows - 1) / kTileRows;
+        const uint32_t nq = f.swiglu_pair ? 2 : 1;
+        for (uint32_t share = 3; share > 1; share--) {
+            const uint32_t ctas = (uint32_t)sm_count * share, stages = (n_tiles + ctas - 1) / ctas * nq * ((f.n_cols / 256 + 7) / 8);
+            if (share == 2 && stages > 8) break;
+            if ((stages > 1 ? 2 : 1) * (size_t)kStageBytes<F, 8> + fixed_bytes<F, 8>(f.n_cols, 3, nq) <= max_smem(share))
+                return launch_format<F, 8>(f, sm_count, share, s, launches);
+        }
+    }
+    return launch_format<F, 16>(f, sm_count, 1, s, launches);
 }
 
 }  // namespace
@@ -766,11 +795,11 @@ cudaError_t launch_qmv_digits(const QmvDigits &f, int sm_count, cudaStream_t s, 
     if (f.n_seg == 0 || f.n_seg > 3 || (reinterpret_cast<uintptr_t>(f.x) & 15)) return cudaErrorInvalidValue;
     if (f.swiglu_pair && (f.n_seg != 2 || !qmv_digits_can_pair(f.n_cols))) return cudaErrorInvalidValue;
     switch (f.type) {
-        case YULE_DTYPE_Q4_K: return launch_format<kQ4K>(f, sm_count, s, launches);
-        case YULE_DTYPE_Q5_K: return launch_format<kQ5K>(f, sm_count, s, launches);
-        case YULE_DTYPE_Q6_K: return launch_format<kQ6K>(f, sm_count, s, launches);
-        case YULE_DTYPE_Q8_0: return launch_format<kQ8>(f, sm_count, s, launches);
-        case YULE_DTYPE_Q4_0: return launch_format<kQ4>(f, sm_count, s, launches);
+        case YULE_DTYPE_Q4_K: return launch_sized<kQ4K>(f, sm_count, s, launches);
+        case YULE_DTYPE_Q5_K: return launch_sized<kQ5K>(f, sm_count, s, launches);
+        case YULE_DTYPE_Q6_K: return launch_sized<kQ6K>(f, sm_count, s, launches);
+        case YULE_DTYPE_Q8_0: return launch_sized<kQ8>(f, sm_count, s, launches);
+        case YULE_DTYPE_Q4_0: return launch_sized<kQ4>(f, sm_count, s, launches);
         default: return cudaErrorInvalidValue;
     }
 }
