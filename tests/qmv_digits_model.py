@@ -11,8 +11,8 @@ set and no copy lands any more; a warp that finds its stage missing gives up wai
 The sums of a unit meet at a named barrier: an arrival count that starts over when it is full, whoever arrived, and
 waits that have no bound; ``more_barriers`` than buffers, because a warp may give up one unit further on than the ring would
 let it come.  ``dead_waits``: a warp that gave up waits for the others at every unit (as the kernel has it), or
-(False) arrives and goes on, as a healthy one that does not finish the unit.  ``copier_checks``: the copying warp stops once
-somebody has given up; without it, it asks for a stage again whose last copy may still be on its way.
+(False) arrives and goes on, as a healthy one that does not finish the unit.  ``dead_keeps``: a warp that gave
+up releases no stage; where it does, the copying warp asks for a stage again whose last copy may still be on its way.
 
 Checks: sums are complete when they are added up and not overwritten before (runs without a failure), no barrier gets more
 arrivals than its phase takes, and everybody gets to the end."""
@@ -33,7 +33,7 @@ class Config:
     units: int = 12
     stages_per_unit: int = 1
     dead_waits: bool = True
-    copier_checks: bool = True
+    dead_keeps: bool = True
     more_barriers: int = 1
     fail_at: int | None = None
 
@@ -64,7 +64,6 @@ class State:
         self.added = [False] * cfg.units
         self.in_flight = []
         self.failed = False   # the status word
-        self.gave_up = False  # some warp has released a stage without waiting for it
 
 
 # What an agent yields is (condition, bounded): it goes on once the condition holds (sent True), or, if the wait is bounded
@@ -73,7 +72,7 @@ def copier(st: State):
     c = st.cfg
     for j in range(c.units * c.stages_per_unit):
         s, ph = j % c.slots, (j // c.slots) & 1
-        if not (yield (lambda: st.empty[s].test(ph ^ 1)), True) or (st.gave_up and c.copier_checks):
+        if not (yield (lambda: st.empty[s].test(ph ^ 1)), True):
             return
         st.full[s].arrive_expect_tx()
         st.in_flight.append(s)
@@ -97,8 +96,8 @@ def warp(st: State, w: int):
             j += 1
             if not dead:
                 dead = not (yield (lambda: st.full[s].test(ph)), True)
-                st.gave_up = st.gave_up or dead
-            st.empty[s].arrive()
+            if not (dead and c.dead_keeps):
+                st.empty[s].arrive()
             yield (lambda: True), False
         if not st.failed:
             if k >= c.finish and not st.added[k - c.finish]:

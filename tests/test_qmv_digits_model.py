@@ -1,6 +1,6 @@
 """The hand-off protocol of the one-vector matvec (yule_b200/csrc/qmv_digits.cu) on a model under random interleavings: with
 copies that arrive, and with copies that stop arriving.  The variants that go wrong then (a warp that gave up does not wait for
-the others; as many barriers as buffers; the copying warp goes on) must be caught, so that a green run means something."""
+the others; as many barriers as buffers; it releases its stages) must be caught, so that a green run means something."""
 
 import pytest
 
@@ -40,6 +40,6 @@ def test_model_catches_warps_that_run_ahead_and_too_few_buffers():
     assert any("deadlock" in why for _, why in failures(ahead, range(60)))
     as_many = Config(slots=4, finish=5, units=14, fail_at=150, more_barriers=0)
     assert any("deadlock" in why for _, why in failures(as_many, range(60)))
-    again = Config(slots=2, finish=3, units=12, fail_at=150, copier_checks=False)
+    again = Config(slots=2, finish=3, units=12, fail_at=150, dead_keeps=False)
     assert any("arrival beyond" in why for _, why in failures(again, range(60)))
     assert failures(Config(slots=6, finish=2, units=14), range(40))

@@ -97,7 +97,7 @@ struct Smem {
     unsigned char *img;   // digits of x: 4 bytes per column
     float *f, *sx;        // 2^-e per 128 columns; (offset constant ·) Σx per scale group
     float *red;           // sums of squares per warp
-    float *inv;           // 1/rms; behind it a word that a warp sets when it gives up waiting for a copy
+    float *inv;           // 1/rms
     float *part;          // [finish][matrix of a pair whose tiles go one by one][warp][row]
     uint64_t *bars;       // full[kMaxSlots], empty[kMaxSlots]
 };
@@ -408,7 +408,6 @@ __global__ void __launch_bounds__(cta_threads(W), ctas_per_sm(W)) qmv_digits_ker
     const uint32_t slots = p.slots;
     const Smem sm = carve<F, W>(smem_raw, p.n_cols, slots, p.finish, nq);
     const uint32_t bar_full = smem_u32(sm.bars), bar_empty = bar_full + 8 * kMaxSlots;
-    volatile uint32_t *gave_up = reinterpret_cast<volatile uint32_t *>(sm.inv + 1);
 
     // Tile `half` of unit k (q: matrix of a pair whose tiles go one by one): its matrix and its number there.
     auto locate = [&](uint32_t k, uint32_t q, uint32_t half, uint32_t &seg) {
@@ -434,7 +433,6 @@ __global__ void __launch_bounds__(cta_threads(W), ctas_per_sm(W)) qmv_digits_ker
     if (warp == W) {
         // ── the copying warp (one thread) ──
         if (lane == 0) {
-            *gave_up = 0;
             for (uint32_t i = 0; i < slots; i++) {
                 mbar_init(bar_full + 8 * i, 1);
                 mbar_init(bar_empty + 8 * i, W);
@@ -491,7 +489,6 @@ __global__ void __launch_bounds__(cta_threads(W), ctas_per_sm(W)) qmv_digits_ker
         if (lane == 0)
             while (n < total) {
                 if (!ring_wait(bar_empty + 8 * slot, phase ^ 1u, p.status, p.wait_cycles)) break;
-                if (*gave_up) break;  // the slot was released by a warp that did not wait for it: its copy may still be on its way
                 issue();
             }
         return;
@@ -569,11 +566,9 @@ __global__ void __launch_bounds__(cta_threads(W), ctas_per_sm(W)) qmv_digits_ker
             Acc acc;
             uint32_t blk = two ? local : warp;
             for (uint32_t c = 0; c < chunks; c++, blk += chunk_blocks) {
-                // A copy that never arrives: the lane waits for no other one, what the warp multiplies from here on means nothing.
-                if (!dead && !ring_wait(bar_full + 8 * slot, phase, p.status, p.wait_cycles)) {
-                    dead = true;
-                    *gave_up = 1;
-                }
+                // A copy that never arrives: the lane waits for no other one and releases no slot (whose copy may still be on its way);
+                // what the warp multiplies from here on means nothing.
+                if (!dead) dead = !ring_wait(bar_full + 8 * slot, phase, p.status, p.wait_cycles);
                 if (blk < bpr && mine) {
                     const unsigned char *r0 = r_base + slot * kStage;
                     if constexpr (F == kQ6K)
@@ -584,7 +579,7 @@ __global__ void __launch_bounds__(cta_threads(W), ctas_per_sm(W)) qmv_digits_ker
                         consume_q32<F == kQ8>(r0, blk, t, lv, sm, b, acc);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_empty + 8 * slot);
+                if (lane == 0 && !dead) mbar_arrive(bar_empty + 8 * slot);
                 if (++slot == slots) {
                     slot = 0;
                     phase ^= 1u;
