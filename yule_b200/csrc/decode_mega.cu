@@ -220,9 +220,8 @@ __device__ __forceinline__ uint4 ld_pairs2(const uint2 *p) {
 }
 
 // Builds the shared-memory image of x for one matvec phase from the (value, epoch) pairs of the vector, by the
-// whole CTA: optional RMSNorm, power-of-two normalisation, fp16 hi/lo split, per-sub-block sums — the arithmetic
-// of stage_activations in q4k_mma_common.cuh / q6k_ring_common.cuh, ordered for latency and for registers (this
-// kernel has 128 per thread and must not spill: behind its shared-memory carve-out L1 is tiny, a spill is an L2
+// whole CTA: optional RMSNorm, power-of-two normalisation, fp16 hi/lo split, per-sub-block sums, ordered for latency and for
+// registers (this kernel has 128 per thread and must not spill: behind its shared-memory carve-out L1 is tiny, a spill is an L2
 // round trip).  The norm weights (static) are requested before any waiting.  A thread's first 8 columns stay in
 // registers between the reduction and the conversion; further chunks (vectors longer than 4096) wait in shared
 // memory, in the 32 bytes of the image that the same thread later overwrites with their converted form.

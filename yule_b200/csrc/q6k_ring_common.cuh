@@ -36,120 +36,8 @@ __host__ __device__ inline size_t row_record_bytes(uint32_t bpr) { return (size_
 //   s32      −32 · Σx over each 16-column scale group (fp32);
 //   zb       zeros for lanes that feed an all-zero B column (and for the lanes that must not
 //            charge the −32 term a second time).
-struct XImage {
-    __half *xh, *xl;
-    float *s32;
-    uint4 *zb;
-    float *inv_scale;
-    float *red;
-};
-
 __host__ __device__ inline uint32_t padded_cols(uint32_t n_cols) { return n_cols + 8 * (n_cols / 128); }
 __host__ __device__ inline size_t x_plane_bytes(uint32_t n_cols) { return (((size_t)padded_cols(n_cols) * 2 + 127) / 128) * 128; }
-
-// RMSNorm (optional), power-of-two normalisation, fp16 hi/lo split and per-16-column sums of x, by the
-// whole CTA.  Each thread keeps its first kCache groups of 8 columns in registers between the reduction
-// pass and the conversion pass; longer vectors re-read the remainder from L2.
-// `load8(c, a)` fetches columns c..c+7 (plain loads in the matvec kernel, polled (value, epoch) pairs in the
-// persistent decode kernel).
-template <class Load8>
-__device__ __forceinline__ void stage_activations(const XImage &sm, Load8 load8, uint32_t n_cols, const float *__restrict__ norm_w,
-                                                  float eps) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int NW = kThreadsCta / 32;
-    constexpr int kCache = 2;
-    if (threadIdx.x < 4) sm.zb[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
-    float cache[kCache][8];
-    float ss = 0.f, mx = 0.f;
-    auto reduce8 = [&](uint32_t c, const float (&a)[8]) {
-        float gw[8];
-        if (norm_w) {
-            *reinterpret_cast<float4 *>(gw) = *reinterpret_cast<const float4 *>(norm_w + c);
-            *reinterpret_cast<float4 *>(gw + 4) = *reinterpret_cast<const float4 *>(norm_w + c + 4);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            ss = fmaf(a[i], a[i], ss);
-            mx = fmaxf(mx, fabsf(norm_w ? a[i] * gw[i] : a[i]));
-        }
-    };
-#pragma unroll
-    for (int k = 0; k < kCache; k++) {
-        const uint32_t c = (threadIdx.x + k * kThreadsCta) * 8;
-        if (c < n_cols) {
-            load8(c, cache[k]);
-            reduce8(c, cache[k]);
-        }
-    }
-    for (uint32_t c = (threadIdx.x + kCache * kThreadsCta) * 8; c < n_cols; c += kThreadsCta * 8) {
-        float a[8];
-        load8(c, a);
-        reduce8(c, a);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    if (lane == 0) {
-        sm.red[wid] = ss;
-        sm.red[32 + wid] = mx;
-    }
-    __syncthreads();
-    ss = 0.f;
-    mx = 0.f;
-#pragma unroll
-    for (int i = 0; i < NW; i++) {
-        ss += sm.red[i];
-        mx = fmaxf(mx, sm.red[32 + i]);
-    }
-    // RMSNorm scale as the CPU runner forms it: 1 / sqrt(ss / n + eps) (yule-infer/src/model_runner.rs:254-258)
-    const float inv_rms = norm_w ? 1.0f / sqrtf(ss / (float)n_cols + eps) : 1.0f;
-    mx *= inv_rms;
-    int eb = (int)((__float_as_uint(mx) >> 23) & 0xFFu);
-    if (mx == 0.f || eb == 0xFF) eb = 127 + 13;
-    int se = 127 + 13 - (eb - 127);
-    se = se < 1 ? 1 : (se > 253 ? 253 : se);
-    const float scale = __uint_as_float((uint32_t)se << 23);
-    if (threadIdx.x == 0) sm.inv_scale[0] = __uint_as_float((uint32_t)(254 - se) << 23);
-    auto convert8 = [&](uint32_t c, float (&a)[8]) {
-        if (norm_w) {
-            float gw[8];
-            *reinterpret_cast<float4 *>(gw) = *reinterpret_cast<const float4 *>(norm_w + c);
-            *reinterpret_cast<float4 *>(gw + 4) = *reinterpret_cast<const float4 *>(norm_w + c + 4);
-#pragma unroll
-            for (int i = 0; i < 8; i++) a[i] = a[i] * inv_rms * gw[i];
-        }
-        __half hi[8], lo[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            a[i] *= scale;
-            hi[i] = __float2half_rn(a[i]);
-            lo[i] = __float2half_rn(a[i] - __half2float(hi[i]));
-        }
-        const uint32_t pc = c + 8 * (c >> 7);
-        *reinterpret_cast<uint4 *>(sm.xh + pc) =
-            make_uint4(h2_as_u32(__halves2half2(hi[0], hi[1])), h2_as_u32(__halves2half2(hi[2], hi[3])),
-                       h2_as_u32(__halves2half2(hi[4], hi[5])), h2_as_u32(__halves2half2(hi[6], hi[7])));
-        *reinterpret_cast<uint4 *>(sm.xl + pc) =
-            make_uint4(h2_as_u32(__halves2half2(lo[0], lo[1])), h2_as_u32(__halves2half2(lo[2], lo[3])),
-                       h2_as_u32(__halves2half2(lo[4], lo[5])), h2_as_u32(__halves2half2(lo[6], lo[7])));
-        float s8 = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-        s8 += __shfl_xor_sync(0xffffffffu, s8, 1);  // two consecutive threads hold one 16-column group
-        if ((lane & 1) == 0) sm.s32[c >> 4] = -32.0f * s8;
-    };
-#pragma unroll
-    for (int k = 0; k < kCache; k++) {
-        const uint32_t c = (threadIdx.x + k * kThreadsCta) * 8;
-        if (c < n_cols) convert8(c, cache[k]);
-    }
-    for (uint32_t c = (threadIdx.x + kCache * kThreadsCta) * 8; c < n_cols; c += kThreadsCta * 8) {
-        float a[8];
-        load8(c, a);
-        convert8(c, a);
-    }
-    __syncthreads();
-}
 
 __device__ __forceinline__ uint32_t word4(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 

@@ -76,17 +76,12 @@ __device__ __forceinline__ float byte_to_float(uint32_t w) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + I)) - 8388608.0f;
 }
 
-constexpr int kMaxSegs = 3;  // matrices that share their activations (Q/K/V; gate/up) in one launch
 struct KBatchParams {
-    CUtensorMap map[kMaxSegs][4];  // per matrix — Q4_K: [0] = the raw tensor; Q6_K: the four planes of the row-planar copy
-    float *out[kMaxSegs];
-    uint32_t n_rows[kMaxSegs], out_stride[kMaxSegs];
-    uint32_t tile0[kMaxSegs + 1];  // first 16-row tile of each matrix in the launch's tile numbering; [n_seg] = n_tiles
-    uint32_t n_seg;
+    CUtensorMap map[4];  // Q4_K: [0] = the raw tensor; Q6_K: the four planes of the row-planar copy
+    float *out;
+    uint32_t n_rows, out_stride;
     const float *x;
-    const float *residual;  // added to the results of matrix 0 (single-matrix launches only)
-    const float *norm_w;    // RMSNorm prologue: the rows are x · inv_rms · norm_w (yule-infer/src/model_runner.rs:254-263), or null
-    float eps;
+    const float *residual;  // added to the results, or null
     uint32_t n_cols, n_tiles, stages, chunks;
     uint32_t nb, x_stride, late_wait;
     uint32_t blk_off;  // first super-block of the rows this launch covers (a launch takes a range of the columns)
@@ -136,9 +131,7 @@ __device__ __forceinline__ void issue_stage(const KBatchParams &p, uint32_t tile
     // Tiled copies by the first lane; every box is as wide as its plane's shared-memory row pitch (what lies beyond the
     // eight super-blocks is never read), rows past the end of the matrix arrive as zeros.
     if (lane == 0) {
-        uint32_t seg = 0;
-        while (seg + 1 < p.n_seg && tile >= p.tile0[seg + 1]) seg++;
-        const uint32_t row0 = (tile - p.tile0[seg]) * kStageRows, blk0 = p.blk_off + chunk * kStageBlocks;
+        const uint32_t row0 = tile * kStageRows, blk0 = p.blk_off + chunk * kStageBlocks;
         mbar_arrive_expect_tx(bar, stage_bytes<Q6>());
         auto box = [&](uint32_t off, const CUtensorMap *m, uint32_t x) {
             asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -147,12 +140,12 @@ __device__ __forceinline__ void issue_stage(const KBatchParams &p, uint32_t tile
                          : "memory");
         };
         if (Q6) {
-            box(kQlOff, &p.map[seg][0], blk0 * 16u);
-            box(kQhOff, &p.map[seg][1], blk0 * 8u);
-            box(kScOff, &p.map[seg][2], blk0 * 2u);
-            box(kDOff, &p.map[seg][3], blk0 / 4u);
+            box(kQlOff, &p.map[0], blk0 * 16u);
+            box(kQhOff, &p.map[1], blk0 * 8u);
+            box(kScOff, &p.map[2], blk0 * 2u);
+            box(kDOff, &p.map[3], blk0 / 4u);
         } else {
-            box(0, &p.map[seg][0], blk0 * 18u);
+            box(0, &p.map[0], blk0 * 18u);
         }
     }
     __syncwarp();
@@ -162,18 +155,14 @@ __device__ __forceinline__ void issue_stage(const KBatchParams &p, uint32_t tile
 // l the four columns 4l..4l+3; two CTA barriers (the per-vector power-of-two scales, then the finished image).
 // Returns 2^-e of vector `want`.
 __device__ __forceinline__ float stage_x(const KBatchSmem &sm, const float *__restrict__ x, uint32_t x_stride, uint32_t nb, uint32_t n_sg,
-                                         int lane, uint32_t want, const float *__restrict__ norm_w, float eps) {
+                                         int lane, uint32_t want) {
     constexpr int KC = 2;  // groups per vector kept in registers between the two passes (all of them up to 4096 columns)
     constexpr uint32_t kAllWarps = kGroups * kWarps;
     const uint32_t W = threadIdx.x >> 5;
     if (threadIdx.x < 64) reinterpret_cast<uint32_t *>(sm.zb)[threadIdx.x] = 0u;
     float4 cache[4][KC];
-    float mx[4] = {0.f, 0.f, 0.f, 0.f}, ss[4] = {0.f, 0.f, 0.f, 0.f};
-    // With the RMSNorm prologue the image holds x · inv_rms · w: max |x · w| and Σx² are reduced together, the
-    // vector's 1/rms enters the maximum afterwards.
-    auto wts = [&](uint32_t s) { return norm_w ? *reinterpret_cast<const float4 *>(norm_w + s * 128u + lane * 4u) : make_float4(1.f, 1.f, 1.f, 1.f); };
-    auto amax4 = [](float4 a, float4 g) { return fmaxf(fmaxf(fabsf(a.x * g.x), fabsf(a.y * g.y)), fmaxf(fabsf(a.z * g.z), fabsf(a.w * g.w))); };
-    auto sq4 = [](float4 a, float acc) { return fmaf(a.w, a.w, fmaf(a.z, a.z, fmaf(a.y, a.y, fmaf(a.x, a.x, acc)))); };
+    float mx[4] = {0.f, 0.f, 0.f, 0.f};
+    auto amax4 = [](float4 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))); };
 #pragma unroll
     for (int v = 0; v < 4; v++) {
         if ((uint32_t)v < nb) {
@@ -191,48 +180,26 @@ __device__ __forceinline__ float stage_x(const KBatchSmem &sm, const float *__re
             const float *xv = x + (size_t)v * x_stride;
 #pragma unroll
             for (int i = 0; i < KC; i++)
-                if (W + kAllWarps * i < n_sg) {
-                    mx[v] = fmaxf(mx[v], amax4(cache[v][i], wts(W + kAllWarps * i)));
-                    ss[v] = sq4(cache[v][i], ss[v]);
-                }
-            for (uint32_t s = W + kAllWarps * KC; s < n_sg; s += kAllWarps) {
-                const float4 a = *reinterpret_cast<const float4 *>(xv + s * 128u + lane * 4u);
-                mx[v] = fmaxf(mx[v], amax4(a, wts(s)));
-                ss[v] = sq4(a, ss[v]);
-            }
+                if (W + kAllWarps * i < n_sg) mx[v] = fmaxf(mx[v], amax4(cache[v][i]));
+            for (uint32_t s = W + kAllWarps * KC; s < n_sg; s += kAllWarps)
+                mx[v] = fmaxf(mx[v], amax4(*reinterpret_cast<const float4 *>(xv + s * 128u + lane * 4u)));
         }
     }
 #pragma unroll
     for (int v = 0; v < 4; v++)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mx[v] = fmaxf(mx[v], __shfl_xor_sync(0xffffffffu, mx[v], o));
-            ss[v] += __shfl_xor_sync(0xffffffffu, ss[v], o);
-        }
+        for (int o = 16; o > 0; o >>= 1) mx[v] = fmaxf(mx[v], __shfl_xor_sync(0xffffffffu, mx[v], o));
     float4 *red = reinterpret_cast<float4 *>(sm.red);
-    if (lane == 0) {
-        red[W] = make_float4(mx[0], mx[1], mx[2], mx[3]);
-        red[kAllWarps + W] = make_float4(ss[0], ss[1], ss[2], ss[3]);
-    }
+    if (lane == 0) red[W] = make_float4(mx[0], mx[1], mx[2], mx[3]);
     __syncthreads();
-    float inv_rms[4] = {1.f, 1.f, 1.f, 1.f};
     {
-        float4 m = red[0], q = red[kAllWarps];
+        float4 m = red[0];
 #pragma unroll
         for (uint32_t w = 1; w < kAllWarps; w++) {
-            const float4 o = red[w], o2 = red[kAllWarps + w];
+            const float4 o = red[w];
             m.x = fmaxf(m.x, o.x), m.y = fmaxf(m.y, o.y), m.z = fmaxf(m.z, o.z), m.w = fmaxf(m.w, o.w);
-            q.x += o2.x, q.y += o2.y, q.z += o2.z, q.w += o2.w;
         }
         mx[0] = m.x, mx[1] = m.y, mx[2] = m.z, mx[3] = m.w;
-        if (norm_w) {
-            // 1 / sqrt(Σx² / n + eps), as the CPU runner forms it (model_runner.rs:254-258)
-            const float n = (float)(n_sg * 128u);
-            inv_rms[0] = 1.0f / sqrtf(q.x / n + eps), inv_rms[1] = 1.0f / sqrtf(q.y / n + eps);
-            inv_rms[2] = 1.0f / sqrtf(q.z / n + eps), inv_rms[3] = 1.0f / sqrtf(q.w / n + eps);
-#pragma unroll
-            for (int v = 0; v < 4; v++) mx[v] *= inv_rms[v];
-        }
     }
     float scale[4], inv_want = 1.f;
 #pragma unroll
@@ -247,11 +214,6 @@ __device__ __forceinline__ float stage_x(const KBatchSmem &sm, const float *__re
     }
     const uint32_t chunk_bytes = nb * 64u;
     auto convert = [&](uint32_t s, uint32_t v, float4 a, float sc) {
-        if (norm_w) {
-            const float4 g = wts(s);
-            const float ir = inv_rms[v];
-            a.x = a.x * ir * g.x, a.y = a.y * ir * g.y, a.z = a.z * ir * g.z, a.w = a.w * ir * g.w;
-        }
         a.x *= sc;  // exact (power of two)
         a.y *= sc;
         a.z *= sc;
@@ -444,7 +406,7 @@ qmv_kquant_batch_kernel(const __grid_constant__ KBatchParams p) {
 
     if (!p.late_wait) yule_pdl_wait();  // the activations (and the residual) come from the previous kernel
     const uint32_t tid = threadIdx.x & (kWarps * 32 - 1);
-    const float inv_scale = stage_x(sm, p.x, p.x_stride, nb, p.n_cols / 128, lane, tid >> 4, p.norm_w, p.eps);
+    const float inv_scale = stage_x(sm, p.x, p.x_stride, nb, p.n_cols / 128, lane, tid >> 4);
     if (total == 0) return;
 
     // B column n = g carries vector g / 2 (hi for even g, lo for odd); columns past 2·nb read zeros
@@ -502,15 +464,12 @@ qmv_kquant_batch_kernel(const __grid_constant__ KBatchParams p) {
                 const uint32_t v = tid >> 4, rr = tid & 15u;
                 float sacc = 0.f;
                 for (uint32_t w2 = 0; w2 < n_warps_used; w2++) sacc += part[w2 * 64 + rr * 4 + v];
-                const uint32_t tile = first_tile + ck * tile_stride;
-                uint32_t seg = 0;
-                while (seg + 1 < p.n_seg && tile >= p.tile0[seg + 1]) seg++;
-                const uint32_t row = (tile - p.tile0[seg]) * kStageRows + rr;
-                if (row < p.n_rows[seg]) {
+                const uint32_t row = (first_tile + ck * tile_stride) * kStageRows + rr;
+                if (row < p.n_rows) {
                     sacc = (sacc * 16777216.0f) * inv_scale;
-                    const size_t o = (size_t)v * p.out_stride[seg] + row;
+                    const size_t o = (size_t)v * p.out_stride + row;
                     if (p.residual) sacc += p.residual[o];
-                    p.out[seg][o] = sacc;
+                    p.out[o] = sacc;
                 }
             }
             cc = 0;
@@ -534,46 +493,34 @@ uint32_t batch_stages(bool q6, uint32_t n_cols, uint32_t nb) {
     return st > (size_t)kMaxStages ? (uint32_t)kMaxStages : (uint32_t)st;
 }
 
-// One launch over the columns [256·blk_off, 256·blk_off + part_cols) of every row of `n_seg` matrices that share their
-// activations (same type, columns, vectors); `residual` is added to the results (single matrix only).
+// One launch over the columns [256·blk_off, 256·blk_off + part_cols) of every row; `residual` is added to the results.
 template <bool Q6>
-cudaError_t launch_variant(const QmvArgs *segs, uint32_t n_seg, uint32_t nb, uint32_t stages, uint32_t blk_off, uint32_t part_cols,
-                           const float *residual, int sm_count, cudaStream_t s) {
-    const QmvArgs &a = segs[0];
+cudaError_t launch_variant(const QmvArgs &a, uint32_t nb, uint32_t stages, uint32_t blk_off, uint32_t part_cols, const float *residual, int sm_count,
+                           cudaStream_t s) {
     KBatchParams p = {};
     const uint32_t bpr = a.n_cols / 256;
-    p.n_seg = n_seg;
-    uint32_t tiles = 0;
-    for (uint32_t i = 0; i < n_seg; i++) {
-        const QmvArgs &g = segs[i];
-        if (Q6) {
-            const uint64_t rec = row_record_bytes(bpr);
-            const uint64_t off[4] = {0, (uint64_t)bpr * 128, (uint64_t)bpr * 192, (uint64_t)bpr * 208};
-            const uint64_t len[4] = {(uint64_t)bpr * 128, (uint64_t)bpr * 64, (uint64_t)bpr * 16, d_section_bytes(bpr)};
-            const uint32_t pitch[4] = {kQlPitch, kQhPitch, kScPitch, kDPitch};
-            for (int pl = 0; pl < 4; pl++) {
-                cudaError_t me = cached_tensor_map_2d(g.planar + off[pl], 8, len[pl] / 8, g.n_rows, rec, pitch[pl] / 8, kStageRows, &p.map[i][pl]);
-                if (me != cudaSuccess) return me;
-            }
-        } else {
-            const uint64_t row_bytes = (uint64_t)bpr * 144;
-            cudaError_t me = cached_tensor_map_2d(g.w, 8, row_bytes / 8, g.n_rows, row_bytes, kQ4RowPitch / 8, kStageRows, &p.map[i][0]);
+    if (Q6) {
+        const uint64_t rec = row_record_bytes(bpr);
+        const uint64_t off[4] = {0, (uint64_t)bpr * 128, (uint64_t)bpr * 192, (uint64_t)bpr * 208};
+        const uint64_t len[4] = {(uint64_t)bpr * 128, (uint64_t)bpr * 64, (uint64_t)bpr * 16, d_section_bytes(bpr)};
+        const uint32_t pitch[4] = {kQlPitch, kQhPitch, kScPitch, kDPitch};
+        for (int pl = 0; pl < 4; pl++) {
+            cudaError_t me = cached_tensor_map_2d(a.planar + off[pl], 8, len[pl] / 8, a.n_rows, rec, pitch[pl] / 8, kStageRows, &p.map[pl]);
             if (me != cudaSuccess) return me;
         }
-        p.out[i] = g.out;
-        p.n_rows[i] = g.n_rows;
-        p.out_stride[i] = g.out_stride;
-        p.tile0[i] = tiles;
-        tiles += (g.n_rows + kStageRows - 1) / kStageRows;
+    } else {
+        const uint64_t row_bytes = (uint64_t)bpr * 144;
+        cudaError_t me = cached_tensor_map_2d(a.w, 8, row_bytes / 8, a.n_rows, row_bytes, kQ4RowPitch / 8, kStageRows, &p.map[0]);
+        if (me != cudaSuccess) return me;
     }
-    for (uint32_t i = n_seg; i <= (uint32_t)kMaxSegs; i++) p.tile0[i] = tiles;
+    p.out = a.out;
+    p.n_rows = a.n_rows;
+    p.out_stride = a.out_stride;
     p.x = a.x + (size_t)blk_off * 256;
     p.residual = residual;
-    p.norm_w = a.norm_w;
-    p.eps = a.eps;
     p.n_cols = part_cols;
     p.blk_off = blk_off;
-    p.n_tiles = tiles;
+    p.n_tiles = (a.n_rows + kStageRows - 1) / kStageRows;
     p.chunks = (part_cols / 256 + kStageBlocks - 1) / kStageBlocks;
     p.nb = nb;
     p.x_stride = a.x_stride;
@@ -624,12 +571,11 @@ uint32_t kquant_batch_width(const QmvArgs &a) {
     if (!q6 && a.type != YULE_DTYPE_Q4_K) return 0;
     if (q6 && !a.planar) return 0;
     if (a.batch < 2 || a.n_cols == 0 || a.n_cols % 256 || a.n_rows == 0 || a.x_stride % 4) return 0;
-    if (a.tp.push || a.tp.wait) return 0;  // fused exchanges stay with the one-vector kernels
+    if (a.tp.push || a.tp.wait || a.norm_w) return 0;  // fused exchanges and RMSNorms stay with the other kernels
     if ((reinterpret_cast<uintptr_t>(q6 ? (const void *)a.planar : (const void *)a.w) & 15) || (reinterpret_cast<uintptr_t>(a.x) & 15)) return 0;
     // the widest pass whose image fits whole; for longer rows the widest that fits in parts of at least two stages
     for (uint32_t nb = a.batch < 4 ? a.batch : 4; nb >= 2; nb--)
         if (part_cols_for(q6, a.n_cols, nb) == a.n_cols) return nb;
-    if (a.norm_w) return 0;  // the RMSNorm prologue needs the whole row in one launch
     for (uint32_t nb = a.batch < 4 ? a.batch : 4; nb >= 2; nb--)
         if (part_cols_for(q6, a.n_cols, nb) != 0) return nb;
     return 0;
@@ -651,8 +597,8 @@ cudaError_t launch_kquant_batch(const QmvArgs &a, uint32_t nb, int sm_count, cud
         if (col + cols > a.n_cols) cols = a.n_cols - col;
         const uint32_t stages = batch_stages(q6, cols, nb);
         const float *residual = i == 0 ? a.residual : a.out;  // later parts add to what the earlier ones stored
-        cudaError_t e = q6 ? launch_variant<true>(&a, 1, nb, stages, col / 256, cols, residual, sm_count, s)
-                           : launch_variant<false>(&a, 1, nb, stages, col / 256, cols, residual, sm_count, s);
+        cudaError_t e = q6 ? launch_variant<true>(a, nb, stages, col / 256, cols, residual, sm_count, s)
+                           : launch_variant<false>(a, nb, stages, col / 256, cols, residual, sm_count, s);
         if (e != cudaSuccess) return e;
         *launches += 1;
         col += cols;
