@@ -287,10 +287,9 @@ typedef struct {
     /* 0: one kernel per reference dispatch (RmsNorm, Qmv, Rope, KV copy,
      *    MultiheadAttn, Add, SiluMul), launched one by one.
      * 1: fused kernels replayed from a CUDA graph (same arithmetic per row).
-     * 2: as 1, with the token step as ONE persistent kernel where the model allows it and gains by it (up to three
-     *    layers, one GPU, the Llama op sequence, Q4_K attn_q/k/v and ffn_gate/up, Q4_K or Q6_K attn_output / ffn_down / output matrix,
+     * 2: as 1, with the token step as ONE persistent kernel where the model allows it (up to three layers, one GPU, the Llama op sequence, Q4_K attn_q/k/v and ffn_gate/up, Q4_K or Q6_K attn_output / ffn_down / output matrix,
      *    grouped-query head shapes 64 or 128 wide); any other model runs as with 1.
-     *    yule_cuda_runner_step_kind tells which one a runner uses. */
+     *    1 is the faster of the two on every shape measured.  yule_cuda_runner_step_kind tells which one a runner uses. */
     uint32_t fused;
     /* Architecture variants of the dense path, as RunnerConfig derives them from the file
      * (yule-infer/src/model_runner.rs:417-460); all zero = the Llama default.  The reference's GPU runner drops

@@ -740,12 +740,13 @@ int32_t setup_mega(yule_cuda_runner *r) {
         r->mega_why = "architecture variant";
         return YULE_OK;
     }
-    // The graph's one-vector kernels hand over faster than the phases of the persistent kernel once there are a few layers: per token,
-    // persistent against graph, 1.1B shape 22 layers 589 against 530 us, 4 layers 134 against 118; dim 1024, 16 layers 352 against
-    // 335; dim 512, 12 layers 230 against 218, 3 layers 60 against 61.  Models of up to three layers keep what fused = 2 asks for: the
-    // very small ones lose nothing, others some (1.1B shape, 2 layers 76 against 67).
+    // The graph is the faster step on every shape measured: per token, persistent against graph, dim 256 27 and 25 us (one layer),
+    // 44 and 41 (two), dim 512 27.3 and 26.5, 45 and 43, 63 and 61 (three), 81 and 78 (four); dim 1024 52 and 47 (two), 94 and 84 (four);
+    // the 1.1B shape 68 and 57 (two), 124 and 109 (four), 589 and 530 (22); with a vocabulary of 32000 the gap is wider.  So a caller who
+    // wants the fastest step asks for fused = 1.  fused = 2 asks for the persistent kernel: models of up to three layers, where it costs
+    // 10 us or so per token, get it; deeper ones, where the cost grows with every layer, keep the graph.
     if (c.n_layers > kMegaMaxLayers && !knob("YULE_CUDA_MEGA")) {
-        r->mega_why = "the graph is faster on a model of this depth";
+        r->mega_why = "the graph is faster, and by more with every layer";
         return YULE_OK;
     }
     MegaModel m;

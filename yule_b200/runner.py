@@ -83,7 +83,8 @@ class CudaTransformerRunner:
 
     ``weights`` maps GGUF tensor names to ``(bytes-like or uint8/float array, DType)``.  ``fused=False``
     issues one kernel per reference dispatch; ``fused=True`` replays fused kernels from a CUDA graph; ``fused=2``
-    additionally runs the token step as one persistent kernel where the model allows it (``step_kind`` tells).
+    additionally runs the token step as one persistent kernel where the model allows it (up to three layers; ``step_kind``
+    tells), which is not the faster step.
     """
 
     def __init__(self, backend: CudaB200Backend, config: ModelConfig, weights: dict, fused: bool = True):
