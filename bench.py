@@ -2,7 +2,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-Workload (BASELINE.json configs[1]): TinyLlama-1.1B-architecture decode — 22 layers, hidden 2048, 32 query /
+Workload: TinyLlama-1.1B-architecture decode — 22 layers, hidden 2048, 32 query /
 4 KV heads (head_dim 64), SwiGLU FFN 5632, vocab 32000; random-init N(0, 0.02) weights quantised to
 Q4_K (output and ffn_down Q6_K), fp32 KV cache, batch 1, 32-token random prompt, 128 greedy tokens.
 One *step* is one such job.  The metric is decode tokens per second (the 128 generated tokens; the
@@ -13,8 +13,7 @@ prompt pass is timed separately).
 `e2e`    — the same job through the reference-facing ModelRunner calls (prefill / decode_step) with
            host buffers: every step uploads the token and position and downloads the vocab-sized logits, and the
            argmax runs on the host.
-`roofline` — the Q4_K dequant-matvec kernel at the TinyLlama FFN-up shape (
-           5632x2048, 1000 launches) over a ring of weight copies larger than L2, replayed from a
+`roofline` — the Q4_K dequant-matvec kernel at the TinyLlama FFN-up shape (5632x2048, 1000 launches) over a ring of weight copies larger than L2, replayed from a
            CUDA graph and timed with CUDA events; achieved = algorithmic bytes per launch / average
            launch duration, peak = measured copy bandwidth of this pool's B200s.
 `cpu_baseline` — the CPU restatement of the reference's runner (its own AVX2 Q4_K assembly kernel where
@@ -25,7 +24,7 @@ sequence with its own replica of the model — batch-1 decode of a model that fi
 exchange step — and `value` is the sum over ranks divided by the slowest rank's time (weak scaling).
 
 `tp` — measured in the same run at every N: batch-1 decode of the Llama-3-70B-architecture model
-       (BASELINE.json configs[4], every linear Q4_K, ~39 GB) with the output rows of every linear sharded over
+       (every linear Q4_K, ~39 GB) with the output rows of every linear sharded over
        the N GPUs and the activations exchanged over NVLink peer memory (strong scaling: one sequence, N GPUs).
        Carries ms/token, tokens/s, the per-GPU fraction of the HBM roofline, and `tp_check`: a two-layer model
        of the same layer shapes run on N GPUs and on one, logits compared bit for bit and greedy tokens compared.
@@ -53,9 +52,9 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 N_PROMPT, N_GEN = 32, 128
-# DRAM bytes of one 5632x2048 launch of the ring kernel, from the ncu capture summarised in the named file
-RING_TRAFFIC_BYTES = 6534144
-RING_TRAFFIC_SOURCE = "profiles/qmv_q4k_ring_5632x2048.md (dram__bytes_read.sum + dram__bytes_write.sum of one launch, ncu capture)"
+# DRAM bytes of one independent 5632x2048 launch, from the ncu capture summarised in the named file
+RING_TRAFFIC_BYTES = 6524416
+RING_TRAFFIC_SOURCE = "profiles/qmv_digits_q4k_5632x2048.md (dram__bytes_read.sum + dram__bytes_write.sum of one launch, ncu capture)"
 METRIC = "batch-1 decode tokens/s; Q4_K matvec achieved HBM GB/s vs B200 peak"
 UNIT = "tokens/s"
 
@@ -126,8 +125,8 @@ def host_argmax_last(logits: np.ndarray) -> int:
 
 
 def build_model_70b(rank: int, world: int, which: str = "c4"):
-    """BASELINE.json configs[4]: Llama-3-70B architecture, every linear Q4_K (~39 GB), row-sharded over `world` ranks;
-    Llama-3-8B architecture, Q4_K linears with a Q6_K output matrix.
+    """c4: Llama-3-70B architecture, every linear Q4_K (~39 GB), row-sharded over `world` ranks;
+    c3: Llama-3-8B architecture, Q4_K linears with a Q6_K output matrix.
     To bound host time the quantised N(0, 0.02) tensors of one layer are generated once and uploaded for all
     the layers (distinct device buffers, so HBM traffic is that of different layers)."""
     from yule_b200 import DType, parallel, synth
@@ -164,8 +163,8 @@ def build_model(rank: int, linear: str = "Q4_K"):
 
 def small_batch_decode(backend, cfg, weights, n_prompt: int = 8, n_gen: int = 64):
     """The same model serving a few independent sequences per step (own KV caches and positions, device picks):
-    every linear reads its weights once per step for up to four sequences (batched matvec kernels) or for all of
-    them (GEMM, from thirteen sequences).  Device time per step over `n_prompt + n_gen` steps, tokens/s over all sequences."""
+    every linear reads its weights once per step.  Device time of `n_gen` steps, that of the prompts (one pass, then the first
+    step) taken off: a run that generates nothing.  Tokens/s over all sequences."""
     from yule_b200 import CudaTransformerRunner, synth
     out = {}
     for batch in (4, 8, 12, 16):
@@ -176,13 +175,16 @@ def small_batch_decode(backend, cfg, weights, n_prompt: int = 8, n_gen: int = 64
         backend.synchronize()
         backend.event_reset()
         e0 = backend.event_record()
-        run.generate_greedy_batch(prompts, n_gen)  # the prompt tokens are steps of the same kind
+        run.generate_greedy_batch(prompts, 0)
         e1 = backend.event_record()
-        ms = backend.event_elapsed_ms(e0, e1)
-        steps = n_prompt + n_gen
-        out[f"batch_{batch}"] = {"steps": steps, "ms_per_step": round(ms / steps, 4),
-                                 "tokens_per_s": round(batch * steps / (ms * 1e-3), 1),
-                                 "linears": "batched matvec kernels" if batch <= 12 else "tcgen05 GEMM"}
+        run.generate_greedy_batch(prompts, n_gen)
+        e2 = backend.event_record()
+        prompt_ms = backend.event_elapsed_ms(e0, e1)
+        ms = backend.event_elapsed_ms(e1, e2) - prompt_ms
+        out[f"batch_{batch}"] = {"steps": n_gen, "ms_per_step": round(ms / n_gen, 4), "prompts_ms": round(prompt_ms, 4),
+                                 "tokens_per_s": round(batch * n_gen / (ms * 1e-3), 1),
+                                 "linears": "qmv_rows (up to sixteen vectors per pass)" if batch <= 12 else
+                                            "qmv_rows (Q6_K, small Q4_K matrices), tcgen05 GEMM"}
         run.close()
     return out
 
@@ -201,7 +203,7 @@ def decode_bytes_per_token(cfg, weights, pos: int, tp_world: int = 1) -> int:
 
 
 def matvec_ring_roofline(backend, peaks, peak_kind, iters: int = 1000) -> dict:
-    """configs[0]: Q4_K 5632x2048 matvec, `iters` launches rotating over copies that together exceed
+    """Q4_K 5632x2048 matvec, `iters` launches rotating over copies that together exceed
     twice the L2, captured once into a CUDA graph and replayed; CUDA-event time / launches."""
     from yule_b200 import DType, matvec_bytes, synth
     n_rows, n_cols, dt = 5632, 2048, DType.Q4_K
@@ -233,7 +235,7 @@ def matvec_ring_roofline(backend, peaks, peak_kind, iters: int = 1000) -> dict:
     bytes_per_launch = matvec_bytes(dt, n_rows, n_cols)
     achieved = bytes_per_launch * iters / (ms * 1e-3) / 1e9
     peak = float(peaks["hbm_gbs"])
-    return {"bound": "hbm", "kernel": "qmv_q4k_ring_kernel",
+    return {"bound": "hbm", "kernel": "qmv_digits_kernel",
             "workload": "Q4_K 5632x2048 matvec x1000 over an 80-copy ring (519 MB); the launches are independent calls of the "
                         "trait method (same input vector), so each overlaps with its predecessor and only its stores wait for it",
             "achieved": round(achieved, 1), "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
@@ -267,7 +269,7 @@ def reference_cuda_kernel_leg(peaks) -> dict:
 
 
 def large_shape_rooflines(backend, peaks) -> dict:
-    """The same matvec kernels on shapes large enough to be bandwidth-bound (BASELINE.json configs[2]'s 128256x4096,
+    """The same matvec kernels on shapes large enough to be bandwidth-bound (128256x4096,
     Q4_K and Q6_K, batch 1) and the tcgen05 GEMM on a prefill-sized problem: what the kernels do when launch
     and dependency latency do not dominate.  Weights stream from HBM over a ring of copies."""
     from yule_b200 import DType, microbench
@@ -312,7 +314,7 @@ def cpu_forward_tokens_per_s(cfg, weights, prompt, budget_s: float, max_tokens: 
     return n / dt_s, cores, kind, sample, n, dt_s
 
 
-WORKLOAD_C1 = ("configs[1] TinyLlama-1.1B-arch decode, {linear} linears, Q6_K output+ffn_down, fp32 KV, batch 1, "
+WORKLOAD_C1 = ("TinyLlama-1.1B-arch decode, {linear} linears, Q6_K output+ffn_down, fp32 KV, batch 1, "
                "{n_prompt}-token prompt + {n_gen} greedy tokens per step")
 
 
@@ -343,7 +345,7 @@ def run_reference(args, rank: int, world: int) -> int:
 
 
 def measure_tp(args, rank: int, world: int, local_rank: int, dist, peaks) -> dict | None:
-    """configs[4] at world size N: batch-1 decode of the Llama-3-70B-architecture model, output rows of every
+    """70B at world size N: batch-1 decode of the Llama-3-70B-architecture model, output rows of every
     linear sharded over the N GPUs (one layer's tensors generated once and uploaded for all 80 layers, each
     rank generating only its own rows).  Before the timing, a two-layer model of the same layer shapes is run
     on N GPUs and (on rank 0) on one GPU: logits compared bit for bit, greedy tokens compared."""
@@ -360,7 +362,7 @@ def measure_tp(args, rank: int, world: int, local_rank: int, dist, peaks) -> dic
 
     n_prompt, n_gen = (8, 8) if args.small else (args.tp_prompt, args.tp_gen)
     full = synth.LLAMA3_70B
-    out = {"workload": f"configs[4] Llama-3-70B-arch decode, all linears Q4_K (one layer's tensors repeated for the "
+    out = {"workload": f"Llama-3-70B-arch decode, all linears Q4_K (one layer's tensors repeated for the "
                        f"{full.n_layers} layers), fp32 KV, batch 1, {n_prompt}-token prompt + {n_gen} greedy tokens",
            "world": world, "scaling": "strong",
            "exchange": ("none (one GPU)" if world == 1 else
@@ -447,9 +449,9 @@ def measure_tp(args, rank: int, world: int, local_rank: int, dist, peaks) -> dic
                     "prefill_tokens_per_s": round(n_prompt * reps / (pre_ms * 1e-3), 1),
                     "hbm_bytes_per_token_per_gpu": bpt, "achieved_gbs_per_gpu": round(gbs, 1),
                     "frac_of_peak_per_gpu": round(gbs / float(peaks["hbm_gbs"]), 4),
-                    "dominant_kernel": "qmv_q4k_mma_kernel (Q4_K matvec, about 95 % of the token step; attention and the "
+                    "dominant_kernel": "qmv_digits_kernel (Q4_K matvec, about 95 % of the token step; attention and the "
                                        "logits exchange are the rest)"})
-        # ── configs[4] batch 32: 32 independent sequences decoded together, every linear one GEMM per step ──
+        # ── batch 32: 32 independent sequences decoded together, every linear one GEMM per step ──
         nb, bp, bg = (8, 4, 4) if args.small else (32, args.tp_prompt, args.tp_gen // 2)
         prompts = synth.tokens(17, nb * bp, cfg.vocab_size).reshape(nb, bp)
         run.generate_greedy_batch(prompts, bg)  # warm-up: allocations, graph capture
@@ -457,20 +459,23 @@ def measure_tp(args, rank: int, world: int, local_rank: int, dist, peaks) -> dic
         tpb.event_reset()
         if dist is not None:
             dist.barrier()
+        # the prompts go through in passes of many rows: their time, that of a run that generates nothing, is taken off
         e0 = tpb.event_record()
-        run.generate_greedy_batch(prompts, bg)
+        run.generate_greedy_batch(prompts, 0)
         e1 = tpb.event_record()
-        b_ms = gather_max(tpb.event_elapsed_ms(e0, e1))
-        steps = bp + bg
-        step_ms = b_ms / steps
+        run.generate_greedy_batch(prompts, bg)
+        e2 = tpb.event_record()
+        prompts_ms = gather_max(tpb.event_elapsed_ms(e0, e1))
+        step_ms = (gather_max(tpb.event_elapsed_ms(e1, e2)) - prompts_ms) / bg
         kv_bytes = 2 * cfg.n_layers * nb * (bp + bg // 2) * (cfg.n_kv_heads // world) * cfg.head_dim * 4
         wbytes = decode_bytes_per_token(cfg, weights, 0, tp_world=world)
-        out["batch32"] = {"sequences": nb, "prompt_tokens": bp, "generated_tokens": bg, "ms_per_step": round(step_ms, 4),
+        out["batch32"] = {"sequences": nb, "prompt_tokens": bp, "generated_tokens": bg, "steps": bg, "ms_per_step": round(step_ms, 4),
+                          "prompts_ms": round(prompts_ms, 4),
                           "tokens_per_s": round(nb * 1e3 / step_ms, 1),
                           "weight_bytes_per_step_per_gpu": wbytes,
                           "achieved_gbs_per_gpu": round((wbytes + kv_bytes) / (step_ms * 1e-3) / 1e9, 1),
                           "frac_of_peak_per_gpu": round((wbytes + kv_bytes) / (step_ms * 1e-3) / 1e9 / float(peaks["hbm_gbs"]), 4),
-                          "path": "tcgen05 GEMM per linear over the 32 rows (prompt positions are steps of the same kind)"}
+                          "path": "tcgen05 GEMM per linear over the 32 rows"}
         run.close()
     except YuleGpuError as e:
         out["error"] = f"{e.code}: {e.message}"
@@ -517,7 +522,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> int:
     step_kind = runner.step_kind
 
     def job():
-        """One configs[1] job on the device; returns (prefill ms, decode ms, tokens)."""
+        """One job on the device; returns (prefill ms, decode ms, tokens)."""
         runner.reset()
         e0 = backend.event_record()
         runner.generate_greedy(prompt, 0)
@@ -599,8 +604,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> int:
             "warmup": max(args.warmup, 3), "warmup_requested": args.warmup, "ms_per_step": round((prefill_ms + decode_ms) / args.steps, 3),
             "higher_is_better": True, "scaling": "strong" if tp else "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic",
-            "config": ({"workload": ("configs[4] Llama-3-70B-arch decode, all linears Q4_K" if args.workload == "c4" else
-                                     "configs[3] Llama-3-8B-arch, Q4_K linears, Q6_K output, prompt through the chunked GEMM prefill on one GPU") +
+            "config": ({"workload": ("Llama-3-70B-arch decode, all linears Q4_K" if args.workload == "c4" else
+                                     "Llama-3-8B-arch, Q4_K linears, Q6_K output, prompt through the chunked GEMM prefill on one GPU") +
                                     f" (one layer's tensors repeated for the {cfg.n_layers} layers), fp32 KV, batch 1, "
                                     f"{N_PROMPT}-token prompt + {N_GEN} greedy tokens per step",
                         "parallelism": f"tp{world}: output rows of every linear sharded over {world} GPU(s), "
@@ -646,7 +651,7 @@ def main() -> int:
                          "256 tokens).  c3/c4 shard the output rows of every linear over the GPUs (tensor parallelism)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--step", choices=["persistent", "graph"], default="persistent",
-                    help="token step of the configs[1] runner: one persistent kernel (default) or the multi-kernel CUDA graph")
+                    help="token step of the c1 runner: the multi-kernel CUDA graph (graph), or as the library picks it when asked for the persistent kernel (default)")
     ap.add_argument("--no-tp", action="store_true", help="leave out the `tp` object (the 70B-arch tensor-parallel decode)")
     ap.add_argument("--tp-prompt", type=int, default=64, help="prompt tokens of the `tp` measurement")
     ap.add_argument("--tp-gen", type=int, default=128, help="generated tokens of the `tp` measurement")

@@ -115,7 +115,7 @@ def test_long_context_uses_several_passes_and_splits(backend, oracle):
 
 
 def test_tinyllama_shape_against_the_multi_kernel_step(backend):
-    """Two layers of the configs[1] architecture: the persistent kernel against the multi-kernel graph on the
+    """Two layers of the 1.1B architecture: the persistent kernel against the multi-kernel graph on the
     same weights (the oracle comparison at this size is the job of test_gpu_layer_shapes)."""
     cfg = ModelConfig(dim=2048, n_layers=2, n_heads=32, n_kv_heads=4, head_dim=64, vocab_size=32000, ff_dim=5632,
                       max_seq_len=256)

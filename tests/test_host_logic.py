@@ -38,7 +38,7 @@ def test_quantisers_round_trip_through_the_oracle(oracle):
 
 
 def test_random_field_scales_follow_the_spec(oracle):
-    """configs[0]: f16 d and dmin drawn as |N(0, 0.002)|; some of them are f16-subnormal (< 6.1e-5)."""
+    """f16 d and dmin drawn as |N(0, 0.002)|; some of them are f16-subnormal (< 6.1e-5)."""
     b = synth.random_blocks(DType.Q4_K, 1, 20000).reshape(-1, 144)
     d = b[:, 0:2].copy().view(np.float16).astype(np.float32).reshape(-1)
     assert (d >= 0).all() and abs(np.sqrt(np.mean(d ** 2)) - 0.002) < 2e-4
