@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import REL_TOL, guarded_rel_err
-from yule_b200 import YuleGpuError, synth
+from yule_b200 import CudaB200Backend, DType, YuleGpuError, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -197,3 +197,41 @@ def test_attention_around_the_lines_between_its_kernels(backend, oracle, hd, seq
         assert guarded_rel_err(backend.download(oh, n_heads * hd), ref) <= REL_TOL
         for h in (qh, kh, vh, oh):
             backend.free(h)
+
+
+@pytest.mark.parametrize("dtype,n_rows,n_cols,batch", [(DType.Q4_K, 5120, 4096, 14), (DType.Q4_K, 1024, 1024, 24), (DType.Q5_K, 1024, 1024, 56)])
+def test_capture_of_a_batch_without_scratch(oracle, dtype, n_rows, n_cols, batch):
+    """The first call of a context inside a graph capture, where the GEMM's scratch cannot be allocated: batches that the matvec
+    kernels can take go to them."""
+    b = CudaB200Backend(0)
+    w, x = synth.random_quantized(dtype, 11, n_rows * n_cols), synth.normal(12, batch * n_cols)
+    wh, xh, oh = b.upload(w), b.upload(x), b.allocate(batch * n_rows * 4)
+    b.graph_begin()
+    b.quantized_matmul_batched(wh, xh, oh, n_rows, n_cols, dtype, batch)
+    graph = b.graph_end()
+    b.graph_launch(graph)
+    y = b.download(oh, batch * n_rows).reshape(batch, n_rows)
+    b.graph_destroy(graph)
+    b.close()
+    for i in (0, batch - 1):
+        assert guarded_rel_err(y[i], oracle.qmv(int(dtype), w, x[i * n_cols:(i + 1) * n_cols], n_rows, n_cols)) <= REL_TOL
+
+
+@pytest.mark.parametrize("hd,seq", [(64, 256), (128, 100), (128, 256)])
+def test_capture_of_attention_without_scratch(oracle, hd, seq):
+    """Likewise up to 256 positions, which need no merge when a query head has a CTA; from 257 on the call is refused and the
+    context stays usable."""
+    n_heads, n_kv = 8, 2
+    b = CudaB200Backend(0)
+    q, K, V = synth.normal(1, n_heads * hd), synth.normal(2, 300 * n_kv * hd), synth.normal(3, 300 * n_kv * hd)
+    qh, kh, vh, oh = b.upload(q), b.upload(K), b.upload(V), b.allocate(n_heads * hd * 4)
+    b.graph_begin()
+    b.multihead_attention(qh, kh, vh, oh, hd, seq, n_heads, n_kv, n_kv * hd)
+    with pytest.raises(YuleGpuError):
+        b.multihead_attention(qh, kh, vh, oh, hd, 300, n_heads, n_kv, n_kv * hd)
+    graph = b.graph_end()
+    b.graph_launch(graph)
+    ref = oracle.attention(q, K.reshape(300, -1)[:seq], V.reshape(300, -1)[:seq], n_heads, n_kv, hd, seq)
+    assert guarded_rel_err(b.download(oh, n_heads * hd), ref) <= REL_TOL
+    b.graph_destroy(graph)
+    b.close()

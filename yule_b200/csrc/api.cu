@@ -494,20 +494,25 @@ int32_t yule_cuda_attn_value(yule_cuda_ctx *ctx, yule_buffer weights, yule_buffe
 // (measured on 1024x4096 .. 128256x4096): the exact Q4_K kernel from 16 (from 32 on matrices of up to 8M weights,
 // where four passes of the batched matvec cost less than the GEMM's fixed part), the generic kernel of the other
 // formats from 32, except Q5_K (tensor-pipe matvec at 3.5 us per row against a 195 us GEMM) from 64; from 8 where the
-// rows are too long for a batched matvec kernel to hold its activation image.  YULE_GEMM_MIN_BATCH overrides all of
-// them (at least 8).
-static uint32_t gemm_min_batch(const QmvArgs &a) {
-    if (const char *e = knob("YULE_GEMM_MIN_BATCH")) {
-        const int v = atoi(e);
-        return v < 8 ? 8u : (uint32_t)v;
-    }
-    // the matvec over sixteen vectors a pass wins up to the line that qmv_rows_preferred draws
-    const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
-    if (a.batch >= 8 && qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) return qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) ? ~0u : 8u;
+// rows are too long for a batched matvec kernel to hold its activation image.
+static uint32_t gemm_line(const QmvArgs &a) {
     const bool tuned = a.type == YULE_DTYPE_Q4_K || a.type == YULE_DTYPE_Q6_K || a.type == YULE_DTYPE_Q8_0 || a.type == YULE_DTYPE_Q4_0;
     if (tuned && a.batch >= 8 && kquant_batch_width(a) < 2 && q8q4_ring_batch_width(a) < 2) return 8u;
     if (a.type == YULE_DTYPE_Q4_K) return (uint64_t)a.n_rows * a.n_cols <= (8ull << 20) ? 32u : 16u;
     return a.type == YULE_DTYPE_Q5_K ? 64u : 32u;
+}
+
+// Whether a call goes to the GEMM.  YULE_GEMM_MIN_BATCH overrides all of the lines (at least 8).
+static bool takes_gemm(const yule_cuda_ctx *ctx, const QmvArgs &a) {
+    if (a.batch < 8 || !qgemm_supported(a.type, a.n_cols, a.batch)) return false;
+    uint32_t line = gemm_line(a);
+    // While a graph is captured its scratch cannot grow: then the matvec kernels, which need none, keep what they can do as well.
+    if (ctx->capturing && ctx->gemm_scratch_bytes < qgemm_scratch_bytes(a.batch, a.n_cols) && a.batch < line) return false;
+    // the matvec over sixteen vectors a pass wins up to the line that qmv_rows_preferred draws
+    const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
+    if (qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) line = qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) ? ~0u : 8u;
+    if (const char *e = knob("YULE_GEMM_MIN_BATCH")) line = atoi(e) < 8 ? 8u : (uint32_t)atoi(e);
+    return a.batch >= line;
 }
 
 static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight_offset, yule_buffer input,
@@ -548,7 +553,7 @@ static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight
     if (type == YULE_DTYPE_Q6_K && W.planar && weight_offset == 0 && W.planar_cols == n_cols &&
         W.planar_blocks == (uint64_t)n_rows * (n_cols / 256))
         a.planar = W.planar;
-    if (batch >= 8 && batch >= gemm_min_batch(a) && qgemm_supported(type, n_cols, batch)) {
+    if (takes_gemm(ctx, a)) {
         // enough activation rows: one pass over the weights on the tcgen05 GEMM
         int32_t rc = ensure_gemm_scratch(ctx, qgemm_scratch_bytes(batch, n_cols));
         if (rc) return rc;
@@ -709,10 +714,16 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
         const size_t need = attn_scratch_floats(n_heads, a.n_splits, head_dim);
         {
             std::lock_guard<std::mutex> lock(ctx->mu);
-            if (a.n_splits > 1 && (ctx->attn_scratch_floats < need || ctx->attn_tickets_n < n_heads)) {
-                YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            bool grow = a.n_splits > 1 && (ctx->attn_scratch_floats < need || ctx->attn_tickets_n < n_heads);
+            if (grow && ctx->capturing && a.gqa && attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount) == 1) {
+                // no scratch to be had while a graph is captured: one query head per CTA, all positions, needs none
+                a.gqa = grow = false;
+                a.n_splits = 1;
+            }
+            if (grow) {
                 if (ctx->capturing)
                     return fail(YULE_ERR_INVALID_ARGUMENT, "the attention scratch cannot grow during graph capture: run the call once outside the capture first");
+                YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
                 // graphs captured earlier may still replay into the old blocks: retire them, do not free them
                 if (ctx->attn_scratch) ctx->retired_scratch.push_back(ctx->attn_scratch);
                 if (ctx->attn_tickets) ctx->retired_scratch.push_back(ctx->attn_tickets);
