@@ -179,15 +179,16 @@ int32_t yule_cuda_sample(yule_cuda_ctx *ctx, yule_buffer logits, uint32_t n, con
 
 /* `batch` activation vectors against one weight read: input is
  * [batch][x_stride] floats, output [batch][out_stride] floats.  Same per-row
- * arithmetic as quantized_matmul.  Small batches go through the matvec kernels
- * four vectors at a time (Q4_K, Q6_K, Q8_0, Q4_0: four vectors share the
- * tensor-core instructions of one, so a pass costs about one vector's time);
- * from 16 vectors of Q4_K (32 on matrices of up to 8M weights), 64 of Q5_K, or
- * 32 of the other block formats (n_cols a multiple of 256), the tcgen05 GEMM
+ * arithmetic as quantized_matmul.  Small batches go through the matvec kernels,
+ * up to sixteen vectors per pass over the weights (Q4_K, Q5_K, Q6_K, Q8_0,
+ * Q4_0); from 13 vectors of Q4_K (17 on matrices of up to 17M weights) or 33 to
+ * 49 of the other block formats (n_cols a multiple of 256), the tcgen05 GEMM
  * takes one pass over the weights.
  * The GEMM keeps its activation tiles in a scratch owned by the context, grown
  * on demand; growing is not possible while a graph is being captured, so run
- * one call of the largest batch before yule_cuda_graph_begin. */
+ * one call of the largest batch before yule_cuda_graph_begin.  (Up to 15 vectors
+ * of Q4_K, 31 on matrices of up to 8M weights, 63 of Q5_K and 31 of the other
+ * formats need no such call: the matvec kernels take them then.) */
 int32_t yule_cuda_quantized_matmul_batched(yule_cuda_ctx *ctx, yule_buffer weights,
                                            yule_buffer input, yule_buffer output, uint32_t n_rows,
                                            uint32_t n_cols, uint32_t gguf_type, uint32_t batch,
@@ -287,8 +288,9 @@ typedef struct {
     /* 0: one kernel per reference dispatch (RmsNorm, Qmv, Rope, KV copy,
      *    MultiheadAttn, Add, SiluMul), launched one by one.
      * 1: fused kernels replayed from a CUDA graph (same arithmetic per row).
-     * 2: as 1, with the token step as ONE persistent kernel where the model allows it (up to three layers, one GPU, the Llama op sequence, Q4_K attn_q/k/v and ffn_gate/up, Q4_K or Q6_K attn_output / ffn_down / output matrix,
-     *    grouped-query head shapes 64 or 128 wide); any other model runs as with 1.
+     * 2: as 1, with the token step as ONE persistent kernel where the model allows it (up to three layers, one
+     *    GPU, the Llama op sequence, Q4_K attn_q/k/v and ffn_gate/up, Q4_K or Q6_K attn_output / ffn_down / output
+     *    matrix, grouped-query head shapes 64 or 128 wide); any other model runs as with 1.
      *    1 is the faster of the two on every shape measured.  yule_cuda_runner_step_kind tells which one a runner uses. */
     uint32_t fused;
     /* Architecture variants of the dense path, as RunnerConfig derives them from the file
