@@ -1,0 +1,60 @@
+"""Decode attention on thread-block clusters (csrc/attn_cluster.cu) at the sizes where its split changes: fewer positions than
+CTAs, a tile of 32 and its neighbours, one cluster and several, the line to the kernel with splits, full contexts."""
+
+import numpy as np
+import pytest
+
+from test_gpu_runner import make_oracle_model
+from yule_b200 import CudaTransformerRunner, DType, ModelConfig, synth
+
+pytestmark = pytest.mark.gpu
+
+# A score is a sum of head_dim products, off by at most head_dim * 2^-24 of the sum of their magnitudes (about sqrt(head_dim) after the
+# scaling, for N(0, 1) values): 8e-5 at 128 in the worst case, a tenth of that with roundings of random sign; the weights carry it on.
+TOL = 1e-5
+
+
+def attention64(q, K, V, n_heads, n_kv, hd):
+    q, K, V = (a.astype(np.float64) for a in (q.reshape(n_heads, hd), K, V))
+    out = np.empty((n_heads, hd))
+    for h in range(n_heads):
+        kv = h // (n_heads // n_kv)
+        s = K[:, kv * hd:(kv + 1) * hd] @ q[h] / np.sqrt(hd)
+        e = np.exp(s - s.max())
+        out[h] = e @ V[:, kv * hd:(kv + 1) * hd] / e.sum()
+    return out.reshape(-1)
+
+
+@pytest.mark.parametrize("hd,n_heads,n_kv,seqs", [
+    (64, 32, 4, (1, 2, 7, 8, 9, 31, 33, 255, 256, 257, 1000, 5119, 5120, 5121)),
+    (128, 32, 8, (1, 3, 32, 64, 65, 511, 513, 768, 769, 2560, 2561)),
+    (128, 64, 8, (5, 100, 1023)), (64, 4, 4, (6, 300, 1500)), (128, 2, 1, (4, 700)), (64, 16, 8, (33, 600))])
+def test_one_query(backend, hd, n_heads, n_kv, seqs):
+    stride = n_kv * hd + 4  # rows that are not packed
+    for seq in seqs:
+        q, K, V = synth.normal(seq, n_heads * hd), synth.normal(seq + 1, seq * stride), synth.normal(seq + 2, seq * stride)
+        q *= 3  # some positions dominate
+        handles = [backend.upload(a) for a in (q, K, V)] + [backend.allocate(n_heads * hd * 4)]
+        qh, kh, vh, oh = handles
+        for _ in range(2):  # the second call finds the tickets of the first
+            backend.multihead_attention(qh, kh, vh, oh, hd, seq, n_heads, n_kv, stride)
+        y = backend.download(oh, n_heads * hd)
+        ref = attention64(q, K.reshape(seq, stride), V.reshape(seq, stride), n_heads, n_kv, hd)
+        assert np.abs(y - ref).max() <= TOL * np.abs(ref).max(), (hd, n_heads, n_kv, seq)
+        for h in handles:
+            backend.free(h)
+
+
+@pytest.mark.parametrize("hd,n_heads,n_kv,ctx,prompt", [(64, 4, 2, 24, 3), (64, 8, 1, 40, 30), (64, 8, 4, 300, 250), (128, 4, 4, 130, 120),
+                                                        (128, 8, 2, 800, 760), (64, 16, 2, 700, 500)])
+def test_runner_up_to_the_full_context(backend, oracle, hd, n_heads, n_kv, ctx, prompt):
+    cfg = ModelConfig(dim=256, n_layers=2, n_heads=n_heads, n_kv_heads=n_kv, head_dim=hd, vocab_size=512, ff_dim=512, max_seq_len=ctx)
+    weights = synth.synthetic_model(cfg, seed=3, std=0.08, linear=DType.Q8_0)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    tokens = [(7 * i + 3) % 512 for i in range(ctx)]
+    got, want = run.prefill(tokens[:prompt]), ref.prefill(tokens[:prompt])
+    for t in tokens[prompt:]:
+        assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+        got, want = run.decode_step(t), ref.decode_step(t)
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+    run.close()

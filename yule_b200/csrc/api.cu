@@ -706,18 +706,28 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
     if (attn_decode_supported(head_dim) && kv_stride % 4 == 0) {
         // split over positions; the partial results live in a context-owned scratch grown on demand
         AttnDecode a;
-        // One KV head's queries together from 100 rows of 128 or 200 of 64 values: 8 KV heads of 128, 101 positions 7.5 -> 6.4 us,
-        // 400 13.7 -> 7.6; 4 of 64, 200 positions 7.2 -> 6.9, but 101 5.2 -> 6.1 (splits of 32 positions that have to be merged).
-        a.gqa = attn_gqa_supported(head_dim, n_heads, n_kv_heads) && (uint64_t)seq_len * head_dim >= 12800;
-        a.n_splits = a.gqa ? attn_gqa_pick_splits(n_kv_heads, seq_len, ctx->prop.multiProcessorCount)
-                           : attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount);
+        a.gqa = attn_gqa_supported(head_dim, n_heads, n_kv_heads);
+        // Clusters up to 5120 rows of 64 values or 2560 of 128, beyond them splits that meet in global memory.  us, splits -> clusters:
+        // 32 heads of 64 on 4, 250 positions 7.1 -> 5.0, 1500 12.6 -> 8.0, 6000 15.5 -> 12.4, 16000 20.3 -> 21.2; 32 heads of 128 on 8, 250 6.8 ->
+        // 5.1, 1500 11.6 -> 10.3, 2500 12.4 -> 12.1, 3500 12.9 -> 13.9; 64 heads on 8, 700 11.6 -> 10.2, 2500 16.6 -> 14.9, 3500 17.3 -> 17.5.
+        const bool clustered = a.gqa && (uint64_t)seq_len * head_dim <= 327680;
+        uint32_t ranks = 0, tickets_n = n_heads;
+        if (clustered) {
+            attn_cluster_shape(n_kv_heads, head_dim, seq_len, true, ctx->prop.multiProcessorCount, &ranks, &a.n_splits);
+            tickets_n = n_kv_heads * kAttnMaxRanks;
+        } else {
+            a.n_splits = a.gqa ? attn_gqa_pick_splits(n_kv_heads, seq_len, ctx->prop.multiProcessorCount)
+                               : attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount);
+        }
         const size_t need = attn_scratch_floats(n_heads, a.n_splits, head_dim);
         {
             std::lock_guard<std::mutex> lock(ctx->mu);
-            bool grow = a.n_splits > 1 && (ctx->attn_scratch_floats < need || ctx->attn_tickets_n < n_heads);
-            if (grow && ctx->capturing && a.gqa && attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount) == 1) {
-                // no scratch to be had while a graph is captured: one query head per CTA, all positions, needs none
-                a.gqa = grow = false;
+            // (more than 256 positions need the scratch of this entry point, whatever the clusters make of it: a capture that cannot have it is refused)
+            const bool longer = attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount) > 1;
+            bool grow = (a.n_splits > 1 || longer) && (ctx->attn_scratch_floats < need || ctx->attn_tickets_n < tickets_n);
+            if (grow && ctx->capturing && !longer) {
+                // no scratch to be had while a graph is captured: one cluster per KV head, which needs none
+                grow = false;
                 a.n_splits = 1;
             }
             if (grow) {
@@ -731,10 +741,10 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
                 ctx->attn_tickets = nullptr;
                 ctx->attn_scratch_floats = ctx->attn_tickets_n = 0;
                 YULE_CUDA_TRY(cudaMalloc((void **)&ctx->attn_scratch, need * sizeof(float)));
-                YULE_CUDA_TRY(cudaMalloc((void **)&ctx->attn_tickets, (size_t)n_heads * sizeof(uint32_t)));
-                YULE_CUDA_TRY(cudaMemsetAsync(ctx->attn_tickets, 0, (size_t)n_heads * sizeof(uint32_t), ctx->stream));
+                YULE_CUDA_TRY(cudaMalloc((void **)&ctx->attn_tickets, (size_t)tickets_n * sizeof(uint32_t)));
+                YULE_CUDA_TRY(cudaMemsetAsync(ctx->attn_tickets, 0, (size_t)tickets_n * sizeof(uint32_t), ctx->stream));
                 ctx->attn_scratch_floats = need;
-                ctx->attn_tickets_n = n_heads;
+                ctx->attn_tickets_n = tickets_n;
             }
             a.scratch = ctx->attn_scratch;
             a.tickets = ctx->attn_tickets;
@@ -749,7 +759,10 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
         a.n_kv_heads = n_kv_heads;
         a.kv_stride = kv_stride;
         a.max_seq_len = seq_len;
-        LAUNCHED(ctx, launch_attn_decode(a, ctx->stream, &_n));
+        if (clustered)
+            LAUNCHED(ctx, launch_attn_cluster(a, ctx->prop.multiProcessorCount, ctx->stream, &_n));
+        else
+            LAUNCHED(ctx, launch_attn_decode(a, ctx->stream, &_n));
         return YULE_OK;
     }
     LAUNCHED(ctx, launch_multihead_attention((const float *)Q.ptr, (const float *)K.ptr, (const float *)V.ptr,

@@ -200,53 +200,23 @@ __global__ void __launch_bounds__(kThreads) attn_decode_kernel(const AttnParams 
 }
 
 
-// Tensor parallelism: element o of this rank's slice of the attention output as a (value, epoch) pair into
-// every rank's pair buffer, one 8-byte store each (the reader polls the pairs; see TpFuse).
-__device__ __noinline__ void tp_push_value(const TpFuse &tp, size_t o, float v) {
-    const uint32_t epoch = *tp.tick * tp.epochs_per_tick + tp.push_index + 1u;
-    for (uint32_t pp = 0; pp < tp.world; pp++)
-        asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(tp.pair_out[pp] + o), "r"(__float_as_uint(v)), "r"(epoch) : "memory");
-}
-
-// TP = true only for launches of a tensor-parallel runner that also push (value, epoch) pairs.
-template <int GROUP, int HD, bool TP>
+template <int GROUP, int HD>
 __global__ void __launch_bounds__(kThreads) attn_decode_gqa_kernel(const __grid_constant__ AttnParams p) {
     extern __shared__ __align__(16) float sm[];
     __shared__ uint32_t s_last;
     yule_pdl_launch_dependents();
     yule_pdl_wait();
-    // prefill: query z of the launch sits z positions further on and has its own rows and scratch
-    const uint32_t z = blockIdx.z;
-    AttnUnit au;
-    au.pos = p.pos_ptr ? (p.pos_per_query ? p.pos_ptr[z] : *p.pos_ptr) : p.seq_len - 1 + z;
-    au.k_cache = p.k_cache + (size_t)z * p.kv_batch_stride;
-    au.v_cache = p.v_cache + (size_t)z * p.kv_batch_stride;
-    au.q_in = p.q + (size_t)z * p.q_stride;
-    au.k_new = p.k_new ? p.k_new + (size_t)z * p.kv_stride : nullptr;
-    au.v_new = p.v_new ? p.v_new + (size_t)z * p.kv_stride : nullptr;
-    au.scratch = p.scratch + (size_t)z * p.n_heads * p.n_splits * (HD + 2);
-    au.tickets = p.tickets + (size_t)z * p.n_heads;
-    au.q_pairs = au.k_pairs = au.v_pairs = nullptr;
-    au.in_epoch = 0;
-    au.prof = nullptr;
-    float *out_z = p.out + (size_t)z * p.out_stride;
-    attn_gqa_unit<GROUP, HD, false>(
-        p, au, blockIdx.x, blockIdx.y, threadIdx.x, sm, &s_last, [] { __syncthreads(); },
-        [&](uint32_t i, float v) {
-            out_z[i] = v;
-            if (TP && p.tp.push) tp_push_value(p.tp, i, v);
-        });
+    attn_gqa_unit<GROUP, HD>(p, blockIdx.x, blockIdx.y, threadIdx.x, sm, &s_last);
 }
 
-
 template <int GROUP, int HD>
-cudaError_t launch_gqa_variant(const AttnParams &p, size_t smem, bool pdl, cudaStream_t s, uint32_t n_tokens = 1) {
-    auto kern = p.tp.push ? attn_decode_gqa_kernel<GROUP, HD, true> : attn_decode_gqa_kernel<GROUP, HD, false>;
+cudaError_t launch_gqa_variant(const AttnParams &p, size_t smem, bool pdl, cudaStream_t s) {
+    auto kern = attn_decode_gqa_kernel<GROUP, HD>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    return launch_kernel(kern, dim3(p.n_kv_heads, p.n_splits, n_tokens), dim3(kThreads), smem, s, pdl, p);
+    return launch_kernel(kern, dim3(p.n_kv_heads, p.n_splits), dim3(kThreads), smem, s, pdl, p);
 }
 
 }  // namespace
@@ -301,9 +271,7 @@ cudaError_t launch_attn_decode(const AttnDecode &a, cudaStream_t s, uint64_t *la
     p.n_splits = a.n_splits;
     p.window = a.window;
     p.softcap = a.softcap;
-    p.pos_per_query = a.pos_per_query ? 1u : 0u;
-    p.kv_batch_stride = a.kv_batch_stride;
-    if ((a.pos_per_query || a.kv_batch_stride) && !a.gqa) return cudaErrorInvalidValue;
+    if (a.pos_per_query || a.kv_batch_stride || a.n_tokens > 1 || a.tp.push) return cudaErrorInvalidValue;  // launch_attn_cluster
     if (a.gqa) {
         if (!attn_gqa_supported(a.hd, a.n_heads, a.n_kv_heads) || a.n_splits > (uint32_t)kGqaMaxSplits) return cudaErrorInvalidValue;
         const uint32_t g = a.n_heads / a.n_kv_heads;
@@ -312,18 +280,12 @@ cudaError_t launch_attn_decode(const AttnDecode &a, cudaStream_t s, uint64_t *la
         if (mc < p.min_chunk) mc = p.min_chunk;
         p.max_chunk = ((mc + 3) / 4) * 4;
         const uint32_t nsl = kThreads / (a.hd / 4);
-        const size_t smem = ((size_t)g * a.hd + 2 * a.hd + 16 + (size_t)g * p.max_chunk + (size_t)nsl * g * a.hd +
+        const size_t smem = ((size_t)g * a.hd + 16 + (size_t)g * p.max_chunk + (size_t)nsl * g * a.hd +
                              2 * (size_t)g * kGqaMaxSplits) * sizeof(float);
         if (smem > 200 * 1024) return cudaErrorInvalidValue;
         *launches += 1;
-        p.q_stride = a.q_stride;
-        p.out_stride = a.out_stride;
-        p.tp = a.tp;
-        // several queries per launch: consecutive positions of one cache, which they only read, or (batched decode) each with a
-        // device position, a cache and new rows of its own
-        if (a.n_tokens > 1 && (a.k_new || a.pos_ptr) && !a.pos_per_query) return cudaErrorInvalidValue;
-        if (a.n_tokens > 1 && a.k_new && !a.kv_batch_stride) return cudaErrorInvalidValue;
-#define YULE_GQA_CASE(G, H) if (g == G && a.hd == H) return launch_gqa_variant<G, H>(p, smem, a.pdl, s, a.n_tokens)
+        if (a.k_new || a.pos_ptr || a.cos_table) return cudaErrorInvalidValue;
+#define YULE_GQA_CASE(G, H) if (g == G && a.hd == H) return launch_gqa_variant<G, H>(p, smem, a.pdl, s)
         YULE_GQA_CASE(1, 64); YULE_GQA_CASE(2, 64); YULE_GQA_CASE(4, 64); YULE_GQA_CASE(8, 64);
         YULE_GQA_CASE(1, 128); YULE_GQA_CASE(2, 128); YULE_GQA_CASE(4, 128); YULE_GQA_CASE(8, 128);
 #undef YULE_GQA_CASE

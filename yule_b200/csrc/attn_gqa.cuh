@@ -37,6 +37,7 @@ struct AttnParams {
     size_t kv_batch_stride;              // floats between the caches of consecutive queries (batched decode)
     uint32_t window;                     // sliding window (model_runner.rs:688-696), 0 = none
     float softcap;                       // attention logit softcap (model_runner.rs:716-721), 0 = none
+    uint32_t settled;                    // attn_cluster_kernel: position and cache rows may be read ahead of the dependency wait
     TpFuse tp;                           // tensor parallelism: the output also goes out as (value, epoch) pairs
     int *status;                         // bounded waits of the pair inputs (persistent decode kernel)
     long long wait_cycles;
@@ -194,31 +195,19 @@ __device__ __forceinline__ void attn_gqa_finish(const AttnParams &p, float *scra
     }
     if (tid == 0) tickets_z[kvh] = 0;  // ready for the next launch on this stream
 }
-// One (KV head, split) unit of work, by 256 threads (`tid` 0..255) that can meet at `sync()`.
-//   PAIRS  the query and the new K / V rows arrive as (value, epoch) pairs that are polled (persistent decode
-//          kernel); otherwise they are plain floats written by an earlier kernel.
-//   sm     dynamic shared memory of the unit (attn_gqa_smem_floats), s_last one more word
-//   store  store(i, v): element i of the [n_heads][HD] output of this query
-template <int GROUP, int HD, bool PAIRS, class Sync, class Store>
-__device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUnit &au, uint32_t kvh, uint32_t split, uint32_t tid,
-                                              float *sm, uint32_t *s_last, Sync sync, Store store) {
+// One (KV head, split) unit of work of a query whose rows are all in the caches, by the 256 threads of a CTA.
+//   sm     dynamic shared memory of the unit, s_last one more word
+template <int GROUP, int HD>
+__device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, uint32_t kvh, uint32_t split, uint32_t tid, float *sm, uint32_t *s_last) {
     constexpr int J = HD / 32;                               // 16-byte steps per lane and row
-    // query heads scored per pass over K: 16 float4 of queries in registers, 8 inside the persistent kernel (which
-    // has 128 registers per thread for everything and a tiny L1 behind its shared-memory carve-out: it must not spill)
-    constexpr int QREGS = PAIRS ? 8 : 16;
-    constexpr int GH = (GROUP * J > QREGS) ? (QREGS / J) : GROUP;
+    constexpr int GH = (GROUP * J > 16) ? (16 / J) : GROUP;  // query heads scored per pass over K: 16 float4 of queries in registers
     constexpr int HD4 = HD / 4;
     constexpr int NSL = kThreads / HD4;                      // position slices of the V pass
     constexpr int NOUT = (GROUP * HD + kThreads - 1) / kThreads;
     const uint32_t head0 = kvh * GROUP;
-    const uint32_t pos = au.pos;
-    float *const k_cache = au.k_cache;
-    float *const v_cache = au.v_cache;
-    const float *q_in = au.q_in;
-    float *scratch_z = au.scratch;
-    uint32_t *tickets_z = au.tickets;
-    const uint32_t seq = pos + 1;
-    const bool fused = PAIRS || au.k_new != nullptr;
+    const float *const k_cache = p.k_cache;
+    const float *const v_cache = p.v_cache;
+    const uint32_t seq = p.seq_len, pos = seq - 1;
     // Sliding window: the reference masks positions t < pos − window to −inf once pos >= window; they then carry
     // no weight, so the splits simply cover [begin, seq) instead of [0, seq).  With an attention softcap as well
     // the reference caps after masking (model_runner.rs:688-721), and cap·tanh(−inf / cap) is −cap, a finite
@@ -234,15 +223,13 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
     const uint32_t hi = lo + chunk < seq ? lo + chunk : seq;
     const int lane = tid & 31, wid = tid >> 5;
 
-    float *qs = sm;                               // GROUP × HD rotated queries
-    float *kcur = qs + GROUP * HD;                // HD: rotated K row of the current token
-    float *vcur = kcur + HD;                      // HD: V row of the current token
-    float *ml = vcur + HD;                        // (max, sum) per head, 16 floats
+    float *qs = sm;                               // GROUP × HD queries
+    float *ml = qs + GROUP * HD;                  // (max, sum) per head, 16 floats
     float *scores = ml + 16;                      // GROUP × max_chunk
     float *partial = scores + (size_t)GROUP * p.max_chunk;  // NSL × GROUP × HD
     // (the merge of attn_gqa_finish works in `partial` and the 2 × GROUP × kGqaMaxSplits floats behind it)
 
-    // The first K tile does not depend on the query: its loads go out before the RoPE prologue.
+    // the first K tile goes out before the queries are staged
     const int qtr = lane >> 3, l8 = lane & 7;
     auto k_row = [&](uint32_t tb) {
         const uint32_t t = tb + wid * 4 + qtr;
@@ -255,83 +242,8 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
         for (int j = 0; j < J; j++) kv_next[j] = *reinterpret_cast<const float4 *>(kp + j * 32);
     }
 
-    // RoPE as in apply_rope (model_runner.rs:277-293): products and sums rounded separately.
-    // Pair inputs: every load of this thread goes out before the first one is checked (an L2 round trip each).
-    constexpr int QIT = (GROUP * (HD / 2) + kThreads - 1) / kThreads;
-    uint2 pq[QIT][2] = {}, pk[2] = {}, pv = {};
-    // the rotation of this thread's pairs: plain loads, asked for before the polled ones (which nothing may overtake)
-    float rot_c[QIT], rot_s[QIT];
-#pragma unroll
-    for (int it = 0; it < QIT; it++) {
-        const uint32_t idx = tid + it * kThreads;
-        rot_c[it] = 1.f;
-        rot_s[it] = 0.f;
-        if (p.cos_table && idx < GROUP * (HD / 2)) {
-            rot_c[it] = p.cos_table[(size_t)pos * (HD / 2) + idx % (HD / 2)];
-            rot_s[it] = p.sin_table[(size_t)pos * (HD / 2) + idx % (HD / 2)];
-        }
-    }
-    if (PAIRS) {
-#pragma unroll
-        for (int it = 0; it < QIT; it++) {
-            const uint32_t idx = tid + it * kThreads;
-            if (idx < GROUP * (HD / 2)) {
-                pq[it][0] = pair_peek(au.q_pairs + (size_t)head0 * HD + 2 * idx);
-                pq[it][1] = pair_peek(au.q_pairs + (size_t)head0 * HD + 2 * idx + 1);
-            }
-        }
-        if (tid < HD / 2) {
-            pk[0] = pair_peek(au.k_pairs + (size_t)kvh * HD + 2 * tid);
-            pk[1] = pair_peek(au.k_pairs + (size_t)kvh * HD + 2 * tid + 1);
-        }
-        if (tid < HD) pv = pair_peek(au.v_pairs + (size_t)kvh * HD + tid);
-    }
-    auto k_at = [&](size_t i) {
-        if (!PAIRS) return au.k_new[i];
-        return pair_settle(pk[i & 1], au.k_pairs + i, au.in_epoch, p.status, p.wait_cycles);  // i = kvh·HD + 2·tid + {0, 1}
-    };
-    auto v_at = [&](size_t i) {
-        if (!PAIRS) return au.v_new[i];
-        return pair_settle(pv, au.v_pairs + i, au.in_epoch, p.status, p.wait_cycles);  // i = kvh·HD + tid
-    };
-#pragma unroll
-    for (int it = 0; it < QIT; it++) {
-        const uint32_t idx = tid + it * kThreads;
-        if (idx >= GROUP * (HD / 2)) break;
-        const uint32_t h = idx / (HD / 2), i = idx % (HD / 2);
-        const size_t qi = (size_t)(head0 + h) * HD + 2 * i;
-        float q0 = PAIRS ? pair_settle(pq[it][0], au.q_pairs + qi, au.in_epoch, p.status, p.wait_cycles) : q_in[qi];
-        float q1 = PAIRS ? pair_settle(pq[it][1], au.q_pairs + qi + 1, au.in_epoch, p.status, p.wait_cycles) : q_in[qi + 1];
-        if (p.cos_table) {
-            const float c = rot_c[it], sn = rot_s[it];
-            const float r0 = __fsub_rn(__fmul_rn(q0, c), __fmul_rn(q1, sn));
-            const float r1 = __fadd_rn(__fmul_rn(q0, sn), __fmul_rn(q1, c));
-            q0 = r0;
-            q1 = r1;
-            if (fused && h == 0) {
-                const float k0 = k_at((size_t)kvh * HD + 2 * i), k1 = k_at((size_t)kvh * HD + 2 * i + 1);
-                kcur[2 * i] = __fsub_rn(__fmul_rn(k0, c), __fmul_rn(k1, sn));
-                kcur[2 * i + 1] = __fadd_rn(__fmul_rn(k0, sn), __fmul_rn(k1, c));
-            }
-        } else if (fused && h == 0) {
-            kcur[2 * i] = k_at((size_t)kvh * HD + 2 * i);
-            kcur[2 * i + 1] = k_at((size_t)kvh * HD + 2 * i + 1);
-        }
-        qs[h * HD + 2 * i] = q0;
-        qs[h * HD + 2 * i + 1] = q1;
-    }
-    if (fused)
-        for (uint32_t d = tid; d < HD; d += kThreads) vcur[d] = v_at((size_t)kvh * HD + d);
-    sync();
-
-    // the split that owns the current position appends the new K and V rows (readers of this launch
-    // take that row from kcur / v_new, never from the cache)
-    if (fused && pos >= lo && pos < hi) {
-        for (uint32_t d = tid; d < HD; d += kThreads) {
-            k_cache[(size_t)pos * p.kv_stride + (size_t)kvh * HD + d] = kcur[d];
-            v_cache[(size_t)pos * p.kv_stride + (size_t)kvh * HD + d] = vcur[d];
-        }
-    }
+    for (uint32_t i = tid; i < GROUP * HD; i += kThreads) qs[i] = p.q[(size_t)head0 * HD + i];
+    __syncthreads();
 
     // scores; the loads of tile i+1 are in flight while tile i is multiplied
     const float scale = 1.0f / sqrtf((float)HD);
@@ -357,10 +269,6 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
                 const float *kp = k_row(tb + 32);
 #pragma unroll
                 for (int j = 0; j < J; j++) kv_next[j] = *reinterpret_cast<const float4 *>(kp + j * 32);
-            }
-            if (fused && t == pos) {
-#pragma unroll
-                for (int j = 0; j < J; j++) kv[j] = *reinterpret_cast<const float4 *>(kcur + j * 32 + l8 * 4);
             }
             float d[GH];
 #pragma unroll
@@ -391,7 +299,7 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
             }
         }
     }
-    sync();
+    __syncthreads();
 
     // softmax statistics: one warp per head
     for (int h = wid; h < GROUP; h += kThreads / 32) {
@@ -411,7 +319,7 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
             ml[2 * h + 1] = sum;
         }
     }
-    sync();
+    __syncthreads();
 
     // Σ_t e_t · V[t] for all GROUP heads from one read of V
     const uint32_t d4 = tid % HD4, slice = tid / HD4;
@@ -419,8 +327,7 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
 #pragma unroll
     for (int h = 0; h < GROUP; h++) acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
     auto v_row = [&](uint32_t t) {
-        return (fused && t == pos) ? reinterpret_cast<const float4 *>(vcur) + d4
-                                   : reinterpret_cast<const float4 *>(v_cache + (size_t)t * p.kv_stride + (size_t)kvh * HD) + d4;
+        return reinterpret_cast<const float4 *>(v_cache + (size_t)t * p.kv_stride + (size_t)kvh * HD) + d4;
     };
     uint32_t t = lo + slice;
     for (; t + 3 * NSL < hi; t += 4 * NSL) {  // four rows in flight
@@ -451,7 +358,7 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
     }
 #pragma unroll
     for (int h = 0; h < GROUP; h++) reinterpret_cast<float4 *>(partial)[((size_t)slice * GROUP + h) * HD4 + d4] = acc[h];
-    sync();
+    __syncthreads();
     float o[NOUT];
 #pragma unroll
     for (int k = 0; k < NOUT; k++) {
@@ -463,7 +370,8 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, const AttnUni
         }
     }
 
-    attn_gqa_finish<GROUP, HD>(p, scratch_z, tickets_z, kvh, split, eff, lo < hi, tid, o, ml, partial, s_last, sync, store);
+    attn_gqa_finish<GROUP, HD>(p, p.scratch, p.tickets, kvh, split, eff, lo < hi, tid, o, ml, partial, s_last, [] { __syncthreads(); },
+                               [&](uint32_t i, float v) { p.out[i] = v; });
 }
 
 // ── the same unit with its keys and values staged in shared memory ──────────────────────────────────────────────

@@ -430,6 +430,9 @@ struct AttnDecode {
     uint32_t window = 0;     // sliding window (yule-infer/src/model_runner.rs:688-696): positions < pos − window are not attended; 0 = none
     float softcap = 0.f;     // attention logit softcap (:716-721): score = cap · tanh(score / cap); 0 = none
     bool gqa = false;        // grouped-query kernel: one CTA per (KV head, split); n_splits from attn_gqa_pick_splits
+    // launch_attn_cluster: the position and the cache rows before it were written by launches that are over when the one before
+    // this one starts (the token before, in a graph of its own), so they may be read ahead of the dependency wait.
+    bool settled = false;
 };
 // Causal attention of n_seq sequences x n_tokens queries (attn_prefill.cu): row b·n_tokens + i of q / out is the query at
 // position pos0 + i of sequence b, whose caches lie b · kv_batch_stride floats on and hold positions [0, pos0 + n_tokens).
@@ -448,6 +451,11 @@ size_t attn_scratch_floats(uint32_t n_heads, uint32_t n_splits, uint32_t hd);
 uint32_t attn_pick_splits(uint32_t n_heads, uint32_t seq_len_hint, int sm_count);
 bool attn_decode_supported(uint32_t hd);
 cudaError_t launch_attn_decode(const AttnDecode &a, cudaStream_t s, uint64_t *launches);
+// A cluster of CTAs per (KV head, query), at long contexts several (attn_cluster.cu): n_splits is the number of clusters that
+// `scratch` has room for, `tickets` are n_kv_heads * kAttnMaxRanks words per query, and min_chunk is not used.
+constexpr uint32_t kAttnMaxRanks = 8;
+void attn_cluster_shape(uint32_t units, uint32_t hd, uint32_t max_seq_len, bool known_length, int sm_count, uint32_t *ranks, uint32_t *clusters);
+cudaError_t launch_attn_cluster(const AttnDecode &a, int sm_count, cudaStream_t s, uint64_t *launches);
 
 // Runner kernels that read the position from device memory (graph-replayable).
 cudaError_t launch_rope_kv_write(float *q, const float *k_tmp, const float *v_tmp, float *k_cache,

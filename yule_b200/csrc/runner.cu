@@ -512,9 +512,11 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches, bool 
         st.ok(launch_qmv_digits(f, sms, s, &st.n));
     };
 
+    // Without its own pick the step follows the sampler in one graph, which writes the position: nothing of the step may start before
+    // that is over, because the attention launches read the position ahead of their dependency wait (AttnDecode::settled).
     if (!(skip & 256))
         st.ok(launch_embed_gather((const uint8_t *)r->token_embd.buf.ptr, r->token_embd.type, dim, 0, tok_ptr,
-                                  r->hidden, s, &st.n, pdl));
+                                  r->hidden, s, &st.n, pdl && pick));
     // Gemma: embeddings scaled by sqrt(dim) (model_runner.rs:568-574)
     if (c.norm_weight_offset > 0.f)
         st.ok(launch_elementwise(kElemScale, r->hidden, nullptr, r->hidden, dim, sqrtf((float)dim), s, &st.n, pdl));
@@ -567,7 +569,8 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches, bool 
             a.window = c.sliding_window;
             a.softcap = c.attn_logit_softcap;
             if (folded(l, 0)) a.tp = push_of(r->x_pair_attn, qdim_l, l, 0);
-            if (!(skip & 4)) st.ok(launch_attn_decode(a, s, &st.n));
+            a.settled = true;
+            if (!(skip & 4)) st.ok(a.gqa ? launch_attn_cluster(a, sms, s, &st.n) : launch_attn_decode(a, s, &st.n));
         } else {
             if (!(skip & 2))
                 st.ok(launch_rope_kv_write(r->q, r->k_tmp, r->v_tmp, L.k_cache, L.v_cache, r->rope_cos, r->rope_sin,
@@ -873,7 +876,7 @@ int32_t ensure_pinned(yule_cuda_runner *r, size_t n_words) {
 // Tensor-parallel runs read the device status word every this many tokens and stop enqueuing once a bounded
 // wait has given up (the waits themselves return at once after the first failure).
 constexpr uint32_t kStatusCheckTokens = 32;
-constexpr uint32_t kPrefillChunk = 512, kPrefillMinTokens = 16, kPrefillMinChunk = 256;
+constexpr uint32_t kPrefillChunk = 512, kPrefillMinTokens = 16;
 // One GPU: passes of up to this many rows.  A launch's fixed part (about 10 us per GEMM) and the last, partly filled wave of
 // tiles count once per pass.
 constexpr uint32_t kPrefillMaxRows = 2048;
@@ -960,7 +963,7 @@ int32_t alloc_chunk_buffers(yule_cuda_runner *r, uint32_t C) {
     }
     if ((rc = alloc((size_t)C * (qdim / N), &r->pf_q)) || (rc = alloc((size_t)C * (kvdim / N), &r->pf_k)) ||
         (rc = alloc((size_t)C * (kvdim / N), &r->pf_v)) || (rc = alloc(C > c.max_seq_len ? C : c.max_seq_len, &tok_f)) ||
-        (rc = alloc((size_t)A * c.n_heads, &tick_f)) ||
+        (rc = alloc((size_t)A * c.n_heads * kAttnMaxRanks, &tick_f)) ||
         (rc = alloc((size_t)A * attn_scratch_floats(c.n_heads / N, r->pf_splits, hd) + 4, &r->pf_attn_scratch)) ||
         (rc = alloc((size_t)kRowsMatvecMax * dim, &r->pf_norm)) || (rc = ensure_pass_scratch(r, C)))
         return rc;
@@ -1286,12 +1289,12 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         a.kv_stride = kvdim_l;
         a.n_splits = r->pf_splits;
         a.max_seq_len = c.max_seq_len;
-        a.min_chunk = kPrefillMinChunk;
         a.gqa = true;
         a.n_tokens = ps.n_live;
         a.q_stride = qdim_l;
         a.out_stride = qdim;
-        if (!tiled) ok(launch_attn_decode(a, s, launches));
+        a.settled = ps.batch;
+        if (!tiled) ok(launch_attn_cluster(a, sms, s, launches));
         exchange(r->xb_att, qdim_l, qdim);
         prep(r->pf_att, qdim, nullptr, nullptr);
         lin(L.attn_output, dim_l, qdim, r->pf_x + (size_t)R * dim_l, dim, r->pf_x + (size_t)R * dim_l);  // x += Wo · attention
@@ -1616,7 +1619,7 @@ int32_t yule_cuda_runner_create(yule_cuda_ctx *ctx, const yule_runner_config *cf
                                                         ctx->prop.multiProcessorCount)
                                  : attn_pick_splits(c.n_heads, c.max_seq_len, ctx->prop.multiProcessorCount);
     A(attn_scratch_floats(c.n_heads, r->attn_splits, hd) + 4, &r->attn_scratch);
-    A(c.n_heads, &tmp);
+    A((size_t)c.n_heads * kAttnMaxRanks, &tmp);
     r->attn_tickets = (uint32_t *)tmp;  // zero-filled by the allocator
     A(4, &tmp);
     r->d_state = (uint32_t *)tmp;
