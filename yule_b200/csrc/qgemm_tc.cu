@@ -29,27 +29,31 @@
 //
 // One CTA per SM, 20 warps, persistent over the work items:
 //   warps 0-7   drain warps: tcgen05.ld of their 32 TMEM lanes × half of the columns after every
-//               stage, FMA by d (and −dmin) into registers; at the end of a tile scale, residual, store
+//               stage, FMA by d (and −dmin) into registers, two columns per instruction; at the end of a tile
+//               scale, residual, store
 //   warp  8     one thread: bulk copies (TMA engine) of the pre-arranged activation tiles
-//   warps 9, 11 one thread each: tcgen05.mma issue, even stages from one, odd stages from the other
-//               (a single thread issues about one MMA per 63 cycles, less than the tensor core
-//               takes); warp 9 also owns the TMEM allocation
+//   warps 9, 11 tcgen05.mma issue, even stages from one, odd stages from the other; warp 9 also owns
+//               the TMEM allocation
 //   warp  10    one thread: tiled TMA loads (cp.async.bulk.tensor.2d) of the raw Q4_K bytes, one
-//               128-row × 144-byte box per super-block, four boxes in flight (two at 128 activation
-//               rows, where the room goes to a third operand stage; three at 32); rows past the end of
-//               the matrix arrive as zeros
-//   warps 12-19 unpack Q4_K from that shared-memory copy → fp16 sc·q in the operand layout (about
-//               1.4 instructions per weight)
-// A stage is a 128-row × 64-column slab of W (16 KB) plus the matching hi and lo slabs of x; the last
-// stage of a super-block also carries the 4 KB m slab and the sub-block sums of x.  At 32 activation rows
-// a stage is two such column groups (a chain of eight MMAs, as at 128 rows, and half the hand-offs per
-// column), and three raw boxes are in flight.
+//               128-row × 144-byte box per super-block, three boxes in flight at 128 activation rows, six
+//               below; rows past the end of the matrix arrive as zeros
+//   warps 12-19 unpack Q4_K from that shared-memory copy → fp16 sc·q in tensor memory, where the MMA takes its
+//               W operand from: a row is a lane, a column two weights, and 64 weights of a row are 32 columns
+// A stage is a 128-row × 64-column slab of W plus the matching hi and lo slabs of x in shared memory; the last
+// stage of a super-block also carries the 4 KB m slab (shared memory) and the sub-block sums of x.  At 32 activation rows
+// a stage is two such column groups (a chain of eight MMAs, as at 128 rows, and half the hand-offs per column).  Tensor memory holds
+// four stages of W and behind them a ring of accumulators, three of 128 columns (four of 64 at 32 rows), in which the min term of a
+// super-block takes its turn like a stage.
 // One launch can run over up to three matrices that read the same activations (Q/K/V; gate/up): their row
 // tiles are numbered one after the other.
-// Operands use the no-swizzle K-major core-matrix layout: 8 rows × 16 bytes per core matrix,
-// core matrices of one 8-column step contiguous along the rows.  Inside a core-matrix row the eight
-// columns sit in the order 0,2,1,3,4,6,5,7 (the order in which nibble pairs fall out of a 32-bit
-// word); both operands use it, so the products pair up correctly.
+// The activation operand is the no-swizzle K-major core-matrix layout: 8 rows × 16 bytes per core matrix,
+// core matrices of one 8-column step contiguous along the rows.  Of eight columns the order is
+// 0,2,1,3,4,6,5,7 (the order in which nibble pairs fall out of a 32-bit word) in both operands, so the products pair up correctly.
+//
+// What bounds it, at 128 activation rows, clocks per stage of an SM: the tensor pipe 512 (+ 16 for the min term).  With W in shared memory a
+// stage moved 121 KB through it (970 clocks) and took 1400.  Measured with one role's work taken out at a time, no role alone bounds it
+// now: hand-offs and issue slots do (a stage takes some 850 clocks, the tensor pipe is busy for 60 % of them, the issue slots for 59 %).  8192x8192 by 256 rows 113 -> 78 us (re-layout included);
+// 32 rows 32.6 -> 26.4; the 8B model's 2048-token prompt 115.7 -> 94.2 ms.
 //
 // Every wait is bounded: a pipeline that stops making progress sets the context's status word,
 // raises the CTA's abort flag, lets all roles fall through to the common exit and frees its TMEM.
@@ -76,32 +80,21 @@ constexpr int kEpiWarps = 8, kProdWarps = 8;
 constexpr int kLoaderWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kRawWarp = kEpiWarps + 2, kMmaWarp2 = kEpiWarps + 3,
               kFirstProdWarp = kEpiWarps + 4;
 constexpr int kGemmThreads = (kEpiWarps + 4 + kProdWarps) * 32;  // 640
-constexpr int kMaxStages = 6;
-#ifndef YULE_GEMM_RAW_SLOTS
-#define YULE_GEMM_RAW_SLOTS 4
-#endif
-constexpr int kRawSlots = YULE_GEMM_RAW_SLOTS;                       // super-blocks of raw Q4_K bytes in flight per CTA (at most)
-// At 128 activation rows a stage is 56 KB: two raw slots instead of four make room for a third stage, which together
-// with the third accumulator set lets the unpacking, MMA-issuing and drain roles overlap.
-// At 32 rows a stage is two column groups wide (53 KB): three raw slots leave room for three of them.
-#ifndef YULE_GEMM_WIDE_32
-#define YULE_GEMM_WIDE_32 1   // two column groups per stage at 32 activation rows
-#endif
-#ifndef YULE_GEMM_RAW_SLOTS_32
-#define YULE_GEMM_RAW_SLOTS_32 (YULE_GEMM_WIDE_32 ? 3 : 4)
-#endif
-__host__ __device__ constexpr uint32_t raw_slots_for(uint32_t bn) {
-    return bn >= 128 ? 2u : (bn <= 32 ? (uint32_t)YULE_GEMM_RAW_SLOTS_32 : (uint32_t)(kRawSlots < 4 ? kRawSlots : 4));
-}
+constexpr int kLaunchRegs = 96;  // registers per thread that 640 threads are launched with
+constexpr int kDrainRegs = 144, kControlRegs = 32, kProdRegs = 80;
+static_assert(kEpiWarps * kDrainRegs + 4 * kControlRegs + kProdWarps * kProdRegs <= (kEpiWarps + 4 + kProdWarps) * kLaunchRegs, "register split");
+constexpr uint32_t kStages = 4;  // of the operand ring: W in tensor memory, x in shared memory
+// Super-blocks of raw Q4_K bytes in flight per CTA: what the activation stages leave room for
+constexpr uint32_t kRawSlots = 6;
+__host__ __device__ constexpr uint32_t raw_slots_for(uint32_t bn) { return bn >= 128 ? 3u : kRawSlots; }
 // 64-column groups of W per stage.  The exact kernel at 32 activation rows takes two: its MMAs are narrow and its
 // drains short, so the waits, fences and barrier arrivals of a stage, not its work, set the pace, and a stage of
 // twice the columns halves them.  A chain is then eight MMAs (one per 16 columns against hi | lo), the same length as
 // at 128 rows.
 __host__ __device__ constexpr uint32_t groups_per_stage(uint32_t bn, bool generic) {
-    return (YULE_GEMM_WIDE_32 && !generic && bn <= 32) ? 2u : 1u;
+    return (!generic && bn <= 32) ? 2u : 1u;
 }
 constexpr uint32_t kRawBytes = kBM * 144;          // one super-block of 128 rows: 18 KB
-constexpr uint32_t kABytes = kBM * kBK * 2;  // the W slab of a stage: 16 KB
 constexpr float kSumScale = 1.0f / 32.0f;     // the sub-block sums of x are stored divided by 32
 // 1 + 2^-23: what truncation takes of a stage's sum on average (measured 0.9e-7 of the result, exact kernel 0.7e-7, at 32 rows
 // 1.2e-7) is given back.
@@ -109,15 +102,6 @@ constexpr float kTruncation = 1.00000012f;
 constexpr float kGenericWScale = 1024.f;      // generic kernel: weights are scaled by 2^10 before the fp16 hi/lo split
 constexpr uint32_t kAmBytes = kBM * 16 * 2;  // the m slab of a super-block: 128 rows × 16 columns, 4 KB
 constexpr long long kWaitCycles = 2000000000LL;  // ~1 s: far beyond any real stall
-
-// Cycle counters of CTA 0's roles (YULE_GEMM_PROF=1 prints them after the launch): a timing aid, compiled in only
-// with -DYULE_GEMM_PROFILE (its counters cost the drain warps registers they do not have to spare).
-#ifdef YULE_GEMM_PROFILE
-constexpr bool kProfile = true;
-#else
-constexpr bool kProfile = false;
-#endif
-__device__ long long g_gemm_prof[16];
 
 constexpr int kGemmSegs = 3;  // matrices that share their activation tiles (Q/K/V; gate/up) in one launch
 struct GemmMaps {
@@ -134,7 +118,7 @@ struct GemmParams {
     uint32_t n_seg;
     uint32_t n_cols, n_tokens;
     uint32_t bn;           // activation rows per tile: 32, 64 or 128
-    uint32_t n_mtiles, n_ntiles, stages;
+    uint32_t n_mtiles, n_ntiles;
     uint32_t ksplit, sb_per;  // split of the columns: `ksplit` work items per tile, `sb_per` super-blocks each (the last may be shorter)
     float *split_part;        // ksplit > 1: per work item a [bn][128] block of partial results
     uint32_t *split_tickets;  // ksplit > 1: per (tile, drain warp) the number of items that have stored theirs; left at zero
@@ -145,9 +129,6 @@ struct GemmParams {
     uint32_t raw_chunks;   // generic kernel: 16-byte chunks copied per row and unit
     uint32_t raw_ring_bytes;  // generic kernel: two slots of 128 rows
     float out_scale;       // kTruncation; generic kernel: / kGenericWScale
-    uint32_t prof;         // timing aid: record cycle counters of CTA 0
-    uint32_t skip;         // timing aid (YULE_GEMM_SKIP, bits): 1 no unpacking, 2 no MMAs, 4 no draining, 8 no activation copies,
-                           // 64 no weight copies, 256 the MMA threads wait for their own commits; results meaningless
     int *status;
 };
 
@@ -162,14 +143,15 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+constexpr uint32_t kSuspendNs = 20000;  // a waiting warp sleeps up to this long instead of spending issue slots on polls
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "n"(kSuspendNs)
         : "memory");
     return ok != 0;
 }
@@ -201,6 +183,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
 
+// True in one lane of the warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one)::"memory");
+    return one != 0;
+}
+
 // D[tmem] (+)= A[smem] · B[smem], fp16 operands, fp32 accumulate, one CTA.
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -210,16 +199,26 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// The same with the accumulate flag known at compile time (an immediate: no register, a predicate ptxas can fold).
+// A from tensor memory (lane = row, a column two fp16 values), the accumulate flag known at compile time.
 template <int ACC>
-__device__ __forceinline__ void umma_f16_c(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(ACC)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(ACC)
         : "memory");
 }
+// 4 or 8 words per lane into as many columns of the warp's 32 lanes; in tensor memory after tmem_st_wait().
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint4 &v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4 &a, const uint4 &b) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // The mbarrier gets one arrival when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -235,16 +234,45 @@ __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t *v) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t *v) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
+          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr)
         : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Two fp32 operations per instruction, each rounded as the single one is.  The drain's arithmetic and the unpacking share the issue
+// slots of an SM with everything else; a stage has to get by with fewer of them than its MMAs take clocks.
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // The eight 6-bit scales and mins of a super-block from its 12 packed bytes
@@ -510,6 +538,16 @@ __device__ __forceinline__ bool unpack32(const unsigned char *unit, uint32_t typ
     return false;
 }
 
+// At 128 activation rows the drain warps hold 64 sums and 32 fresh accumulators each: registers move to them from the others.  Called
+// by every warp of a warpgroup.
+template <int BN, int REGS>
+__device__ __forceinline__ void split_registers() {
+    if constexpr (BN == 128) {
+        if constexpr (REGS > kLaunchRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
+    }
+}
+
 // Position in the stage ring without a runtime division (an integer division runs on the same
 // slow pipe as the half conversions): slot and phase parity, advanced once per stage.
 struct RingPos {
@@ -578,28 +616,23 @@ struct RowBlock {
 template <int BN, bool GENERIC>
 struct Tile {
     // Up to 64 activation rows the hi and lo terms of the activations sit side by side as one operand of 2·BN rows:
-    // one MMA per 16 columns instead of two (an MMA reads its 4 KB of W from shared memory whatever its width, which
-    // is what a narrow MMA costs), the two products land in neighbouring accumulator columns and the drain adds them.
+    // one MMA per 16 columns instead of two, the two products land in neighbouring accumulator columns and the drain adds them.
     static constexpr bool MERGED = BN <= 64;
-    // TMEM accumulator sets in flight.  Up to 64 rows every set has its own min accumulator.  At 128 rows the min
-    // accumulator (written by one MMA per super-block, read by the drain of that stage) is shared by all sets, which
-    // leaves room for three main accumulators instead of two: the MMA of stage i + 3 waits for the drain of stage i,
-    // which is after the drain of any earlier min term.  With two sets the issue-then-drain cycle of a set (about
-    // 600 cycles each at 128 rows) bounded a stage at 750 cycles whatever the other buffers.
-    static constexpr bool SHARED_MIN = BN == 128;
-    static constexpr uint32_t NBUF = BN == 32 ? 4 : (SHARED_MIN ? (GENERIC ? 4 : 3) : 2);
+    // Tensor memory: accumulators in a ring, behind them the W operand of every stage.  The min term of a super-block (exact kernel)
+    // takes a place in the ring of accumulators like a stage does.
     static constexpr uint32_t kMainCols = MERGED ? 2 * BN : BN;
-    static constexpr uint32_t kBufCols = SHARED_MIN ? kMainCols : kMainCols + BN;  // main (+ min) accumulator of a set
-    static constexpr uint32_t kMinBase = SHARED_MIN ? 3 * kMainCols : kMainCols;   // shared: column 384; else behind the set's main
-    static constexpr uint32_t kTmemCols = 512;               // allocated as a power of two
     static constexpr uint32_t CW = BN / 2;                   // columns per drain warp
     static constexpr uint32_t kXHalfBytes = BN * kBK * 2;    // one fp16 term of the activation slab
     static constexpr uint32_t kBmBytes = BN * 16 * 2;        // sub-block sums of x: BN rows × (8 hi + 8 lo)
     static constexpr uint32_t KG = groups_per_stage(BN, GENERIC);  // 64-column groups per stage
     static constexpr uint32_t SPB = 4 / KG;                        // stages per super-block
-    // stage (exact):   W (KG groups) | m | KG × (x_hi | x_lo) | sums   (everything after m arrives in one bulk copy)
-    // stage (generic): W_hi | W_lo | x_hi | x_lo
-    static constexpr uint32_t kOffAm = KG * kABytes, kOffX = GENERIC ? 2 * kABytes : KG * kABytes + kAmBytes;
+    static constexpr uint32_t kACols = (GENERIC ? 2 : 1) * KG * kBK / 2;  // tensor-memory columns of a stage's W (generic: hi, then lo)
+    static constexpr uint32_t NBUF = (512 - kStages * kACols) / kMainCols;
+    static constexpr uint32_t kABase = NBUF * kMainCols;
+    static_assert(NBUF >= (GENERIC ? 2 : 3) && kABase + kStages * kACols <= 512, "tensor memory");
+    // stage (exact):   m | KG × (x_hi | x_lo) | sums   (everything after m arrives in one bulk copy)
+    // stage (generic): x_hi | x_lo
+    static constexpr uint32_t kOffX = GENERIC ? 0u : kAmBytes;
     static constexpr uint32_t kOffSums = kOffX + KG * 2 * kXHalfBytes;
     static constexpr uint32_t kStageBytes = kOffSums + (GENERIC ? 0u : kBmBytes);
     static constexpr uint32_t kRaw = raw_slots_for(BN);
@@ -614,21 +647,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
     constexpr uint32_t NBUF = T::NBUF, CW = T::CW, kXHalfBytes = T::kXHalfBytes, kStageBytes = T::kStageBytes;
     extern __shared__ __align__(128) unsigned char smem[];
     yule_pdl_launch_dependents();
-    const uint32_t skip = kProfile ? p.skip : 0u;  // the timing aids exist only in profiling builds
-    const long long t_entry = (kProfile && p.prof) ? clock64() : 0;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char *tail = smem + (size_t)p.stages * kStageBytes;
-    unsigned char *raw = tail;                               // kRawSlots boxes of raw Q4_K bytes
-    uint64_t *bars = reinterpret_cast<uint64_t *>(tail + (GENERIC ? p.raw_ring_bytes : T::kRawRingBytes));  // full[6] empty[6] acc_full[4] acc_empty[4] raw_full[4] raw_empty[4]
-    const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kMaxStages;
-    const uint32_t bar_acc_full = bar_empty + 8 * kMaxStages, bar_acc_empty = bar_acc_full + 32;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (the shuffles tell the compiler what is the same in a warp)
+    unsigned char *raw = smem + (size_t)kStages * kStageBytes;  // boxes of raw Q4_K bytes
+    uint64_t *bars = reinterpret_cast<uint64_t *>(raw + (GENERIC ? p.raw_ring_bytes : T::kRawRingBytes));  // full[4] empty[4] acc_full[4] acc_empty[4] raw_full[6] raw_empty[6]
+    const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kStages;
+    const uint32_t bar_acc_full = bar_empty + 8 * kStages, bar_acc_empty = bar_acc_full + 32;
     const uint32_t bar_raw_full = bar_acc_empty + 32, bar_raw_empty = bar_raw_full + 8 * kRawSlots;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kMaxStages + 8 + 2 * kRawSlots);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 8 + 2 * kRawSlots);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    volatile uint32_t *mma_progress = reinterpret_cast<volatile uint32_t *>(tmem_slot + 2);  // per MMA thread: stages seen full
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < p.stages; s++) {
+        for (uint32_t s = 0; s < kStages; s++) {
             mbar_init(bar_full + 8 * s, kProdWarps + 1);  // one arrival per producer warp + the loader's expect_tx
             mbar_init(bar_empty + 8 * s, 1);              // tcgen05.commit
         }
@@ -641,33 +670,33 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             mbar_init(bar_raw_empty + 8 * b, kProdWarps);  // every producer warp is done with the box
         }
         *abort_flag = 0;
-        mma_progress[0] = mma_progress[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
     }
     if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T::kTmemCols)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     const uint32_t n_items = p.n_mtiles * p.n_ntiles * p.ksplit;
     const uint32_t bpr = p.n_cols / 256;  // super-blocks per row
 
+    if (warp >= kEpiWarps && warp < kFirstProdWarp) {
+    split_registers<BN, kControlRegs>();  // (one instruction for the warpgroup)
     if (warp == kLoaderWarp) {
         if (lane == 0) {
             yule_pdl_wait();  // the activation tiles come from the kernel before this one
-            uint32_t it = 0;
             RingPos ring;
             bool ok = true;
             for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 const Item wi = decode_item(p, item, bpr);
                 const unsigned char *src = reinterpret_cast<const unsigned char *>(p.xb) + (size_t)wi.nt * bpr * T::kSuperBytes;
-                for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, it++, ring.advance(p.stages)) {
+                for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
                     const uint32_t s = ring.s, ph = ring.ph;
                     if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, p.status)) {
                         ok = false;
@@ -676,10 +705,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                     const uint32_t g = kb % T::SPB;
                     const uint32_t bytes = T::KG * 2 * kXHalfBytes + ((!GENERIC && g == T::SPB - 1) ? T::kBmBytes : 0u);  // the sums ride with the last stage
                     const uint32_t dst = smem_u32(smem + (size_t)s * kStageBytes + T::kOffX);
-                    if (skip & 8u) {
-                        mbar_arrive(bar_full + 8 * s);
-                        continue;
-                    }
                     mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                                  "l"(src + (size_t)(kb / T::SPB) * T::kSuperBytes + (size_t)g * T::KG * 2 * kXHalfBytes), "r"(bytes),
@@ -689,120 +714,96 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             }
         }
     } else if (warp == kMmaWarp || warp == kMmaWarp2) {
-        if (lane == 0) {
-            const uint32_t parity_of_mine = warp == kMmaWarp ? 0u : 1u;  // this thread issues the stages with it % 2 == parity
-            // fp16 × fp16 → fp32, both operands K-major, M = 128, N = BN
-            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-            [[maybe_unused]] constexpr uint32_t idesc2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // N = 2·BN
-            constexpr uint32_t x_lbo = BN * 16;  // bytes of one 8-column step of an activation slab (of its hi or lo rows)
-            uint32_t it = 0;
-            bool ok = true;
-            RingPos ring;
-            long long tw0 = 0, tw1 = 0, ti = 0, tc = 0;
-            const long long tstart = (kProfile && p.prof) ? clock64() : 0;
-            for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const Item wi = decode_item(p, item, bpr);
-                for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, it++, ring.advance(p.stages)) {
-                    const bool mine = (it & 1u) == parity_of_mine;  // the threads alternate stages
-                    const uint32_t s = ring.s, ph = ring.ph;
-                    const uint32_t buf = it % NBUF, aph = (it / NBUF) & 1u;
-                    const long long c0 = (kProfile && p.prof) ? clock64() : 0;
-                    if (mine && !(skip & 16u) && !mbar_wait(bar_acc_empty + 8 * buf, aph ^ 1u, abort_flag, p.status)) {
-                        ok = false;
-                        break;
-                    }
-                    if (!mine) continue;
-                    const long long c1 = (kProfile && p.prof) ? clock64() : 0;
-                    // A parity wait only tells phase k of a barrier from phase k - 1.  The previous use of this
-                    // stage may belong to the other thread: wait until it has seen that phase complete, so that
-                    // this thread never asks for a phase two ahead of the barrier's.
-                    if (it >= p.stages && ((it - p.stages) & 1u) != parity_of_mine) {
-                        const long long t0 = clock64();
-                        while (mma_progress[parity_of_mine ^ 1u] < it - p.stages + 1) {
-                            if (*abort_flag || clock64() - t0 > kWaitCycles) {
-                                *abort_flag = 1;
-                                atomicExch(p.status, kStatusGemmTimeout);
-                                ok = false;
-                                break;
-                            }
-                        }
-                        if (!ok) break;
-                    }
-                    if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, p.status)) {
-                        ok = false;
-                        break;
-                    }
-                    mma_progress[parity_of_mine] = it + 1;
-                    const long long c2 = (kProfile && p.prof) ? clock64() : 0;
-                    tw0 += c1 - c0;
-                    tw1 += c2 - c1;
-                    tc_fence_after();
-                    const uint32_t d_main = tmem_base + buf * T::kBufCols;
-                    [[maybe_unused]] const uint32_t d_min = T::SHARED_MIN ? tmem_base + T::kMinBase : d_main + T::kMinBase;
-                    const uint32_t a = smem_u32(smem + (size_t)s * kStageBytes);
-                    const uint32_t x_hi = a + T::kOffX;
-                    // One descriptor per operand and stage; the 16-column steps are constants added to its address field (the
-                    // issuing thread's own instruction stream, not the tensor pipe, bounded the MMA rate).
-                    const uint64_t da0 = smem_desc(a, 2048, 128);
-                    const uint64_t db0 = T::MERGED ? smem_desc(x_hi, 2 * x_lbo, 128) : smem_desc(x_hi, x_lbo, 128);
-                    // The tensor core truncates when it adds to an accumulator, which costs a part of what the accumulator holds.  So
-                    // the products with lo terms go first, or to the columns of their own: the hi·hi sums see four additions (eight at two
-                    // column groups per stage), not eight or twelve.
-                    auto steps = [&](auto f) {
-                        f(std::integral_constant<uint32_t, 0>{});
-                        f(std::integral_constant<uint32_t, 1>{});
-                        f(std::integral_constant<uint32_t, 2>{});
-                        f(std::integral_constant<uint32_t, 3>{});
-                        if constexpr (T::KG == 2) {  // the second group's slabs follow the first's in both operands
-                            f(std::integral_constant<uint32_t, 4>{});
-                            f(std::integral_constant<uint32_t, 5>{});
-                            f(std::integral_constant<uint32_t, 6>{});
-                            f(std::integral_constant<uint32_t, 7>{});
-                        }
-                    };
-                    if (!(skip & 2u)) {
-                        if constexpr (T::MERGED) {
-                            steps([&](auto k16c) {
-                                constexpr uint32_t k16 = decltype(k16c)::value;
-                                const uint64_t da = da0 + (uint64_t)((k16 * 4096u) >> 4);
-                                // rows [0, BN) of an 8-column step are the hi terms, rows [BN, 2·BN) the lo terms
-                                const uint64_t db = db0 + (uint64_t)((k16 * 4u * x_lbo) >> 4);
-                                umma_f16_c<(k16 != 0)>(d_main, da, db, idesc2);  // every stage starts a fresh accumulator
-                                if (GENERIC)  // the lo term of the weights against the hi term of the activations: beside the other small products
-                                    umma_f16_c<1>(d_main + BN, da + (uint64_t)(kABytes >> 4), db, idesc);
-                            });
-                        } else {
-                            steps([&](auto k16c) {
-                                constexpr uint32_t k16 = decltype(k16c)::value;
-                                const uint64_t da = da0 + (uint64_t)((k16 * 4096u) >> 4), dbh = db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4);
-                                umma_f16_c<(k16 != 0)>(d_main, da, dbh + (uint64_t)(kXHalfBytes >> 4), idesc);  // every stage starts a fresh accumulator
-                                if (GENERIC)  // the lo term of the weights against the hi term of the activations
-                                    umma_f16_c<1>(d_main, da + (uint64_t)(kABytes >> 4), dbh, idesc);
-                            });
-                            steps([&](auto k16c) {
-                                constexpr uint32_t k16 = decltype(k16c)::value;
-                                umma_f16_c<1>(d_main, da0 + (uint64_t)((k16 * 4096u) >> 4), db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4), idesc);
-                            });
-                        }
-                    }
-                    if (!GENERIC && kb % T::SPB == T::SPB - 1)  // Σ_s m_s · (sum of x over sub-block s), hi and lo sums side by side
-                        umma_f16(d_min, smem_desc(a + T::kOffAm, 2048, 128), smem_desc(a + T::kOffSums, x_lbo, 128), idesc, 0u);
-                    const long long c3 = (kProfile && p.prof) ? clock64() : 0;
-                    umma_commit(bar_empty + 8 * s);       // the slabs may be overwritten once these MMAs are done
-                    if (!(skip & 32u)) umma_commit(bar_acc_full + 8 * buf);  // and the accumulators may be drained
-                    if (skip & 256u) mbar_wait(bar_empty + 8 * s, ph, abort_flag, p.status);  // timing aid: the commit's own latency, charged to `commit`
-                    const long long c4 = (kProfile && p.prof) ? clock64() : 0;
-                    ti += c3 - c2;
-                    tc += c4 - c3;
+        // The whole warp goes through the loop, so that addresses and descriptors are uniform registers, and one lane issues: with the loop
+        // in one lane every MMA moved its operands there first, which took the issuing thread 47 clocks an MMA alone and 140 beside the
+        // other roles.  The warps alternate stages, so that one waits, fences and commits while the other's MMAs run.
+        //   A parity wait cannot tell a phase from the one two before it, and need not: a stage slot always belongs to the same warp (an
+        // even number of slots), and of an accumulator slot's uses a warp skips so few that the drain of the use before the one it asks
+        // for is known to be over: drains end in order, and it has waited for one that is at most NBUF + 3 uses back (NBUF >= 3), or
+        // NBUF + 2 where no min term sits between the stages (NBUF >= 2).
+        const uint32_t mine = warp == kMmaWarp ? 0u : 1u;
+        // fp16 × fp16 → fp32, both operands K-major, M = 128, N = BN
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+        [[maybe_unused]] constexpr uint32_t idesc2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // N = 2·BN
+        constexpr uint32_t x_lbo = BN * 16;  // bytes of one 8-column step of an activation slab (of its hi or lo rows)
+        bool ok = true;
+        RingPos ring, acc;
+        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            const Item wi = decode_item(p, item, bpr);
+            for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
+                const uint32_t s = ring.s;
+                if ((kb & 1u) != mine) {  // (a super-block has an even number of stages)
+                    acc.advance(NBUF);
+                    if (!GENERIC && kb % T::SPB == T::SPB - 1) acc.advance(NBUF);
+                    continue;
                 }
-            }
-            if ((kProfile && p.prof) && blockIdx.x == 0 && warp == kMmaWarp) {
-                g_gemm_prof[0] = clock64() - tstart;
-                g_gemm_prof[1] = tw0;
-                g_gemm_prof[2] = tw1;
-                g_gemm_prof[3] = ti;
-                g_gemm_prof[4] = tc;
-                g_gemm_prof[5] = it;
+                ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status) && mbar_wait(bar_full + 8 * s, ring.ph, abort_flag, p.status);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d_main = tmem_base + acc.s * T::kMainCols;
+                const uint32_t stage = smem_u32(smem + (size_t)s * kStageBytes);
+                const uint32_t x_hi = stage + T::kOffX, w0 = tmem_base + T::kABase + s * T::kACols;
+                // One descriptor per stage; the 16-column steps are constants added to its address field (the
+                // issuing thread's own instruction stream, not the tensor pipe, can bound the MMA rate).
+                const uint64_t db0 = T::MERGED ? smem_desc(x_hi, 2 * x_lbo, 128) : smem_desc(x_hi, x_lbo, 128);
+                // The tensor core truncates when it adds to an accumulator, which costs a part of what the accumulator holds.  So
+                // the products with lo terms go first, or to the columns of their own: the hi·hi sums see four additions (eight at two
+                // column groups per stage), not eight or twelve.
+                auto steps = [&](auto f) {
+                    f(std::integral_constant<uint32_t, 0>{});
+                    f(std::integral_constant<uint32_t, 1>{});
+                    f(std::integral_constant<uint32_t, 2>{});
+                    f(std::integral_constant<uint32_t, 3>{});
+                    if constexpr (T::KG == 2) {  // the second group's slabs follow the first's in both operands
+                        f(std::integral_constant<uint32_t, 4>{});
+                        f(std::integral_constant<uint32_t, 5>{});
+                        f(std::integral_constant<uint32_t, 6>{});
+                        f(std::integral_constant<uint32_t, 7>{});
+                    }
+                };
+                constexpr uint32_t w_lo = T::kACols / 2;  // generic: the columns of the weights' lo terms
+                if (elect_one()) {
+                    if constexpr (T::MERGED) {
+                        steps([&](auto k16c) {
+                            constexpr uint32_t k16 = decltype(k16c)::value;
+                            // rows [0, BN) of an 8-column step are the hi terms, rows [BN, 2·BN) the lo terms
+                            const uint64_t db = db0 + (uint64_t)((k16 * 4u * x_lbo) >> 4);
+                            umma_f16_ts<(k16 != 0)>(d_main, w0 + 8 * k16, db, idesc2);  // every stage starts a fresh accumulator
+                            if (GENERIC)  // the lo term of the weights against the hi term of the activations: beside the other small products
+                                umma_f16_ts<1>(d_main + BN, w0 + w_lo + 8 * k16, db, idesc);
+                        });
+                    } else {
+                        steps([&](auto k16c) {
+                            constexpr uint32_t k16 = decltype(k16c)::value;
+                            const uint64_t dbh = db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4);
+                            umma_f16_ts<(k16 != 0)>(d_main, w0 + 8 * k16, dbh + (uint64_t)(kXHalfBytes >> 4), idesc);  // every stage starts a fresh accumulator
+                            if (GENERIC)  // the lo term of the weights against the hi term of the activations
+                                umma_f16_ts<1>(d_main, w0 + w_lo + 8 * k16, dbh, idesc);
+                        });
+                        steps([&](auto k16c) {
+                            constexpr uint32_t k16 = decltype(k16c)::value;
+                            umma_f16_ts<1>(d_main, w0 + 8 * k16, db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4), idesc);
+                        });
+                }
+                umma_commit(bar_acc_full + 8 * acc.s);  // the accumulators may be drained once these MMAs are done
+                if (GENERIC || kb % T::SPB != T::SPB - 1) umma_commit(bar_empty + 8 * s);  // and the operands overwritten
+                }
+                __syncwarp();
+                acc.advance(NBUF);
+                if (!GENERIC && kb % T::SPB == T::SPB - 1) {  // Σ_s m_s · (sum of x over sub-block s), hi and lo sums side by side
+                    ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        umma_f16(tmem_base + acc.s * T::kMainCols, smem_desc(stage, 2048, 128), smem_desc(stage + T::kOffSums, x_lbo, 128), idesc, 0u);
+                        umma_commit(bar_acc_full + 8 * acc.s);
+                        umma_commit(bar_empty + 8 * s);
+                    }
+                    __syncwarp();
+                    acc.advance(NBUF);
+                }
             }
         }
     } else if (warp == kRawWarp) {
@@ -813,10 +814,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
                 if (!mbar_wait(bar_raw_empty + 8 * slot, ph ^ 1u, abort_flag, p.status)) break;
                 const uint32_t x = walk.sb * 144u, y = walk.mt * kBM;  // byte column (a multiple of 16), first row
-                if (skip & 64u) {  // timing aid: no raw bytes
-                    mbar_arrive(bar_raw_full + 8 * slot);
-                    continue;
-                }
                 mbar_arrive_expect_tx(bar_raw_full + 8 * slot, kRawBytes);
                 asm volatile(
                     "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -825,7 +822,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                     : "memory");
             }
         }
+    }
     } else if (warp >= kFirstProdWarp) {
+        split_registers<BN, kProdRegs>();
         const uint32_t ptid = threadIdx.x - kFirstProdWarp * 32;  // 0..255
         const uint32_t r = ptid & 127u, hf = ptid >> 7;           // row of the tile, which 16 bytes of the 32
         if (GENERIC) {
@@ -835,7 +834,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             // one being unpacked; thread (r, hf) then dequantises columns [32·hf, 32·hf + 32) of every stage for
             // row r from that copy with the arithmetic of the bit-exact per-element routines, scales by 2^10 and
             // splits into fp16 hi + lo.
-            const uint32_t in_core = (r >> 3) * 128 + (r & 7u) * 16;
+            const uint32_t w_at = tmem_base + T::kABase + ((warp & 3u) << 21) + hf * 16;  // this warp's lanes, this thread's columns of a stage
             const uint32_t ub = p.unit_bytes, rstride = p.raw_stride, c16 = p.raw_chunks;
             const uint32_t slot_bytes = kBM * rstride;
             auto unit_start = [&](const UnitWalk &w, uint32_t tile_row) {  // address of row `tile_row`'s bytes of the unit
@@ -876,39 +875,45 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 asm volatile("bar.sync 2, 256;" ::: "memory");         // and everyone else's
                 const bool live = cur.mt * kBM + r < p.n_rows[cur.seg];
                 const unsigned char *rawrow = raw + (size_t)(u & 1u) * slot_bytes + (size_t)r * rstride + (unit_start(cur, r) & 15u);
-                for (uint32_t g = 0; g < 4 && ok; g++, ring.advance(p.stages)) {
-                    if (!mbar_wait(bar_empty + 8 * ring.s, ring.ph ^ 1u, abort_flag, p.status)) {
-                        ok = false;
-                        break;
-                    }
-                    unsigned char *a_hi = smem + (size_t)ring.s * kStageBytes, *a_lo = a_hi + kABytes;
-                    const bool done = unpack32(rawrow, p.type, g * kBK + hf * 32, live, [&](uint32_t c8, const uint4 &h, const uint4 &l) {
-                        const uint32_t kc = hf * 4 + c8;
-                        *reinterpret_cast<uint4 *>(a_hi + kc * 2048 + in_core) = h;
-                        *reinterpret_cast<uint4 *>(a_lo + kc * 2048 + in_core) = l;
-                    });
-#pragma unroll 1
-                    for (uint32_t c8 = 0; c8 < 4 && !done; c8++) {
-                        const uint32_t col0 = g * kBK + hf * 32 + c8 * 8;  // column inside the unit
-                        float v[8];
-                        dequant8_unit(rawrow, p.type, col0, v);
+                for (uint32_t g = 0; g < 4 && ok; g++, ring.advance(kStages)) {
+                    ok = mbar_wait(bar_empty + 8 * ring.s, ring.ph ^ 1u, abort_flag, p.status);
+                    ok = __all_sync(0xffffffffu, ok);  // (a warp stays together: its stores are the warp's)
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t w_hi = w_at + ring.s * T::kACols, w_lo = w_hi + T::kACols / 2;
+                    uint4 hi[4], lo[4];
+                    const bool done = unpack32(rawrow, p.type, g * kBK + hf * 32, live, [&](uint32_t c8, const uint4 &h, const uint4 &l) { hi[c8] = h, lo[c8] = l; });
+                    if (__all_sync(0xffffffffu, done)) {
 #pragma unroll
-                        for (int i = 0; i < 8; i++) v[i] = live ? v[i] * kGenericWScale : 0.f;
-                        // positions 0..7 of the 16 bytes hold columns 0,2,1,3,4,6,5,7 (the order of the activation tiles)
-                        const float o[8] = {v[0], v[2], v[1], v[3], v[4], v[6], v[5], v[7]};
-                        uint32_t h[4], l[4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const __half2 hh = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
-                            const float2 back = __half22float2(hh);
-                            h[i] = as_u32(hh);
-                            l[i] = as_u32(__floats2half2_rn(o[2 * i] - back.x, o[2 * i + 1] - back.y));
+                        for (uint32_t c8 = 0; c8 < 4; c8 += 2) {
+                            tmem_st8(w_hi + 4 * c8, hi[c8], hi[c8 + 1]);
+                            tmem_st8(w_lo + 4 * c8, lo[c8], lo[c8 + 1]);
                         }
-                        const uint32_t kc = hf * 4 + c8;
-                        *reinterpret_cast<uint4 *>(a_hi + kc * 2048 + in_core) = make_uint4(h[0], h[1], h[2], h[3]);
-                        *reinterpret_cast<uint4 *>(a_lo + kc * 2048 + in_core) = make_uint4(l[0], l[1], l[2], l[3]);
+                    } else {
+#pragma unroll 1
+                        for (uint32_t c8 = 0; c8 < 4; c8++) {
+                            const uint32_t col0 = g * kBK + hf * 32 + c8 * 8;  // column inside the unit
+                            float v[8];
+                            dequant8_unit(rawrow, p.type, col0, v);
+#pragma unroll
+                            for (int i = 0; i < 8; i++) v[i] = live ? v[i] * kGenericWScale : 0.f;
+                            // positions 0..7 of the 16 bytes hold columns 0,2,1,3,4,6,5,7 (the order of the activation tiles)
+                            const float o[8] = {v[0], v[2], v[1], v[3], v[4], v[6], v[5], v[7]};
+                            uint32_t h[4], l[4];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                const __half2 hh = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
+                                const float2 back = __half22float2(hh);
+                                h[i] = as_u32(hh);
+                                l[i] = as_u32(__floats2half2_rn(o[2 * i] - back.x, o[2 * i + 1] - back.y));
+                            }
+                            __syncwarp();
+                            tmem_st4(w_hi + 4 * c8, make_uint4(h[0], h[1], h[2], h[3]));
+                            tmem_st4(w_lo + 4 * c8, make_uint4(l[0], l[1], l[2], l[3]));
+                        }
                     }
-                    fence_async_smem();
+                    tmem_st_wait();
+                    tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_full + 8 * ring.s);
                 }
@@ -916,56 +921,47 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             }
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else {
-        uint32_t it = 0;
         bool ok = true;
-        const uint32_t in_core = (r >> 3) * 128 + (r & 7u) * 16;
+        const uint32_t in_core = (r >> 3) * 128 + (r & 7u) * 16;  // place of this row in the m slab
+        const uint32_t w_at = tmem_base + T::kABase + ((warp & 3u) << 21) + hf * 8;  // this warp's lanes, this thread's columns of a stage
         const __half2 k1024 = __half2half2(__ushort_as_half(0x6400)), kneg1024 = __half2half2(__ushort_as_half(0xE400));
+        const __half2 kneg64 = __half2half2(__ushort_as_half(0xD400)), k16th = __half2half2(__ushort_as_half(0x2C00));
         RingPos ring;
-        long long pw = 0, pk = 0, pf = 0;
-        const long long pstart = (kProfile && p.prof) ? clock64() : 0;
         // the four stages of one super-block
         auto unpack_block = [&](const RowBlock &cur) {
             const ScalesMins sm = q4k_scales_mins(cur.hdr.y, cur.hdr.z, cur.hdr.w);
 #pragma unroll
-            for (uint32_t g = 0; g < 4; g++, it++) {
-                const uint32_t s = ring.s, ph = ring.ph;
+            for (uint32_t g = 0; g < 4; g++) {
+                const uint32_t s = ring.s;
                 const bool opens = g % T::KG == 0, closes = g % T::KG == T::KG - 1;  // first / last group of its stage
                 // scales of sub-blocks 2g (low nibbles) and 2g + 1 (high nibbles) as fp16 pairs (sc, sc)
                 const uint32_t scw = g < 2 ? sm.sc_lo : sm.sc_hi, j0 = (2 * g) & 3u;
                 const __half2 sc0 = __hsub2(as_half2(biased_pair(scw, 0x4040u + j0 * 0x0101u)), k1024);
                 const __half2 sc1 = __hsub2(as_half2(biased_pair(scw, 0x4040u + (j0 + 1) * 0x0101u)), k1024);
-                const __half2 nb0 = __hmul2(sc0, kneg1024), nb1 = __hmul2(sc1, kneg1024);  // −1024·sc ≥ −64512: exact
-                const long long c0 = (kProfile && p.prof) ? clock64() : 0;
-                if (opens && !mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, p.status)) {
-                    ok = false;
-                    return;
+                // low nibbles: (1024 + q)·sc − 1024·sc, high nibbles where they lie: (1024 + 16·q)·(sc / 16) − 64·sc; both q·sc, exact
+                const __half2 nb0 = __hmul2(sc0, kneg1024), nb1 = __hmul2(sc1, kneg64), sc1_16 = __hmul2(sc1, k16th);  // −1024·sc ≥ −64512
+                if (opens) {
+                    ok = mbar_wait(bar_empty + 8 * s, ring.ph ^ 1u, abort_flag, p.status);
+                    ok = __all_sync(0xffffffffu, ok);  // (a warp stays together: its stores are the warp's)
+                    if (!ok) return;
+                    tc_fence_after();
                 }
-                const long long c1 = (kProfile && p.prof) ? clock64() : 0;
-                pw += c1 - c0;
-                unsigned char *stage = smem + (size_t)s * kStageBytes, *a = stage + (g % T::KG) * kABytes;
                 // byte b of the 32 holds column b (low nibble, sub-block 2g) and column 32 + b (high nibble)
                 const uint32_t qw[4] = {cur.q[g].x, cur.q[g].y, cur.q[g].z, cur.q[g].w};
+                uint4 lo[2], hi[2];
 #pragma unroll
                 for (int half8 = 0; half8 < 2; half8++) {
-                    if (skip & 1u) break;
-                    const uint32_t w0 = qw[2 * half8], w1 = qw[2 * half8 + 1];
-                    const uint32_t kc_lo = hf * 2 + half8;  // 8-column step of the low-nibble columns
-                    // (1024 + q)·sc − 1024·sc = q·sc, exact; pairs are bytes (0, 2) and (1, 3) of a word
-                    auto mul = [&](uint32_t nib_pair, __half2 sc, __half2 nb) {
-                        return as_u32(__hfma2(as_half2((nib_pair & 0x000F000Fu) | 0x64006400u), sc, nb));
-                    };
-                    uint4 lo, hi;
-                    lo.x = mul(w0, sc0, nb0);
-                    lo.y = mul(w0 >> 8, sc0, nb0);
-                    lo.z = mul(w1, sc0, nb0);
-                    lo.w = mul(w1 >> 8, sc0, nb0);
-                    hi.x = mul(w0 >> 4, sc1, nb1);
-                    hi.y = mul(w0 >> 12, sc1, nb1);
-                    hi.z = mul(w1 >> 4, sc1, nb1);
-                    hi.w = mul(w1 >> 12, sc1, nb1);
-                    *reinterpret_cast<uint4 *>(a + kc_lo * 2048 + in_core) = lo;
-                    *reinterpret_cast<uint4 *>(a + (4 + kc_lo) * 2048 + in_core) = hi;
+                    const uint32_t w0 = qw[2 * half8], w1 = qw[2 * half8 + 1], w0s = w0 >> 8, w1s = w1 >> 8;
+                    // pairs are bytes (0, 2) and (1, 3) of a word
+                    auto low = [&](uint32_t w) { return as_u32(__hfma2(as_half2((w & 0x000F000Fu) | 0x64006400u), sc0, nb0)); };
+                    auto high = [&](uint32_t w) { return as_u32(__hfma2(as_half2((w & 0x00F000F0u) | 0x64006400u), sc1_16, nb1)); };
+                    lo[half8] = make_uint4(low(w0), low(w0s), low(w1), low(w1s));
+                    hi[half8] = make_uint4(high(w0), high(w0s), high(w1), high(w1s));
                 }
+                // eight columns are four words of tensor memory: 16·hf of the first 32, 16·hf of the last
+                const uint32_t w = w_at + s * T::kACols + (g % T::KG) * 32;
+                tmem_st8(w, lo[0], lo[1]);
+                tmem_st8(w + 16, hi[0], hi[1]);
                 if (g == 3) {
                     // the eight mins of the super-block, twice: columns 0-7 meet the hi sums, 8-15 the lo sums
                     uint4 m;
@@ -973,25 +969,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                     m.y = as_u32(__hsub2(as_half2(biased_pair(sm.m_lo, 0x5342u)), k1024));
                     m.z = as_u32(__hsub2(as_half2(biased_pair(sm.m_hi, 0x5140u)), k1024));
                     m.w = as_u32(__hsub2(as_half2(biased_pair(sm.m_hi, 0x5342u)), k1024));
-                    *reinterpret_cast<uint4 *>(stage + T::kOffAm + hf * 2048 + in_core) = m;
-                }
-                const long long c2 = (kProfile && p.prof) ? clock64() : 0;
-                if (closes) {
+                    *reinterpret_cast<uint4 *>(smem + (size_t)s * kStageBytes + hf * 2048 + in_core) = m;
                     fence_async_smem();  // generic-proxy stores → visible to the tensor core's reads
+                }
+                if (closes) {
+                    tmem_st_wait();
+                    tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_full + 8 * s);
-                    ring.advance(p.stages);
+                    ring.advance(kStages);
                 }
-                const long long c3 = (kProfile && p.prof) ? clock64() : 0;
-                pk += c2 - c1;
-                pf += c3 - c2;
             }
         };
         UnitWalk walk;
         walk.start(p, n_items, bpr);
         for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, n_items, bpr)) {
             const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
-            if (!mbar_wait(bar_raw_full + 8 * slot, ph, abort_flag, p.status)) break;
+            ok = mbar_wait(bar_raw_full + 8 * slot, ph, abort_flag, p.status);
+            if (!__all_sync(0xffffffffu, ok)) break;
             // row r of the box: 144 bytes; rows are 36 words apart, so eight lanes cover all 32 banks
             const unsigned char *bp = raw + (size_t)slot * kRawBytes + r * 144u;
             RowBlock cur;
@@ -1002,86 +997,96 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_raw_empty + 8 * slot);  // this warp is done with the box
         }
-        if ((kProfile && p.prof) && blockIdx.x == 0 && ptid == 0) {
-            g_gemm_prof[6] = clock64() - pstart;
-            g_gemm_prof[7] = pw;
-            g_gemm_prof[8] = pk;
-            g_gemm_prof[9] = pf;
-        }
         }  // exact Q4_K producer
     } else {
+        split_registers<BN, kDrainRegs>();
         // drain warp: TMEM lanes [32·(warp % 4), +32) = rows of the tile, columns [CW·(warp / 4), +CW)
-        const long long t_ready = (kProfile && p.prof) ? clock64() : 0;
         yule_pdl_wait();
         const uint32_t lane_base = (warp & 3u) * 32u, col_base = (warp >> 2) * CW;
-        uint32_t it = 0;
+        RingPos ring;
         bool ok = true;
-        long long dw = 0, t_loop_end = 0;
-        const long long dstart = (kProfile && p.prof) ? clock64() : 0;
         for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
             const Item wi = decode_item(p, item, bpr);
             const uint32_t mt = wi.mt, nt = wi.nt;
             const uint32_t row = mt * kBM + lane_base + lane;
             const uint8_t *rowp = p.w[wi.seg] + (size_t)(row < p.n_rows[wi.seg] ? row : p.n_rows[wi.seg] - 1) * bpr * 144;
-            float acc[CW];
+            uint64_t acc2[CW / 2];  // pairs of sums: columns 2j, 2j + 1
 #pragma unroll
-            for (uint32_t j = 0; j < CW; j++) acc[j] = 0.f;
+            for (uint32_t j = 0; j < CW / 2; j++) acc2[j] = 0;
             uint32_t dd_cur = 0, dd_next = GENERIC ? 0u : __ldg(reinterpret_cast<const uint32_t *>(rowp + (size_t)wi.sb0 * 144));  // (d, dmin) of the first super-block
+            // the accumulator at the head of the ring: wait for it, and give it back
+            auto await = [&]() {
+                const bool full = mbar_wait(bar_acc_full + 8 * ring.s, ring.ph, abort_flag, p.status);
+                ok = __all_sync(0xffffffffu, full);  // (a warp stays together: its loads are the warp's)
+                tc_fence_after();
+                return tmem_base + (lane_base << 16) + ring.s * T::kMainCols + col_base;
+            };
+            auto release = [&]() {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_acc_empty + 8 * ring.s);
+                ring.advance(NBUF);
+            };
             const uint32_t kb_end = T::SPB * wi.sb1;
-            for (uint32_t kb = T::SPB * wi.sb0; kb < kb_end; kb++, it++) {
-                if (skip & 32u) break;
-                const uint32_t buf = it % NBUF, aph = (it / NBUF) & 1u;
+            for (uint32_t kb = T::SPB * wi.sb0; kb < kb_end; kb++) {
                 if (!GENERIC && kb % T::SPB == 0u) {  // new super-block: take its (d, dmin), ask for the next one's
                     dd_cur = dd_next;
                     if (kb + T::SPB < kb_end) dd_next = __ldg(reinterpret_cast<const uint32_t *>(rowp + (size_t)(kb / T::SPB + 1) * 144));
                 }
                 const float2 dd = GENERIC ? make_float2(1.f, 0.f) : __half22float2(as_half2(dd_cur));
-                const long long c0 = (kProfile && p.prof) ? clock64() : 0;
-                if (!mbar_wait(bar_acc_full + 8 * buf, aph, abort_flag, p.status)) {
-                    ok = false;
-                    break;
-                }
-                if ((kProfile && p.prof)) dw += clock64() - c0;
-                tc_fence_after();
-                const uint32_t t_main = tmem_base + (lane_base << 16) + buf * T::kBufCols + col_base;
+                const uint64_t d2 = pair(dd.x, dd.x);
+                uint32_t at = await();
+                if (!ok) break;
+                // the accumulators go back before the arithmetic on what was read last
                 if constexpr (T::MERGED) {
-                    // all the loads of the stage in flight together, one wait
                     uint32_t v[CW], vl[CW];
-                    if (!(skip & 4u)) {
 #pragma unroll
-                        for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-                            tmem_ld16_issue(t_main + c0, v + c0);
-                            tmem_ld16_issue(t_main + BN + c0, vl + c0);  // the products with the lo terms
-                        }
-                        tmem_ld_wait();
-#pragma unroll
-                        for (uint32_t j = 0; j < CW; j++) acc[j] = fmaf(dd.x, __uint_as_float(v[j]) + __uint_as_float(vl[j]), acc[j]);
+                    for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
+                        tmem_ld16_issue(at + c0, v + c0);
+                        tmem_ld16_issue(at + BN + c0, vl + c0);  // the products with the lo terms
                     }
+                    tmem_ld_wait();
+                    release();
+#pragma unroll
+                    for (uint32_t j = 0; j < CW; j += 2) acc2[j / 2] = fma2(d2, add2(pair_bits(v[j], v[j + 1]), pair_bits(vl[j], vl[j + 1])), acc2[j / 2]);
                 } else {
+                    uint32_t v[32];
+                    tmem_ld32_issue(at, v);
+                    tmem_ld_wait();
 #pragma unroll
-                    for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-                        if (skip & 4u) break;
-                        uint32_t v[16];
-                        tmem_ld16(t_main + c0, v);
+                    for (uint32_t j = 0; j < 32; j += 2) acc2[j / 2] = fma2(d2, pair_bits(v[j], v[j + 1]), acc2[j / 2]);
+                    tmem_ld32_issue(at + 32, v);
+                    tmem_ld_wait();
+                    release();
 #pragma unroll
-                        for (int j = 0; j < 16; j++) acc[c0 + j] = fmaf(dd.x, __uint_as_float(v[j]), acc[c0 + j]);
+                    for (uint32_t j = 0; j < 32; j += 2) acc2[16 + j / 2] = fma2(d2, pair_bits(v[j], v[j + 1]), acc2[16 + j / 2]);
+                }
+                if (!GENERIC && kb % T::SPB == T::SPB - 1) {  // the stage that ends a super-block is followed by the min term
+                    at = await();
+                    if (!ok) break;
+                    constexpr uint32_t R = CW < 32 ? CW : 32;
+                    const float minus_dmin = -dd.y * (1.0f / kSumScale);
+                    const uint64_t m2 = pair(minus_dmin, minus_dmin);
+#pragma unroll
+                    for (uint32_t c0 = 0; c0 < CW; c0 += R) {
+                        uint32_t v[R];
+#pragma unroll
+                        for (uint32_t c1 = 0; c1 < R; c1 += 16) tmem_ld16_issue(at + c0 + c1, v + c1);
+                        tmem_ld_wait();
+                        if (c0 + R == CW) release();
+#pragma unroll
+                        for (uint32_t j = 0; j < R; j += 2) acc2[(c0 + j) / 2] = fma2(m2, pair_bits(v[j], v[j + 1]), acc2[(c0 + j) / 2]);
                     }
                 }
-                if (!GENERIC && kb % T::SPB == T::SPB - 1) {  // the stage that ends a super-block carries the min term
-#pragma unroll
-                    for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-                        uint32_t v[16];
-                        tmem_ld16((T::SHARED_MIN ? tmem_base + (lane_base << 16) + col_base : t_main) + T::kMinBase + c0, v);
-#pragma unroll
-                        for (int j = 0; j < 16; j++) acc[c0 + j] = fmaf(-dd.y * (1.0f / kSumScale), __uint_as_float(v[j]), acc[c0 + j]);
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
             }
             if (!ok) break;
-            if ((kProfile && p.prof)) t_loop_end = clock64();
+            float acc[CW];
+#pragma unroll
+            for (uint32_t j = 0; j < CW; j += 2) {
+                const float2 a = unpair(acc2[j / 2]);
+                acc[j] = a.x;
+                acc[j + 1] = a.y;
+            }
             const uint32_t n0 = nt * BN + col_base;
             if (p.ksplit > 1) {
                 // This item covers a part of the columns.  Every drain warp stores its block of scaled partial sums, then
@@ -1163,13 +1168,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 }
             }
         }
-        if ((kProfile && p.prof) && blockIdx.x == 0 && threadIdx.x == 0) {
-            g_gemm_prof[10] = clock64() - dstart;
-            g_gemm_prof[11] = dw;
-            g_gemm_prof[12] = t_ready - t_entry;
-            g_gemm_prof[13] = dstart - t_ready;
-            g_gemm_prof[14] = clock64() - t_loop_end;
-        }
     }
 
     // common exit: nothing of this CTA may still be in flight when its TMEM and shared memory go
@@ -1184,9 +1182,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
         __syncthreads();
     }
     if (warp == kMmaWarp) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T::kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
-    if ((kProfile && p.prof) && blockIdx.x == 0 && threadIdx.x == 0) g_gemm_prof[15] = clock64() - t_entry;
 }
 
 // Activation rows → the GEMM's operand tiles, one CTA per (padded) row: power-of-two row scale,
@@ -1363,6 +1360,28 @@ cudaError_t encode_weight_map(const uint8_t *w, uint32_t n_rows, uint32_t n_cols
     return cached_tensor_map_2d(w, 1, row_bytes, n_rows, row_bytes, 144, kBM, out);  // one driver call per (tensor, shape), not per launch
 }
 
+template <int BN, bool GENERIC>
+cudaError_t launch_gemm(const GemmParams &p, const GemmMaps &w_maps, uint32_t grid, size_t smem, bool pdl, cudaStream_t s) {
+    auto kern = qgemm_tc_kernel<BN, GENERIC>;
+    static bool attr_done[64] = {};  // the opt-in for large dynamic shared memory belongs to the device
+    static std::mutex mu;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+            cudaFuncAttributes fa;  // the split of the registers counts on what the launch brings
+            e = cudaFuncGetAttributes(&fa, kern);
+            if (e == cudaSuccess && BN == 128 && fa.numRegs < kLaunchRegs) e = cudaErrorInvalidValue;
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024);
+            if (e != cudaSuccess) return e;
+            if (dev >= 0 && dev < 64) attr_done[dev] = true;
+        }
+    }
+    return launch_kernel(kern, dim3(grid), dim3(kGemmThreads), smem, s, pdl, p, w_maps);
+}
+
 uint32_t pick_bn(uint32_t n_tokens) { return n_tokens <= 32 ? 32 : (n_tokens <= 64 ? 64 : 128); }
 
 }  // namespace
@@ -1537,23 +1556,18 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     }
     const bool generic = g.type != YULE_DTYPE_Q4_K || (knob("YULE_GEMM_GENERIC") && atoi(knob("YULE_GEMM_GENERIC")));
     const uint32_t kg = groups_per_stage(bn, generic);
-    const uint32_t stage_bytes = generic ? 2 * kABytes + 2 * bn * kBK * 2 : kg * kABytes + kAmBytes + kg * 2 * bn * kBK * 2 + bn * 32;
+    const uint32_t stage_bytes = kg * 2 * bn * kBK * 2 + (generic ? 0u : kAmBytes + bn * 32);
     p.unit_bytes = 256 / block_size(g.type) * block_bytes(g.type);
     p.raw_chunks = (p.unit_bytes + 14 + 15) / 16;      // covers the unit from any 2-byte-aligned start
     p.raw_stride = (p.raw_chunks | 1u) * 16;            // an odd multiple of 16 bytes
     p.raw_ring_bytes = (2 * kBM * p.raw_stride + 127u) & ~127u;
     const size_t raw_ring = generic ? p.raw_ring_bytes : (size_t)raw_slots_for(bn) * kRawBytes;
-    uint32_t stages = (uint32_t)((220u * 1024u - (raw_ring + 512u)) / stage_bytes);
-    if (stages < 2) return cudaErrorInvalidValue;
-    p.stages = stages > (uint32_t)kMaxStages ? (uint32_t)kMaxStages : stages;
     p.type = g.type;
     p.w_row_bytes = (uint64_t)(g.n_cols / block_size(g.type)) * block_bytes(g.type);
     p.out_scale = (generic ? 1.0f / kGenericWScale : 1.0f) * kTruncation;
     p.status = g.status;
-    p.prof = (kProfile && knob("YULE_GEMM_PROF")) ? 1u : 0u;
-    p.skip = (kProfile && knob("YULE_GEMM_SKIP")) ? (uint32_t)atoi(knob("YULE_GEMM_SKIP")) : 0u;
-    const size_t tail_bytes = raw_ring + (2 * kMaxStages + 8 + 2 * kRawSlots) * 8 + 32;
-    const size_t smem = (size_t)p.stages * stage_bytes + tail_bytes;
+    const size_t tail_bytes = raw_ring + (2 * kStages + 8 + 2 * kRawSlots) * 8 + 32;
+    const size_t smem = kStages * stage_bytes + tail_bytes;
     GemmMaps w_maps;
     memset(&w_maps, 0, sizeof(w_maps));
     if (!generic) {
@@ -1564,30 +1578,12 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     }
     uint32_t grid = p.n_mtiles * p.n_ntiles * p.ksplit;
     if (grid > (uint32_t)sm_count) grid = (uint32_t)sm_count;
-    auto launch = [&](auto kern) {
-        cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024);
-        if (e2 != cudaSuccess) return e2;
-        return launch_kernel(kern, dim3(grid), dim3(kGemmThreads), smem, s, g.pdl, p, w_maps);
-    };
     if (generic)
-        e = bn == 32 ? launch(qgemm_tc_kernel<32, true>) : (bn == 64 ? launch(qgemm_tc_kernel<64, true>) : launch(qgemm_tc_kernel<128, true>));
+        e = bn == 32 ? launch_gemm<32, true>(p, w_maps, grid, smem, g.pdl, s) : (bn == 64 ? launch_gemm<64, true>(p, w_maps, grid, smem, g.pdl, s) : launch_gemm<128, true>(p, w_maps, grid, smem, g.pdl, s));
     else
-        e = bn == 32 ? launch(qgemm_tc_kernel<32, false>) : (bn == 64 ? launch(qgemm_tc_kernel<64, false>) : launch(qgemm_tc_kernel<128, false>));
+        e = bn == 32 ? launch_gemm<32, false>(p, w_maps, grid, smem, g.pdl, s) : (bn == 64 ? launch_gemm<64, false>(p, w_maps, grid, smem, g.pdl, s) : launch_gemm<128, false>(p, w_maps, grid, smem, g.pdl, s));
     if (e != cudaSuccess) return e;
     *launches += 1;
-    if (p.prof) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(s, &cs);
-        if (cs == cudaStreamCaptureStatusNone && cudaStreamSynchronize(s) == cudaSuccess) {
-            long long h[16];
-            if (cudaMemcpyFromSymbol(h, g_gemm_prof, sizeof(h)) == cudaSuccess)
-                fprintf(stderr,
-                        "[qgemm prof, CTA 0, cycles] mma: total %lld wait_acc_empty %lld wait_full %lld issue %lld commit %lld stages %lld | "
-                        "producer: total %lld wait_empty %lld unpack %lld fence+arrive %lld | drain: total %lld wait_acc_full %lld | "
-                        "set-up %lld wait for the re-layout %lld epilogue %lld kernel %lld\n",
-                        h[0], h[1], h[2], h[3], h[4], h[5], h[6], h[7], h[8], h[9], h[10], h[11], h[12], h[13], h[14], h[15]);
-        }
-    }
     return cudaSuccess;
 }
 
