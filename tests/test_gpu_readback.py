@@ -1,0 +1,52 @@
+"""Small results to the host (csrc/readback.cu): sizes around its vector width, its CTAs' shares and the line to the copy engine, into
+pageable, unaligned and pinned memory; behind a matvec as its dependent launch; from several threads."""
+
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from yule_b200 import DType, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4095, 4096, 4097, 64 * 4096 + 5, (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
+def test_sizes_and_destinations(backend, n):
+    data = np.random.default_rng(n).integers(0, 256, n, dtype=np.uint8)
+    h = backend.upload(data)
+    pinned = torch.zeros(n + 64, dtype=torch.uint8).pin_memory().numpy()
+    for dst in (np.zeros(n, np.uint8), np.zeros(n + 8, np.uint8)[3:3 + n], pinned[:n], pinned[16:16 + n], pinned[5:5 + n]):
+        dst[:] = 0
+        backend.copy_from_device(h, dst)
+        assert np.array_equal(dst, data)
+    assert pinned[16 + n:].max(initial=0) == 0  # nothing behind the end
+    backend.free(h)
+
+
+def test_behind_a_matvec_and_from_threads(backend, oracle):
+    rows, cols = 1000, 2048
+    w, x = synth.random_quantized(DType.Q4_K, 5, rows * cols), synth.normal(6, cols)
+    wh, xh = backend.upload(w), backend.upload(x)
+    outs = [backend.allocate(rows * 4) for _ in range(4)]
+    ref = oracle.qmv(int(DType.Q4_K), w, x, rows, cols)
+    for _ in range(20):
+        backend.quantized_matmul(wh, xh, outs[0], rows, cols, DType.Q4_K)
+        assert np.abs(backend.download(outs[0], rows) - ref).max() <= 1e-5 * np.abs(ref).max()
+    for o in outs[1:]:
+        backend.quantized_matmul(wh, xh, o, rows, cols, DType.Q4_K)
+    good = [0] * 4
+
+    def read(i):
+        for _ in range(200):
+            y = np.zeros(rows, np.float32)
+            backend.copy_from_device(outs[i], y)
+            good[i] += int(np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max())
+
+    threads = [threading.Thread(target=read, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert good == [200] * 4

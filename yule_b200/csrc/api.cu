@@ -158,6 +158,7 @@ int32_t yule_cuda_create(int32_t ordinal, yule_cuda_ctx **out_ctx) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->device_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->device_status, 0, sizeof(int));
+    if (e == cudaSuccess) e = read_back_create(ctx);
     if (e != cudaSuccess) {
         delete ctx;
         return fail_cuda(e, "context setup");
@@ -166,6 +167,7 @@ int32_t yule_cuda_create(int32_t ordinal, yule_cuda_ctx **out_ctx) {
         int major = ctx->prop.major, minor = ctx->prop.minor;
         cudaStreamDestroy(ctx->stream);
         cudaFree(ctx->device_status);
+        read_back_destroy(ctx);
         delete ctx;
         return fail(YULE_ERR_CUDA, "device is sm_%d%d; this library carries sm_100a kernels only", major,
                     minor);
@@ -190,6 +192,7 @@ int32_t yule_cuda_destroy(yule_cuda_ctx *ctx) {
     if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
     if (ctx->attn_tickets) cudaFree(ctx->attn_tickets);
     if (ctx->device_status) cudaFree(ctx->device_status);
+    read_back_destroy(ctx);
     if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
     for (void *p : ctx->retired_scratch) cudaFree(p);
     if (ctx->sampler_scratch) cudaFree(ctx->sampler_scratch);
@@ -297,8 +300,7 @@ int32_t yule_cuda_copy_from_device(yule_cuda_ctx *ctx, yule_buffer src, void *da
     FIND(ctx, src, s);
     if (len && !data) return fail(YULE_ERR_INVALID_ARGUMENT, "null data");
     size_t n = len < s.size ? len : s.size;
-    if (n) YULE_CUDA_TRY(cudaMemcpyAsync(data, s.ptr, n, cudaMemcpyDeviceToHost, ctx->stream));
-    YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    YULE_CUDA_TRY(read_back(ctx, s.ptr, data, n, _pdl_chain));
     return YULE_OK;
 }
 

@@ -98,6 +98,10 @@ struct yule_cuda_ctx {
     // may still replay into them, so they are kept until the context is destroyed instead of being freed.
     std::vector<void *> retired_scratch;
     std::atomic<uint64_t> launches{0};
+    // read-back of small results (readback.cu): landing area in mapped host memory with the epoch behind it, both views; the kernel's ticket
+    std::mutex rb_mu;
+    unsigned char *rb_host = nullptr, *rb_device = nullptr;
+    uint32_t *rb_ticket = nullptr, rb_epoch = 0;
     // Word the kernels with bounded waits write when they give up; read by synchronize.
     int *device_status = nullptr;
     long long wait_cycles = yule::kDefaultWaitCycles;  // budget of every bounded device-side wait
@@ -116,6 +120,16 @@ struct yule_cuda_ctx {
 };
 
 namespace yule {
+
+// Results of up to this size reach the host by a kernel's own stores (readback.cu).
+constexpr size_t kReadBackBytes = 1024 * 1024;
+cudaError_t read_back_create(yule_cuda_ctx *ctx);
+void read_back_destroy(yule_cuda_ctx *ctx);
+// Blocks until `n` bytes at `src` (device), as everything enqueued before leaves them, are at `data` (host).  pdl: the operation before is a
+// launch that lets its dependents start early.
+cudaError_t read_back(yule_cuda_ctx *ctx, const void *src, void *data, size_t n, bool pdl);
+// Two words of device memory from arguments of the launch: nothing on the host has to stay as it is until the copy has run.
+cudaError_t launch_set_words(uint32_t *at, uint32_t a, uint32_t b, cudaStream_t s);
 
 // The four formats with tuned matvec and tensor-core GEMM kernels.
 inline bool is_tuned_format(uint32_t t) {

@@ -1459,12 +1459,8 @@ int32_t step(yule_cuda_runner *r, uint32_t token, bool token_from_device) {
         int32_t rc = ensure_graph(r);
         if (rc) return rc;
         if (!token_from_device) {
-            // h_pinned[0..1] = {token, pos}: the position is rewritten too, so a reset() or a
-            // failed step cannot leave the device counter out of step with the host's.
-            YULE_CUDA_TRY(cudaStreamSynchronize(s));  // staging words may still be in flight
-            r->h_pinned[0] = token;
-            r->h_pinned[1] = r->pos;
-            YULE_CUDA_TRY(cudaMemcpyAsync(r->d_state, r->h_pinned, 8, cudaMemcpyHostToDevice, s));
+            // the position is rewritten too, so a reset() or a failed step cannot leave the device counter out of step with the host's
+            YULE_CUDA_TRY(launch_set_words(r->d_state, token, r->pos, s));
         }
         YULE_CUDA_TRY(cudaGraphLaunch(r->graph_exec, s));
         r->ctx->launches.fetch_add(graph_kernels(r));
@@ -1478,10 +1474,14 @@ int32_t read_logits(yule_cuda_runner *r, float *logits_out) {
     if (!logits_out) return YULE_OK;
     cudaStream_t s = r->ctx->stream;
     const size_t bytes = (size_t)r->cfg.vocab_size * 4;
-    if (!r->h_logits) YULE_CUDA_TRY(cudaMallocHost((void **)&r->h_logits, bytes));
-    YULE_CUDA_TRY(cudaMemcpyAsync(r->h_logits, r->logits, bytes, cudaMemcpyDeviceToHost, s));
-    YULE_CUDA_TRY(cudaStreamSynchronize(s));
-    memcpy(logits_out, r->h_logits, bytes);
+    if (bytes <= kReadBackBytes) {
+        YULE_CUDA_TRY(read_back(r->ctx, r->logits, logits_out, bytes, false));
+    } else {
+        if (!r->h_logits) YULE_CUDA_TRY(cudaMallocHost((void **)&r->h_logits, bytes));
+        YULE_CUDA_TRY(cudaMemcpyAsync(r->h_logits, r->logits, bytes, cudaMemcpyDeviceToHost, s));
+        YULE_CUDA_TRY(cudaStreamSynchronize(s));
+        memcpy(logits_out, r->h_logits, bytes);
+    }
     return r->xchg ? yule_cuda_synchronize(r->ctx) : YULE_OK;  // reports a peer that never arrived
 }
 
