@@ -310,7 +310,7 @@ size_t qgemm_scratch_bytes(uint32_t n_tokens, uint32_t n_cols);
 cudaError_t launch_qgemm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
 // The two halves of launch_qgemm, for matrices that share their activations (Q/K/V, gate/up):
 // one re-layout, then one GEMM per matrix with the same n_tokens, n_cols and scratch.
-cudaError_t launch_qgemm_xprep(const QGemm &g, cudaStream_t s, uint64_t *launches);
+cudaError_t launch_qgemm_xprep(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
 cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
 
 // Row-planar device copy of a Q6_K tensor (q6k_planar.cu): n_cols a multiple of 256.

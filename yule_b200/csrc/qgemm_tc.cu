@@ -1200,17 +1200,21 @@ struct XprepParams {
     float *oscale;
 };
 
-// One CTA per row, as many threads (up to 1024) as have columns to work on; a thread keeps its 8·CHUNKS columns in registers from
-// the single read of the row to the stores, so a row of up to 8192·CHUNKS columns costs one round trip to memory and two block
-// reductions whatever its length.  (With 1024 threads whatever the row length 2048 rows of 4096 columns took 42 us, now 31: half of the
-// threads of an SM held no data.)
+// ROWS rows per CTA, as many threads (up to 1024) as have columns to work on; a thread keeps its 8·CHUNKS columns of a row in registers from
+// the single read to the stores, so rows of up to 8192·CHUNKS / ROWS columns cost one round trip to memory and two block reductions
+// whatever their length.  A thread's 16 bytes of a term lie alone in their 8-column step, the next row's 16 bytes behind them: with two rows in
+// neighbouring lanes a warp writes whole 32-byte sectors, with one it writes halves.  2048 rows of 14336 columns with SwiGLU 137 -> 102 us,
+// of 4096 columns with RMSNorm 29 -> 24.  Where there are not rows enough to give every SM
+// two, one per CTA keeps more SMs at work.
 constexpr int kXprepThreads = 1024;
-template <int CHUNKS>
+template <int CHUNKS, int ROWS>
 __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepParams p) {
     yule_pdl_launch_dependents();
     yule_pdl_wait();
-    __shared__ float red[32];
-    const uint32_t n = blockIdx.x, nt = n / p.bn, r = n % p.bn;
+    __shared__ float red[32 * ROWS];
+    const uint32_t lane_row = threadIdx.x % ROWS, tc = threadIdx.x / ROWS, row_threads = blockDim.x / ROWS;
+    const uint32_t n = blockIdx.x * ROWS + lane_row, nt = n / p.bn, r = n % p.bn;
+    const bool live = n < p.n_tokens;  // else a padding row of the last tile: all zeros
     const uint32_t bpr = p.n_cols / 256;
     const uint32_t x_half_bytes = p.bn * kBK * 2, bm_bytes = p.bn * 32, super_bytes = 8 * x_half_bytes + bm_bytes;
     const uint32_t core = ((r >> 3) * 64 + (r & 7u) * 8) * 2;  // byte offset of this row inside an 8-column step
@@ -1226,50 +1230,37 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         return reinterpret_cast<__half *>(p.xb + ((size_t)nt * bpr + sb) * super_bytes + 8 * (size_t)x_half_bytes +
                                           term * (p.bn * 16) + core) + s;
     };
-    if (n >= p.n_tokens) {  // padding row of the last tile
-        for (uint32_t k0 = threadIdx.x * 8; k0 < p.n_cols; k0 += blockDim.x * 8) {
-            *reinterpret_cast<uint4 *>(slab16(k0, 0)) = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4 *>(slab16(k0, 1)) = make_uint4(0, 0, 0, 0);
-            if ((k0 & 31u) == 0) {
-                *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 0) = __ushort_as_half(0);
-                *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 1) = __ushort_as_half(0);
-            }
-        }
-        if (threadIdx.x == 0) p.oscale[n] = 0.f;
-        return;
-    }
     const float *x = p.x + (size_t)n * p.x_stride;
     const float *gate = p.gate ? p.gate + (size_t)n * p.x_stride : nullptr;
-    auto block_reduce = [&](float v, bool is_max) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const float other = __shfl_xor_sync(0xffffffffu, v, o);
-            v = is_max ? fmaxf(v, other) : v + other;
-        }
+    // over the threads of a row, which are every ROWS-th lane
+    auto row_reduce = [&](float v, bool is_max) {
+        auto both = [&](float a, float b) { return is_max ? fmaxf(a, b) : a + b; };
+        for (int o = 16; o >= ROWS; o >>= 1) v = both(v, __shfl_xor_sync(0xffffffffu, v, o));
         __syncthreads();
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        if ((threadIdx.x & 31u) < ROWS) red[(threadIdx.x >> 5) * ROWS + lane_row] = v;
         __syncthreads();
-        const uint32_t lane = threadIdx.x & 31u, n_warps = blockDim.x >> 5;
-        v = lane < n_warps ? red[lane] : 0.f;  // (sums of squares, magnitudes: nothing is below zero)
-        for (int o = 16; o > 0; o >>= 1) {
-            const float other = __shfl_xor_sync(0xffffffffu, v, o);
-            v = is_max ? fmaxf(v, other) : v + other;
-        }
+        const uint32_t n_warps = blockDim.x >> 5, first = (threadIdx.x & 31u) / ROWS;
+        v = 0.f;  // (sums of squares, magnitudes: nothing is below zero)
+        for (uint32_t w = first; w < n_warps; w += 32 / ROWS) v = both(v, red[w * ROWS + lane_row]);
+        for (int o = 16; o >= ROWS; o >>= 1) v = both(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     };
     // rows start on a 16-byte boundary when the stride is a multiple of four floats; otherwise scalar loads
-    const bool vec = ((reinterpret_cast<uintptr_t>(x) | (gate ? reinterpret_cast<uintptr_t>(gate) : 0)) & 15u) == 0;
+    auto load8 = [&](const float *from, float (&to)[8]) {
+        if ((reinterpret_cast<uintptr_t>(from) & 15u) == 0) {
+            const float4 a = *reinterpret_cast<const float4 *>(from), b = *reinterpret_cast<const float4 *>(from + 4);
+            to[0] = a.x, to[1] = a.y, to[2] = a.z, to[3] = a.w, to[4] = b.x, to[5] = b.y, to[6] = b.z, to[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) to[i] = from[i];
+        }
+    };
     float v[CHUNKS][8];
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
-        const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
-        if (k0 < p.n_cols) {
-            if (vec) {
-                const float4 a = *reinterpret_cast<const float4 *>(x + k0), b = *reinterpret_cast<const float4 *>(x + k0 + 4);
-                v[c][0] = a.x, v[c][1] = a.y, v[c][2] = a.z, v[c][3] = a.w, v[c][4] = b.x, v[c][5] = b.y, v[c][6] = b.z, v[c][7] = b.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[c][i] = x[k0 + i];
-            }
+        const uint32_t k0 = ((uint32_t)c * row_threads + tc) * 8;
+        if (live && k0 < p.n_cols) {
+            load8(x + k0, v[c]);
         } else {
 #pragma unroll
             for (int i = 0; i < 8; i++) v[c][i] = 0.f;
@@ -1281,27 +1272,28 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         for (int c = 0; c < CHUNKS; c++)
 #pragma unroll
             for (int i = 0; i < 8; i++) ss = fmaf(v[c][i], v[c][i], ss);
-        ss = block_reduce(ss, false);
+        ss = row_reduce(ss, false);
         const float inv = 1.0f / sqrtf(ss / (float)p.n_cols + p.eps);
 #pragma unroll
         for (int c = 0; c < CHUNKS; c++) {
-            const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
-            if (k0 < p.n_cols) {
+            const uint32_t k0 = ((uint32_t)c * row_threads + tc) * 8;
+            if (live && k0 < p.n_cols) {
+                float w[8];
+                load8(p.norm_w + k0, w);
 #pragma unroll
-                for (int i = 0; i < 8; i++) v[c][i] = v[c][i] * inv * p.norm_w[k0 + i];
+                for (int i = 0; i < 8; i++) v[c][i] = v[c][i] * inv * w[i];
             }
         }
     }
     if (gate) {
 #pragma unroll
         for (int c = 0; c < CHUNKS; c++) {
-            const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
-            if (k0 < p.n_cols) {
+            const uint32_t k0 = ((uint32_t)c * row_threads + tc) * 8;
+            if (live && k0 < p.n_cols) {
+                float gt[8];
+                load8(gate + k0, gt);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float gt = gate[k0 + i];
-                    v[c][i] = (gt / (1.0f + expf(-gt))) * v[c][i];
-                }
+                for (int i = 0; i < 8; i++) v[c][i] = (gt[i] / (1.0f + expf(-gt[i]))) * v[c][i];
             }
         }
     }
@@ -1310,7 +1302,7 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
     for (int c = 0; c < CHUNKS; c++)
 #pragma unroll
         for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[c][i]));
-    amax = block_reduce(amax, true);
+    amax = row_reduce(amax, true);
     // power of two that puts the largest element in [2^13, 2^14)
     float scale = 1.f;
     if (amax > 1e-30f && amax < 1e30f) {
@@ -1318,11 +1310,11 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         frexpf(amax, &ex);  // amax = m · 2^ex, m in [0.5, 1)
         scale = ldexpf(1.f, 14 - ex);
     }
-    if (threadIdx.x == 0) p.oscale[n] = 1.0f / scale;
+    if (tc == 0) p.oscale[n] = live ? 1.0f / scale : 0.f;
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
-        const uint32_t k0 = ((uint32_t)c * blockDim.x + threadIdx.x) * 8;
-        if (k0 >= p.n_cols) break;  // whole groups of four threads (32 columns) leave together
+        const uint32_t k0 = ((uint32_t)c * row_threads + tc) * 8;
+        if (k0 >= p.n_cols) break;  // whole warps leave together (256 columns are 32 threads of a row)
         float sum = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -1341,10 +1333,10 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         }
         *reinterpret_cast<uint4 *>(slab16(k0, 0)) = make_uint4(h[0], h[1], h[2], h[3]);
         *reinterpret_cast<uint4 *>(slab16(k0, 1)) = make_uint4(l[0], l[1], l[2], l[3]);
-        // four consecutive threads cover one 32-column sub-block
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if ((threadIdx.x & 3u) == 0) {
+        // four consecutive threads of a row cover one 32-column sub-block
+        sum += __shfl_xor_sync(0xffffffffu, sum, ROWS);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2 * ROWS);
+        if ((tc & 3u) == 0) {
             sum *= kSumScale;  // 32 elements of up to 2^14 each: keep the sum inside fp16's range
             const __half sh = __float2half_rn(sum);
             *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 0) = sh;
@@ -1468,7 +1460,7 @@ size_t qgemm_scratch_bytes(uint32_t n_tokens, uint32_t n_cols) {
     return kGemmSplitBytes + padded * n_cols * 4 + padded * (n_cols / 256) * 32 + padded * sizeof(float) + 512;
 }
 
-cudaError_t launch_qgemm_xprep(const QGemm &g, cudaStream_t s, uint64_t *launches) {
+cudaError_t launch_qgemm_xprep(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches) {
     if (!qgemm_supported(g.type, g.n_cols, g.n_tokens)) return cudaErrorInvalidValue;
     const uint32_t bn = pick_bn(g.n_tokens);
     const uint32_t n_ntiles = (g.n_tokens + bn - 1) / bn, padded = n_ntiles * bn;
@@ -1488,15 +1480,19 @@ cudaError_t launch_qgemm_xprep(const QGemm &g, cudaStream_t s, uint64_t *launche
     xp.xb = xb;
     xp.oscale = oscale;
     cudaError_t e;
-    auto threads = [&](uint32_t chunks) { return dim3(((g.n_cols / 8 + chunks - 1) / chunks + 31) / 32 * 32); };
-    if (g.n_cols <= 8192)
-        e = launch_kernel(gemm_xprep_kernel<1>, dim3(padded), threads(1), 0, s, g.pdl, xp);
+    auto launch = [&](auto kern, uint32_t chunks, uint32_t rows) {
+        return launch_kernel(kern, dim3(padded / rows), dim3(rows * (((g.n_cols / 8 + chunks - 1) / chunks + 31) / 32 * 32)), 0, s, g.pdl, xp);
+    };
+    if (padded >= 2 * (uint32_t)sm_count && g.n_cols <= 16384)  // (padded is a multiple of 32)
+        e = g.n_cols <= 4096 ? launch(gemm_xprep_kernel<1, 2>, 1, 2) : (g.n_cols <= 8192 ? launch(gemm_xprep_kernel<2, 2>, 2, 2) : launch(gemm_xprep_kernel<4, 2>, 4, 2));
+    else if (g.n_cols <= 8192)
+        e = launch(gemm_xprep_kernel<1, 1>, 1, 1);
     else if (g.n_cols <= 16384)
-        e = launch_kernel(gemm_xprep_kernel<2>, dim3(padded), threads(2), 0, s, g.pdl, xp);
+        e = launch(gemm_xprep_kernel<2, 1>, 2, 1);
     else if (g.n_cols <= 32768)
-        e = launch_kernel(gemm_xprep_kernel<4>, dim3(padded), threads(4), 0, s, g.pdl, xp);
+        e = launch(gemm_xprep_kernel<4, 1>, 4, 1);
     else if (g.n_cols <= 65536)
-        e = launch_kernel(gemm_xprep_kernel<8>, dim3(padded), threads(8), 0, s, g.pdl, xp);
+        e = launch(gemm_xprep_kernel<8, 1>, 8, 1);
     else
         return cudaErrorInvalidValue;
     if (e != cudaSuccess) return e;
@@ -1589,7 +1585,7 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
 
 cudaError_t launch_qgemm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches) {
     if (g.n_rows == 0) return cudaErrorInvalidValue;
-    cudaError_t e = launch_qgemm_xprep(g, s, launches);
+    cudaError_t e = launch_qgemm_xprep(g, sm_count, s, launches);
     if (e != cudaSuccess) return e;
     QGemm mm = g;
     mm.pdl = true;  // behind the re-layout of its own activations: only the weight copies run ahead of it

@@ -1044,7 +1044,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         g.n_tokens = m;
         g.scratch = ctx->gemm_scratch;
         g.pdl = true;  // starts under the tail of its predecessor; reads and writes only after the dependency wait
-        ok(launch_qgemm_xprep(g, s, launches));
+        ok(launch_qgemm_xprep(g, sms, s, launches));
     };
     // `rows` output rows of this rank, written at `out` with `stride` floats between the rows of the result.  Matrices
     // of one format that read the same re-laid-out rows and add no residual (Q/K/V; gate/up) wait in `gq` and go out
