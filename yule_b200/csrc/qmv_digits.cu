@@ -759,9 +759,16 @@ cudaError_t launch_format(const QmvDigits &f, int sm_count, uint32_t share, cuda
 // not keep fed.  us per independent call, 16-warp CTAs against these: Q4_K 2048x2048 2.26, 0.95, 5632x2048 3.29, 2.30, 14336x4096
 // 9.1, 6.7, 28672x8192 23.3, 22.7; Q8_0 2048x2048 2.45, 1.14; two to an SM Q6_K 14336x4096 11.3, 9.5, Q8_0 4096x4096 4.5, 3.4;
 // beyond the lines Q4_K 4096x14336 7.2, 8.6, Q5_K 28672x8192 27.7, 29.7.
+//   In a chain of dependent launches nothing overlaps, but a launch over many rows ends sooner: more CTAs, each with fewer units, leave a smaller
+// last round.  From 30000 rows on, for the two formats whose unpacking is shortest: us per token, 16-warp CTAs against these, 8 layers of
+// the 8B shape in Q4_0 (128256x4096 output) 503, 491; 4 layers of the 70B shape in Q4_K (57344x8192) 628, 626.  With the line at 12000 rows
+// (28672x4096 in Q4_K) 8B 1563, 1650; the outputs of Q8_0 and Q6_K (32000x2048, 128256x4096) gain nothing.
 template <int F>
 cudaError_t launch_sized(const QmvDigits &f, int sm_count, cudaStream_t s, uint64_t *launches) {
-    if (f.pdl && f.late_wait && f.n_cols <= 8192 && !f.tp.push && !f.tp.wait) {
+    uint32_t all_rows = 0;
+    for (uint32_t i = 0; i < f.n_seg; i++) all_rows += f.rows[i];
+    const bool many_rows = all_rows >= 30000 && (F == kQ4K || F == kQ4);
+    if (f.pdl && (f.late_wait || many_rows) && f.n_cols <= 8192 && !f.tp.push && !f.tp.wait) {
         uint32_t n_tiles = 0;
         for (uint32_t i = 0; i < (f.swiglu_pair ? 1 : f.n_seg); i++) n_tiles += (f.rows[i] + kTileRows - 1) / kTileRows;
         const uint32_t nq = f.swiglu_pair ? 2 : 1;
