@@ -1,0 +1,72 @@
+"""Lines of the dispatch, from both sides: dependent one-vector matvecs over many rows on half-size CTAs (qmv_digits.cu), activation rows that
+share a CTA in the GEMM's re-layout (qgemm_tc.cu)."""
+
+import numpy as np
+import pytest
+
+from conftest import guarded_rel_err, REL_TOL
+from test_gpu_runner import make_oracle_model
+from yule_b200 import CudaB200Backend, CudaTransformerRunner, DType, ModelConfig, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q8_0, DType.Q4_0, DType.Q6_K])
+@pytest.mark.parametrize("vocab", [29984, 30000, 30016])
+def test_output_matrix_in_the_token_step(backend, oracle, dtype, vocab):
+    cfg = ModelConfig(dim=512, n_layers=1, n_heads=8, n_kv_heads=2, head_dim=64, vocab_size=vocab, ff_dim=512, max_seq_len=16)
+    weights = synth.synthetic_model(cfg, seed=7, std=0.05, linear=DType.Q8_0, output=dtype)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    got, want = run.prefill([3, 17, 4]), ref.prefill([3, 17, 4])
+    for t in (29983, 5):
+        assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()  # 22-bit activations, fp32 sums over 512 columns: some 1e-6
+        got, want = run.decode_step(t), ref.decode_step(t)
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+    run.close()
+
+
+@pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q8_0])
+@pytest.mark.parametrize("cols", [256, 4096, 4352, 8192, 8448, 16384, 16640])
+@pytest.mark.parametrize("batch,odd", [(255, 0), (257, 0), (300, 1), (384, 2)])
+def test_re_layout(backend, oracle, dtype, cols, batch, odd):
+    """Two rows per CTA from 296 padded rows on; rows that start off a 16-byte boundary (odd = extra floats per row); a padded last tile."""
+    rows, stride = 40, cols + odd
+    w, x = synth.random_quantized(dtype, 11, rows * cols), synth.normal(12, batch * stride)
+    wh, xh, oh = backend.upload(w), backend.upload(x), backend.allocate(batch * rows * 4)
+    backend.quantized_matmul_batched(wh, xh, oh, rows, cols, dtype, batch, stride, rows)
+    y = backend.download(oh, batch * rows).reshape(batch, rows)
+    for b in (0, 1, 2, batch // 2, batch - 2, batch - 1):
+        ref = oracle.qmv(int(dtype), w, x[b * stride:b * stride + cols], rows, cols)
+        assert guarded_rel_err(y[b], ref) <= REL_TOL
+        assert np.abs(y[b] - ref).max() <= 1e-5 * np.abs(ref).max()
+    for h in (wh, xh, oh):
+        backend.free(h)
+
+
+def test_long_prompt_through_two_row_re_layout(backend, oracle):
+    cfg = ModelConfig(dim=512, n_layers=2, n_heads=8, n_kv_heads=2, head_dim=64, vocab_size=600, ff_dim=768, max_seq_len=400)
+    weights = synth.synthetic_model(cfg, seed=9, std=0.05, linear=DType.Q4_K, ffn_down=DType.Q6_K)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    prompt = synth.tokens(10, 333, cfg.vocab_size)
+    got, want = run.prefill(prompt), ref.prefill(list(prompt))
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+    run.close()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("rows,batch", [(4352, 9), (4608, 10), (4608, 12)])  # 119, 126 and 126 Mi weights: the line is 120 Mi
+def test_nine_to_twelve_vectors_over_a_large_matrix(oracle, rows, batch, captured):
+    """Where the GEMM takes over it needs a scratch; the first call of a context inside a capture goes without."""
+    cols = 28672
+    b = CudaB200Backend(0)
+    w, x = synth.random_quantized(DType.Q4_K, 21, rows * cols), synth.normal(22, batch * cols)
+    wh, xh, oh = b.upload(w), b.upload(x), b.allocate(batch * rows * 4)
+    if captured:
+        b.graph_begin()
+    b.quantized_matmul_batched(wh, xh, oh, rows, cols, DType.Q4_K, batch)
+    if captured:
+        b.graph_launch(b.graph_end())
+    y = b.download(oh, batch * rows).reshape(batch, rows)
+    b.close()
+    for i in (0, batch - 1):
+        assert guarded_rel_err(y[i], oracle.qmv(int(DType.Q4_K), w, x[i * cols:(i + 1) * cols], rows, cols)) <= REL_TOL
