@@ -689,6 +689,32 @@ int32_t yule_cuda_dequantize(yule_cuda_ctx *ctx, yule_buffer weights, uint32_t g
     return YULE_OK;
 }
 
+// Grows the split scratch of the attention entry point, each block by itself and never below what it was.  The context's lock is held.  What is
+// outgrown is kept: a graph captured earlier may still replay into it.
+static int32_t grow_attn_scratch(yule_cuda_ctx *ctx, size_t floats, uint32_t tickets) {
+    auto fresh = [&](void **block, size_t bytes) {
+        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e == cudaSuccess) e = cudaMalloc(block, bytes);
+        if (e == cudaSuccess && (e = cudaMemsetAsync(*block, 0, bytes, ctx->stream)) != cudaSuccess) cudaFree(*block);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e;
+    };
+    void *block = nullptr;
+    if (ctx->attn_scratch_floats < floats) {
+        YULE_CUDA_TRY(fresh(&block, floats * sizeof(float)));
+        if (ctx->attn_scratch) ctx->retired_scratch.push_back(ctx->attn_scratch);
+        ctx->attn_scratch = (float *)block;
+        ctx->attn_scratch_floats = floats;
+    }
+    if (ctx->attn_tickets_n < tickets) {
+        YULE_CUDA_TRY(fresh(&block, (size_t)tickets * sizeof(uint32_t)));
+        if (ctx->attn_tickets) ctx->retired_scratch.push_back(ctx->attn_tickets);
+        ctx->attn_tickets = (uint32_t *)block;
+        ctx->attn_tickets_n = tickets;
+    }
+    return YULE_OK;
+}
+
 int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k_cache, yule_buffer v_cache,
                                       yule_buffer out, uint32_t head_dim, uint32_t seq_len, uint32_t n_heads,
                                       uint32_t n_kv_heads, uint32_t kv_stride) {
@@ -714,40 +740,32 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
         // 32 heads of 64 on 4, 250 positions 7.1 -> 5.0, 1500 12.6 -> 8.0, 6000 15.5 -> 12.4, 16000 20.3 -> 21.2; 32 heads of 128 on 8, 250 6.8 ->
         // 5.1, 1500 11.6 -> 10.3, 2500 12.4 -> 12.1, 3500 12.9 -> 13.9; 64 heads on 8, 700 11.6 -> 10.2, 2500 16.6 -> 14.9, 3500 17.3 -> 17.5.
         const bool clustered = a.gqa && (uint64_t)seq_len * head_dim <= 327680;
-        uint32_t ranks = 0, tickets_n = n_heads;
+        const uint32_t splits = a.gqa ? attn_gqa_pick_splits(n_kv_heads, seq_len, ctx->prop.multiProcessorCount)
+                                      : attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount);
+        const uint32_t cluster_tickets = a.gqa ? n_kv_heads * kAttnMaxRanks : 0;
+        a.n_splits = splits;
         if (clustered) {
+            uint32_t ranks;
             attn_cluster_shape(n_kv_heads, head_dim, seq_len, true, ctx->prop.multiProcessorCount, &ranks, &a.n_splits);
-            tickets_n = n_kv_heads * kAttnMaxRanks;
-        } else {
-            a.n_splits = a.gqa ? attn_gqa_pick_splits(n_kv_heads, seq_len, ctx->prop.multiProcessorCount)
-                               : attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount);
         }
-        const size_t need = attn_scratch_floats(n_heads, a.n_splits, head_dim);
         {
             std::lock_guard<std::mutex> lock(ctx->mu);
             // (more than 256 positions need the scratch of this entry point, whatever the clusters make of it: a capture that cannot have it is refused)
             const bool longer = attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount) > 1;
-            bool grow = (a.n_splits > 1 || longer) && (ctx->attn_scratch_floats < need || ctx->attn_tickets_n < tickets_n);
-            if (grow && ctx->capturing && !longer) {
-                // no scratch to be had while a graph is captured: one cluster per KV head, which needs none
-                grow = false;
-                a.n_splits = 1;
-            }
-            if (grow) {
-                if (ctx->capturing)
+            auto holds = [&](uint32_t n, uint32_t tickets) {
+                return ctx->attn_scratch_floats >= attn_scratch_floats(n_heads, n, head_dim) && ctx->attn_tickets_n >= tickets;
+            };
+            if (a.n_splits == 1 && !longer) {
+                // one cluster per KV head, or one CTA per query head: no scratch
+            } else if (!ctx->capturing) {
+                // What either route takes at this length: a host that takes turns between long and short contexts allocates once, and after one
+                // call outside it a capture has what both need.
+                const uint32_t n = splits > a.n_splits ? splits : a.n_splits;
+                if (int32_t rc = grow_attn_scratch(ctx, attn_scratch_floats(n_heads, n, head_dim), n_heads > cluster_tickets ? n_heads : cluster_tickets)) return rc;
+            } else if (!holds(a.n_splits, clustered ? cluster_tickets : n_heads)) {
+                if (longer && !(clustered && holds(splits, n_heads)))
                     return fail(YULE_ERR_INVALID_ARGUMENT, "the attention scratch cannot grow during graph capture: run the call once outside the capture first");
-                YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-                // graphs captured earlier may still replay into the old blocks: retire them, do not free them
-                if (ctx->attn_scratch) ctx->retired_scratch.push_back(ctx->attn_scratch);
-                if (ctx->attn_tickets) ctx->retired_scratch.push_back(ctx->attn_tickets);
-                ctx->attn_scratch = nullptr;
-                ctx->attn_tickets = nullptr;
-                ctx->attn_scratch_floats = ctx->attn_tickets_n = 0;
-                YULE_CUDA_TRY(cudaMalloc((void **)&ctx->attn_scratch, need * sizeof(float)));
-                YULE_CUDA_TRY(cudaMalloc((void **)&ctx->attn_tickets, (size_t)tickets_n * sizeof(uint32_t)));
-                YULE_CUDA_TRY(cudaMemsetAsync(ctx->attn_tickets, 0, (size_t)tickets_n * sizeof(uint32_t), ctx->stream));
-                ctx->attn_scratch_floats = need;
-                ctx->attn_tickets_n = tickets_n;
+                a.n_splits = 1;  // one cluster per KV head, or one CTA per query head
             }
             a.scratch = ctx->attn_scratch;
             a.tickets = ctx->attn_tickets;
