@@ -181,8 +181,7 @@ int32_t yule_cuda_sample(yule_cuda_ctx *ctx, yule_buffer logits, uint32_t n, con
  * [batch][x_stride] floats, output [batch][out_stride] floats.  Same per-row
  * arithmetic as quantized_matmul.  Small batches go through the matvec kernels,
  * up to sixteen vectors per pass over the weights (Q4_K, Q5_K, Q6_K, Q8_0,
- * Q4_0); from 13 vectors of Q4_K (9 on matrices of
- * more than 120 Mi weights, 17 on up to 17 Mi) or 33 to
+ * Q4_0); from 13 vectors of Q4_K (17 on matrices of up to 17 Mi weights) or 33 to
  * 49 of the other block formats (n_cols a multiple of 256), the tcgen05 GEMM
  * takes one pass over the weights.
  * The GEMM keeps its activation tiles in a scratch owned by the context, grown

@@ -508,12 +508,11 @@ static uint32_t gemm_line(const QmvArgs &a) {
 static bool takes_gemm(const yule_cuda_ctx *ctx, const QmvArgs &a) {
     if (a.batch < 8 || !qgemm_supported(a.type, a.n_cols, a.batch)) return false;
     uint32_t line = gemm_line(a);
-    const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
-    const bool rows = qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride);
     // While a graph is captured its scratch cannot grow: then the matvec kernels, which need none, keep what they can do as well.
-    if (ctx->capturing && ctx->gemm_scratch_bytes < qgemm_scratch_bytes(a.batch, a.n_cols) && (a.batch < line || (rows && a.batch <= 12))) return false;
+    if (ctx->capturing && ctx->gemm_scratch_bytes < qgemm_scratch_bytes(a.batch, a.n_cols) && a.batch < line) return false;
     // the matvec over sixteen vectors a pass wins up to the line that qmv_rows_preferred draws
-    if (rows) line = qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) ? ~0u : 8u;
+    const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
+    if (qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) line = qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) ? ~0u : 8u;
     if (const char *e = knob("YULE_GEMM_MIN_BATCH")) line = atoi(e) < 8 ? 8u : (uint32_t)atoi(e);
     return a.batch >= line;
 }

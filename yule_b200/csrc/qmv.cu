@@ -551,9 +551,7 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
     // several vectors, up to sixteen per pass (YULE_QMV_ROWS=0 / 1: never / wherever it can)
     if (a.batch >= 2) {
         const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
-        // (nine to twelve vectors that the GEMM would be faster for, here because it has no scratch, are still best off together)
-        const bool wanted = knob("YULE_QMV_ROWS") ? atoi(knob("YULE_QMV_ROWS")) != 0
-                                                  : qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) || (a.batch > 8 && a.batch <= 12);
+        const bool wanted = knob("YULE_QMV_ROWS") ? atoi(knob("YULE_QMV_ROWS")) != 0 : qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch);
         if (wanted && qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) {
             QmvRows f;
             f.type = a.type;

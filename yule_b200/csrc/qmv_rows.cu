@@ -852,12 +852,13 @@ cudaError_t launch_format(const QmvRows &f, cudaStream_t s, uint64_t *launches) 
 // whole and overlap independent calls (Q4_K 2048x2048, 4 vectors: 2.8 against 4.0 us), longer ones take several launches there (8192x8192
 // 29 against 17 us).  Q4_K, GEMM with its re-layout against this: 8 vectors 8192x28672 67.5, 68.3 us, smaller ones 6 to 9 us for this; 9 to 12 vectors
 // 14336x4096 26.7, 24.0, 28672x4096 42.3, 42.4, 28672x8192 71.8, 83.5, 8192x28672 67.8, 84.4; 16 vectors 4096x4096 17.7, 13.7, 14336x4096 27.2, 29.2,
-// 8192x8192 28.8, 33.4.  The other formats' GEMM is slower: Q8_0 16 vectors 14336x4096 99, 27, 32 vectors 4096x14336 91, 81; 48 vectors
-// 4096x4096 37 against 44 (Q4_0 34 against 32), 14336x4096 116 against 80 (both as measured with W in shared memory).
+// 8192x8192 28.8, 33.4.  (Up to twelve vectors it is this one also where the GEMM is faster: its accumulators truncate, and the error against
+// 64 bits would go from 1.6e-7 to 3.2e-7 to 4.0e-7, 4608x28672.)  The other formats' GEMM is slower: Q8_0 16 vectors 14336x4096 99, 27, 32 vectors
+// 4096x14336 91, 81; 48 vectors 4096x4096 37 against 44 (Q4_0 34 against 32), 14336x4096 116 against 80 (both as measured with W in shared memory).
 bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch) {
     if (batch < 2) return false;
     if (batch <= 4 && type != YULE_DTYPE_Q5_K) return n_cols > 4096;
-    if (type == YULE_DTYPE_Q4_K) return batch <= 8 || n_rows * n_cols <= (batch <= 12 ? 120ull << 20 : batch <= 16 ? 17ull << 20 : 0ull);
+    if (type == YULE_DTYPE_Q4_K) return batch <= 12 || (batch <= 16 && n_rows * n_cols <= (17ull << 20));
     return batch <= 32 || (batch <= 48 && (n_rows * n_cols > (17ull << 20) || type == YULE_DTYPE_Q4_0 || type == YULE_DTYPE_Q5_K));
 }
 
