@@ -1,6 +1,8 @@
 """Small results to the host (csrc/readback.cu): sizes around its vector width, its CTAs' shares and the line to the copy engine, into
 pageable, unaligned and pinned memory; behind a matvec as its dependent launch; from several threads."""
 
+import ctypes
+import mmap
 import threading
 
 import numpy as np
@@ -50,3 +52,42 @@ def test_behind_a_matvec_and_from_threads(backend, oracle):
     for t in threads:
         t.join()
     assert good == [200] * 4
+
+
+@pytest.mark.parametrize("registered", [
+    [(0, 4096, 3), (12288, 4096, 3)],   # the ends of the destination, not its middle: a kernel's stores to the middle would fault
+    [(0, 8192, 3)],                     # its beginning
+    [(8192, 8192, 3)],                  # its end
+    [(0, 16384, 3)],                    # all of it
+    [(0, 16384, 8 | 3)],                # all of it, read-only for the device
+])
+def test_destinations_that_a_kernel_may_not_store_to(backend, registered):
+    """Memory that is registered in part, or read-only, gets its bytes from the host."""
+    cuda = ctypes.CDLL("libcuda.so.1")
+    data = np.random.default_rng(2).integers(0, 256, 16384, dtype=np.uint8)
+    h, area = backend.upload(data), mmap.mmap(-1, 16384)
+    dst = np.frombuffer(area, np.uint8)
+    base = dst.ctypes.data
+    for at, size, flags in registered:
+        assert cuda.cuMemHostRegister_v2(ctypes.c_void_p(base + at), ctypes.c_size_t(size), flags) == 0
+    try:
+        for lo, hi in ((0, 16384), (16, 16384), (0, 16000)):
+            dst[:] = 0
+            backend.copy_from_device(h, dst[lo:hi])
+            assert np.array_equal(dst[lo:hi], data[:hi - lo])
+    finally:
+        for at, _, _ in registered:
+            cuda.cuMemHostUnregister(ctypes.c_void_p(base + at))
+        backend.free(h)
+
+
+def test_managed_memory(backend):
+    cuda = ctypes.CDLL("libcuda.so.1")
+    data = np.random.default_rng(3).integers(0, 256, 10000, dtype=np.uint8)
+    h, ptr = backend.upload(data), ctypes.c_ulonglong()
+    assert cuda.cuMemAllocManaged(ctypes.byref(ptr), ctypes.c_size_t(10000), 1) == 0
+    dst = np.frombuffer((ctypes.c_ubyte * 10000).from_address(ptr.value), np.uint8)
+    backend.copy_from_device(h, dst)
+    assert np.array_equal(dst, data)
+    cuda.cuMemFree_v2(ptr)
+    backend.free(h)

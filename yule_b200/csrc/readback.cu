@@ -10,6 +10,8 @@
 #include <chrono>
 #include <cstring>
 
+#include <cuda.h>
+
 #include "internal.h"
 
 namespace yule {
@@ -42,15 +44,32 @@ __global__ void set_words_kernel(uint32_t *at, uint32_t a, uint32_t b) {
     at[1] = b;
 }
 
-// The device's view of n bytes of host memory, or null where it has none (pageable memory).
-unsigned char *mapped_view(void *data, size_t n) {
-    cudaPointerAttributes a, z;
-    if (cudaPointerGetAttributes(&a, data) != cudaSuccess || cudaPointerGetAttributes(&z, (char *)data + n - 1) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-    return (char *)z.devicePointer - (char *)a.devicePointer == (ptrdiff_t)(n - 1) ? (unsigned char *)a.devicePointer : nullptr;
+// Whether the n bytes at `data` are host memory that is not managed, by one driver query.  `view`: the device's view of them where a kernel may store there, all
+// n inside one allocation or registration that the device may write (stores to memory registered read-only, or past a registration, would fault), else null.
+bool host_destination(void *data, size_t n, unsigned char **view) {
+    typedef CUresult (*QueryFn)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr);
+    static const QueryFn query = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<QueryFn>(fn);
+    }();
+    unsigned int type = 0, managed = 0, access = 0;
+    CUdeviceptr device = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void *values[] = {&type, &managed, &device, &start, &size, &access};
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(data);
+    *view = nullptr;
+    if (!query || query(6, which, values, at) != CUDA_SUCCESS || managed || (type != 0 && type != CU_MEMORYTYPE_HOST)) return false;
+    // (type 0: pageable memory, of which CUDA knows nothing; the range is in host addresses)
+    if (type != 0 && device && access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE && at >= start && n <= size && at - start <= size - n)
+        *view = reinterpret_cast<unsigned char *>(device);
+    return true;
 }
 
 }  // namespace
@@ -71,12 +90,13 @@ void read_back_destroy(yule_cuda_ctx *ctx) {
 // The stream's work so far is over and its bytes are in `data` when this returns.  Calls of several threads take turns: landing area,
 // ticket and epoch are one set.
 cudaError_t read_back(yule_cuda_ctx *ctx, const void *src, void *data, size_t n, bool pdl) {
-    if (n == 0 || n > kReadBackBytes || ctx->capturing || (reinterpret_cast<uintptr_t>(src) & 15)) {
+    unsigned char *view = nullptr;
+    if (n == 0 || n > kReadBackBytes || ctx->capturing || (reinterpret_cast<uintptr_t>(src) & 15) || !host_destination(data, n, &view)) {
         cudaError_t e = n ? cudaMemcpyAsync(data, src, n, cudaMemcpyDeviceToHost, ctx->stream) : cudaSuccess;
         return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
     }
     std::lock_guard<std::mutex> lock(ctx->rb_mu);
-    unsigned char *direct = (reinterpret_cast<uintptr_t>(data) & 15) == 0 ? mapped_view(data, n) : nullptr;
+    unsigned char *direct = (reinterpret_cast<uintptr_t>(data) & 15) == 0 ? view : nullptr;
     const uint32_t epoch = ++ctx->rb_epoch, grid = (uint32_t)(n < 64 * 4096 ? (n + 4095) / 4096 : 64);
     volatile uint32_t *flag = reinterpret_cast<volatile uint32_t *>(ctx->rb_host + kFlagOffset);
     cudaError_t e = launch_kernel(read_back_kernel, dim3(grid), dim3(kThreads), 0, ctx->stream, pdl, (const unsigned char *)src, direct ? direct : ctx->rb_device,
