@@ -54,6 +54,21 @@ def test_behind_a_matvec_and_from_threads(backend, oracle):
     assert good == [200] * 4
 
 
+def test_every_byte_is_there_when_the_call_returns(backend):
+    """The last CTA's fence has to cover the stores of the others: the destination is looked at at once, each time with other contents."""
+    n = 1 << 20
+    a = np.random.default_rng(1).integers(0, 256, n, dtype=np.uint8)
+    both = a, ~a
+    handles = [backend.upload(x) for x in both]
+    pinned = torch.zeros(n, dtype=torch.uint8).pin_memory().numpy()
+    for size in (5000, 70000, n):
+        for i in range(200):
+            backend.copy_from_device(handles[i & 1], pinned[:size])
+            assert np.array_equal(pinned[:size], both[i & 1][:size])
+    for h in handles:
+        backend.free(h)
+
+
 @pytest.mark.parametrize("registered", [
     [(0, 4096, 3), (12288, 4096, 3)],   # the ends of the destination, not its middle: a kernel's stores to the middle would fault
     [(0, 8192, 3)],                     # its beginning

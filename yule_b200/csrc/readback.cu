@@ -3,8 +3,11 @@
 // A host that drives the layers itself reads a vector back after every few launches, and what that costs is not the transfer (22 KB
 // over PCIe are 0.5 us) but its dressing: a copy on a copy engine, which has to be told by the launch queue, and a wait for the
 // whole stream.  Up to kReadBackBytes a kernel on the same stream stores the bytes into host memory itself, behind a matvec as its
-// dependent launch, and writes an epoch behind them that the host polls.  One 5632x2048 matvec and its result: 21.2 -> 18.1 us; 4096x14336 by
-// four rows 43.5 -> 37.8; from Python, a third of the rest is the calls.
+// dependent launch, and writes an epoch behind them that the host polls.  What bounds it is the trip over PCIe that a system-wide fence waits for: with two
+// fences per CTA, and a second driver query for the destination, pinned memory was slower than the copy engine on every call behind anything but a matvec.
+//   us, copy engine, two fences, one: idle stream, 16 KB pinned 12.5, 13.8, 11.6, pageable 15.7, 14.6, 12.3; 512 KB pinned 21.6, 25.4, 21.0, 1 MB 30.7, 35.2, 30.8
+// (beyond it, the copy engine).  5632x2048 matvec and its result 22.0, 18.4, 16.5; 4096x14336 by four rows 33.7, 33.2, 28.9; RMSNorm of 5632 values and its
+// result 19.1, 17.8, 15.8.  What a trip costs depends on the host: on another one the 5632x2048 matvec took 21.7 and, with two fences, 21.2.
 
 #include <atomic>
 #include <chrono>
@@ -30,9 +33,14 @@ __global__ void __launch_bounds__(kThreads) read_back_kernel(const unsigned char
     if (first < (n & 15u)) dst[(n & ~15u) + first] = __ldcg(src + (n & ~15u) + first);
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence_system();
-        if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
-            *ticket = 0;  // for the next launch on this stream
+        // The CTAs meet on the device; one fence of the last of them, which a trip to the host takes, then orders all their stores before the epoch.
+        bool last = true;
+        if (gridDim.x > 1) {
+            __threadfence();
+            last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+            if (last) *ticket = 0;  // for the next launch on this stream
+        }
+        if (last) {
             __threadfence_system();
             *reinterpret_cast<volatile uint32_t *>(flag) = epoch;
         }
