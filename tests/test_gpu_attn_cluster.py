@@ -58,3 +58,19 @@ def test_runner_up_to_the_full_context(backend, oracle, hd, n_heads, n_kv, ctx, 
         got, want = run.decode_step(t), ref.decode_step(t)
     assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
     run.close()
+
+
+@pytest.mark.parametrize("route", [None, "0", "1"])  # as the runner picks, clusters, splits
+@pytest.mark.parametrize("hd,n_heads,n_kv,turns", [(64, 8, 2, (40, 20, 35, 17, 300, 30)), (64, 4, 4, (96, 17)), (128, 8, 2, (17, 31, 400, 40)), (128, 8, 1, (280, 60))])
+def test_prompts_of_several_turns(backend, oracle, monkeypatch, route, hd, n_heads, n_kv, turns):
+    """Short prompts after others: their queries, each with one key more than the one before, on either side of the line between the kernels."""
+    if route:
+        monkeypatch.setenv("YULE_CUDA_ROWS_SPLITS", route)
+    cfg = ModelConfig(dim=256, n_layers=2, n_heads=n_heads, n_kv_heads=n_kv, head_dim=hd, vocab_size=512, ff_dim=512, max_seq_len=2048)
+    weights = synth.synthetic_model(cfg, seed=4, std=0.08, linear=DType.Q8_0)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    for i, n in enumerate(turns):
+        prompt = synth.tokens(20 + i, n, 512)
+        got, want = run.prefill(prompt), ref.prefill(list(prompt))
+        assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max(), (i, n)
+    run.close()

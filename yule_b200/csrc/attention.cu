@@ -206,17 +206,17 @@ __global__ void __launch_bounds__(kThreads) attn_decode_gqa_kernel(const __grid_
     __shared__ uint32_t s_last;
     yule_pdl_launch_dependents();
     yule_pdl_wait();
-    attn_gqa_unit<GROUP, HD>(p, blockIdx.x, blockIdx.y, threadIdx.x, sm, &s_last);
+    attn_gqa_unit<GROUP, HD>(p, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, sm, &s_last);
 }
 
 template <int GROUP, int HD>
-cudaError_t launch_gqa_variant(const AttnParams &p, size_t smem, bool pdl, cudaStream_t s) {
+cudaError_t launch_gqa_variant(const AttnParams &p, size_t smem, uint32_t n_tokens, bool pdl, cudaStream_t s) {
     auto kern = attn_decode_gqa_kernel<GROUP, HD>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    return launch_kernel(kern, dim3(p.n_kv_heads, p.n_splits), dim3(kThreads), smem, s, pdl, p);
+    return launch_kernel(kern, dim3(p.n_kv_heads, p.n_splits, n_tokens), dim3(kThreads), smem, s, pdl, p);
 }
 
 }  // namespace
@@ -271,7 +271,9 @@ cudaError_t launch_attn_decode(const AttnDecode &a, cudaStream_t s, uint64_t *la
     p.n_splits = a.n_splits;
     p.window = a.window;
     p.softcap = a.softcap;
-    if (a.pos_per_query || a.kv_batch_stride || a.n_tokens > 1 || a.tp.push) return cudaErrorInvalidValue;  // launch_attn_cluster
+    if (a.pos_per_query || a.kv_batch_stride || a.tp.push || (a.n_tokens > 1 && !a.gqa)) return cudaErrorInvalidValue;  // launch_attn_cluster
+    p.q_stride = a.q_stride;
+    p.out_stride = a.out_stride;
     if (a.gqa) {
         if (!attn_gqa_supported(a.hd, a.n_heads, a.n_kv_heads) || a.n_splits > (uint32_t)kGqaMaxSplits) return cudaErrorInvalidValue;
         const uint32_t g = a.n_heads / a.n_kv_heads;
@@ -285,7 +287,7 @@ cudaError_t launch_attn_decode(const AttnDecode &a, cudaStream_t s, uint64_t *la
         if (smem > 200 * 1024) return cudaErrorInvalidValue;
         *launches += 1;
         if (a.k_new || a.pos_ptr || a.cos_table) return cudaErrorInvalidValue;
-#define YULE_GQA_CASE(G, H) if (g == G && a.hd == H) return launch_gqa_variant<G, H>(p, smem, a.pdl, s)
+#define YULE_GQA_CASE(G, H) if (g == G && a.hd == H) return launch_gqa_variant<G, H>(p, smem, a.n_tokens, a.pdl, s)
         YULE_GQA_CASE(1, 64); YULE_GQA_CASE(2, 64); YULE_GQA_CASE(4, 64); YULE_GQA_CASE(8, 64);
         YULE_GQA_CASE(1, 128); YULE_GQA_CASE(2, 128); YULE_GQA_CASE(4, 128); YULE_GQA_CASE(8, 128);
 #undef YULE_GQA_CASE

@@ -196,9 +196,10 @@ __device__ __forceinline__ void attn_gqa_finish(const AttnParams &p, float *scra
     if (tid == 0) tickets_z[kvh] = 0;  // ready for the next launch on this stream
 }
 // One (KV head, split) unit of work of a query whose rows are all in the caches, by the 256 threads of a CTA.
+//   z      query of the launch: it sits z positions further on and has its own rows, scratch and tickets
 //   sm     dynamic shared memory of the unit, s_last one more word
 template <int GROUP, int HD>
-__device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, uint32_t kvh, uint32_t split, uint32_t tid, float *sm, uint32_t *s_last) {
+__device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, uint32_t kvh, uint32_t split, uint32_t z, uint32_t tid, float *sm, uint32_t *s_last) {
     constexpr int J = HD / 32;                               // 16-byte steps per lane and row
     constexpr int GH = (GROUP * J > 16) ? (16 / J) : GROUP;  // query heads scored per pass over K: 16 float4 of queries in registers
     constexpr int HD4 = HD / 4;
@@ -207,7 +208,7 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, uint32_t kvh,
     const uint32_t head0 = kvh * GROUP;
     const float *const k_cache = p.k_cache;
     const float *const v_cache = p.v_cache;
-    const uint32_t seq = p.seq_len, pos = seq - 1;
+    const uint32_t seq = p.seq_len + z, pos = seq - 1;
     // Sliding window: the reference masks positions t < pos − window to −inf once pos >= window; they then carry
     // no weight, so the splits simply cover [begin, seq) instead of [0, seq).  With an attention softcap as well
     // the reference caps after masking (model_runner.rs:688-721), and cap·tanh(−inf / cap) is −cap, a finite
@@ -242,7 +243,8 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, uint32_t kvh,
         for (int j = 0; j < J; j++) kv_next[j] = *reinterpret_cast<const float4 *>(kp + j * 32);
     }
 
-    for (uint32_t i = tid; i < GROUP * HD; i += kThreads) qs[i] = p.q[(size_t)head0 * HD + i];
+    const float *q = p.q + (size_t)z * p.q_stride + (size_t)head0 * HD;
+    for (uint32_t i = tid; i < GROUP * HD; i += kThreads) qs[i] = q[i];
     __syncthreads();
 
     // scores; the loads of tile i+1 are in flight while tile i is multiplied
@@ -370,8 +372,9 @@ __device__ __forceinline__ void attn_gqa_unit(const AttnParams &p, uint32_t kvh,
         }
     }
 
-    attn_gqa_finish<GROUP, HD>(p, p.scratch, p.tickets, kvh, split, eff, lo < hi, tid, o, ml, partial, s_last, [] { __syncthreads(); },
-                               [&](uint32_t i, float v) { p.out[i] = v; });
+    float *out = p.out + (size_t)z * p.out_stride;
+    attn_gqa_finish<GROUP, HD>(p, p.scratch + (size_t)z * p.n_heads * p.n_splits * (HD + 2), p.tickets + (size_t)z * p.n_heads, kvh, split, eff, lo < hi, tid, o, ml,
+                               partial, s_last, [] { __syncthreads(); }, [&](uint32_t i, float v) { out[i] = v; });
 }
 
 // ── the same unit with its keys and values staged in shared memory ──────────────────────────────────────────────

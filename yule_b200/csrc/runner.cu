@@ -876,7 +876,7 @@ int32_t ensure_pinned(yule_cuda_runner *r, size_t n_words) {
 // Tensor-parallel runs read the device status word every this many tokens and stop enqueuing once a bounded
 // wait has given up (the waits themselves return at once after the first failure).
 constexpr uint32_t kStatusCheckTokens = 32;
-constexpr uint32_t kPrefillChunk = 512, kPrefillMinTokens = 16;
+constexpr uint32_t kPrefillChunk = 512, kPrefillMinTokens = 16, kPrefillMinChunk = 256;
 // One GPU: passes of up to this many rows.  A launch's fixed part (about 10 us per GEMM) and the last, partly filled wave of
 // tiles count once per pass.
 constexpr uint32_t kPrefillMaxRows = 2048;
@@ -1294,7 +1294,16 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         a.q_stride = qdim_l;
         a.out_stride = qdim;
         a.settled = ps.batch;
-        if (!tiled) ok(launch_attn_cluster(a, sms, s, launches));
+        // Queries of a prompt share no tiles but are many, and then it is not latency that counts: the splits take fewer instructions per position.  us a pass
+        // after so many positions, clusters, splits, 30 / 90 tokens: 11 layers of the 1.1B shape after 0 813, 818 / 1354, 1362 (60 tokens 1066, 1096), after 100 895, 872 / 1503,
+        // 1452, after 1900 1417, 1268 / 3007, 2328; 6 layers of the 8B shape after 0 574, 582 / 980, 947, after 1900 1238, 992 / 2622, 1918, after 3800 1829, 1285 / 4194, 2642.
+        const bool splits = knob("YULE_CUDA_ROWS_SPLITS") ? atoi(knob("YULE_CUDA_ROWS_SPLITS")) != 0 : (uint64_t)(ps.pos0 + ps.n_live) * hd > 96 * 64;
+        if (!tiled && !ps.batch && splits) {
+            a.min_chunk = kPrefillMinChunk;
+            ok(launch_attn_decode(a, s, launches));
+        } else if (!tiled) {
+            ok(launch_attn_cluster(a, sms, s, launches));
+        }
         exchange(r->xb_att, qdim_l, qdim);
         prep(r->pf_att, qdim, nullptr, nullptr);
         lin(L.attn_output, dim_l, qdim, r->pf_x + (size_t)R * dim_l, dim, r->pf_x + (size_t)R * dim_l);  // x += Wo · attention
