@@ -25,6 +25,21 @@ def test_output_matrix_in_the_token_step(backend, oracle, dtype, vocab):
     run.close()
 
 
+@pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q4_0])
+@pytest.mark.parametrize("dim,ff,vocab", [(2048, 15104, 512), (2304, 15104, 512), (4096, 512, 30016), (4352, 512, 30016)])
+def test_columns_of_a_pair_and_of_an_output_matrix(backend, oracle, dtype, dim, ff, vocab):
+    """30208 rows of gate and up, 30016 of an output matrix: half-size CTAs up to 2048 and 4096 columns."""
+    cfg = ModelConfig(dim=dim, n_layers=1, n_heads=8, n_kv_heads=2, head_dim=64, vocab_size=vocab, ff_dim=ff, max_seq_len=16)
+    weights = synth.synthetic_model(cfg, seed=8, std=0.05, linear=dtype)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    got, want = run.prefill([3, 17]), ref.prefill([3, 17])
+    for t in (500, 5):
+        assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+        got, want = run.decode_step(t), ref.decode_step(t)
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+    run.close()
+
+
 @pytest.mark.parametrize("dtype", [DType.Q4_K, DType.Q8_0])
 @pytest.mark.parametrize("cols", [256, 4096, 4352, 8192, 8448, 16384, 16640])
 @pytest.mark.parametrize("batch,pad", [(255, 0), (257, 0), (300, 4), (384, 8)])

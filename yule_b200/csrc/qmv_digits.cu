@@ -759,15 +759,17 @@ cudaError_t launch_format(const QmvDigits &f, int sm_count, uint32_t share, cuda
 // not keep fed.  us per independent call, 16-warp CTAs against these: Q4_K 2048x2048 2.26, 0.95, 5632x2048 3.29, 2.30, 14336x4096
 // 9.1, 6.7, 28672x8192 23.3, 22.7; Q8_0 2048x2048 2.45, 1.14; two to an SM Q6_K 14336x4096 11.3, 9.5, Q8_0 4096x4096 4.5, 3.4;
 // beyond the lines Q4_K 4096x14336 7.2, 8.6, Q5_K 28672x8192 27.7, 29.7.
-//   In a chain of dependent launches nothing overlaps, but a launch over many rows ends sooner: more CTAs, each with fewer units, leave a smaller
-// last round.  From 30000 rows on, for the two formats whose unpacking is shortest: us per token, 16-warp CTAs against these, 8 layers of
-// the 8B shape in Q4_0 (128256x4096 output) 503, 491; 4 layers of the 70B shape in Q4_K (57344x8192) 628, 626.  With the line at 12000 rows
-// (28672x4096 in Q4_K) 8B 1563, 1650; the outputs of Q8_0 and Q6_K (32000x2048, 128256x4096) gain nothing.
+//   In a chain of dependent launches nothing overlaps, yet over many rows of few columns, where a tile is a stage or two, three half-size CTAs keep an SM
+// busier through the start and the end of a tile than one.  So they are taken from 30000 rows of up to 4096 columns on (a gate / up pair: 2048), for the two
+// formats whose unpacking is shortest.  us per token, 16-warp CTAs, these, two layers and an output in Q4_K: 32000x2048 47.5, 47.1, 32000x4096 64.7, 63.1, 64000x4096
+// 79.9, 74.2, 128256x4096 110.9, 98.5, 256000x3072 159.4, 126.3; 32768x8192 92.1, 93.9, 200064x5120 152.2, 159.5.  Eight layers with a gate / up pair of 30720x1024 205.1,
+// 197.1, 49152x2048 295.9, 285.4; 32768x4096 326.2, 346.9, 30208x5120 389.3, 431.1, 32768x6144 419.6, 463.2.  Q4_0 alike.  28672x4096 in the 8B model
+// 1563, 1650; the outputs of Q8_0 and Q6_K (32000x2048, 128256x4096) gain nothing.
 template <int F>
 cudaError_t launch_sized(const QmvDigits &f, int sm_count, cudaStream_t s, uint64_t *launches) {
     uint32_t all_rows = 0;
     for (uint32_t i = 0; i < f.n_seg; i++) all_rows += f.rows[i];
-    const bool many_rows = all_rows >= 30000 && (F == kQ4K || F == kQ4);
+    const bool many_rows = all_rows >= 30000 && f.n_cols <= (f.swiglu_pair ? 2048u : 4096u) && (F == kQ4K || F == kQ4);
     if (f.pdl && (f.late_wait || many_rows) && f.n_cols <= 8192 && !f.tp.push && !f.tp.wait) {
         uint32_t n_tiles = 0;
         for (uint32_t i = 0; i < (f.swiglu_pair ? 1 : f.n_seg); i++) n_tiles += (f.rows[i] + kTileRows - 1) / kTileRows;
