@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import glob
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -40,6 +41,44 @@ def _stale(target: str, sources: list[str]) -> bool:
     return any(os.path.getmtime(s) > t for s in sources)
 
 
+# The GEMM's 128-row kernel moves registers between its warps (setmaxnreg) out of what its launch brings, and would wait for ever if the compiler had
+# given it fewer than the split adds up to: that is a matter of the compiler, so it is checked where the compiler runs.
+REGISTER_FLOORS = {"qgemm_tc.cu": (r"qgemm_tc_kernelILi128E", r"kLaunchRegs = (\d+);")}
+
+
+def check_registers(report: str, kernel: str, at_least: int) -> None:
+    """Raises unless ``report`` (ptxas -v) gives every instantiation of ``kernel`` (a pattern) at least so many registers."""
+    counts = {}
+    for name, rest in re.findall(r"Compiling entry function '(\S+)'(.*?)(?=Compiling entry function|\Z)", report, re.S):
+        used = re.search(r"Used (\d+) registers", rest)
+        if re.search(kernel, name) and used:
+            counts[name] = int(used.group(1))
+    if not counts:
+        raise RuntimeError(f"the compiler's report names no kernel {kernel}")
+    for name, n in counts.items():
+        if n < at_least:
+            raise RuntimeError(f"{name} was compiled to {n} registers; its register split is made for a launch with {at_least}")
+
+
+def _compile(job: list[str]) -> None:
+    src = job[job.index("-c") + 1]
+    floor = REGISTER_FLOORS.get(os.path.basename(src))
+    if floor is None:
+        subprocess.check_call(job)
+        return
+    done = subprocess.run(job if "-v" in job else job[:1] + ["-Xptxas", "-v"] + job[1:], stderr=subprocess.PIPE, text=True)
+    all_of_it = done.returncode or "-v" in job
+    sys.stderr.write("".join(line for line in done.stderr.splitlines(True) if all_of_it or not line.startswith(("ptxas info", "    "))))
+    if done.returncode:
+        raise subprocess.CalledProcessError(done.returncode, job)
+    try:
+        with open(src) as f:
+            check_registers(done.stderr, floor[0], int(re.search(floor[1], f.read()).group(1)))
+    except RuntimeError:
+        os.remove(job[job.index("-o") + 1])
+        raise
+
+
 def build_cuda(force: bool = False, verbose: bool = False) -> str:
     """One nvcc process per source file (in parallel), objects under ``csrc/build/``, then one link."""
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
@@ -56,7 +95,7 @@ def build_cuda(force: bool = False, verbose: bool = False) -> str:
     if jobs:
         from concurrent.futures import ThreadPoolExecutor
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as pool:
-            list(pool.map(subprocess.check_call, jobs))
+            list(pool.map(_compile, jobs))
     objs = [os.path.join(objdir, os.path.basename(s)[:-3] + ".o") for s in srcs]
     if force or jobs or _stale(CUDA_SO, objs):
         subprocess.check_call([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC"] + objs +

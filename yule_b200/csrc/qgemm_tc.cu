@@ -80,7 +80,7 @@ constexpr int kEpiWarps = 8, kProdWarps = 8;
 constexpr int kLoaderWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kRawWarp = kEpiWarps + 2, kMmaWarp2 = kEpiWarps + 3,
               kFirstProdWarp = kEpiWarps + 4;
 constexpr int kGemmThreads = (kEpiWarps + 4 + kProdWarps) * 32;  // 640
-constexpr int kLaunchRegs = 96;  // registers per thread that 640 threads are launched with
+constexpr int kLaunchRegs = 96;  // registers per thread that 640 threads are launched with (the build checks that the 128-row kernels get them)
 constexpr int kDrainRegs = 144, kControlRegs = 32, kProdRegs = 80;
 static_assert(kEpiWarps * kDrainRegs + 4 * kControlRegs + kProdWarps * kProdRegs <= (kEpiWarps + 4 + kProdWarps) * kLaunchRegs, "register split");
 constexpr uint32_t kStages = 4;  // of the operand ring: W in tensor memory, x in shared memory
@@ -1363,7 +1363,7 @@ cudaError_t launch_gemm(const GemmParams &p, const GemmMaps &w_maps, uint32_t gr
     {
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-            cudaFuncAttributes fa;  // the split of the registers counts on what the launch brings
+            cudaFuncAttributes fa;  // the split of the registers counts on what the launch brings: a library that was not built by build.py must not hang
             e = cudaFuncGetAttributes(&fa, kern);
             if (e == cudaSuccess && BN == 128 && fa.numRegs < kLaunchRegs) e = cudaErrorInvalidValue;
             if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024);
