@@ -5,7 +5,9 @@ import random
 
 import pytest
 
-STAGES, WARPS = 4, 8
+from test_gemm_pipeline_model import RINGS
+
+STAGES, WARPS = RINGS["q4k-128"].stages, 8
 
 
 class Barrier:
@@ -96,8 +98,8 @@ def simulate(seed, nbuf, per_block, with_min, blocks):
             del waits[r]
 
 
-# accumulators, stages per super-block, min term: 128 and 64 rows, 32 rows, the formats without a min term at 64+ and at 32 rows
-@pytest.mark.parametrize("nbuf,per_block,with_min", [(3, 4, True), (4, 2, True), (2, 4, False), (4, 4, False)])
+# accumulators, stages per super-block, min term of every instantiation, as the source has them
+@pytest.mark.parametrize("nbuf,per_block,with_min", sorted({(c.nbuf, c.stages_per_unit, c.min_term) for c in RINGS.values()}))
 def test_rings_hold(nbuf, per_block, with_min):
     for seed in range(60):
         simulate(seed, nbuf, per_block, with_min, 1 + seed % 7)

@@ -868,9 +868,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             cur.start(p, n_items, bpr);
             ahead = cur;
             copy_unit(ahead, 0);
-            for (uint32_t u = 0; cur.live && ok; u++, cur = ahead) {
+            // A warp that has given up goes on through its units, without copying or unpacking: the barriers below count all eight warps and have no
+            // bound, so one that left would keep those that passed its last wait just before it ran out.
+            for (uint32_t u = 0; cur.live; u++, cur = ahead) {
                 ahead.next(p, n_items, bpr);
-                copy_unit(ahead, u + 1);
+                if (ok) copy_unit(ahead, u + 1);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");   // this thread's copies of unit u have landed
                 asm volatile("bar.sync 2, 256;" ::: "memory");         // and everyone else's
                 const bool live = cur.mt * kBM + r < p.n_rows[cur.seg];
