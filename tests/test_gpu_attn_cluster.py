@@ -74,3 +74,35 @@ def test_prompts_of_several_turns(backend, oracle, monkeypatch, route, hd, n_hea
         got, want = run.prefill(prompt), ref.prefill(list(prompt))
         assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max(), (i, n)
     run.close()
+
+
+@pytest.mark.parametrize("hd,n_heads,n_kv", [(64, 8, 2), (128, 8, 1), (128, 4, 4)])
+@pytest.mark.parametrize("window,softcap", [(130, 0.0), (300, 0.0), (0, 1.5), (300, 0.7), (45, 0.7)])
+def test_window_and_softcap(backend, oracle, hd, n_heads, n_kv, window, softcap):
+    """Positions over one CTA, several and several clusters; window edges inside a tile.  Under a soft-cap masked positions keep a weight."""
+    cfg = ModelConfig(dim=256, n_layers=2, n_heads=n_heads, n_kv_heads=n_kv, head_dim=hd, vocab_size=512, ff_dim=512, max_seq_len=2048,
+                      sliding_window=window, attn_logit_softcap=softcap)
+    weights = synth.synthetic_model(cfg, seed=6, std=0.15, linear=DType.Q8_0)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    tokens, at = list(synth.tokens(7, 901, 512)), 0
+    for upto in (20, 46, 131, 260, 301, 431, 700, 901):
+        got, want = run.prefill(tokens[at:upto]), ref.prefill(tokens[at:upto])
+        assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max(), upto
+        at = upto
+    run.close()
+
+
+@pytest.mark.parametrize("batch,hd,n_heads,n_kv,ctx", [(3, 64, 8, 2, 4096), (16, 128, 8, 4, 2048), (2, 128, 8, 1, 4096), (40, 64, 4, 4, 2048)])
+def test_batches_at_long_contexts(backend, oracle, batch, hd, n_heads, n_kv, ctx):
+    """Several clusters per KV head and sequence (the contexts are long enough for scratch): the first and the last sequence against the CPU runner."""
+    cfg = ModelConfig(dim=256, n_layers=2, n_heads=n_heads, n_kv_heads=n_kv, head_dim=hd, vocab_size=512, ff_dim=512, max_seq_len=ctx)
+    weights = synth.synthetic_model(cfg, seed=8, std=0.08, linear=DType.Q8_0)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), [make_oracle_model(oracle, cfg, weights) for _ in range(2)]
+    steps = 520
+    tokens = synth.tokens(9, batch * steps, 512).reshape(batch, steps)
+    for i in range(steps):
+        got = run.decode_batch(tokens[:, i])
+        for b, m in zip((0, batch - 1), ref):
+            want = m.decode_step(int(tokens[b, i]))
+            assert np.abs(got[b] - want).max() <= 1e-4 * np.abs(want).max(), (b, i)
+    run.close()

@@ -106,3 +106,18 @@ def test_managed_memory(backend):
     assert np.array_equal(dst, data)
     cuda.cuMemFree_v2(ptr)
     backend.free(h)
+
+
+def test_logits_beyond_the_line_to_the_copy_engine(backend, oracle):
+    """262144 logits are 1 MiB."""
+    from test_gpu_runner import make_oracle_model
+    from yule_b200 import CudaTransformerRunner, ModelConfig
+    cfg = ModelConfig(dim=256, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, vocab_size=262400, ff_dim=256, max_seq_len=16)
+    weights = synth.synthetic_model(cfg, seed=3, std=0.05, linear=DType.Q8_0)
+    run, ref = CudaTransformerRunner(backend, cfg, weights, fused=1), make_oracle_model(oracle, cfg, weights)
+    got, want = run.prefill([1, 2]), ref.prefill([1, 2])
+    for t in (262399, 5):
+        assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+        got, want = run.decode_step(t), ref.decode_step(t)
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()
+    run.close()
