@@ -159,18 +159,16 @@ int32_t yule_cuda_create(int32_t ordinal, yule_cuda_ctx **out_ctx) {
     if (e == cudaSuccess) e = cudaMalloc(&ctx->device_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->device_status, 0, sizeof(int));
     if (e == cudaSuccess) e = read_back_create(ctx);
-    if (e != cudaSuccess) {
-        delete ctx;
-        return fail_cuda(e, "context setup");
-    }
-    if (ctx->prop.major < 10) {
-        int major = ctx->prop.major, minor = ctx->prop.minor;
-        cudaStreamDestroy(ctx->stream);
-        cudaFree(ctx->device_status);
+    const bool too_old = e == cudaSuccess && ctx->prop.major < 10;
+    if (e != cudaSuccess || too_old) {
+        const int major = ctx->prop.major, minor = ctx->prop.minor;
         read_back_destroy(ctx);
+        if (ctx->device_status) cudaFree(ctx->device_status);
+        if (ctx->stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
-        return fail(YULE_ERR_CUDA, "device is sm_%d%d; this library carries sm_100a kernels only", major,
-                    minor);
+        if (too_old) return fail(YULE_ERR_CUDA, "device is sm_%d%d; this library carries sm_100a kernels only", major, minor);
+        cudaGetLastError();
+        return fail_cuda(e, "context setup");
     }
     *out_ctx = ctx;
     return YULE_OK;
