@@ -687,142 +687,142 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
     const uint32_t bpr = p.n_cols / 256;  // super-blocks per row
 
     if (warp >= kEpiWarps && warp < kFirstProdWarp) {
-    split_registers<BN, kControlRegs>();  // (one instruction for the warpgroup)
-    if (warp == kLoaderWarp) {
-        if (lane == 0) {
-            yule_pdl_wait();  // the activation tiles come from the kernel before this one
-            RingPos ring;
-            bool ok = true;
-            for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const Item wi = decode_item(p, item, bpr);
-                const unsigned char *src = reinterpret_cast<const unsigned char *>(p.xb) + (size_t)wi.nt * bpr * T::kSuperBytes;
-                for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
-                    const uint32_t s = ring.s, ph = ring.ph;
-                    if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, p.status)) {
-                        ok = false;
-                        break;
+        split_registers<BN, kControlRegs>();  // (one instruction for the warpgroup)
+        if (warp == kLoaderWarp) {
+            if (lane == 0) {
+                yule_pdl_wait();  // the activation tiles come from the kernel before this one
+                RingPos ring;
+                bool ok = true;
+                for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                    const Item wi = decode_item(p, item, bpr);
+                    const unsigned char *src = reinterpret_cast<const unsigned char *>(p.xb) + (size_t)wi.nt * bpr * T::kSuperBytes;
+                    for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
+                        const uint32_t s = ring.s, ph = ring.ph;
+                        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, p.status)) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t g = kb % T::SPB;
+                        const uint32_t bytes = T::KG * 2 * kXHalfBytes + ((!GENERIC && g == T::SPB - 1) ? T::kBmBytes : 0u);  // the sums ride with the last stage
+                        const uint32_t dst = smem_u32(smem + (size_t)s * kStageBytes + T::kOffX);
+                        mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                                     "l"(src + (size_t)(kb / T::SPB) * T::kSuperBytes + (size_t)g * T::KG * 2 * kXHalfBytes), "r"(bytes),
+                                     "r"(bar_full + 8 * s)
+                                     : "memory");
                     }
-                    const uint32_t g = kb % T::SPB;
-                    const uint32_t bytes = T::KG * 2 * kXHalfBytes + ((!GENERIC && g == T::SPB - 1) ? T::kBmBytes : 0u);  // the sums ride with the last stage
-                    const uint32_t dst = smem_u32(smem + (size_t)s * kStageBytes + T::kOffX);
-                    mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                                 "l"(src + (size_t)(kb / T::SPB) * T::kSuperBytes + (size_t)g * T::KG * 2 * kXHalfBytes), "r"(bytes),
-                                 "r"(bar_full + 8 * s)
-                                 : "memory");
                 }
             }
-        }
-    } else if (warp == kMmaWarp || warp == kMmaWarp2) {
-        // The whole warp goes through the loop, so that addresses and descriptors are uniform registers, and one lane issues: with the loop
-        // in one lane every MMA moved its operands there first, which took the issuing thread 47 clocks an MMA alone and 140 beside the
-        // other roles.  The warps alternate stages, so that one waits, fences and commits while the other's MMAs run.
-        //   A parity wait cannot tell a phase from the one two before it, and need not: a stage slot always belongs to the same warp (an
-        // even number of slots), and of an accumulator slot's uses a warp skips so few that the drain of the use before the one it asks
-        // for is known to be over: drains end in order, and it has waited for one that is at most NBUF + 3 uses back (NBUF >= 3), or
-        // NBUF + 2 where no min term sits between the stages (NBUF >= 2).
-        const uint32_t mine = warp == kMmaWarp ? 0u : 1u;
-        // fp16 × fp16 → fp32, both operands K-major, M = 128, N = BN
-        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-        [[maybe_unused]] constexpr uint32_t idesc2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // N = 2·BN
-        constexpr uint32_t x_lbo = BN * 16;  // bytes of one 8-column step of an activation slab (of its hi or lo rows)
-        bool ok = true;
-        RingPos ring, acc;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const Item wi = decode_item(p, item, bpr);
-            for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
-                const uint32_t s = ring.s;
-                if ((kb & 1u) != mine) {  // (a super-block has an even number of stages)
-                    acc.advance(NBUF);
-                    if (!GENERIC && kb % T::SPB == T::SPB - 1) acc.advance(NBUF);
-                    continue;
-                }
-                ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status) && mbar_wait(bar_full + 8 * s, ring.ph, abort_flag, p.status);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t d_main = tmem_base + acc.s * T::kMainCols;
-                const uint32_t stage = smem_u32(smem + (size_t)s * kStageBytes);
-                const uint32_t x_hi = stage + T::kOffX, w0 = tmem_base + T::kABase + s * T::kACols;
-                // One descriptor per stage; the 16-column steps are constants added to its address field (the
-                // issuing thread's own instruction stream, not the tensor pipe, can bound the MMA rate).
-                const uint64_t db0 = T::MERGED ? smem_desc(x_hi, 2 * x_lbo, 128) : smem_desc(x_hi, x_lbo, 128);
-                // The tensor core truncates when it adds to an accumulator, which costs a part of what the accumulator holds.  So
-                // the products with lo terms go first, or to the columns of their own: the hi·hi sums see four additions (eight at two
-                // column groups per stage), not eight or twelve.
-                auto steps = [&](auto f) {
-                    f(std::integral_constant<uint32_t, 0>{});
-                    f(std::integral_constant<uint32_t, 1>{});
-                    f(std::integral_constant<uint32_t, 2>{});
-                    f(std::integral_constant<uint32_t, 3>{});
-                    if constexpr (T::KG == 2) {  // the second group's slabs follow the first's in both operands
-                        f(std::integral_constant<uint32_t, 4>{});
-                        f(std::integral_constant<uint32_t, 5>{});
-                        f(std::integral_constant<uint32_t, 6>{});
-                        f(std::integral_constant<uint32_t, 7>{});
+        } else if (warp == kMmaWarp || warp == kMmaWarp2) {
+            // The whole warp goes through the loop, so that addresses and descriptors are uniform registers, and one lane issues: with the loop
+            // in one lane every MMA moved its operands there first, which took the issuing thread 47 clocks an MMA alone and 140 beside the
+            // other roles.  The warps alternate stages, so that one waits, fences and commits while the other's MMAs run.
+            //   A parity wait cannot tell a phase from the one two before it, and need not: a stage slot always belongs to the same warp (an
+            // even number of slots), and of an accumulator slot's uses a warp skips so few that the drain of the use before the one it asks
+            // for is known to be over: drains end in order, and it has waited for one that is at most NBUF + 3 uses back (NBUF >= 3), or
+            // NBUF + 2 where no min term sits between the stages (NBUF >= 2).
+            const uint32_t mine = warp == kMmaWarp ? 0u : 1u;
+            // fp16 × fp16 → fp32, both operands K-major, M = 128, N = BN
+            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+            [[maybe_unused]] constexpr uint32_t idesc2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // N = 2·BN
+            constexpr uint32_t x_lbo = BN * 16;  // bytes of one 8-column step of an activation slab (of its hi or lo rows)
+            bool ok = true;
+            RingPos ring, acc;
+            for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                const Item wi = decode_item(p, item, bpr);
+                for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
+                    const uint32_t s = ring.s;
+                    if ((kb & 1u) != mine) {  // (a super-block has an even number of stages)
+                        acc.advance(NBUF);
+                        if (!GENERIC && kb % T::SPB == T::SPB - 1) acc.advance(NBUF);
+                        continue;
                     }
-                };
-                constexpr uint32_t w_lo = T::kACols / 2;  // generic: the columns of the weights' lo terms
-                if (elect_one()) {
-                    if constexpr (T::MERGED) {
-                        steps([&](auto k16c) {
-                            constexpr uint32_t k16 = decltype(k16c)::value;
-                            // rows [0, BN) of an 8-column step are the hi terms, rows [BN, 2·BN) the lo terms
-                            const uint64_t db = db0 + (uint64_t)((k16 * 4u * x_lbo) >> 4);
-                            umma_f16_ts<(k16 != 0)>(d_main, w0 + 8 * k16, db, idesc2);  // every stage starts a fresh accumulator
-                            if (GENERIC)  // the lo term of the weights against the hi term of the activations: beside the other small products
-                                umma_f16_ts<1>(d_main + BN, w0 + w_lo + 8 * k16, db, idesc);
-                        });
-                    } else {
-                        steps([&](auto k16c) {
-                            constexpr uint32_t k16 = decltype(k16c)::value;
-                            const uint64_t dbh = db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4);
-                            umma_f16_ts<(k16 != 0)>(d_main, w0 + 8 * k16, dbh + (uint64_t)(kXHalfBytes >> 4), idesc);  // every stage starts a fresh accumulator
-                            if (GENERIC)  // the lo term of the weights against the hi term of the activations
-                                umma_f16_ts<1>(d_main, w0 + w_lo + 8 * k16, dbh, idesc);
-                        });
-                        steps([&](auto k16c) {
-                            constexpr uint32_t k16 = decltype(k16c)::value;
-                            umma_f16_ts<1>(d_main, w0 + 8 * k16, db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4), idesc);
-                        });
-                }
-                umma_commit(bar_acc_full + 8 * acc.s);  // the accumulators may be drained once these MMAs are done
-                if (GENERIC || kb % T::SPB != T::SPB - 1) umma_commit(bar_empty + 8 * s);  // and the operands overwritten
-                }
-                __syncwarp();
-                acc.advance(NBUF);
-                if (!GENERIC && kb % T::SPB == T::SPB - 1) {  // Σ_s m_s · (sum of x over sub-block s), hi and lo sums side by side
-                    ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status);
+                    ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status) && mbar_wait(bar_full + 8 * s, ring.ph, abort_flag, p.status);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
+                    const uint32_t d_main = tmem_base + acc.s * T::kMainCols;
+                    const uint32_t stage = smem_u32(smem + (size_t)s * kStageBytes);
+                    const uint32_t x_hi = stage + T::kOffX, w0 = tmem_base + T::kABase + s * T::kACols;
+                    // One descriptor per stage; the 16-column steps are constants added to its address field (the
+                    // issuing thread's own instruction stream, not the tensor pipe, can bound the MMA rate).
+                    const uint64_t db0 = T::MERGED ? smem_desc(x_hi, 2 * x_lbo, 128) : smem_desc(x_hi, x_lbo, 128);
+                    // The tensor core truncates when it adds to an accumulator, which costs a part of what the accumulator holds.  So
+                    // the products with lo terms go first, or to the columns of their own: the hi·hi sums see four additions (eight at two
+                    // column groups per stage), not eight or twelve.
+                    auto steps = [&](auto f) {
+                        f(std::integral_constant<uint32_t, 0>{});
+                        f(std::integral_constant<uint32_t, 1>{});
+                        f(std::integral_constant<uint32_t, 2>{});
+                        f(std::integral_constant<uint32_t, 3>{});
+                        if constexpr (T::KG == 2) {  // the second group's slabs follow the first's in both operands
+                            f(std::integral_constant<uint32_t, 4>{});
+                            f(std::integral_constant<uint32_t, 5>{});
+                            f(std::integral_constant<uint32_t, 6>{});
+                            f(std::integral_constant<uint32_t, 7>{});
+                        }
+                    };
+                    constexpr uint32_t w_lo = T::kACols / 2;  // generic: the columns of the weights' lo terms
                     if (elect_one()) {
-                        umma_f16(tmem_base + acc.s * T::kMainCols, smem_desc(stage, 2048, 128), smem_desc(stage + T::kOffSums, x_lbo, 128), idesc, 0u);
-                        umma_commit(bar_acc_full + 8 * acc.s);
-                        umma_commit(bar_empty + 8 * s);
+                        if constexpr (T::MERGED) {
+                            steps([&](auto k16c) {
+                                constexpr uint32_t k16 = decltype(k16c)::value;
+                                // rows [0, BN) of an 8-column step are the hi terms, rows [BN, 2·BN) the lo terms
+                                const uint64_t db = db0 + (uint64_t)((k16 * 4u * x_lbo) >> 4);
+                                umma_f16_ts<(k16 != 0)>(d_main, w0 + 8 * k16, db, idesc2);  // every stage starts a fresh accumulator
+                                if (GENERIC)  // the lo term of the weights against the hi term of the activations: beside the other small products
+                                    umma_f16_ts<1>(d_main + BN, w0 + w_lo + 8 * k16, db, idesc);
+                            });
+                        } else {
+                            steps([&](auto k16c) {
+                                constexpr uint32_t k16 = decltype(k16c)::value;
+                                const uint64_t dbh = db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4);
+                                umma_f16_ts<(k16 != 0)>(d_main, w0 + 8 * k16, dbh + (uint64_t)(kXHalfBytes >> 4), idesc);  // every stage starts a fresh accumulator
+                                if (GENERIC)  // the lo term of the weights against the hi term of the activations
+                                    umma_f16_ts<1>(d_main, w0 + w_lo + 8 * k16, dbh, idesc);
+                            });
+                            steps([&](auto k16c) {
+                                constexpr uint32_t k16 = decltype(k16c)::value;
+                                umma_f16_ts<1>(d_main, w0 + 8 * k16, db0 + (uint64_t)((k16 * 2u * x_lbo) >> 4), idesc);
+                            });
+                        }
+                        umma_commit(bar_acc_full + 8 * acc.s);  // the accumulators may be drained once these MMAs are done
+                        if (GENERIC || kb % T::SPB != T::SPB - 1) umma_commit(bar_empty + 8 * s);  // and the operands overwritten
                     }
                     __syncwarp();
                     acc.advance(NBUF);
+                    if (!GENERIC && kb % T::SPB == T::SPB - 1) {  // Σ_s m_s · (sum of x over sub-block s), hi and lo sums side by side
+                        ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {
+                            umma_f16(tmem_base + acc.s * T::kMainCols, smem_desc(stage, 2048, 128), smem_desc(stage + T::kOffSums, x_lbo, 128), idesc, 0u);
+                            umma_commit(bar_acc_full + 8 * acc.s);
+                            umma_commit(bar_empty + 8 * s);
+                        }
+                        __syncwarp();
+                        acc.advance(NBUF);
+                    }
+                }
+            }
+        } else if (warp == kRawWarp) {
+            if (!GENERIC && lane == 0) {
+                UnitWalk walk;
+                walk.start(p, n_items, bpr);
+                for (uint32_t u = 0; walk.live; u++, walk.next(p, n_items, bpr)) {
+                    const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
+                    if (!mbar_wait(bar_raw_empty + 8 * slot, ph ^ 1u, abort_flag, p.status)) break;
+                    const uint32_t x = walk.sb * 144u, y = walk.mt * kBM;  // byte column (a multiple of 16), first row
+                    mbar_arrive_expect_tx(bar_raw_full + 8 * slot, kRawBytes);
+                    asm volatile(
+                        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+                            smem_u32(raw + (size_t)slot * kRawBytes)),
+                        "l"(reinterpret_cast<uint64_t>(&w_maps.m[walk.seg])), "r"(bar_raw_full + 8 * slot), "r"(x), "r"(y)
+                        : "memory");
                 }
             }
         }
-    } else if (warp == kRawWarp) {
-        if (!GENERIC && lane == 0) {
-            UnitWalk walk;
-            walk.start(p, n_items, bpr);
-            for (uint32_t u = 0; walk.live; u++, walk.next(p, n_items, bpr)) {
-                const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
-                if (!mbar_wait(bar_raw_empty + 8 * slot, ph ^ 1u, abort_flag, p.status)) break;
-                const uint32_t x = walk.sb * 144u, y = walk.mt * kBM;  // byte column (a multiple of 16), first row
-                mbar_arrive_expect_tx(bar_raw_full + 8 * slot, kRawBytes);
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-                        smem_u32(raw + (size_t)slot * kRawBytes)),
-                    "l"(reinterpret_cast<uint64_t>(&w_maps.m[walk.seg])), "r"(bar_raw_full + 8 * slot), "r"(x), "r"(y)
-                    : "memory");
-            }
-        }
-    }
     } else if (warp >= kFirstProdWarp) {
         split_registers<BN, kProdRegs>();
         const uint32_t ptid = threadIdx.x - kFirstProdWarp * 32;  // 0..255
@@ -923,82 +923,82 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             }
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else {
-        bool ok = true;
-        const uint32_t in_core = (r >> 3) * 128 + (r & 7u) * 16;  // place of this row in the m slab
-        const uint32_t w_at = tmem_base + T::kABase + ((warp & 3u) << 21) + hf * 8;  // this warp's lanes, this thread's columns of a stage
-        const __half2 k1024 = __half2half2(__ushort_as_half(0x6400)), kneg1024 = __half2half2(__ushort_as_half(0xE400));
-        const __half2 kneg64 = __half2half2(__ushort_as_half(0xD400)), k16th = __half2half2(__ushort_as_half(0x2C00));
-        RingPos ring;
-        // the four stages of one super-block
-        auto unpack_block = [&](const RowBlock &cur) {
-            const ScalesMins sm = q4k_scales_mins(cur.hdr.y, cur.hdr.z, cur.hdr.w);
-#pragma unroll
-            for (uint32_t g = 0; g < 4; g++) {
-                const uint32_t s = ring.s;
-                const bool opens = g % T::KG == 0, closes = g % T::KG == T::KG - 1;  // first / last group of its stage
-                // scales of sub-blocks 2g (low nibbles) and 2g + 1 (high nibbles) as fp16 pairs (sc, sc)
-                const uint32_t scw = g < 2 ? sm.sc_lo : sm.sc_hi, j0 = (2 * g) & 3u;
-                const __half2 sc0 = __hsub2(as_half2(biased_pair(scw, 0x4040u + j0 * 0x0101u)), k1024);
-                const __half2 sc1 = __hsub2(as_half2(biased_pair(scw, 0x4040u + (j0 + 1) * 0x0101u)), k1024);
-                // low nibbles: (1024 + q)·sc − 1024·sc, high nibbles where they lie: (1024 + 16·q)·(sc / 16) − 64·sc; both q·sc, exact
-                const __half2 nb0 = __hmul2(sc0, kneg1024), nb1 = __hmul2(sc1, kneg64), sc1_16 = __hmul2(sc1, k16th);  // −1024·sc ≥ −64512
-                if (opens) {
-                    ok = mbar_wait(bar_empty + 8 * s, ring.ph ^ 1u, abort_flag, p.status);
-                    ok = __all_sync(0xffffffffu, ok);  // (a warp stays together: its stores are the warp's)
-                    if (!ok) return;
-                    tc_fence_after();
+            bool ok = true;
+            const uint32_t in_core = (r >> 3) * 128 + (r & 7u) * 16;  // place of this row in the m slab
+            const uint32_t w_at = tmem_base + T::kABase + ((warp & 3u) << 21) + hf * 8;  // this warp's lanes, this thread's columns of a stage
+            const __half2 k1024 = __half2half2(__ushort_as_half(0x6400)), kneg1024 = __half2half2(__ushort_as_half(0xE400));
+            const __half2 kneg64 = __half2half2(__ushort_as_half(0xD400)), k16th = __half2half2(__ushort_as_half(0x2C00));
+            RingPos ring;
+            // the four stages of one super-block
+            auto unpack_block = [&](const RowBlock &cur) {
+                const ScalesMins sm = q4k_scales_mins(cur.hdr.y, cur.hdr.z, cur.hdr.w);
+    #pragma unroll
+                for (uint32_t g = 0; g < 4; g++) {
+                    const uint32_t s = ring.s;
+                    const bool opens = g % T::KG == 0, closes = g % T::KG == T::KG - 1;  // first / last group of its stage
+                    // scales of sub-blocks 2g (low nibbles) and 2g + 1 (high nibbles) as fp16 pairs (sc, sc)
+                    const uint32_t scw = g < 2 ? sm.sc_lo : sm.sc_hi, j0 = (2 * g) & 3u;
+                    const __half2 sc0 = __hsub2(as_half2(biased_pair(scw, 0x4040u + j0 * 0x0101u)), k1024);
+                    const __half2 sc1 = __hsub2(as_half2(biased_pair(scw, 0x4040u + (j0 + 1) * 0x0101u)), k1024);
+                    // low nibbles: (1024 + q)·sc − 1024·sc, high nibbles where they lie: (1024 + 16·q)·(sc / 16) − 64·sc; both q·sc, exact
+                    const __half2 nb0 = __hmul2(sc0, kneg1024), nb1 = __hmul2(sc1, kneg64), sc1_16 = __hmul2(sc1, k16th);  // −1024·sc ≥ −64512
+                    if (opens) {
+                        ok = mbar_wait(bar_empty + 8 * s, ring.ph ^ 1u, abort_flag, p.status);
+                        ok = __all_sync(0xffffffffu, ok);  // (a warp stays together: its stores are the warp's)
+                        if (!ok) return;
+                        tc_fence_after();
+                    }
+                    // byte b of the 32 holds column b (low nibble, sub-block 2g) and column 32 + b (high nibble)
+                    const uint32_t qw[4] = {cur.q[g].x, cur.q[g].y, cur.q[g].z, cur.q[g].w};
+                    uint4 lo[2], hi[2];
+    #pragma unroll
+                    for (int half8 = 0; half8 < 2; half8++) {
+                        const uint32_t w0 = qw[2 * half8], w1 = qw[2 * half8 + 1], w0s = w0 >> 8, w1s = w1 >> 8;
+                        // pairs are bytes (0, 2) and (1, 3) of a word
+                        auto low = [&](uint32_t w) { return as_u32(__hfma2(as_half2((w & 0x000F000Fu) | 0x64006400u), sc0, nb0)); };
+                        auto high = [&](uint32_t w) { return as_u32(__hfma2(as_half2((w & 0x00F000F0u) | 0x64006400u), sc1_16, nb1)); };
+                        lo[half8] = make_uint4(low(w0), low(w0s), low(w1), low(w1s));
+                        hi[half8] = make_uint4(high(w0), high(w0s), high(w1), high(w1s));
+                    }
+                    // eight columns are four words of tensor memory: 16·hf of the first 32, 16·hf of the last
+                    const uint32_t w = w_at + s * T::kACols + (g % T::KG) * 32;
+                    tmem_st8(w, lo[0], lo[1]);
+                    tmem_st8(w + 16, hi[0], hi[1]);
+                    if (g == 3) {
+                        // the eight mins of the super-block, twice: columns 0-7 meet the hi sums, 8-15 the lo sums
+                        uint4 m;
+                        m.x = as_u32(__hsub2(as_half2(biased_pair(sm.m_lo, 0x5140u)), k1024));
+                        m.y = as_u32(__hsub2(as_half2(biased_pair(sm.m_lo, 0x5342u)), k1024));
+                        m.z = as_u32(__hsub2(as_half2(biased_pair(sm.m_hi, 0x5140u)), k1024));
+                        m.w = as_u32(__hsub2(as_half2(biased_pair(sm.m_hi, 0x5342u)), k1024));
+                        *reinterpret_cast<uint4 *>(smem + (size_t)s * kStageBytes + hf * 2048 + in_core) = m;
+                        fence_async_smem();  // generic-proxy stores → visible to the tensor core's reads
+                    }
+                    if (closes) {
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_full + 8 * s);
+                        ring.advance(kStages);
+                    }
                 }
-                // byte b of the 32 holds column b (low nibble, sub-block 2g) and column 32 + b (high nibble)
-                const uint32_t qw[4] = {cur.q[g].x, cur.q[g].y, cur.q[g].z, cur.q[g].w};
-                uint4 lo[2], hi[2];
-#pragma unroll
-                for (int half8 = 0; half8 < 2; half8++) {
-                    const uint32_t w0 = qw[2 * half8], w1 = qw[2 * half8 + 1], w0s = w0 >> 8, w1s = w1 >> 8;
-                    // pairs are bytes (0, 2) and (1, 3) of a word
-                    auto low = [&](uint32_t w) { return as_u32(__hfma2(as_half2((w & 0x000F000Fu) | 0x64006400u), sc0, nb0)); };
-                    auto high = [&](uint32_t w) { return as_u32(__hfma2(as_half2((w & 0x00F000F0u) | 0x64006400u), sc1_16, nb1)); };
-                    lo[half8] = make_uint4(low(w0), low(w0s), low(w1), low(w1s));
-                    hi[half8] = make_uint4(high(w0), high(w0s), high(w1), high(w1s));
-                }
-                // eight columns are four words of tensor memory: 16·hf of the first 32, 16·hf of the last
-                const uint32_t w = w_at + s * T::kACols + (g % T::KG) * 32;
-                tmem_st8(w, lo[0], lo[1]);
-                tmem_st8(w + 16, hi[0], hi[1]);
-                if (g == 3) {
-                    // the eight mins of the super-block, twice: columns 0-7 meet the hi sums, 8-15 the lo sums
-                    uint4 m;
-                    m.x = as_u32(__hsub2(as_half2(biased_pair(sm.m_lo, 0x5140u)), k1024));
-                    m.y = as_u32(__hsub2(as_half2(biased_pair(sm.m_lo, 0x5342u)), k1024));
-                    m.z = as_u32(__hsub2(as_half2(biased_pair(sm.m_hi, 0x5140u)), k1024));
-                    m.w = as_u32(__hsub2(as_half2(biased_pair(sm.m_hi, 0x5342u)), k1024));
-                    *reinterpret_cast<uint4 *>(smem + (size_t)s * kStageBytes + hf * 2048 + in_core) = m;
-                    fence_async_smem();  // generic-proxy stores → visible to the tensor core's reads
-                }
-                if (closes) {
-                    tmem_st_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_full + 8 * s);
-                    ring.advance(kStages);
-                }
+            };
+            UnitWalk walk;
+            walk.start(p, n_items, bpr);
+            for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, n_items, bpr)) {
+                const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
+                ok = mbar_wait(bar_raw_full + 8 * slot, ph, abort_flag, p.status);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                // row r of the box: 144 bytes; rows are 36 words apart, so eight lanes cover all 32 banks
+                const unsigned char *bp = raw + (size_t)slot * kRawBytes + r * 144u;
+                RowBlock cur;
+                cur.hdr = *reinterpret_cast<const uint4 *>(bp);
+    #pragma unroll
+                for (int g = 0; g < 4; g++) cur.q[g] = *reinterpret_cast<const uint4 *>(bp + 16 + g * 32 + hf * 16);
+                unpack_block(cur);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_raw_empty + 8 * slot);  // this warp is done with the box
             }
-        };
-        UnitWalk walk;
-        walk.start(p, n_items, bpr);
-        for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, n_items, bpr)) {
-            const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
-            ok = mbar_wait(bar_raw_full + 8 * slot, ph, abort_flag, p.status);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            // row r of the box: 144 bytes; rows are 36 words apart, so eight lanes cover all 32 banks
-            const unsigned char *bp = raw + (size_t)slot * kRawBytes + r * 144u;
-            RowBlock cur;
-            cur.hdr = *reinterpret_cast<const uint4 *>(bp);
-#pragma unroll
-            for (int g = 0; g < 4; g++) cur.q[g] = *reinterpret_cast<const uint4 *>(bp + 16 + g * 32 + hf * 16);
-            unpack_block(cur);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_raw_empty + 8 * slot);  // this warp is done with the box
-        }
         }  // exact Q4_K producer
     } else {
         split_registers<BN, kDrainRegs>();
