@@ -1247,15 +1247,9 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         for (int o = 16; o >= ROWS; o >>= 1) v = both(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     };
-    // rows start on a 16-byte boundary when the stride is a multiple of four floats; otherwise scalar loads
-    auto load8 = [&](const float *from, float (&to)[8]) {
-        if ((reinterpret_cast<uintptr_t>(from) & 15u) == 0) {
-            const float4 a = *reinterpret_cast<const float4 *>(from), b = *reinterpret_cast<const float4 *>(from + 4);
-            to[0] = a.x, to[1] = a.y, to[2] = a.z, to[3] = a.w, to[4] = b.x, to[5] = b.y, to[6] = b.z, to[7] = b.w;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; i++) to[i] = from[i];
-        }
+    auto load8 = [&](const float *from, float (&to)[8]) {  // (the host has checked the alignment)
+        const float4 a = *reinterpret_cast<const float4 *>(from), b = *reinterpret_cast<const float4 *>(from + 4);
+        to[0] = a.x, to[1] = a.y, to[2] = a.z, to[3] = a.w, to[4] = b.x, to[5] = b.y, to[6] = b.z, to[7] = b.w;
     };
     float v[CHUNKS][8];
 #pragma unroll
@@ -1464,6 +1458,8 @@ size_t qgemm_scratch_bytes(uint32_t n_tokens, uint32_t n_cols) {
 
 cudaError_t launch_qgemm_xprep(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches) {
     if (!qgemm_supported(g.type, g.n_cols, g.n_tokens)) return cudaErrorInvalidValue;
+    // rows are read 16 bytes at a time: buffers start on 256-byte boundaries, and the entry points take strides of whole float4s only
+    if (((reinterpret_cast<uintptr_t>(g.x) | reinterpret_cast<uintptr_t>(g.gate) | reinterpret_cast<uintptr_t>(g.norm_w)) & 15) || g.x_stride % 4) return cudaErrorInvalidValue;
     const uint32_t bn = pick_bn(g.n_tokens);
     const uint32_t n_ntiles = (g.n_tokens + bn - 1) / bn, padded = n_ntiles * bn;
     unsigned char *xb = reinterpret_cast<unsigned char *>(g.scratch) + kGemmSplitBytes;
