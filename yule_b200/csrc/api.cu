@@ -736,6 +736,7 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
         // Clusters up to 5120 rows of 64 values or 2560 of 128, beyond them splits that meet in global memory.  us, splits -> clusters:
         // 32 heads of 64 on 4, 250 positions 7.1 -> 5.0, 1500 12.6 -> 8.0, 6000 15.5 -> 12.4, 16000 20.3 -> 21.2; 32 heads of 128 on 8, 250 6.8 ->
         // 5.1, 1500 11.6 -> 10.3, 2500 12.4 -> 12.1, 3500 12.9 -> 13.9; 64 heads on 8, 700 11.6 -> 10.2, 2500 16.6 -> 14.9, 3500 17.3 -> 17.5.
+        // (For heads of 64 the two meet between 6000 and 16000 positions, so their line could lie further out; it has not been looked for.)
         const bool clustered = a.gqa && (uint64_t)seq_len * head_dim <= 327680;
         const uint32_t splits = a.gqa ? attn_gqa_pick_splits(n_kv_heads, seq_len, ctx->prop.multiProcessorCount)
                                       : attn_pick_splits(n_heads, seq_len, ctx->prop.multiProcessorCount);

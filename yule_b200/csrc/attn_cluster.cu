@@ -11,8 +11,9 @@
 // ticket and two more passes of loads.  At long contexts it is a stream: tiles of 32 positions through a ring of asynchronous
 // copies, running maximum and sum per head.
 //
-// Measured, us a token and layer in the chain of a token step, against the split kernel this replaced there: 1.1B shape (32 heads of 64
-// on 4) at 100 positions 8.2 -> 4.2, at 1930 10 -> 7; 8B shape (32 of 128 on 8) at 130 positions 9.7 -> 5.5.
+// Measured, us by which the launch moves the end of a token step on, against the split kernel this replaced there: 1.1B shape (32 heads of 64
+// on 4) at 50 positions 7.8 -> 3.9, at 100 7.8 -> 4.1, at 1930 15.0 -> 8.9; 8B shape (32 of 128 on 8) at 50 9.4 -> 4.5, at 130 9.6 -> 5.6.  Not for the many
+// queries of a prompt: per position it takes more instructions than the splits (runner.cu has the line).
 //
 // Every warp has four rows of a tile to itself, from the copy to the weighted sum, with a running maximum of its own, so the
 // stream has no CTA barrier; 16000 positions of the 8B shape take 35 us (3.7 TB/s), 42 with three barriers a tile.
@@ -34,8 +35,9 @@ namespace {
 
 constexpr uint32_t kTile = 32;        // positions per tile: eight warps of four
 constexpr uint32_t kMaxRanks = kAttnMaxRanks;  // CTAs of a cluster
-// Tiles per CTA from which another cluster joins in.  us per token and layer, two against four: 1.1B shape at 1930 positions 10.3,
-// 12.0, at 430 9.9, 9.7; 8B at 1920 29.2, 31.4, at 320 49.0, 48.5 (whole layer).
+// Tiles per CTA from which another cluster joins in.  us per token and layer, heads of 64, two against four: 1.1B shape at 1930 positions 10.3, 12.0, at
+// 430 9.9, 9.7.  Heads of 128, two, three, four (8B shape with a narrow feed-forward, whole layer): at 300 positions 31.2, 30.6, 30.7, at 500 31.6, 32.4, 32.7, at 1500
+// 33.3, 34.4, 35.5, at 4000 the same: three is right up to some 400 positions, two would be beyond.
 constexpr uint32_t cluster_tiles(uint32_t hd) { return hd == 64 ? 2u : 3u; }
 constexpr int kWarps = kThreads / 32;
 template <int HD>
