@@ -1,0 +1,113 @@
+"""The rings of csrc/qgemm_int.cu under random interleavings, on the CPU: as test_gemm_rings.py, with one or two accumulators per stage, the offset's
+accumulator behind the last stage of a super-block, and the ring of block scales that the unpacking warps store and the drain warps read."""
+
+import os
+import random
+import re
+
+import pytest
+
+from test_gemm_rings import Barrier
+
+with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "yule_b200", "csrc", "qgemm_int.cu")) as f:
+    SOURCE = f.read()
+STAGES, SCALES = (int(re.search(rf"{n} = (\d+);", SOURCE).group(1)) for n in ("kStages", "kScaleRing"))
+WARPS = 8
+
+
+def accumulators(bn, w_cols):
+    """kMainCols, kAccFit and NBUF of the source."""
+    return min(8, (512 - STAGES * w_cols) // (2 * bn if bn <= 64 else bn))
+
+
+CASES = [(bn, name, accumulators(bn, 64 if name == "q6" else 32)) for bn in (32, 64, 128) for name in ("block32", "q5", "q6")]
+
+
+def simulate(seed, nbuf, name, blocks, scale_ring=SCALES):
+    rng = random.Random(seed)
+    n, per = 4 * blocks, 2 if name == "block32" else 1
+    closes = lambda i: name == "q5" and i % 4 == 3  # noqa: E731
+    full, empty = [[Barrier(c) for _ in range(STAGES)] for c in (WARPS + 1, 1)]
+    acc_full, acc_empty = [[Barrier(c) for _ in range(nbuf)] for c in (2 if name == "block32" else 1, WARPS)]
+    w = [[-1] * (WARPS + 1) for _ in range(STAGES)]
+    ran, acc, readers = {-1}, [-1] * nbuf, [WARPS] * nbuf
+    scales = [[-1] * WARPS for _ in range(scale_ring)]
+    queues = [[], []]
+
+    def producer(p):
+        for i in range(n):
+            s = i % STAGES
+            yield lambda: empty[s].over(i // STAGES & 1 ^ 1)
+            assert w[s][p] in ran, "operand overwritten before it was read"
+            w[s][p] = i
+            if p < WARPS:
+                scales[i % scale_ring][p] = i
+            full[s].arrive()
+
+    def mma(s, i, slot, a, last):
+        def go():
+            assert all(t == i for t in w[s]), "MMA on operands of another stage"
+            assert readers[slot] == WARPS, "accumulator overwritten before it was drained"
+            acc[slot], readers[slot] = a, 0
+            if last:
+                ran.add(i)
+        return go
+
+    def issuer(mine):
+        a = 0
+        for i in range(n):
+            s, uses = i % STAGES, per + closes(i)
+            if i & 1 == mine:
+                for k in range(uses):
+                    slot, ph = (a + k) % nbuf, (a + k) // nbuf & 1
+                    yield lambda: acc_empty[slot].over(ph ^ 1)
+                    if k == 0:
+                        yield lambda: full[s].over(i // STAGES & 1)
+                    last = k == uses - 1
+                    queues[mine] += [mma(s, i, slot, a + k, last), acc_full[slot].arrive]
+                    if last:
+                        queues[mine].append(empty[s].arrive)
+                    if name == "block32":
+                        acc_full[slot].arrive()
+            a += uses
+
+    def drain():
+        a = 0
+        for i in range(n):
+            for k in range(per + closes(i)):
+                slot = a % nbuf
+                yield lambda: acc_full[slot].over(a // nbuf & 1)
+                assert acc[slot] == a, "drained another step's sums"
+                assert name != "block32" or all(t == i for t in scales[i % scale_ring]), "scales of another stage"
+                readers[slot] += 1
+                acc_empty[slot].arrive()
+                a += 1
+
+    roles = [producer(p) for p in range(WARPS + 1)] + [issuer(0), issuer(1)] + [drain() for _ in range(WARPS)]
+    waits = {r: next(r, None) for r in roles}
+    speed = {r: rng.choice([1, 1, 3, 20]) for r in roles}
+    waits = {r: c for r, c in waits.items() if c is not None}
+    while waits or queues[0] or queues[1]:
+        ready = [r for r, c in waits.items() if c()]
+        pipe = [q for q in queues if q]
+        assert ready or pipe, "nothing can go on"
+        if pipe and (not ready or rng.random() < 0.3):
+            rng.choice(pipe).pop(0)()
+            continue
+        r = rng.choices(ready, [1 / speed[x] for x in ready])[0]
+        waits[r] = next(r, None)
+        if waits[r] is None:
+            del waits[r]
+
+
+@pytest.mark.parametrize("bn,name,nbuf", CASES)
+def test_rings_hold(bn, name, nbuf):
+    for seed in range(50):
+        simulate(seed, nbuf, name, 1 + seed % 7)
+
+
+def test_the_model_catches_rings_that_are_too_short():
+    for nbuf, name, ring in ((2, "block32", SCALES), (2, "q5", SCALES), (3, "block32", 4)):
+        with pytest.raises(AssertionError):
+            for seed in range(400):
+                simulate(seed, nbuf, name, 6, ring)

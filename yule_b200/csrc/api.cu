@@ -490,10 +490,9 @@ int32_t yule_cuda_attn_value(yule_cuda_ctx *ctx, yule_buffer weights, yule_buffe
     return YULE_OK;
 }
 
-// From how many activation rows the tcgen05 GEMM beats ceil(batch / 4) passes of the matvec kernels
-// (measured on 1024x4096 .. 128256x4096): the exact Q4_K kernel from 16 (from 32 on matrices of up to 8M weights,
-// where four passes of the batched matvec cost less than the GEMM's fixed part), the generic kernel of the other
-// formats from 32, except Q5_K (tensor-pipe matvec at 3.5 us per row against a 195 us GEMM) from 64; from 8 where the
+// From how many activation rows the tcgen05 GEMM beats ceil(batch / 4) passes of the matvec kernels for two to four vectors, where those are the
+// alternative (rows that qmv_rows cannot take; measured on 1024x4096 .. 128256x4096): Q4_K from 16 (from 32 on matrices of up to 8M weights,
+// where four passes of the batched matvec cost less than the GEMM's fixed part), other formats from 32, Q5_K from 64; from 8 where the
 // rows are too long for a batched matvec kernel to hold its activation image.
 static uint32_t gemm_line(const QmvArgs &a) {
     const bool tuned = a.type == YULE_DTYPE_Q4_K || a.type == YULE_DTYPE_Q6_K || a.type == YULE_DTYPE_Q8_0 || a.type == YULE_DTYPE_Q4_0;
@@ -502,12 +501,17 @@ static uint32_t gemm_line(const QmvArgs &a) {
     return a.type == YULE_DTYPE_Q5_K ? 64u : 32u;
 }
 
+// Whether the matvec over sixteen vectors a pass takes the call where the GEMM does not.
+static bool rows_can(const QmvArgs &a) {
+    return qmv_rows_supported(a.type, a.type == YULE_DTYPE_Q6_K ? a.planar : a.w, a.x, a.n_cols, a.x_stride) && qmv_rows_over_matvecs(a.type, a.n_rows, a.n_cols, a.batch);
+}
+
 // Whether a call goes to the GEMM.  YULE_GEMM_MIN_BATCH overrides all of the lines (at least 8).
 static bool takes_gemm(const yule_cuda_ctx *ctx, const QmvArgs &a) {
     if (a.batch < 8 || !qgemm_supported(a.type, a.n_cols, a.batch)) return false;
     uint32_t line = gemm_line(a);
     // While a graph is captured its scratch cannot grow: then the matvec kernels, which need none, keep what they can do as well.
-    if (ctx->capturing && ctx->gemm_scratch_bytes < qgemm_scratch_bytes(a.batch, a.n_cols) && a.batch < line) return false;
+    if (ctx->capturing && ctx->gemm_scratch_bytes < qgemm_scratch_bytes(a.batch, a.n_cols) && (a.batch < line || rows_can(a))) return false;
     // the matvec over sixteen vectors a pass wins up to the line that qmv_rows_preferred draws
     const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
     if (qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) line = qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch) ? ~0u : 8u;
@@ -553,12 +557,17 @@ static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight
     if (type == YULE_DTYPE_Q6_K && W.planar && weight_offset == 0 && W.planar_cols == n_cols &&
         W.planar_blocks == (uint64_t)n_rows * (n_cols / 256))
         a.planar = W.planar;
-    if (takes_gemm(ctx, a)) {
+    bool gemm = takes_gemm(ctx, a);
+    if (gemm) {
+        const int32_t rc = ensure_gemm_scratch(ctx, qgemm_scratch_bytes(batch, n_cols));
+        if (rc && !rows_can(a)) return rc;
+        gemm = rc == YULE_OK;  // (no memory for its scratch: the matvec needs none)
+    }
+    if (gemm) {
         // enough activation rows: one pass over the weights on the tcgen05 GEMM
-        int32_t rc = ensure_gemm_scratch(ctx, qgemm_scratch_bytes(batch, n_cols));
-        if (rc) return rc;
         QGemm g;
         g.w = a.w;
+        g.planar = a.planar;
         g.type = type;
         g.x = a.x;
         g.out = a.out;

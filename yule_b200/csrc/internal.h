@@ -259,8 +259,9 @@ struct QmvRows {
     int *status = nullptr;            // device status word for the kernel's bounded waits, or null
     long long wait_cycles = kDefaultWaitCycles;
 };
-// Whether `batch` vectors (two or more) against a matrix of this format belong to qmv_rows rather than to the kernels for two to four
-// vectors per pass or to the GEMM (the pointers and strides have to be qmv_rows_supported besides).
+// Whether `batch` vectors (two or more) against a matrix of this format belong to qmv_rows rather than to the other matvecs, and whether
+// rather than to those or to the GEMM (the pointers and strides have to be qmv_rows_supported besides).
+bool qmv_rows_over_matvecs(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch);
 bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch);
 bool qmv_rows_supported(uint32_t type, const void *w, const float *x, uint32_t n_cols, uint32_t x_stride);
 cudaError_t launch_qmv_rows(const QmvRows &f, cudaStream_t s, uint64_t *launches);
@@ -293,6 +294,7 @@ struct QGemm {
     const uint8_t *w_more[2] = {nullptr, nullptr};
     float *out_more[2] = {nullptr, nullptr};
     uint32_t n_rows_more[2] = {0, 0}, out_stride_more[2] = {0, 0};
+    const uint8_t *planar = nullptr, *planar_more[2] = {nullptr, nullptr};  // Q6_K: the row-planar copies of w and w_more, where there are any
     void *scratch = nullptr;
     int *status = nullptr;  // the context's device status word
     bool pdl = false;
@@ -312,9 +314,13 @@ cudaError_t launch_qgemm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t 
 // one re-layout, then one GEMM per matrix with the same n_tokens, n_cols and scratch.
 cudaError_t launch_qgemm_xprep(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
 cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64_t *launches);
+// The kernel of Q8_0, Q4_0, Q5_K and Q6_K (qgemm_int.cu), with the parameters that launch_qgemm_mm fills in.
+bool qgemm_int_supported(const QGemm &g);
+cudaError_t launch_qgemm_int(const QGemm &g, const void *params, uint32_t grid, cudaStream_t s);
 
 // Row-planar device copy of a Q6_K tensor (q6k_planar.cu): n_cols a multiple of 256.
 size_t q6k_planar_bytes(uint64_t n_rows, uint32_t n_cols);
+size_t q6k_planar_row_bytes(uint32_t n_cols);
 cudaError_t launch_q6k_repack(const uint8_t *raw, uint8_t *planar, uint64_t n_rows, uint32_t n_cols, cudaStream_t s,
                               uint64_t *launches);
 

@@ -44,6 +44,7 @@ __global__ void repack_q6k_rows_kernel(const uint8_t *__restrict__ raw, uint8_t 
 }  // namespace
 
 size_t q6k_planar_bytes(uint64_t n_rows, uint32_t n_cols) { return (size_t)n_rows * row_record_bytes(n_cols / 256) + 256; }
+size_t q6k_planar_row_bytes(uint32_t n_cols) { return row_record_bytes(n_cols / 256); }
 
 cudaError_t launch_q6k_repack(const uint8_t *raw, uint8_t *planar, uint64_t n_rows, uint32_t n_cols, cudaStream_t s,
                               uint64_t *launches) {

@@ -19,8 +19,7 @@
 // bias that grows with the chain length; draining after every stage, and the small products before the
 // large ones, keep a chain of large ones at 4 MMAs (8 at 32 rows) and leave the long sum to ordinary
 // round-to-nearest fp32; the mean of the bias is given back at the end.  Error against 64 bits (2-norm) at
-// 200 rows: Q8_0 and Q6_K 1.2e-7 to 1.4e-7, Q4_K 2.4e-7 to 2.7e-7; with large and small
-// products in turn, 3.2e-7 and 3.9e-7, in the same time.
+// 200 rows: Q4_K 2.4e-7 to 2.7e-7; with large and small products in turn, 3.9e-7, in the same time.
 //
 // Work items: (row tile, activation tile) pairs; when these are few (small matrices, tensor-parallel
 // shards, few activation rows) the super-blocks of a row are split into up to 16 parts, one item each,
@@ -70,13 +69,14 @@
 
 #include "dequant_device.cuh"
 #include "internal.h"
+#include "qgemm_common.cuh"
 
 namespace yule {
 namespace {
 
 constexpr int kBM = 128;  // rows of W per tile = TMEM lanes
 constexpr int kBK = 64;   // columns per stage (a quarter of a super-block)
-constexpr int kEpiWarps = 8, kProdWarps = 8;
+constexpr int kProdWarps = 8;
 constexpr int kLoaderWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kRawWarp = kEpiWarps + 2, kMmaWarp2 = kEpiWarps + 3,
               kFirstProdWarp = kEpiWarps + 4;
 constexpr int kGemmThreads = (kEpiWarps + 4 + kProdWarps) * 32;  // 640
@@ -95,203 +95,15 @@ __host__ __device__ constexpr uint32_t groups_per_stage(uint32_t bn, bool generi
     return (!generic && bn <= 32) ? 2u : 1u;
 }
 constexpr uint32_t kRawBytes = kBM * 144;          // one super-block of 128 rows: 18 KB
-constexpr float kSumScale = 1.0f / 32.0f;     // the sub-block sums of x are stored divided by 32
-// 1 + 2^-23: what truncation takes of a stage's sum on average (measured 0.9e-7 of the result, exact kernel 0.7e-7, at 32 rows
+// 2^-23: what truncation takes of a stage's sum on average (measured 0.9e-7 of the result, exact kernel 0.7e-7, at 32 rows
 // 1.2e-7) is given back.
-constexpr float kTruncation = 1.00000012f;
+constexpr float kTruncation = 0.00000011920929f;
 constexpr float kGenericWScale = 1024.f;      // generic kernel: weights are scaled by 2^10 before the fp16 hi/lo split
 constexpr uint32_t kAmBytes = kBM * 16 * 2;  // the m slab of a super-block: 128 rows × 16 columns, 4 KB
-constexpr long long kWaitCycles = 2000000000LL;  // ~1 s: far beyond any real stall
 
-constexpr int kGemmSegs = 3;  // matrices that share their activation tiles (Q/K/V; gate/up) in one launch
 struct GemmMaps {
     CUtensorMap m[kGemmSegs];  // exact kernel: tiled view of each weight matrix
 };
-struct GemmParams {
-    const uint8_t *w[kGemmSegs];  // blocks, row-major, per matrix
-    const __half *xb;      // activation tiles written by gemm_xprep_kernel
-    const float *oscale;   // per (padded) activation row: 1 / row scale
-    float *out[kGemmSegs]; // [n_tokens][out_stride] per matrix
-    const float *residual; // added to the results of matrix 0 (same layout; single-matrix launches only) or null
-    uint32_t n_rows[kGemmSegs], out_stride[kGemmSegs];
-    uint32_t mt0[kGemmSegs + 1];  // first row tile of each matrix in the launch's numbering; [n_seg] = n_mtiles
-    uint32_t n_seg;
-    uint32_t n_cols, n_tokens;
-    uint32_t bn;           // activation rows per tile: 32, 64 or 128
-    uint32_t n_mtiles, n_ntiles;
-    uint32_t ksplit, sb_per;  // split of the columns: `ksplit` work items per tile, `sb_per` super-blocks each (the last may be shorter)
-    float *split_part;        // ksplit > 1: per work item a [bn][128] block of partial results
-    uint32_t *split_tickets;  // ksplit > 1: per (tile, drain warp) the number of items that have stored theirs; left at zero
-    uint32_t type;         // GGUF type id of the weights (generic kernel)
-    uint64_t w_row_bytes;  // bytes of one row of the weight tensor
-    uint32_t unit_bytes;   // generic kernel: bytes of 256 columns of one row
-    uint32_t raw_stride;   // generic kernel: shared-memory row stride of the raw copy (an odd multiple of 16 bytes)
-    uint32_t raw_chunks;   // generic kernel: 16-byte chunks copied per row and unit
-    uint32_t raw_ring_bytes;  // generic kernel: two slots of 128 rows
-    float out_scale;       // kTruncation; generic kernel: / kGenericWScale
-    int *status;
-};
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-constexpr uint32_t kSuspendNs = 20000;  // a waiting warp sleeps up to this long instead of spending issue slots on polls
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "n"(kSuspendNs)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait.  False: the CTA is giving up (this thread ran out of time, or another did).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t it = 1;; it++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 255u) == 0u) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > kWaitCycles) {
-                *abort_flag = 1;
-                atomicExch(status, kStatusGemmTimeout);
-                return false;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// Shared-memory operand descriptor, K-major, no swizzle: lbo = bytes between the two core
-// matrices of a 16-column step, sbo = bytes between 8-row groups.  Bit 46 is the descriptor
-// version of this architecture.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
-}
-
-// True in one lane of the warp.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one)::"memory");
-    return one != 0;
-}
-
-// D[tmem] (+)= A[smem] · B[smem], fp16 operands, fp32 accumulate, one CTA.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// A from tensor memory (lane = row, a column two fp16 values), the accumulate flag known at compile time.
-template <int ACC>
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(ACC)
-        : "memory");
-}
-// 4 or 8 words per lane into as many columns of the warp's 32 lanes; in tensor memory after tmem_st_wait().
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint4 &v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4 &a, const uint4 &b) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z),
-                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// The mbarrier gets one arrival when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// The same load without the wait: the registers hold the values only after tmem_ld_wait().
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t *v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t *v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Two fp32 operations per instruction, each rounded as the single one is.  The drain's arithmetic and the unpacking share the issue
-// slots of an SM with everything else; a stage has to get by with fewer of them than its MMAs take clocks.
-__device__ __forceinline__ uint64_t pair(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpair(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// The eight 6-bit scales and mins of a super-block from its 12 packed bytes
-// (yule-core/src/dequant.rs:165-176), four per word, one byte each.
-struct ScalesMins {
-    uint32_t sc_lo, sc_hi, m_lo, m_hi;  // sub-blocks 0-3 and 4-7
-};
-__device__ __forceinline__ ScalesMins q4k_scales_mins(uint32_t s0, uint32_t s1, uint32_t s2) {
-    ScalesMins r;
-    r.sc_lo = s0 & 0x3F3F3F3Fu;
-    r.m_lo = s1 & 0x3F3F3F3Fu;
-    r.sc_hi = (s2 & 0x0F0F0F0Fu) | ((s0 >> 2) & 0x30303030u);
-    r.m_hi = ((s2 >> 4) & 0x0F0F0F0Fu) | ((s1 >> 2) & 0x30303030u);
-    return r;
-}
-// fp16 pair (1024 + a, 1024 + b) from two bytes: 0x6400 | v is the half 1024 + v for v < 1024
-__device__ __forceinline__ uint32_t biased_pair(uint32_t word, uint32_t selector) { return __byte_perm(word, 0x64646464u, selector); }
-__device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
-__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
 
 // Eight consecutive weights (columns col0 .. col0+7 of a 256-column unit, col0 a multiple of 8) from a
 // 2-byte-aligned copy of the unit's blocks, with the arithmetic of the per-element routines
@@ -412,196 +224,55 @@ __device__ __forceinline__ void words_at(const unsigned char *p, uint32_t (&w)[N
         prev = next;
     }
 }
-// 32 consecutive weights (columns col0 .. col0 + 31 of a 256-column unit) times 2^10 as fp16 hi + lo, eight columns at a time to
+// 32 consecutive weights of Q6_K (columns col0 .. col0 + 31 of a super-block) times 2^10 as fp16 hi + lo, eight columns at a time to
 // put(i, hi, lo) in the order 0,2,1,3,4,6,5,7.  The same values as dequant8_unit and its split give, without conversion
-// instructions: a quant is a half after one OR and one subtraction, 2^10·d is a half (fp16 d below 64, subnormals included),
-// hi = rn(d·q) and lo = fma(d, q, -hi), which is exact.  Q6_K: d·sc is a pair of halves itself.  False: not this
-// format, or a scale that is not finite or too large; nothing was written.  Q6_K 2048x5632 against 777 rows: 275 us with dequant8_unit, 185 with this.
+// instructions: a quant is a half after one OR and one subtraction, 2^10·d·sc a pair of halves.  False: a scale that is not finite or too large;
+// nothing was written.  2048x5632 against 777 rows: 275 us with dequant8_unit, 185 with this.  (A tensor with a row-planar copy goes to qgemm_int.cu.)
 template <class Put>
-__device__ __forceinline__ bool unpack32(const unsigned char *unit, uint32_t type, uint32_t col0, bool live, Put put) {
-    const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
+__device__ __forceinline__ bool unpack32_q6k(const unsigned char *unit, uint32_t col0, bool live, Put put) {
     auto finite = [](__half2 d) { return __hle(__habs(__low2half(d)), __ushort_as_half(0x7BFF)); };  // false for infinities and NaN
     auto u16_at = [&](uint32_t off) { return *reinterpret_cast<const unsigned short *>(unit + off); };
-    if (type == YULE_DTYPE_Q8_0 || type == YULE_DTYPE_Q4_0) {
-        const bool q8 = type == YULE_DTYPE_Q8_0;
-        const uint32_t b = (col0 >> 5) * (q8 ? 34u : 18u);
-        const __half2 d = live ? __hmul2(__half2half2(__ushort_as_half(u16_at(b))), k1024) : __half2half2(__ushort_as_half(0));
-        if (!finite(d)) return false;
-        auto split = [&](uint32_t biased, uint32_t bias, uint32_t &hi, uint32_t &lo) {
-            const __half2 q = __hsub2(as_half2(biased), as_half2(bias)), h = __hmul2(d, q);
-            hi = as_u32(h);
-            lo = as_u32(__hfma2(d, q, __hneg2(h)));
+    const uint32_t h = col0 >> 7, g = (col0 >> 5) & 3u;
+    const float d = live ? f16_bits_to_f32(u16_at(208)) * kGenericWScale : 0.f;
+    const uint32_t scw = u16_at(192 + 8 * h + 2 * g);  // the scales of the first and the last sixteen columns
+    __half2 dh[2], dl[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float ds = d * (float)(int)(signed char)(scw >> (8 * k));
+        dh[k] = __float2half2_rn(ds);
+        dl[k] = __float2half2_rn(ds - __low2float(dh[k]));
+    }
+    if (!finite(dh[0]) || !finite(dh[1])) return false;
+    uint32_t ql[8], qh[8];
+    words_at(unit + 64 * h + 32 * (g & 1u), ql);
+    words_at(unit + 128 + 32 * h, qh);
+    const uint32_t sl = 4 * (g >> 1), sh = 2 * g;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        auto split = [&](uint32_t q6, uint32_t &hi, uint32_t &lo) {
+            const __half2 q = __hsub2(as_half2((q6 & 0x00FF00FFu) | 0x64006400u), as_half2(0x64206420u));  // 1056
+            const __half2 a = dh[i >> 1], b = dl[i >> 1], x = __hfma2(a, q, __hmul2(b, q));
+            hi = as_u32(x);
+            lo = as_u32(__hfma2(b, q, __hfma2(a, q, __hneg2(x))));
         };
-        if (q8) {
-            uint32_t w[8];
-            words_at(unit + b + 2, w);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                uint4 h, l;
-                split((w[2 * i] & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.x, l.x);  // byte ^ 128 = byte + 128
-                split(((w[2 * i] >> 8) & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.y, l.y);
-                split((w[2 * i + 1] & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.z, l.z);
-                split(((w[2 * i + 1] >> 8) & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u, h.w, l.w);
-                put(i, h, l);
-            }
-        } else {
-            uint32_t w[4];
-            words_at(unit + b + 2, w);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {  // byte k: columns 2k (low nibble) and 2k + 1
-                const uint32_t v = w[i] & 0x0F0F0F0Fu, u = (w[i] >> 4) & 0x0F0F0F0Fu;
-                uint4 h, l;
-                split(biased_pair(v, 0x4140u), 0x64086408u, h.x, l.x);
-                split(biased_pair(u, 0x4140u), 0x64086408u, h.y, l.y);
-                split(biased_pair(v, 0x4342u), 0x64086408u, h.z, l.z);
-                split(biased_pair(u, 0x4342u), 0x64086408u, h.w, l.w);
-                put(i, h, l);
-            }
-        }
-        return true;
+        const uint32_t v = ((ql[2 * i] >> sl) & 0x0F0F0F0Fu) | (((qh[2 * i] >> sh) & 0x03030303u) << 4);
+        const uint32_t u = ((ql[2 * i + 1] >> sl) & 0x0F0F0F0Fu) | (((qh[2 * i + 1] >> sh) & 0x03030303u) << 4);
+        uint4 hv, lv;
+        split(v, hv.x, lv.x);
+        split(v >> 8, hv.y, lv.y);
+        split(u, hv.z, lv.z);
+        split(u >> 8, hv.w, lv.w);
+        put(i, hv, lv);
     }
-    if (type == YULE_DTYPE_Q6_K) {
-        const uint32_t h = col0 >> 7, g = (col0 >> 5) & 3u;
-        const float d = live ? f16_bits_to_f32(u16_at(208)) * kGenericWScale : 0.f;
-        const uint32_t scw = u16_at(192 + 8 * h + 2 * g);  // the scales of the first and the last sixteen columns
-        __half2 dh[2], dl[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const float ds = d * (float)(int)(signed char)(scw >> (8 * k));
-            dh[k] = __float2half2_rn(ds);
-            dl[k] = __float2half2_rn(ds - __low2float(dh[k]));
-        }
-        if (!finite(dh[0]) || !finite(dh[1])) return false;
-        uint32_t ql[8], qh[8];
-        words_at(unit + 64 * h + 32 * (g & 1u), ql);
-        words_at(unit + 128 + 32 * h, qh);
-        const uint32_t sl = 4 * (g >> 1), sh = 2 * g;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            auto split = [&](uint32_t q6, uint32_t &hi, uint32_t &lo) {
-                const __half2 q = __hsub2(as_half2((q6 & 0x00FF00FFu) | 0x64006400u), as_half2(0x64206420u));  // 1056
-                const __half2 a = dh[i >> 1], b = dl[i >> 1], x = __hfma2(a, q, __hmul2(b, q));
-                hi = as_u32(x);
-                lo = as_u32(__hfma2(b, q, __hfma2(a, q, __hneg2(x))));
-            };
-            const uint32_t v = ((ql[2 * i] >> sl) & 0x0F0F0F0Fu) | (((qh[2 * i] >> sh) & 0x03030303u) << 4);
-            const uint32_t u = ((ql[2 * i + 1] >> sl) & 0x0F0F0F0Fu) | (((qh[2 * i + 1] >> sh) & 0x03030303u) << 4);
-            uint4 hv, lv;
-            split(v, hv.x, lv.x);
-            split(v >> 8, hv.y, lv.y);
-            split(u, hv.z, lv.z);
-            split(u >> 8, hv.w, lv.w);
-            put(i, hv, lv);
-        }
-        return true;
-    }
-    if (type == YULE_DTYPE_Q5_K) {  // the minimum is subtracted in fp32, as the CPU does
-        const uint32_t sb = col0 >> 5;
-        uint32_t sc, mn;
-        if (sb < 4) {
-            sc = unit[4 + sb] & 63u;
-            mn = unit[8 + sb] & 63u;
-        } else {
-            sc = (unit[8 + sb] & 0xFu) | ((unit[sb] >> 6) << 4);
-            mn = (unit[8 + sb] >> 4) | ((unit[4 + sb] >> 6) << 4);
-        }
-        // (scaling by 2^10 commutes with the roundings)
-        const float ds = __fmul_rn(f16_bits_to_f32(u16_at(0)), (float)sc) * kGenericWScale;
-        const float dm = __fmul_rn(f16_bits_to_f32(u16_at(2)), (float)mn) * kGenericWScale;
-        uint32_t ql[8], qh[8];
-        words_at(unit + 48 + 32 * (sb >> 1), ql);
-        words_at(unit + 16, qh);
-        const uint32_t sl = 4 * (sb & 1u);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            auto five = [&](int k) { return ((ql[k] >> sl) & 0x0F0F0F0Fu) | (((qh[k] >> sb) & 0x01010101u) << 4); };
-            auto value = [&](uint32_t q, uint32_t byte) {
-                const float f = __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7440u + byte)) - 8388608.f;
-                return live ? __fsub_rn(__fmul_rn(f, ds), dm) : 0.f;
-            };
-            auto split = [&](float x, float y, uint32_t &hi, uint32_t &lo) {
-                const __half2 hh = __floats2half2_rn(x, y);
-                const float2 back = __half22float2(hh);
-                hi = as_u32(hh);
-                lo = as_u32(__floats2half2_rn(x - back.x, y - back.y));
-            };
-            const uint32_t v = five(2 * i), u = five(2 * i + 1);
-            uint4 h, l;
-            split(value(v, 0), value(v, 2), h.x, l.x);
-            split(value(v, 1), value(v, 3), h.y, l.y);
-            split(value(u, 0), value(u, 2), h.z, l.z);
-            split(value(u, 1), value(u, 3), h.w, l.w);
-            put(i, h, l);
-        }
-        return true;
-    }
-    return false;
+    return true;
 }
 
 // At 128 activation rows the drain warps hold 64 sums and 32 fresh accumulators each: registers move to them from the others.  Called
 // by every warp of a warpgroup.
 template <int BN, int REGS>
 __device__ __forceinline__ void split_registers() {
-    if constexpr (BN == 128) {
-        if constexpr (REGS > kLaunchRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
-        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
-    }
+    move_registers<BN == 128, REGS, kLaunchRegs>();
 }
-
-// Position in the stage ring without a runtime division (an integer division runs on the same
-// slow pipe as the half conversions): slot and phase parity, advanced once per stage.
-struct RingPos {
-    uint32_t s = 0, ph = 0;
-    __device__ __forceinline__ void advance(uint32_t stages) {
-        if (++s == stages) {
-            s = 0;
-            ph ^= 1u;
-        }
-    }
-};
-
-// A work item: tile (row tile x activation tile) and the range of super-blocks [sb0, sb1) of its columns.
-struct Item {
-    uint32_t tile, ks, mt, nt, sb0, sb1, seg;  // mt: row tile inside matrix `seg`
-};
-__device__ __forceinline__ Item decode_item(const GemmParams &p, uint32_t item, uint32_t bpr) {
-    Item r;
-    r.tile = item / p.ksplit;
-    r.ks = item - r.tile * p.ksplit;
-    r.mt = r.tile / p.n_ntiles;
-    r.nt = r.tile - r.mt * p.n_ntiles;
-    r.seg = 0;
-    while (r.seg + 1 < p.n_seg && r.mt >= p.mt0[r.seg + 1]) r.seg++;
-    r.mt -= p.mt0[r.seg];
-    r.sb0 = r.ks * p.sb_per;
-    r.sb1 = r.sb0 + p.sb_per < bpr ? r.sb0 + p.sb_per : bpr;
-    return r;
-}
-// The (work item, super-block) pairs of this CTA in the order every role goes through them.
-struct UnitWalk {
-    uint32_t item, sb, sb1, mt, seg;
-    bool live;
-    __device__ __forceinline__ void load(const GemmParams &p, uint32_t n_items, uint32_t bpr) {
-        live = item < n_items;
-        if (live) {
-            const Item it = decode_item(p, item, bpr);
-            sb = it.sb0;
-            sb1 = it.sb1;
-            mt = it.mt;
-            seg = it.seg;
-        }
-    }
-    __device__ __forceinline__ void start(const GemmParams &p, uint32_t n_items, uint32_t bpr) {
-        item = blockIdx.x;
-        load(p, n_items, bpr);
-    }
-    __device__ __forceinline__ void next(const GemmParams &p, uint32_t n_items, uint32_t bpr) {
-        if (++sb == sb1) {
-            item += gridDim.x;
-            load(p, n_items, bpr);
-        }
-    }
-};
 
 // One row's share of a super-block: the 16-byte header (d, dmin, packed scales) and this thread's
 // 16 of the 32 quant bytes of each of the four 64-column groups.
@@ -884,7 +555,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                     tc_fence_after();
                     const uint32_t w_hi = w_at + ring.s * T::kACols, w_lo = w_hi + T::kACols / 2;
                     uint4 hi[4], lo[4];
-                    const bool done = unpack32(rawrow, p.type, g * kBK + hf * 32, live, [&](uint32_t c8, const uint4 &h, const uint4 &l) { hi[c8] = h, lo[c8] = l; });
+                    const bool done = p.type == YULE_DTYPE_Q6_K && unpack32_q6k(rawrow, g * kBK + hf * 32, live, [&](uint32_t c8, const uint4 &h, const uint4 &l) { hi[c8] = h, lo[c8] = l; });
                     if (__all_sync(0xffffffffu, done)) {
 #pragma unroll
                         for (uint32_t c8 = 0; c8 < 4; c8 += 2) {
@@ -1089,86 +760,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 acc[j] = a.x;
                 acc[j + 1] = a.y;
             }
-            const uint32_t n0 = nt * BN + col_base;
-            if (p.ksplit > 1) {
-                // This item covers a part of the columns.  Every drain warp stores its block of scaled partial sums, then
-                // takes a ticket of its (tile, warp); the warp that finds all the other parts stored adds them in the
-                // order of the parts (its own included, so the sum does not depend on who came last) and writes the result.
-                float *mine = p.split_part + (size_t)item * (BN * kBM) + lane_base + lane;
-#pragma unroll
-                for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-                    const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;
-#pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        const float sc = __shfl_sync(0xffffffffu, osc, j);
-                        __stcg(mine + (size_t)(col_base + c0 + j) * kBM, acc[c0 + j] * sc * p.out_scale);
-                    }
-                }
-                __threadfence();
-                __syncwarp();
-                uint32_t ticket = 0;
-                uint32_t *tk = p.split_tickets + (size_t)wi.tile * kEpiWarps + warp;
-                if (lane == 0) {
-                    ticket = atomicAdd(tk, 1u);
-                    if (ticket == p.ksplit - 1) *tk = 0;  // left at zero for the next launch
-                }
-                ticket = __shfl_sync(0xffffffffu, ticket, 0);
-                if (ticket != p.ksplit - 1) continue;
-                __threadfence();
-                const float *parts = p.split_part + (size_t)(wi.tile * p.ksplit) * (BN * kBM) + (size_t)col_base * kBM + lane_base + lane;
-#pragma unroll
-                for (uint32_t j = 0; j < CW; j++) acc[j] = 0.f;
-                // the loads of up to KS parts are in flight together; the additions keep the order of the parts
-                constexpr uint32_t KS = CW <= 16 ? 4 : (CW <= 32 ? 2 : 1);
-#pragma unroll 1
-                for (uint32_t ks0 = 0; ks0 < p.ksplit; ks0 += KS, parts += KS * BN * kBM) {
-                    float v[KS][CW];
-#pragma unroll
-                    for (uint32_t q = 0; q < KS; q++)
-#pragma unroll
-                        for (uint32_t j = 0; j < CW; j++)
-                            v[q][j] = ks0 + q < p.ksplit ? __ldcg(parts + (size_t)q * (BN * kBM) + (size_t)j * kBM) : 0.f;
-#pragma unroll
-                    for (uint32_t q = 0; q < KS; q++)
-#pragma unroll
-                        for (uint32_t j = 0; j < CW; j++) acc[j] += v[q][j];
-                }
-#pragma unroll
-                for (uint32_t c0 = 0; c0 < CW; c0 += 4) {
-                    const size_t o0 = (size_t)(n0 + c0) * p.out_stride[wi.seg] + row;
-                    const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 < p.n_tokens ? p.n_tokens - (n0 + c0) : 0u;
-                    float res[4];
-                    if (p.residual) {
-#pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
-                    }
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; j++)
-                        if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? acc[c0 + j] + res[j] : acc[c0 + j];
-                }
-                continue;
-            }
-#pragma unroll
-            for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-                const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;  // padded to whole tiles
-                // Four residuals are asked for before the first of their stores (which may be to the same matrix, so nothing but
-                // this order lets them overlap): one by one they took 24 us per tile, so they take 7.
-#pragma unroll
-                for (int j0 = 0; j0 < 16; j0 += 4) {
-                    const size_t o0 = (size_t)(n0 + c0 + j0) * p.out_stride[wi.seg] + row;
-                    const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 + j0 < p.n_tokens ? p.n_tokens - (n0 + c0 + j0) : 0u;
-                    float res[4];
-                    if (p.residual) {
-#pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
-                    }
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; j++) {
-                        const float val = acc[c0 + j0 + j] * __shfl_sync(0xffffffffu, osc, j0 + j) * p.out_scale;
-                        if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? val + res[j] : val;
-                    }
-                }
-            }
+            finish_item<BN, CW>(p, wi, item, warp, lane, lane_base, col_base, acc);
         }
     }
 
@@ -1444,8 +1036,8 @@ cudaError_t encode_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// Q4_K runs on the exact-integer kernel; Q6_K, Q8_0 and Q4_0 on the generic one (YULE_GEMM_GENERIC=1
-// sends Q4_K there too, for comparison).  The activation tiles are laid out per 256 columns.
+// Q4_K runs on the exact-integer kernel, Q8_0, Q4_0, Q5_K and Q6_K on that of qgemm_int.cu, the others on the generic one (YULE_GEMM_GENERIC=1
+// sends all of them there, for comparison).  The activation tiles are laid out per 256 columns.
 bool qgemm_supported(uint32_t type, uint32_t n_cols, uint32_t n_tokens) {
     return is_quantized(type) && n_cols % 256 == 0 && n_cols > 0 && n_cols <= 65536 && n_tokens >= 1;
 }
@@ -1548,7 +1140,20 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
         p.split_tickets = reinterpret_cast<uint32_t *>(g.scratch);
         p.split_part = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(g.scratch) + kGemmTicketBytes);
     }
-    const bool generic = g.type != YULE_DTYPE_Q4_K || (knob("YULE_GEMM_GENERIC") && atoi(knob("YULE_GEMM_GENERIC")));
+    p.status = g.status;
+    p.truncation = kTruncation;
+    p.out_scale = 1.0f;
+    uint32_t grid = p.n_mtiles * p.n_ntiles * p.ksplit;
+    if (grid > (uint32_t)sm_count) grid = (uint32_t)sm_count;
+    p.w_row_bytes = (uint64_t)(g.n_cols / block_size(g.type)) * block_bytes(g.type);
+    const bool forced = knob("YULE_GEMM_GENERIC") && atoi(knob("YULE_GEMM_GENERIC"));
+    if (!forced && qgemm_int_supported(g)) {
+        e = launch_qgemm_int(g, &p, grid, s);
+        if (e != cudaSuccess) return e;
+        *launches += 1;
+        return cudaSuccess;
+    }
+    const bool generic = forced || g.type != YULE_DTYPE_Q4_K;
     const uint32_t kg = groups_per_stage(bn, generic);
     const uint32_t stage_bytes = kg * 2 * bn * kBK * 2 + (generic ? 0u : kAmBytes + bn * 32);
     p.unit_bytes = 256 / block_size(g.type) * block_bytes(g.type);
@@ -1557,9 +1162,7 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     p.raw_ring_bytes = (2 * kBM * p.raw_stride + 127u) & ~127u;
     const size_t raw_ring = generic ? p.raw_ring_bytes : (size_t)raw_slots_for(bn) * kRawBytes;
     p.type = g.type;
-    p.w_row_bytes = (uint64_t)(g.n_cols / block_size(g.type)) * block_bytes(g.type);
-    p.out_scale = (generic ? 1.0f / kGenericWScale : 1.0f) * kTruncation;
-    p.status = g.status;
+    if (generic) p.out_scale /= kGenericWScale;
     const size_t tail_bytes = raw_ring + (2 * kStages + 8 + 2 * kRawSlots) * 8 + 32;
     const size_t smem = kStages * stage_bytes + tail_bytes;
     GemmMaps w_maps;
@@ -1570,8 +1173,6 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
             if (e != cudaSuccess) return e;
         }
     }
-    uint32_t grid = p.n_mtiles * p.n_ntiles * p.ksplit;
-    if (grid > (uint32_t)sm_count) grid = (uint32_t)sm_count;
     if (generic)
         e = bn == 32 ? launch_gemm<32, true>(p, w_maps, grid, smem, g.pdl, s) : (bn == 64 ? launch_gemm<64, true>(p, w_maps, grid, smem, g.pdl, s) : launch_gemm<128, true>(p, w_maps, grid, smem, g.pdl, s));
     else

@@ -551,7 +551,7 @@ cudaError_t launch_qmv(const QmvArgs &a, int sm_count, cudaStream_t s, uint64_t 
     // several vectors, up to sixteen per pass (YULE_QMV_ROWS=0 / 1: never / wherever it can)
     if (a.batch >= 2) {
         const uint8_t *w = a.type == YULE_DTYPE_Q6_K ? a.planar : a.w;
-        const bool wanted = knob("YULE_QMV_ROWS") ? atoi(knob("YULE_QMV_ROWS")) != 0 : qmv_rows_preferred(a.type, a.n_rows, a.n_cols, a.batch);
+        const bool wanted = knob("YULE_QMV_ROWS") ? atoi(knob("YULE_QMV_ROWS")) != 0 : qmv_rows_over_matvecs(a.type, a.n_rows, a.n_cols, a.batch);
         if (wanted && qmv_rows_supported(a.type, w, a.x, a.n_cols, a.x_stride)) {
             QmvRows f;
             f.type = a.type;

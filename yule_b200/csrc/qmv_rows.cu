@@ -848,18 +848,29 @@ cudaError_t launch_format(const QmvRows &f, cudaStream_t s, uint64_t *launches) 
 
 }  // namespace
 
-// Measured per launch, this kernel against the others.  Two to four vectors: the kernels for so few read rows of up to 4096 columns
+// Measured per launch, this kernel against the other matvecs.  Two to four vectors: the kernels for so few read rows of up to 4096 columns
 // whole and overlap independent calls (Q4_K 2048x2048, 4 vectors: 2.8 against 4.0 us), longer ones take several launches there (8192x8192
-// 29 against 17 us).  Q4_K, GEMM with its re-layout against this: 8 vectors 8192x28672 67.5, 68.3 us, smaller ones 6 to 9 us for this; 9 to 12 vectors
-// 14336x4096 26.7, 24.0, 28672x4096 42.3, 42.4, 28672x8192 71.8, 83.5, 8192x28672 67.8, 84.4; 16 vectors 4096x4096 17.7, 13.7, 14336x4096 27.2, 29.2,
-// 8192x8192 28.8, 33.4.  (Up to twelve vectors it is this one also where the GEMM is faster: its accumulators truncate, and the error against
-// 64 bits would go from 1.6e-7 to 3.2e-7 to 4.0e-7, 4608x28672.)  The other formats' GEMM is slower: Q8_0 16 vectors 14336x4096 99, 27, 32 vectors
-// 4096x14336 91, 81; 48 vectors 4096x4096 37 against 44 (Q4_0 34 against 32), 14336x4096 116 against 80 (both as measured with W in shared memory).
-bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch) {
+// 29 against 17 us).  More vectors take several launches there, or run without the tensor pipe.
+bool qmv_rows_over_matvecs(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch) {
     if (batch < 2) return false;
     if (batch <= 4 && type != YULE_DTYPE_Q5_K) return n_cols > 4096;
     if (type == YULE_DTYPE_Q4_K) return batch <= 12 || (batch <= 16 && n_rows * n_cols <= (17ull << 20));
     return batch <= 32 || (batch <= 48 && (n_rows * n_cols > (17ull << 20) || type == YULE_DTYPE_Q4_0 || type == YULE_DTYPE_Q5_K));
+}
+
+// And against the GEMM with its re-layout.  Q4_K (GEMM, this): 8 vectors 8192x28672 67.5, 68.3 us, smaller ones 6 to 9 us for this; 9 to 12 vectors
+// 14336x4096 26.7, 24.0, 28672x4096 42.3, 42.4, 28672x8192 71.8, 83.5, 8192x28672 67.8, 84.4; 16 vectors 4096x4096 17.7, 13.7, 14336x4096 27.2, 29.2,
+// 8192x8192 28.8, 33.4.  (Up to twelve vectors it is this one also where the GEMM is faster: its accumulators truncate, and the error against
+// 64 bits would go from 1.6e-7 to 3.2e-7 to 4.0e-7, 4608x28672.)
+// The other formats' GEMM (qgemm_int.cu) has the error of this kernel (Q8_0 4096 columns and 24 vectors 0.9e-7 both, Q5_K 1.1e-7 against 1.4e-7), so time
+// decides; a seventeenth vector is a second pass here.  17, 24, 32 vectors, GEMM against this: Q5_K 2048x2048 17, 17, 17 against 15, 17, 20 us, 2048x5632 20, 20, 20
+// against 22, 24, 33, 8192x28672 112, 113, 114 against 170, 188, 232; Q6_K 2048x2048 18, 18, 18 against 15, 17, 19, 4096x4096 18, 19, 19 against 23, 24, 27; Q8_0 2048x2048 20, 21, 21
+// against 14, 15, 16, 2048x5632 23, 23, 24 against 21, 24, 27, 8192x8192 47, 47, 47 against 44, 50, 61, 4096x14336 40, 40, 41 against 47, 52, 81; Q4_0 the same within 10 %.
+bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch) {
+    if (batch <= 16 || type == YULE_DTYPE_Q4_K) return qmv_rows_over_matvecs(type, n_rows, n_cols, batch);
+    const bool small = n_rows * n_cols <= (8ull << 20);
+    if (type == YULE_DTYPE_Q5_K || type == YULE_DTYPE_Q6_K) return small && batch <= 24;
+    return batch <= (small ? 32u : n_cols <= 8192 ? 20u : 16u);
 }
 
 bool qmv_rows_supported(uint32_t type, const void *w, const float *x, uint32_t n_cols, uint32_t x_stride) {

@@ -1059,9 +1059,11 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         gq_open = false;
     };
     auto mm = [&](const Tensor &t, uint32_t rows, uint32_t cols, float *out, uint32_t stride, const float *residual) {
+        const uint8_t *planar = t.buf.planar && t.buf.planar_cols == cols ? t.buf.planar : nullptr;
         if (gq_open && share_mm && !residual && gq.type == t.type && gq.n_cols == cols && gq.n_more < 2) {
             const uint32_t i = gq.n_more++;
             gq.w_more[i] = (const uint8_t *)t.buf.ptr;
+            gq.planar_more[i] = planar;
             gq.out_more[i] = out;
             gq.n_rows_more[i] = rows;
             gq.out_stride_more[i] = stride;
@@ -1070,6 +1072,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         mm_flush();
         gq = QGemm();
         gq.w = (const uint8_t *)t.buf.ptr;
+        gq.planar = planar;
         gq.type = t.type;
         gq.out = out;
         gq.residual = residual;
