@@ -29,9 +29,11 @@ struct GemmParams {
     uint32_t n_cols, n_tokens;
     uint32_t bn;           // activation rows per tile: 32, 64 or 128
     uint32_t n_mtiles, n_ntiles;
-    uint32_t ksplit, sb_per;  // split of the columns: `ksplit` work items per tile, `sb_per` super-blocks each (the last may be shorter)
-    float *split_part;        // ksplit > 1: per work item a [bn][128] block of partial results
-    uint32_t *split_tickets;  // ksplit > 1: per (tile, drain warp) the number of items that have stored theirs; left at zero
+    // The first split_tiles tiles are dealt by super-blocks: their split_units = split_tiles · n_cols / 256 in equal runs to split_ctas CTAs; whole
+    // tiles follow, one per CTA and round.
+    uint32_t split_tiles, split_ctas, split_units;
+    float *split_part;        // blocks of [bn][128] partial results: two per CTA (its runs touch at most two tiles), then one per CTA
+    uint32_t *split_tickets;  // per (split tile, drain warp) the number of its parts that are stored; left at zero
     uint32_t type;         // GGUF type id of the weights (generic kernel)
     uint64_t w_row_bytes;  // bytes of one row of the weight tensor
     uint32_t unit_bytes;   // generic kernel: bytes of 256 columns of one row
@@ -241,119 +243,121 @@ struct RingPos {
 
 // A work item: tile (row tile x activation tile) and the range of super-blocks [sb0, sb1) of its columns.
 struct Item {
-    uint32_t tile, ks, mt, nt, sb0, sb1, seg;  // mt: row tile inside matrix `seg`
+    uint32_t tile, mt, nt, sb0, sb1, seg;  // mt: row tile inside matrix `seg`
+    uint32_t part;                         // which of this CTA's runs, where the tile is split
 };
-__device__ __forceinline__ Item decode_item(const GemmParams &p, uint32_t item, uint32_t bpr) {
-    Item r;
-    r.tile = item / p.ksplit;
-    r.ks = item - r.tile * p.ksplit;
-    r.mt = r.tile / p.n_ntiles;
-    r.nt = r.tile - r.mt * p.n_ntiles;
-    r.seg = 0;
-    while (r.seg + 1 < p.n_seg && r.mt >= p.mt0[r.seg + 1]) r.seg++;
-    r.mt -= p.mt0[r.seg];
-    r.sb0 = r.ks * p.sb_per;
-    r.sb1 = r.sb0 + p.sb_per < bpr ? r.sb0 + p.sb_per : bpr;
-    return r;
-}
+// This CTA's work items, in the order in which every role goes through them: its run of the split tiles' super-blocks, which covers a part of one
+// tile or of two, then whole tiles.  (Dealing whole tiles alone leaves the last round as empty as it comes: 448 tiles of a 70B gate / up
+// on 148 SMs are four rounds for 3.03 of work, 112 tiles of a 1.1B down projection one for 0.76.  The parts first, so that adding them up
+// runs under the tiles that follow.)
+// (Selects instead of branches, and nothing that hides from the compiler that all threads have the same item: ring positions and tensor-memory addresses
+// depend on how often loops run, and have to be uniform registers; and with branches the callers' loops came out three times over. Either
+// made the GEMM a tenth to a quarter slower.)
+struct ItemWalk {
+    uint32_t step;
+    __device__ __forceinline__ explicit ItemWalk(const GemmParams &p) : step((uint32_t)(blockIdx.x >= p.split_ctas) << 1) {}
+    __device__ __forceinline__ bool next(const GemmParams &p, uint32_t bpr, Item &r) {
+        const uint32_t ctas = p.split_ctas > 1 ? p.split_ctas : 1;
+        const uint32_t lo = blockIdx.x * p.split_units / ctas, hi = (blockIdx.x + 1) * p.split_units / ctas;  // this CTA's run
+        const uint32_t first = lo / bpr, mid = (first + 1) * bpr;                                                // and where its first tile ends
+        const bool run = step < 2, second = step == 1;
+        r.tile = run ? first + step : p.split_tiles + (step - 2) * gridDim.x + blockIdx.x;
+        r.sb0 = run && !second ? lo + bpr - mid : 0;
+        r.sb1 = !run ? bpr : second ? hi - mid : (hi < mid ? hi : mid) + bpr - mid;
+        r.part = run ? step : 0;
+        step = run && hi <= mid ? 2 : step + 1;
+        r.mt = r.tile / p.n_ntiles;
+        r.nt = r.tile - r.mt * p.n_ntiles;
+        r.seg = 0;
+        while (r.seg + 1 < p.n_seg && r.mt >= p.mt0[r.seg + 1]) r.seg++;
+        r.mt -= p.mt0[r.seg];
+        return r.tile < p.n_mtiles * p.n_ntiles;
+    }
+};
 // The (work item, super-block) pairs of this CTA in the order every role goes through them.
 struct UnitWalk {
-    uint32_t item, sb, sb1, mt, seg;
+    ItemWalk items;
+    Item it;
+    uint32_t sb;
     bool live;
-    __device__ __forceinline__ void load(const GemmParams &p, uint32_t n_items, uint32_t bpr) {
-        live = item < n_items;
-        if (live) {
-            const Item it = decode_item(p, item, bpr);
-            sb = it.sb0;
-            sb1 = it.sb1;
-            mt = it.mt;
-            seg = it.seg;
-        }
+    __device__ __forceinline__ UnitWalk(const GemmParams &p, uint32_t bpr) : items(p) { load(p, bpr); }
+    __device__ __forceinline__ void load(const GemmParams &p, uint32_t bpr) {
+        live = items.next(p, bpr, it);
+        sb = it.sb0;
     }
-    __device__ __forceinline__ void start(const GemmParams &p, uint32_t n_items, uint32_t bpr) {
-        item = blockIdx.x;
-        load(p, n_items, bpr);
-    }
-    __device__ __forceinline__ void next(const GemmParams &p, uint32_t n_items, uint32_t bpr) {
-        if (++sb == sb1) {
-            item += gridDim.x;
-            load(p, n_items, bpr);
-        }
+    __device__ __forceinline__ void next(const GemmParams &p, uint32_t bpr) {
+        if (++sb == it.sb1) load(p, bpr);
     }
 };
+// The block of the work area for an item's partial sums, and one that is no other item's while a whole tile is at work.
+__device__ __forceinline__ float *part_block(const GemmParams &p, uint32_t index, uint32_t bn) { return p.split_part + (size_t)index * (bn * kTileRows); }
+__device__ __forceinline__ uint32_t own_part(const Item &wi) { return 2 * blockIdx.x + wi.part; }
 
 // The end of a work item for one drain warp: its scaled sums to the output, or, where the columns of a tile are split, to the work area.
 // acc[j] is row lane_base + lane, column col_base + j of the tile.
 template <int BN, uint32_t CW>
-__device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi, uint32_t item, uint32_t warp, uint32_t lane, uint32_t lane_base, uint32_t col_base,
+__device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi, uint32_t bpr, uint32_t warp, uint32_t lane, uint32_t lane_base, uint32_t col_base,
                                             float (&acc)[CW]) {
     const uint32_t row = wi.mt * kTileRows + lane_base + lane;
     const uint32_t n0 = wi.nt * BN + col_base;
-    if (p.ksplit > 1) {
+    float truncation = p.truncation, scale = p.out_scale;
+    bool summed = false;
+    if (wi.sb1 - wi.sb0 < bpr) {
         // This item covers a part of the columns.  Every drain warp stores its block of scaled partial sums, then
         // takes a ticket of its (tile, warp); the warp that finds all the other parts stored adds them in the
         // order of the parts (its own included, so the sum does not depend on who came last) and writes the result.
-        float *mine = p.split_part + (size_t)item * (BN * kTileRows) + lane_base + lane;
+        const size_t in_block = (size_t)col_base * kTileRows + lane_base + lane;
+        float *mine = part_block(p, own_part(wi), BN) + in_block;
 #pragma unroll
         for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-            const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;
+            const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;  // padded to whole tiles
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const float sc = __shfl_sync(0xffffffffu, osc, j);
-                __stcg(mine + (size_t)(col_base + c0 + j) * kTileRows, fmaf(acc[c0 + j], p.truncation, acc[c0 + j]) * sc * p.out_scale);
-            }
+            for (uint32_t j = 0; j < 16; j++)
+                __stcg(mine + (size_t)(c0 + j) * kTileRows, fmaf(acc[c0 + j], truncation, acc[c0 + j]) * __shfl_sync(0xffffffffu, osc, j) * scale);
         }
-        __threadfence();
         __syncwarp();
+        // the CTAs whose runs hold the tile's first and its last super-block; the first of them may have begun with the tile before
+        const uint32_t u0 = wi.tile * bpr;
+        const uint32_t cta0 = ((u0 + 1) * p.split_ctas - 1) / p.split_units, n_parts = ((u0 + bpr) * p.split_ctas - 1) / p.split_units - cta0 + 1;
         uint32_t ticket = 0;
         uint32_t *tk = p.split_tickets + (size_t)wi.tile * kEpiWarps + warp;
         if (lane == 0) {
-            ticket = atomicAdd(tk, 1u);
-            if (ticket == p.ksplit - 1) *tk = 0;  // left at zero for the next launch
+            // (release: the stores of the warp, which it has met; acquire: those of the warps that took theirs before)
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(tk) : "memory");
+            if (ticket == n_parts - 1) *tk = 0;  // left at zero for the next launch
         }
         ticket = __shfl_sync(0xffffffffu, ticket, 0);
-        if (ticket != p.ksplit - 1) return;
-        __threadfence();
-        const float *parts = p.split_part + (size_t)(wi.tile * p.ksplit) * (BN * kTileRows) + (size_t)col_base * kTileRows + lane_base + lane;
+        if (ticket != n_parts - 1) return;
+        __syncwarp();
+        const uint32_t first = 2 * cta0 + (cta0 * p.split_units / p.split_ctas < u0 ? 1u : 0u);
 #pragma unroll
         for (uint32_t j = 0; j < CW; j++) acc[j] = 0.f;
         // the loads of up to KS parts are in flight together; the additions keep the order of the parts
         constexpr uint32_t KS = CW <= 16 ? 4 : (CW <= 32 ? 2 : 1);
 #pragma unroll 1
-        for (uint32_t ks0 = 0; ks0 < p.ksplit; ks0 += KS, parts += KS * BN * kTileRows) {
+        for (uint32_t k0 = 0; k0 < n_parts; k0 += KS) {
             float v[KS][CW];
 #pragma unroll
-            for (uint32_t q = 0; q < KS; q++)
+            for (uint32_t q = 0; q < KS; q++) {
+                const uint32_t k = k0 + q;
+                const float *from = part_block(p, k == 0 ? first : 2 * (cta0 + k), BN) + in_block;
 #pragma unroll
-                for (uint32_t j = 0; j < CW; j++)
-                    v[q][j] = ks0 + q < p.ksplit ? __ldcg(parts + (size_t)q * (BN * kTileRows) + (size_t)j * kTileRows) : 0.f;
+                for (uint32_t j = 0; j < CW; j++) v[q][j] = k < n_parts ? __ldcg(from + (size_t)j * kTileRows) : 0.f;
+            }
 #pragma unroll
             for (uint32_t q = 0; q < KS; q++)
 #pragma unroll
                 for (uint32_t j = 0; j < CW; j++) acc[j] += v[q][j];
         }
-#pragma unroll
-        for (uint32_t c0 = 0; c0 < CW; c0 += 4) {
-            const size_t o0 = (size_t)(n0 + c0) * p.out_stride[wi.seg] + row;
-            const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 < p.n_tokens ? p.n_tokens - (n0 + c0) : 0u;
-            float res[4];
-            if (p.residual) {
-#pragma unroll
-                for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
-            }
-#pragma unroll
-            for (uint32_t j = 0; j < 4; j++)
-                if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? acc[c0 + j] + res[j] : acc[c0 + j];
-        }
-        return;
+        summed = true, truncation = 0.f, scale = 1.f;  // the parts were scaled
     }
+    // Four residuals are asked for before the first of their stores (which may be to the same matrix, so nothing but
+    // this order lets them overlap): one by one they took 24 us per tile, so they take 7.
 #pragma unroll
     for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-        const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;  // padded to whole tiles
-        // Four residuals are asked for before the first of their stores (which may be to the same matrix, so nothing but
-        // this order lets them overlap): one by one they took 24 us per tile, so they take 7.
+        const float osc = summed ? 1.f : lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;
 #pragma unroll
-        for (int j0 = 0; j0 < 16; j0 += 4) {
+        for (uint32_t j0 = 0; j0 < 16; j0 += 4) {
             const size_t o0 = (size_t)(n0 + c0 + j0) * p.out_stride[wi.seg] + row;
             const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 + j0 < p.n_tokens ? p.n_tokens - (n0 + c0 + j0) : 0u;
             float res[4];
@@ -363,7 +367,7 @@ __device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi,
             }
 #pragma unroll
             for (uint32_t j = 0; j < 4; j++) {
-                const float val = fmaf(acc[c0 + j0 + j], p.truncation, acc[c0 + j0 + j]) * __shfl_sync(0xffffffffu, osc, j0 + j) * p.out_scale;
+                const float val = fmaf(acc[c0 + j0 + j], truncation, acc[c0 + j0 + j]) * __shfl_sync(0xffffffffu, osc, j0 + j) * scale;
                 if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? val + res[j] : val;
             }
         }

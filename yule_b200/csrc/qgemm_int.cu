@@ -154,7 +154,6 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-    const uint32_t n_items = p.n_mtiles * p.n_ntiles * p.ksplit;
     const uint32_t bpr = p.n_cols / 256;  // super-blocks per row
 
     if (warp >= kEpiWarps && warp < kFirstProdWarp) {
@@ -164,8 +163,8 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                 yule_pdl_wait();  // the activation tiles come from the kernel before this one
                 RingPos ring;
                 bool ok = true;
-                for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                    const Item wi = decode_item(p, item, bpr);
+                ItemWalk items(p);
+                    for (Item wi; ok && items.next(p, bpr, wi);) {
                     const unsigned char *src = reinterpret_cast<const unsigned char *>(p.xb) + (size_t)wi.nt * bpr * T::kSuperBytes;
                     for (uint32_t kb = 4 * wi.sb0; kb < 4 * wi.sb1; kb++, ring.advance(kStages)) {
                         const uint32_t s = ring.s;
@@ -187,8 +186,8 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             constexpr uint32_t x_lbo = BN * 16;  // bytes of one 8-column step of an activation slab (of its hi or lo rows)
             bool ok = true;
             RingPos ring, acc;
-            for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const Item wi = decode_item(p, item, bpr);
+            ItemWalk items(p);
+                for (Item wi; ok && items.next(p, bpr, wi);) {
                 for (uint32_t kb = 4 * wi.sb0; kb < 4 * wi.sb1 && ok; kb++, ring.advance(kStages)) {
                     const uint32_t s = ring.s;
                     const bool closes = T::OFFSET && (kb & 3u) == 3u;
@@ -269,15 +268,14 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             }
         } else if (warp == kRawWarp) {
             if (lane == 0) {
-                UnitWalk walk;
-                walk.start(p, n_items, bpr);
-                for (uint32_t u = 0; walk.live; u++, walk.next(p, n_items, bpr)) {
+                UnitWalk walk(p, bpr);
+                for (uint32_t u = 0; walk.live; u++, walk.next(p, bpr)) {
                     const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
                     if (!mbar_wait(bar_raw_empty + 8 * slot, ph ^ 1u, abort_flag, p.status)) break;
-                    const uint32_t dst = smem_u32(raw + (size_t)slot * T::kRawBytes), bar = bar_raw_full + 8 * slot, y = walk.mt * kTileRows;
+                    const uint32_t dst = smem_u32(raw + (size_t)slot * T::kRawBytes), bar = bar_raw_full + 8 * slot, y = walk.it.mt * kTileRows;
                     auto box = [&](int map, uint32_t x, uint32_t to) {
                         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(to),
-                                     "l"(reinterpret_cast<uint64_t>(&w_maps.m[walk.seg][map])), "r"(bar), "r"(x), "r"(y)
+                                     "l"(reinterpret_cast<uint64_t>(&w_maps.m[walk.it.seg][map])), "r"(bar), "r"(x), "r"(y)
                                      : "memory");
                     };
                     mbar_arrive_expect_tx(bar, T::kRawBytes);
@@ -439,9 +437,8 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             }
             close();
         };
-        UnitWalk walk;
-        walk.start(p, n_items, bpr);
-        for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, n_items, bpr)) {
+        UnitWalk walk(p, bpr);
+        for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, bpr)) {
             const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
             ok = mbar_wait(bar_raw_full + 8 * slot, ph, abort_flag, p.status);
             ok = __all_sync(0xffffffffu, ok);
@@ -491,8 +488,8 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
         RingPos ring;
         bool ok = true;
         [[maybe_unused]] uint32_t n_stage = 0;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const Item wi = decode_item(p, item, bpr);
+        ItemWalk items(p);
+            for (Item wi; ok && items.next(p, bpr, wi);) {
             const uint32_t row = wi.mt * kTileRows + lane_base + lane;
             const uint8_t *rowp = p.w[wi.seg] + (size_t)(row < p.n_rows[wi.seg] ? row : p.n_rows[wi.seg] - 1) * p.w_row_bytes;
             // the scales of a super-block: Q5_K (d, dmin) at its start, Q6_K d in the last plane of the row
@@ -515,11 +512,12 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
 #pragma unroll
                 for (uint32_t j = 0; j < CW / 2; j++) sums[to][j] = add2(sums[to][j], sums[from][j]);
             };
-            // (a block of the work area that is this item's, or where columns are not split this CTA's)
-            [[maybe_unused]] float *const kept = p.split_part + (size_t)(p.ksplit > 1 ? item : blockIdx.x) * (BN * kTileRows) + (size_t)col_base * kTileRows + lane_base + lane;
+            // (a block of the work area that is this item's, or for a whole tile this CTA's)
+            [[maybe_unused]] auto kept = [&] { return part_block(p, wi.sb1 - wi.sb0 < bpr ? own_part(wi) : 2 * kGemmMaxCtas + blockIdx.x, BN) + (size_t)col_base * kTileRows + lane_base + lane; };
             [[maybe_unused]] auto add_kept = [&] {
+                const float *from = kept();
 #pragma unroll
-                for (uint32_t j = 0; j < CW / 2; j++) sums[0][j] = add2(sums[0][j], pair(__ldcg(kept + (2 * j) * kTileRows), __ldcg(kept + (2 * j + 1) * kTileRows)));
+                for (uint32_t j = 0; j < CW / 2; j++) sums[0][j] = add2(sums[0][j], pair(__ldcg(from + (2 * j) * kTileRows), __ldcg(from + (2 * j + 1) * kTileRows)));
             };
             clear(0);
             uint32_t dd_cur = 0, dd_next = scale_at(wi.sb0);
@@ -571,11 +569,12 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                     if (nth == 0) clear(1);
                 } else if (nth == 0 && sb != wi.sb0) {
                     if (sb != wi.sb0 + kLevel) add_kept();
+                    float *to = kept();
 #pragma unroll
                     for (uint32_t j = 0; j < CW / 2; j++) {
                         const float2 a = unpair(sums[0][j]);
-                        __stcg(kept + (2 * j) * kTileRows, a.x);
-                        __stcg(kept + (2 * j + 1) * kTileRows, a.y);
+                        __stcg(to + (2 * j) * kTileRows, a.x);
+                        __stcg(to + (2 * j + 1) * kTileRows, a.y);
                     }
                     clear(0);
                 }
@@ -614,7 +613,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                 acc[j] = a.x;
                 acc[j + 1] = a.y;
             }
-            finish_item<BN, CW>(p, wi, item, warp, lane, lane_base, col_base, acc);
+            finish_item<BN, CW>(p, wi, bpr, warp, lane, lane_base, col_base, acc);
         }
     }
 

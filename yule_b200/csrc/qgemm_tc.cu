@@ -21,10 +21,9 @@
 // round-to-nearest fp32; the mean of the bias is given back at the end.  Error against 64 bits (2-norm) at
 // 200 rows: Q4_K 2.4e-7 to 2.7e-7; with large and small products in turn, 3.9e-7, in the same time.
 //
-// Work items: (row tile, activation tile) pairs; when these are few (small matrices, tensor-parallel
-// shards, few activation rows) the super-blocks of a row are split into up to 16 parts, one item each,
-// whose scaled partial sums the last drain warp of a (tile, warp) to finish adds up in the order of
-// the parts.
+// Work items: (row tile, activation tile) pairs; those that do not fill a round of CTAs (all of them in small matrices, tensor-parallel
+// shards, with few activation rows) are dealt by super-blocks, in equal runs, and the last drain warp of a (tile, warp) to finish adds up
+// the scaled partial sums in the order of the parts.
 //
 // One CTA per SM, 20 warps, persistent over the work items:
 //   warps 0-7   drain warps: tcgen05.ld of their 32 TMEM lanes × half of the columns after every
@@ -354,7 +353,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-    const uint32_t n_items = p.n_mtiles * p.n_ntiles * p.ksplit;
     const uint32_t bpr = p.n_cols / 256;  // super-blocks per row
 
     if (warp >= kEpiWarps && warp < kFirstProdWarp) {
@@ -364,8 +362,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 yule_pdl_wait();  // the activation tiles come from the kernel before this one
                 RingPos ring;
                 bool ok = true;
-                for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                    const Item wi = decode_item(p, item, bpr);
+                ItemWalk items(p);
+                    for (Item wi; ok && items.next(p, bpr, wi);) {
                     const unsigned char *src = reinterpret_cast<const unsigned char *>(p.xb) + (size_t)wi.nt * bpr * T::kSuperBytes;
                     for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
                         const uint32_t s = ring.s, ph = ring.ph;
@@ -399,8 +397,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             constexpr uint32_t x_lbo = BN * 16;  // bytes of one 8-column step of an activation slab (of its hi or lo rows)
             bool ok = true;
             RingPos ring, acc;
-            for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const Item wi = decode_item(p, item, bpr);
+            ItemWalk items(p);
+                for (Item wi; ok && items.next(p, bpr, wi);) {
                 for (uint32_t kb = T::SPB * wi.sb0; kb < T::SPB * wi.sb1; kb++, ring.advance(kStages)) {
                     const uint32_t s = ring.s;
                     if ((kb & 1u) != mine) {  // (a super-block has an even number of stages)
@@ -479,17 +477,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             }
         } else if (warp == kRawWarp) {
             if (!GENERIC && lane == 0) {
-                UnitWalk walk;
-                walk.start(p, n_items, bpr);
-                for (uint32_t u = 0; walk.live; u++, walk.next(p, n_items, bpr)) {
+                UnitWalk walk(p, bpr);
+                for (uint32_t u = 0; walk.live; u++, walk.next(p, bpr)) {
                     const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
                     if (!mbar_wait(bar_raw_empty + 8 * slot, ph ^ 1u, abort_flag, p.status)) break;
-                    const uint32_t x = walk.sb * 144u, y = walk.mt * kBM;  // byte column (a multiple of 16), first row
+                    const uint32_t x = walk.sb * 144u, y = walk.it.mt * kBM;  // byte column (a multiple of 16), first row
                     mbar_arrive_expect_tx(bar_raw_full + 8 * slot, kRawBytes);
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
                             smem_u32(raw + (size_t)slot * kRawBytes)),
-                        "l"(reinterpret_cast<uint64_t>(&w_maps.m[walk.seg])), "r"(bar_raw_full + 8 * slot), "r"(x), "r"(y)
+                        "l"(reinterpret_cast<uint64_t>(&w_maps.m[walk.it.seg])), "r"(bar_raw_full + 8 * slot), "r"(x), "r"(y)
                         : "memory");
                 }
             }
@@ -509,9 +506,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             const uint32_t ub = p.unit_bytes, rstride = p.raw_stride, c16 = p.raw_chunks;
             const uint32_t slot_bytes = kBM * rstride;
             auto unit_start = [&](const UnitWalk &w, uint32_t tile_row) {  // address of row `tile_row`'s bytes of the unit
-                uint32_t grow = w.mt * kBM + tile_row;
-                grow = grow < p.n_rows[w.seg] ? grow : p.n_rows[w.seg] - 1;
-                return reinterpret_cast<uintptr_t>(p.w[w.seg]) + (size_t)grow * p.w_row_bytes + (size_t)w.sb * ub;
+                uint32_t grow = w.it.mt * kBM + tile_row;
+                grow = grow < p.n_rows[w.it.seg] ? grow : p.n_rows[w.it.seg] - 1;
+                return reinterpret_cast<uintptr_t>(p.w[w.it.seg]) + (size_t)grow * p.w_row_bytes + (size_t)w.sb * ub;
             };
             auto copy_unit = [&](const UnitWalk &w, uint32_t u) {
                 if (w.live) {
@@ -535,18 +532,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
             };
             RingPos ring;
             bool ok = true;
-            UnitWalk cur, ahead;  // the unit being unpacked and the one being copied
-            cur.start(p, n_items, bpr);
-            ahead = cur;
+            UnitWalk cur(p, bpr), ahead = cur;  // the unit being unpacked and the one being copied
             copy_unit(ahead, 0);
             // A warp that has given up goes on through its units, without copying or unpacking: the barriers below count all eight warps and have no
             // bound, so one that left would keep those that passed its last wait just before it ran out.
             for (uint32_t u = 0; cur.live; u++, cur = ahead) {
-                ahead.next(p, n_items, bpr);
+                ahead.next(p, bpr);
                 if (ok) copy_unit(ahead, u + 1);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");   // this thread's copies of unit u have landed
                 asm volatile("bar.sync 2, 256;" ::: "memory");         // and everyone else's
-                const bool live = cur.mt * kBM + r < p.n_rows[cur.seg];
+                const bool live = cur.it.mt * kBM + r < p.n_rows[cur.it.seg];
                 const unsigned char *rawrow = raw + (size_t)(u & 1u) * slot_bytes + (size_t)r * rstride + (unit_start(cur, r) & 15u);
                 for (uint32_t g = 0; g < 4 && ok; g++, ring.advance(kStages)) {
                     ok = mbar_wait(bar_empty + 8 * ring.s, ring.ph ^ 1u, abort_flag, p.status);
@@ -654,9 +649,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                     }
                 }
             };
-            UnitWalk walk;
-            walk.start(p, n_items, bpr);
-            for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, n_items, bpr)) {
+            UnitWalk walk(p, bpr);
+            for (uint32_t u = 0; walk.live && ok; u++, walk.next(p, bpr)) {
                 const uint32_t slot = u % T::kRaw, ph = (u / T::kRaw) & 1u;
                 ok = mbar_wait(bar_raw_full + 8 * slot, ph, abort_flag, p.status);
                 if (!__all_sync(0xffffffffu, ok)) break;
@@ -678,8 +672,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
         const uint32_t lane_base = (warp & 3u) * 32u, col_base = (warp >> 2) * CW;
         RingPos ring;
         bool ok = true;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const Item wi = decode_item(p, item, bpr);
+        ItemWalk items(p);
+            for (Item wi; ok && items.next(p, bpr, wi);) {
             const uint32_t mt = wi.mt, nt = wi.nt;
             const uint32_t row = mt * kBM + lane_base + lane;
             const uint8_t *rowp = p.w[wi.seg] + (size_t)(row < p.n_rows[wi.seg] ? row : p.n_rows[wi.seg] - 1) * bpr * 144;
@@ -700,42 +694,44 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 if (lane == 0) mbar_arrive(bar_acc_empty + 8 * ring.s);
                 ring.advance(NBUF);
             };
-            const uint32_t kb_end = T::SPB * wi.sb1;
-            for (uint32_t kb = T::SPB * wi.sb0; kb < kb_end; kb++) {
-                if (!GENERIC && kb % T::SPB == 0u) {  // new super-block: take its (d, dmin), ask for the next one's
+            for (uint32_t sb = wi.sb0; sb < wi.sb1 && ok; sb++) {
+                if (!GENERIC) {  // new super-block: take its (d, dmin), ask for the next one's
                     dd_cur = dd_next;
-                    if (kb + T::SPB < kb_end) dd_next = __ldg(reinterpret_cast<const uint32_t *>(rowp + (size_t)(kb / T::SPB + 1) * 144));
+                    if (sb + 1 < wi.sb1) dd_next = __ldg(reinterpret_cast<const uint32_t *>(rowp + (size_t)(sb + 1) * 144));
                 }
                 const float2 dd = GENERIC ? make_float2(1.f, 0.f) : __half22float2(as_half2(dd_cur));
                 const uint64_t d2 = pair(dd.x, dd.x);
-                uint32_t at = await();
-                if (!ok) break;
-                // the accumulators go back before the arithmetic on what was read last
-                if constexpr (T::MERGED) {
-                    uint32_t v[CW], vl[CW];
 #pragma unroll
-                    for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-                        tmem_ld16_issue(at + c0, v + c0);
-                        tmem_ld16_issue(at + BN + c0, vl + c0);  // the products with the lo terms
+                for (uint32_t g = 0; g < T::SPB; g++) {
+                    uint32_t at = await();
+                    if (!ok) break;
+                    // the accumulators go back before the arithmetic on what was read last
+                    if constexpr (T::MERGED) {
+                        uint32_t v[CW], vl[CW];
+#pragma unroll
+                        for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
+                            tmem_ld16_issue(at + c0, v + c0);
+                            tmem_ld16_issue(at + BN + c0, vl + c0);  // the products with the lo terms
+                        }
+                        tmem_ld_wait();
+                        release();
+#pragma unroll
+                        for (uint32_t j = 0; j < CW; j += 2) acc2[j / 2] = fma2(d2, add2(pair_bits(v[j], v[j + 1]), pair_bits(vl[j], vl[j + 1])), acc2[j / 2]);
+                    } else {
+                        uint32_t v[32];
+                        tmem_ld32_issue(at, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j += 2) acc2[j / 2] = fma2(d2, pair_bits(v[j], v[j + 1]), acc2[j / 2]);
+                        tmem_ld32_issue(at + 32, v);
+                        tmem_ld_wait();
+                        release();
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j += 2) acc2[16 + j / 2] = fma2(d2, pair_bits(v[j], v[j + 1]), acc2[16 + j / 2]);
                     }
-                    tmem_ld_wait();
-                    release();
-#pragma unroll
-                    for (uint32_t j = 0; j < CW; j += 2) acc2[j / 2] = fma2(d2, add2(pair_bits(v[j], v[j + 1]), pair_bits(vl[j], vl[j + 1])), acc2[j / 2]);
-                } else {
-                    uint32_t v[32];
-                    tmem_ld32_issue(at, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; j += 2) acc2[j / 2] = fma2(d2, pair_bits(v[j], v[j + 1]), acc2[j / 2]);
-                    tmem_ld32_issue(at + 32, v);
-                    tmem_ld_wait();
-                    release();
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; j += 2) acc2[16 + j / 2] = fma2(d2, pair_bits(v[j], v[j + 1]), acc2[16 + j / 2]);
                 }
-                if (!GENERIC && kb % T::SPB == T::SPB - 1) {  // the stage that ends a super-block is followed by the min term
-                    at = await();
+                if (!GENERIC && ok) {  // the stage that ends a super-block is followed by the min term
+                    const uint32_t at = await();
                     if (!ok) break;
                     constexpr uint32_t R = CW < 32 ? CW : 32;
                     const float minus_dmin = -dd.y * (1.0f / kSumScale);
@@ -760,7 +756,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
                 acc[j] = a.x;
                 acc[j + 1] = a.y;
             }
-            finish_item<BN, CW>(p, wi, item, warp, lane, lane_base, col_base, acc);
+            finish_item<BN, CW>(p, wi, bpr, warp, lane, lane_base, col_base, acc);
         }
     }
 
@@ -962,6 +958,30 @@ cudaError_t launch_gemm(const GemmParams &p, const GemmMaps &w_maps, uint32_t gr
     return launch_kernel(kern, dim3(grid), dim3(kGemmThreads), smem, s, pdl, p, w_maps);
 }
 
+// Which tiles are dealt by super-blocks: those that do not fill a round of CTAs, a tile to sixteen CTAs at the most (its parts have to be added up), at least
+// four super-blocks to a CTA.  A part costs its stores, a ticket and its share of the sum, some 3 to 5 us that the tensor pipe waits in part, against
+// super-blocks of 1.8 us at 128 activation rows and 1.1 at 32.  So not where that would shorten the round by fewer than three super-blocks, and runs that
+// end inside a tile, with two parts for most CTAs, only where they shorten it by four more (128 rows) or eight (32 rows: 64 tiles of 32 super-blocks in halves
+// 21 us, in 148 equal runs 23.5; 80 tiles 31 us whole, 25 in equal runs; 448 tiles 119.5 us as four rounds, 104 as three and the rest in parts).
+void split_tiles(GemmParams &p, uint32_t tiles, uint32_t bpr, uint32_t ctas) {
+    p.split_tiles = p.split_ctas = p.split_units = 0;
+    const uint32_t rest = tiles % ctas, units = rest * bpr;
+    if (rest == 0) return;
+    uint32_t most = 16, run = 4;
+    if (const char *k = knob("YULE_GEMM_KSPLIT"))
+        if (atoi(k) > 0) most = (uint32_t)atoi(k), run = 1;
+    auto least = [](uint32_t a, uint32_t b, uint32_t c) { return a < b ? (a < c ? a : c) : (b < c ? b : c); };
+    const uint32_t parts = least(ctas / rest, most, bpr / run), even = parts > 1 ? rest * parts : rest;  // every tile in equal parts
+    const uint32_t equal = least(ctas, rest * most, units / run);                                         // runs that may end inside a tile
+    auto longest = [&](uint32_t to) { return (units + to - 1) / to; };
+    uint32_t to = even;
+    if (equal > even && longest(even) >= longest(equal) + (p.bn >= 128 ? 4u : 8u)) to = equal;
+    if (to <= rest || (run > 1 && bpr < longest(to) + 3)) return;
+    p.split_tiles = rest;
+    p.split_ctas = to;
+    p.split_units = units;
+}
+
 uint32_t pick_bn(uint32_t n_tokens) { return n_tokens <= 32 ? 32 : (n_tokens <= 64 ? 64 : 128); }
 
 }  // namespace
@@ -1118,33 +1138,14 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     for (uint32_t i = p.n_seg; i < (uint32_t)kGemmSegs; i++) p.mt0[i + 1] = p.mt0[p.n_seg];
     p.n_mtiles = p.mt0[p.n_seg];
     p.n_ntiles = n_ntiles;
-    // Few tiles and long rows: the columns of a tile are split over several CTAs (whole super-blocks, at least four
-    // per part), whose partial results the last one to finish adds up in a fixed order.
-    p.ksplit = 1;
-    p.sb_per = g.n_cols / 256;
-    {
-        const uint32_t base = p.n_mtiles * p.n_ntiles, bpr = g.n_cols / 256;
-        uint32_t want = 1;
-        if (base * 2 <= (uint32_t)sm_count && bpr >= 8) {
-            want = (uint32_t)sm_count / base;
-            if (want > bpr / 4) want = bpr / 4;
-            if (want > 16) want = 16;
-        }
-        if (const char *k = knob("YULE_GEMM_KSPLIT")) want = (uint32_t)atoi(k) > 0 ? (uint32_t)atoi(k) : want;
-        if (want > bpr) want = bpr;
-        while (want > 1 && base * want > kGemmSplitMaxItems) want--;
-        if (want > 1) {
-            p.sb_per = (bpr + want - 1) / want;
-            p.ksplit = (bpr + p.sb_per - 1) / p.sb_per;
-        }
-        p.split_tickets = reinterpret_cast<uint32_t *>(g.scratch);
-        p.split_part = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(g.scratch) + kGemmTicketBytes);
-    }
+    const uint32_t ctas = (uint32_t)sm_count < kGemmMaxCtas ? (uint32_t)sm_count : kGemmMaxCtas, tiles = p.n_mtiles * p.n_ntiles;
+    split_tiles(p, tiles, g.n_cols / 256, ctas);
+    p.split_tickets = reinterpret_cast<uint32_t *>(g.scratch);
+    p.split_part = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(g.scratch) + kGemmTicketBytes);
     p.status = g.status;
     p.truncation = kTruncation;
     p.out_scale = 1.0f;
-    uint32_t grid = p.n_mtiles * p.n_ntiles * p.ksplit;
-    if (grid > (uint32_t)sm_count) grid = (uint32_t)sm_count;
+    const uint32_t grid = tiles > p.split_tiles ? (tiles < ctas ? tiles : ctas) : p.split_ctas;
     p.w_row_bytes = (uint64_t)(g.n_cols / block_size(g.type)) * block_bytes(g.type);
     const bool forced = knob("YULE_GEMM_GENERIC") && atoi(knob("YULE_GEMM_GENERIC"));
     if (!forced && qgemm_int_supported(g)) {
