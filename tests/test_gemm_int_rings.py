@@ -20,13 +20,14 @@ def accumulators(bn, w_cols):
     return min(8, (512 - STAGES * w_cols) // (2 * bn if bn <= 64 else bn))
 
 
-CASES = [(bn, name, accumulators(bn, 64 if name == "q6" else 32)) for bn in (32, 64, 128) for name in ("block32", "q5", "q6")]
+CASES = [(bn, name, accumulators(bn, 64 if name == "q6" else 32)) for bn in (32, 64, 128) for name in ("block32", "q5", "q6")] + [(128, "q4k", accumulators(128, 32))]
 
 
 def simulate(seed, nbuf, name, blocks, scale_ring=SCALES):
     rng = random.Random(seed)
     n, per = 4 * blocks, 2 if name == "block32" else 1
-    closes = lambda i: name == "q5" and i % 4 == 3  # noqa: E731
+    closes = lambda i: name in ("q5", "q4k") and i % 4 == 3  # noqa: E731
+    span = 2 if name == "q4k" else 1  # stages that share an accumulator
     full, empty = [[Barrier(c) for _ in range(STAGES)] for c in (WARPS + 1, 1)]
     acc_full, acc_empty = [[Barrier(c) for _ in range(nbuf)] for c in (2 if name == "block32" else 1, WARPS)]
     w = [[-1] * (WARPS + 1) for _ in range(STAGES)]
@@ -44,37 +45,40 @@ def simulate(seed, nbuf, name, blocks, scale_ring=SCALES):
                 scales[i % scale_ring][p] = i
             full[s].arrive()
 
-    def mma(s, i, slot, a, last):
+    def mma(stages, slot, a, first, frees):
         def go():
-            assert all(t == i for t in w[s]), "MMA on operands of another stage"
-            assert readers[slot] == WARPS, "accumulator overwritten before it was drained"
+            assert all(t == i for i in stages for t in w[i % STAGES]), "MMA on operands of another stage"
+            assert readers[slot] == WARPS or (not first and acc[slot] == a), "accumulator overwritten before it was drained"
             acc[slot], readers[slot] = a, 0
-            if last:
-                ran.add(i)
+            ran.update(frees)
         return go
 
     def issuer(mine):
         a = 0
-        for i in range(n):
-            s, uses = i % STAGES, per + closes(i)
-            if i & 1 == mine:
+        for i in range(0, n, span):
+            stages = range(i, i + span)
+            uses = per + closes(stages[-1])
+            if i // span & 1 == mine:
                 for k in range(uses):
                     slot, ph = (a + k) % nbuf, (a + k) // nbuf & 1
                     yield lambda: acc_empty[slot].over(ph ^ 1)
                     if k == 0:
-                        yield lambda: full[s].over(i // STAGES & 1)
+                        for j, t in enumerate(stages):
+                            yield lambda: full[t % STAGES].over(t // STAGES & 1)
+                            if j + 1 < span:  # the small products of the first stage go out before the second is there
+                                queues[mine].append(mma([t], slot, a, True, []))
                     last = k == uses - 1
-                    queues[mine] += [mma(s, i, slot, a + k, last), acc_full[slot].arrive]
-                    if last:
-                        queues[mine].append(empty[s].arrive)
+                    frees = (list(stages) if last else list(stages)[:-1]) if k == 0 else [stages[-1]] if last else []
+                    queues[mine] += [mma(list(stages) if k == 0 or span == 1 else [stages[-1]], slot, a + k, k > 0 or span == 1, frees)]
+                    queues[mine] += [empty[t % STAGES].arrive for t in frees] + [acc_full[slot].arrive]
                     if name == "block32":
                         acc_full[slot].arrive()
             a += uses
 
     def drain():
         a = 0
-        for i in range(n):
-            for k in range(per + closes(i)):
+        for i in range(0, n, span):
+            for k in range(per + closes(i + span - 1)):
                 slot = a % nbuf
                 yield lambda: acc_full[slot].over(a // nbuf & 1)
                 assert acc[slot] == a, "drained another step's sums"
@@ -107,7 +111,7 @@ def test_rings_hold(bn, name, nbuf):
 
 
 def test_the_model_catches_rings_that_are_too_short():
-    for nbuf, name, ring in ((2, "block32", SCALES), (2, "q5", SCALES), (3, "block32", 4)):
+    for nbuf, name, ring in ((2, "block32", SCALES), (2, "q5", SCALES), (2, "q4k", SCALES), (3, "block32", 4)):
         with pytest.raises(AssertionError):
             for seed in range(400):
                 simulate(seed, nbuf, name, 6, ring)

@@ -1,25 +1,29 @@
-// Quantised GEMM on tcgen05 for Q8_0, Q4_0, Q5_K and Q6_K (on its row-planar copy), eight or more activation rows:
+// Quantised GEMM on tcgen05 for Q8_0, Q4_0, Q5_K and Q6_K (on its row-planar copy), eight or more activation rows, and for Q4_K from 65 on:
 //
 //     out[n][r] = Σ_k W[r][k] · x[n][k]
 //
-// The sibling of the Q4_K kernel (qgemm_tc.cu): the same roles, activation tiles, work items and two MMAs per product, W·x_hi and W·x_lo, because
+// The sibling of the kernel in qgemm_tc.cu: the same roles, activation tiles, work items and two MMAs per product, W·x_hi and W·x_lo, because
 // the W operand is an exact integer in fp16 and its scale is multiplied in after the drain, in fp32.  What differs is where the scale changes:
 //
 //   Q8_0, Q4_0  one d per 32 columns: q (-128 .. 127; q − 8) is the operand, and a stage of 64 columns fills two accumulators, one per block.  The d
 //               of a (row, block) goes from the unpacking warps to the drain warps through shared memory.
-//   Q5_K        sc·(q − 16) (|.| ≤ 1008), drained with d.  What the centring and the minimum leave, c = 16·d·sc − dmin·m per 32 columns, meets the
-//               sub-block sums of x in one more accumulator per super-block: c is formed in fp32, scaled by a power of two that d and dmin
-//               give (both sides compute it) and split into fp16 hi + lo.  (Summing q and the minimum apart, as the Q4_K kernel does, doubles the error.)
+//   Q4_K, Q5_K  sc·(q − 8), sc·(q − 16) (|.| ≤ 1008), drained with d.  What the centring and the minimum leave, c = 8·d·sc − dmin·m (16) per 32 columns,
+//               meets the sub-block sums of x in one more accumulator per super-block: c is formed in fp32, scaled by a power of two that d and dmin
+//               give (both sides compute it) and split into fp16 hi + lo.  (Summing q and the minimum apart, as qgemm_tc.cu does, doubles the error.)
 //   Q6_K        sc·(q − 32) has up to 13 bits: hi (rounded to 11) and lo (the rest, exact), three MMAs per 16 columns, drained with d.
 //
-// The weights arrive as tiled TMA boxes of one super-block (256 columns) of 128 rows: Q8_0 272 bytes a row, Q4_0 144, Q5_K 176 (odd multiples of 16: eight
+// An accumulator of Q4_K holds two stages, which halves the drains: gate / up of the 8B shape against 2047 rows 894 us in qgemm_tc.cu, 831 here (1160 TFLOP/s of MMAs; cuBLAS
+// sustains 1397), error against 64 bits 2.8e-7 and 1.3e-7.  The others hold one: two would take 7 to 12 % less time, but the adder truncates, and at 2048
+// columns the error would be 1.3e-7 where the kernel that these formats had before gave 1.25e-7.
+//
+// The weights arrive as tiled TMA boxes of one super-block (256 columns) of 128 rows: Q8_0 272 bytes a row, Q4_K and Q4_0 144, Q5_K 176 (odd multiples of 16: eight
 // lanes cover all banks), Q6_K its ql, qh and scale planes, the first two swizzled for the same reason.  Rows past the end of the matrix arrive as zeros.
 //
-// Before, these formats went through the dequantising kernel of qgemm_tc.cu: three MMAs per product, W as fp16 hi + lo of the dequantised value, raw bytes
-// fetched by the unpacking warps themselves between two barriers of theirs.  The linears of an 8B layer against 1000 rows, ms, before and now: Q8_0 2.35, 1.21, Q4_0 2.16,
-// 1.19, Q5_K 3.51, 1.01, Q6_K 2.66, 1.04 (of the tensor pipe at its measured rate 35, 36, 42 and, with three MMAs, 61 %); Q6_K 2048x5632 by 777 rows 162, 68 us.
+// Before, the formats other than Q4_K went through the dequantising kernel of qgemm_tc.cu: three MMAs per product, W as fp16 hi + lo of the dequantised value, raw bytes
+// fetched by the unpacking warps themselves between two barriers of theirs.  The linears of an 8B layer against 1000 rows, ms, before and now: Q8_0 2.35, 1.20, Q4_0 2.16,
+// 1.17, Q5_K 3.51, 1.02, Q6_K 2.66, 1.03 (of the tensor pipe at its measured rate 35, 36, 41 and, with three MMAs, 61 %); Q6_K 2048x5632 by 777 rows 162, 64 us.
 //
-// 20 warps: 0-7 drain, 8 loads x, 9 and 11 issue MMAs (even and odd stages), 10 loads W, 12-19 unpack; barriers, rings and the reasons as in qgemm_tc.cu.
+// 20 warps: 0-7 drain, 8 loads x, 9 and 11 issue MMAs in turns, 10 loads W, 12-19 unpack; barriers, rings and the reasons as in qgemm_tc.cu.
 // Every wait is bounded.
 
 #include <cstring>
@@ -34,7 +38,7 @@
 namespace yule {
 namespace {
 
-enum Fmt { kQ8, kQ4, kQ5K, kQ6K };
+enum Fmt { kQ8, kQ4, kQ5K, kQ6K, kQ4K };
 
 constexpr int kProdWarps = 8;
 constexpr int kLoaderWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kRawWarp = kEpiWarps + 2, kMmaWarp2 = kEpiWarps + 3, kFirstProdWarp = kEpiWarps + 4;
@@ -59,7 +63,7 @@ struct IntMaps {
 template <int FMT, int BN>
 struct Tile {
     static constexpr bool MERGED = BN <= 64;  // hi and lo rows of x as one operand of 2·BN rows, as in the Q4_K kernel
-    static constexpr bool BLOCK32 = FMT == kQ8 || FMT == kQ4, OFFSET = FMT == kQ5K, WLO = FMT == kQ6K;
+    static constexpr bool BLOCK32 = FMT == kQ8 || FMT == kQ4, OFFSET = FMT == kQ5K || FMT == kQ4K, WLO = FMT == kQ6K;
     static constexpr uint32_t kMainCols = MERGED ? 2 * BN : BN;
     static constexpr uint32_t CW = BN / 2;                 // columns per drain warp
     static constexpr uint32_t kXHalfBytes = BN * 64 * 2;   // one fp16 term of the activation slab
@@ -75,14 +79,17 @@ struct Tile {
     static_assert(NBUF >= kAccs + (OFFSET ? 2 : 1) && (!BLOCK32 || 7 + NBUF <= 2 * kScaleRing - 1), "accumulator ring");
     static constexpr uint32_t kABase = NBUF * kMainCols;
     static_assert(kABase + kStages * kACols <= 512, "tensor memory");
-    static constexpr uint32_t kOffsetBytes = OFFSET ? kTileRows * 32 * 2 : 0;  // Q5_K: c_hi | c_hi | c_lo | c_lo, eight columns each
-    static constexpr uint32_t kOffSums = kOffsetBytes + 2 * kXHalfBytes;
-    static constexpr uint32_t kStageBytes = kOffSums + (OFFSET ? kBmBytes : 0u);
-    static constexpr uint32_t kRawRow = FMT == kQ8 ? 272 : FMT == kQ4 ? 144 : 176;
+    static constexpr uint32_t kSpan = FMT == kQ4K ? 2 : 1;  // stages that an accumulator holds (with kSpan = 1 and BLOCK32: half of one)
+    static constexpr uint32_t kStageBytes = 2 * kXHalfBytes;
+    // Behind the last slot, which is where every super-block's last stage lies: the sub-block sums of x (one bulk copy brings them with that stage)
+    // and the offset's operand, c_hi | c_hi | c_lo | c_lo, eight columns each.
+    static constexpr uint32_t kOffSums = kStages * kStageBytes, kOffOffset = kOffSums + (OFFSET ? kBmBytes : 0u);
+    static constexpr uint32_t kOffRaw = kOffOffset + (OFFSET ? kTileRows * 32 * 2 : 0u);
+    static constexpr uint32_t kRawRow = FMT == kQ8 ? 272 : FMT == kQ5K ? 176 : 144;
     static constexpr uint32_t kRawBytes = FMT == kQ6K ? kTileRows * 208 : kTileRows * kRawRow;
     static constexpr uint32_t kScaleBytes = BLOCK32 ? kScaleRing * 2 * kTileRows * 4 : 0;
     static constexpr uint32_t kTailBytes = (2 * kStages + 2 * kMaxAcc + 2 * kMaxRaw) * 8 + 32;
-    static constexpr uint32_t kFixed = 1024 + kStages * kStageBytes + kScaleBytes + kTailBytes;  // (1024: the swizzled planes start on such boundaries)
+    static constexpr uint32_t kFixed = 1024 + kOffRaw + kScaleBytes + kTailBytes;  // (1024: the swizzled planes start on such boundaries)
     static constexpr uint32_t kRawFit = (kMaxSmem - kFixed) / kRawBytes;
     static constexpr uint32_t kRaw = kRawFit < 6 ? kRawFit : 6;  // super-blocks of raw bytes in flight
     static_assert(kRaw >= 2, "shared memory");
@@ -117,8 +124,8 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
     yule_pdl_launch_dependents();
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     unsigned char *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);  // stages | raw boxes | scales | barriers
-    unsigned char *raw = smem + (size_t)kStages * kStageBytes;
-    static_assert((kStages * kStageBytes) % 1024 == 0 && (FMT != kQ6K || T::kRawBytes % 1024 == 0), "swizzle");
+    unsigned char *raw = smem + T::kOffRaw;
+    static_assert(T::kOffRaw % 1024 == 0 && (FMT != kQ6K || T::kRawBytes % 1024 == 0), "swizzle");
     float *scales = reinterpret_cast<float *>(raw + T::kRaw * T::kRawBytes);  // BLOCK32: [kScaleRing][2][128]
     uint64_t *bars = reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(scales) + T::kScaleBytes);
     const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kStages;
@@ -173,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                         const uint32_t g = kb & 3u, bytes = 2 * kXHalfBytes + ((T::OFFSET && g == 3) ? T::kBmBytes : 0u);  // the sums ride with the last stage
                         mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                         smem_u32(smem + (size_t)s * kStageBytes + T::kOffsetBytes)),
+                                         smem_u32(smem + (size_t)s * kStageBytes)),
                                      "l"(src + (size_t)(kb >> 2) * T::kSuperBytes + (size_t)g * 2 * kXHalfBytes), "r"(bytes), "r"(bar_full + 8 * s)
                                      : "memory");
                     }
@@ -188,78 +195,113 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             RingPos ring, acc;
             ItemWalk items(p);
                 for (Item wi; ok && items.next(p, bpr, wi);) {
-                for (uint32_t kb = 4 * wi.sb0; kb < 4 * wi.sb1 && ok; kb++, ring.advance(kStages)) {
-                    const uint32_t s = ring.s;
-                    const bool closes = T::OFFSET && (kb & 3u) == 3u;
-                    if ((kb & 1u) != mine) {
+                for (uint32_t kb = 4 * wi.sb0; kb < 4 * wi.sb1 && ok; kb += T::kSpan, ring.advance(kStages)) {
+                    const bool closes = T::OFFSET && (kb & 3u) == 4u - T::kSpan;
+                    if ((kb / T::kSpan & 1u) != mine) {
 #pragma unroll
                         for (uint32_t i = 0; i < T::kAccs; i++) acc.advance(NBUF);
                         if (closes) acc.advance(NBUF);
+                        if (T::kSpan == 2) ring.advance(kStages);
                         continue;
                     }
-                    const uint32_t stage = smem_u32(smem + (size_t)s * kStageBytes);
-                    const uint32_t x_hi = stage + T::kOffsetBytes, w0 = tmem_base + T::kABase + s * T::kACols;
-                    const uint64_t db0 = smem_desc(x_hi, T::MERGED ? 2 * x_lbo : x_lbo, 128);
-                    // An accumulator of the stage: its 16-column steps [K0, K1).  The adder truncates, which costs a part of what the accumulator
-                    // holds, so the products with lo terms go first, or to columns of their own.
-                    auto fill = [&](auto k0c, auto k1c, bool last) {
-                        constexpr uint32_t K0 = decltype(k0c)::value, K1 = decltype(k1c)::value;
-                        ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status) &&
-                             (K0 != 0 || mbar_wait(bar_full + 8 * s, ring.ph, abort_flag, p.status));
+                    auto await = [&](uint32_t bar, uint32_t parity) { ok = ok && mbar_wait(bar, parity, abort_flag, p.status); };
+                    auto all_ok = [&] {
                         ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) return;
                         tc_fence_after();
-                        const uint32_t d_main = tmem_base + acc.s * T::kMainCols;
-                        if (elect_one()) {
+                        return ok;
+                    };
+                    // The 16-column steps [K0, K1) of ring slot s.  The adder truncates, which costs a part of what the accumulator holds, so the
+                    // products with lo terms go first (`small`), or to columns of their own.
+                    auto w_at = [&](uint32_t s) { return tmem_base + T::kABase + s * T::kACols; };
+                    auto x_at = [&](uint32_t s) { return smem_desc(smem_u32(smem + (size_t)s * kStageBytes), T::MERGED ? 2 * x_lbo : x_lbo, 128); };
+                    auto small = [&](auto k0c, auto k1c, auto freshc, uint32_t d_main, uint32_t s) {
+                        constexpr uint32_t K0 = decltype(k0c)::value, K1 = decltype(k1c)::value;
+                        const uint32_t w0 = w_at(s);
+                        const uint64_t db0 = x_at(s);
+                        mma_steps<K0, K1>([&](auto kc) {
+                            constexpr uint32_t k = decltype(kc)::value;
+                            constexpr int add = k != K0 || !decltype(freshc)::value;
                             if constexpr (T::MERGED) {
-                                mma_steps<K0, K1>([&](auto kc) {
-                                    constexpr uint32_t k = decltype(kc)::value;
-                                    const uint64_t db = db0 + (uint64_t)((k * 4u * x_lbo) >> 4);
-                                    umma_f16_ts<(k != K0)>(d_main, w0 + 8 * k, db, idesc2);
-                                    if (T::WLO) umma_f16_ts<1>(d_main + BN, w0 + 32 + 8 * k, db, idesc);  // W_lo·x_hi beside the other small products
-                                });
+                                const uint64_t db = db0 + (uint64_t)((k * 4u * x_lbo) >> 4);
+                                umma_f16_ts<add>(d_main, w0 + 8 * k, db, idesc2);
+                                if (T::WLO) umma_f16_ts<1>(d_main + BN, w0 + 32 + 8 * k, db, idesc);  // W_lo·x_hi beside the other small products
                             } else {
-                                mma_steps<K0, K1>([&](auto kc) {
-                                    constexpr uint32_t k = decltype(kc)::value;
-                                    const uint64_t db = db0 + (uint64_t)((k * 2u * x_lbo) >> 4);
-                                    umma_f16_ts<(k != K0)>(d_main, w0 + 8 * k, db + (uint64_t)(kXHalfBytes >> 4), idesc);
-                                    if (T::WLO) umma_f16_ts<1>(d_main, w0 + 32 + 8 * k, db, idesc);
-                                });
-                                mma_steps<K0, K1>([&](auto kc) {
-                                    constexpr uint32_t k = decltype(kc)::value;
-                                    umma_f16_ts<1>(d_main, w0 + 8 * k, db0 + (uint64_t)((k * 2u * x_lbo) >> 4), idesc);
-                                });
+                                const uint64_t db = db0 + (uint64_t)((k * 2u * x_lbo) >> 4);
+                                umma_f16_ts<add>(d_main, w0 + 8 * k, db + (uint64_t)(kXHalfBytes >> 4), idesc);
+                                if (T::WLO) umma_f16_ts<1>(d_main, w0 + 32 + 8 * k, db, idesc);
                             }
-                            umma_commit(bar_acc_full + 8 * acc.s);
-                            if (last) umma_commit(bar_empty + 8 * s);
-                            if (T::BLOCK32) mbar_arrive(bar_acc_full + 8 * acc.s);
+                        });
+                    };
+                    auto large = [&](auto k0c, auto k1c, uint32_t d_main, uint32_t s) {
+                        if constexpr (!T::MERGED) {
+                            const uint32_t w0 = w_at(s);
+                            const uint64_t db0 = x_at(s);
+                            mma_steps<decltype(k0c)::value, decltype(k1c)::value>([&](auto kc) {
+                                constexpr uint32_t k = decltype(kc)::value;
+                                umma_f16_ts<1>(d_main, w0 + 8 * k, db0 + (uint64_t)((k * 2u * x_lbo) >> 4), idesc);
+                            });
                         }
-                        __syncwarp();
-                        acc.advance(NBUF);
                     };
                     constexpr std::integral_constant<uint32_t, 0> k0{};
                     constexpr std::integral_constant<uint32_t, 2> k2{};
                     constexpr std::integral_constant<uint32_t, 4> k4{};
-                    if constexpr (T::BLOCK32) {
-                        fill(k0, k2, false);
-                        if (!ok) break;
-                        fill(k2, k4, true);
-                    } else {
-                        fill(k0, k4, !closes);
-                    }
-                    if (!ok) break;
-                    if (closes) {  // Σ_s c_s · (sum of x over sub-block s): the lo terms of c, then the hi terms, against hi and lo sums side by side
-                        ok = mbar_wait(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u, abort_flag, p.status);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) break;
-                        tc_fence_after();
+                    constexpr std::true_type fresh{};
+                    if constexpr (T::kSpan == 2) {
+                        const uint32_t d_main = tmem_base + acc.s * T::kMainCols, s0 = ring.s;
+                        await(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u);
+                        await(bar_full + 8 * s0, ring.ph);
+                        if (!all_ok()) break;
+                        if (elect_one()) small(k0, k4, fresh, d_main, s0);
+                        __syncwarp();
+                        ring.advance(kStages);
+                        await(bar_full + 8 * ring.s, ring.ph);
+                        if (!all_ok()) break;
                         if (elect_one()) {
-                            const uint32_t d_main = tmem_base + acc.s * T::kMainCols;
-                            const uint64_t sums = smem_desc(stage + T::kOffSums, x_lbo, 128);
-                            umma_f16(d_main, smem_desc(stage + 4096, 2048, 128), sums, idesc, 0u);
-                            umma_f16(d_main, smem_desc(stage, 2048, 128), sums, idesc, 1u);
+                            small(k0, k4, std::false_type{}, d_main, ring.s);
+                            large(k0, k4, d_main, s0);
+                            umma_commit(bar_empty + 8 * s0);
+                            large(k0, k4, d_main, ring.s);
                             umma_commit(bar_acc_full + 8 * acc.s);
-                            umma_commit(bar_empty + 8 * s);
+                            if (!closes) umma_commit(bar_empty + 8 * ring.s);
+                        }
+                        __syncwarp();
+                        acc.advance(NBUF);
+                    } else {
+                        const uint32_t s = ring.s;
+                        auto fill = [&](auto k0c, auto k1c, bool last) {
+                            await(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u);
+                            if (decltype(k0c)::value == 0) await(bar_full + 8 * s, ring.ph);
+                            if (!all_ok()) return;
+                            if (elect_one()) {
+                                const uint32_t d_main = tmem_base + acc.s * T::kMainCols;
+                                small(k0c, k1c, fresh, d_main, s);
+                                large(k0c, k1c, d_main, s);
+                                umma_commit(bar_acc_full + 8 * acc.s);
+                                if (last) umma_commit(bar_empty + 8 * s);
+                                if (T::BLOCK32) mbar_arrive(bar_acc_full + 8 * acc.s);
+                            }
+                            __syncwarp();
+                            acc.advance(NBUF);
+                        };
+                        if constexpr (T::BLOCK32) {
+                            fill(k0, k2, false);
+                            if (!ok) break;
+                            fill(k2, k4, true);
+                        } else {
+                            fill(k0, k4, !closes);
+                        }
+                        if (!ok) break;
+                    }
+                    if (closes) {  // Σ_s c_s · (sum of x over sub-block s): the lo terms of c, then the hi terms, against hi and lo sums side by side
+                        await(bar_acc_empty + 8 * acc.s, acc.ph ^ 1u);
+                        if (!all_ok()) break;
+                        if (elect_one()) {
+                            const uint32_t d_off = tmem_base + acc.s * T::kMainCols, c_at = smem_u32(smem + T::kOffOffset);
+                            const uint64_t sums = smem_desc(smem_u32(smem + T::kOffSums), x_lbo, 128);
+                            umma_f16(d_off, smem_desc(c_at + 4096, 2048, 128), sums, idesc, 0u);
+                            umma_f16(d_off, smem_desc(c_at, 2048, 128), sums, idesc, 1u);
+                            umma_commit(bar_acc_full + 8 * acc.s);
+                            umma_commit(bar_empty + 8 * ring.s);
                         }
                         __syncwarp();
                         acc.advance(NBUF);
@@ -348,22 +390,23 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             }
             close();
         };
-        // Q5_K: sixteen bytes of the quants of a 64-column group give sixteen columns of its first and of its second sub-block
-        [[maybe_unused]] auto group_q5 = [&](auto gc, const unsigned char *row, const uint4 &hdr, const ScalesMins &sm, const uint4 &qh) {
+        // Q4_K, Q5_K: sixteen bytes of the quants of a 64-column group give sixteen columns of its first and of its second sub-block
+        [[maybe_unused]] auto group_q45 = [&](auto gc, const unsigned char *row, const uint4 &hdr, const ScalesMins &sm, const uint4 &qh) {
             constexpr uint32_t g = decltype(gc)::value, j0 = (2 * g) & 3u;
+            constexpr float middle = FMT == kQ5K ? 16.f : 8.f;
             const uint32_t scw = g < 2 ? sm.sc_lo : sm.sc_hi;
             const __half2 sc0 = __hsub2(as_half2(biased_pair(scw, 0x4040u + j0 * 0x0101u)), k1024);
             const __half2 sc1 = __hsub2(as_half2(biased_pair(scw, 0x4040u + (j0 + 1) * 0x0101u)), k1024);
-            // (1024 + 16·q)·(sc / 16) − 80·sc = (q − 16)·sc, exact: 80·sc ≤ 5040 = 16·315
-            const __half2 k16th = __float2half2_rn(0.0625f), kneg80 = __float2half2_rn(-80.f);
-            const __half2 a0 = __hmul2(sc0, k16th), b0 = __hmul2(sc0, kneg80), a1 = __hmul2(sc1, k16th), b1 = __hmul2(sc1, kneg80);
-            const uint4 ql = *reinterpret_cast<const uint4 *>(row + 48 + 32 * g + 16 * hf);
+            // (1024 + 16·q)·(sc / 16) − (64 + middle)·sc = (q − middle)·sc, exact: 80·sc ≤ 5040 = 16·315, 72·sc ≤ 4536 = 8·567
+            const __half2 k16th = __float2half2_rn(0.0625f), kbias = __float2half2_rn(-64.f - middle);
+            const __half2 a0 = __hmul2(sc0, k16th), b0 = __hmul2(sc0, kbias), a1 = __hmul2(sc1, k16th), b1 = __hmul2(sc1, kbias);
+            const uint4 ql = *reinterpret_cast<const uint4 *>(row + (FMT == kQ5K ? 48 : 16) + 32 * g + 16 * hf);
             if (!open()) return;
             const uint32_t q[4] = {ql.x, ql.y, ql.z, ql.w}, h[4] = {qh.x, qh.y, qh.z, qh.w};
             const uint32_t to = w_lanes + ring.s * T::kACols + hf * 8;
             // bytes (0, 2) and (1, 3) of a word: nibble to bits 4-7, fifth bit (bit J of its byte) to bit 8 of each half
             auto five = [&](uint32_t nib, uint32_t bit, const __half2 &a, const __half2 &b) {
-                return as_u32(__hfma2(as_half2((nib & 0x00F000F0u) | (bit & 0x01000100u) | 0x64006400u), a, b));
+                return as_u32(__hfma2(as_half2((nib & 0x00F000F0u) | (FMT == kQ5K ? bit & 0x01000100u : 0u) | 0x64006400u), a, b));
             };
             uint4 lo[2], hi[2];
 #pragma unroll
@@ -378,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             if constexpr (g == 3) {
                 const float2 dd = __half22float2(as_half2(hdr.x));
                 const float scale = offset_scale(offset_exponent(dd.x, dd.y));
-                const float ds = 16.f * dd.x;
+                const float ds = middle * dd.x;
                 uint32_t c[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
@@ -397,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                         c[k] = as_u32(__floats2half2_rn(v[0] - back.x, v[1] - back.y));
                     }
                 }
-                unsigned char *slab = smem + (size_t)ring.s * kStageBytes + hf * 4096 + (r >> 3) * 128 + (r & 7u) * 16;
+                unsigned char *slab = smem + T::kOffOffset + hf * 4096 + (r >> 3) * 128 + (r & 7u) * 16;
                 *reinterpret_cast<uint4 *>(slab) = make_uint4(c[0], c[1], c[2], c[3]);
                 *reinterpret_cast<uint4 *>(slab + 2048) = make_uint4(c[0], c[1], c[2], c[3]);
                 fence_async_smem();  // generic-proxy stores → visible to the tensor core's reads
@@ -453,12 +496,12 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                 };
                 if (hf == 0) all(std::integral_constant<uint32_t, 0>{});
                 else all(std::integral_constant<uint32_t, 1>{});
-            } else if constexpr (FMT == kQ5K) {
+            } else if constexpr (T::OFFSET) {
                 const unsigned char *row = box + r * T::kRawRow;
-                const uint4 hdr = *reinterpret_cast<const uint4 *>(row), qh = *reinterpret_cast<const uint4 *>(row + 16 + 16 * hf);
+                const uint4 hdr = *reinterpret_cast<const uint4 *>(row), qh = FMT == kQ5K ? *reinterpret_cast<const uint4 *>(row + 16 + 16 * hf) : hdr;
                 const ScalesMins sm = q4k_scales_mins(hdr.y, hdr.z, hdr.w);
                 mma_steps<0, 4>([&](auto gc) {
-                    if (ok) group_q5(gc, row, hdr, sm, qh);
+                    if (ok) group_q45(gc, row, hdr, sm, qh);
                 });
             } else {
                 // ql: chunk c of row r lies at c ^ (r mod 8), qh: at c ^ (r / 2 mod 4); the scales of a row are sixteen bytes
@@ -492,9 +535,9 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
             for (Item wi; ok && items.next(p, bpr, wi);) {
             const uint32_t row = wi.mt * kTileRows + lane_base + lane;
             const uint8_t *rowp = p.w[wi.seg] + (size_t)(row < p.n_rows[wi.seg] ? row : p.n_rows[wi.seg] - 1) * p.w_row_bytes;
-            // the scales of a super-block: Q5_K (d, dmin) at its start, Q6_K d in the last plane of the row
+            // the scales of a super-block: Q4_K, Q5_K (d, dmin) at its start, Q6_K d in the last plane of the row
             auto scale_at = [&](uint32_t sb) -> uint32_t {
-                if constexpr (FMT == kQ5K) return __ldg(reinterpret_cast<const uint32_t *>(rowp + (size_t)sb * 176));
+                if constexpr (T::OFFSET) return __ldg(reinterpret_cast<const uint32_t *>(rowp + (size_t)sb * T::kRawRow));
                 else if constexpr (FMT == kQ6K) return __ldg(reinterpret_cast<const unsigned short *>(rowp + (size_t)bpr * 208) + sb);
                 else return 0;
             };
@@ -596,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemm_int_kernel(const __grid_con
                     if (sb + 1 < wi.sb1) dd_next = scale_at(sb + 1);
                     const float2 dd = __half22float2(as_half2(dd_cur));
 #pragma unroll 1
-                    for (uint32_t g = 0; g < 4 && ok; g++) drain(sides, chunk, [&] { return dd.x; }, into);
+                    for (uint32_t g = 0; g < 4 / T::kSpan && ok; g++) drain(sides, chunk, [&] { return dd.x; }, into);
                     if (T::OFFSET && ok) drain(std::false_type{}, chunk, [&] { return offset_unscale(offset_exponent(dd.x, dd.y)) * (1.0f / kSumScale); }, into);
                 }
                 if constexpr (T::MERGED) {
@@ -662,7 +705,8 @@ cudaError_t launch_bn(const GemmParams &p, const IntMaps &maps, uint32_t grid, b
 
 }  // namespace
 
-// Every matrix of the launch: Q8_0, Q4_0 and Q5_K rows on 16-byte boundaries (their super-blocks are multiples of 16 bytes), Q6_K with its planar copy.
+// Every matrix of the launch: Q8_0, Q4_0, Q5_K and Q4_K rows on 16-byte boundaries (their super-blocks are multiples of 16 bytes), Q6_K with its planar copy.  Up to
+// 64 activation rows Q4_K stays in qgemm_tc.cu, whose stages of two column groups at 32 rows have fewer hand-offs (8192x28672 by 32 rows 71 us).
 bool qgemm_int_supported(const QGemm &g) {
     if (g.type == YULE_DTYPE_Q6_K) {
         if (!g.planar) return false;
@@ -670,7 +714,7 @@ bool qgemm_int_supported(const QGemm &g) {
             if (!g.planar_more[i]) return false;
         return true;
     }
-    if (g.type != YULE_DTYPE_Q8_0 && g.type != YULE_DTYPE_Q4_0 && g.type != YULE_DTYPE_Q5_K) return false;
+    if (g.type != YULE_DTYPE_Q8_0 && g.type != YULE_DTYPE_Q4_0 && g.type != YULE_DTYPE_Q5_K && (g.type != YULE_DTYPE_Q4_K || g.n_tokens <= 64)) return false;
     uintptr_t all = reinterpret_cast<uintptr_t>(g.w);
     for (uint32_t i = 0; i < g.n_more; i++) all |= reinterpret_cast<uintptr_t>(g.w_more[i]);
     return (all & 15) == 0;
@@ -691,7 +735,7 @@ cudaError_t launch_qgemm_int(const QGemm &g, const void *params, uint32_t grid, 
             if (e == cudaSuccess) e = cached_tensor_map_2d(w + (size_t)bpr * 128, 1, (uint64_t)bpr * 64, p.n_rows[i], p.w_row_bytes, 64, kTileRows, &maps.m[i][1], 64);
             if (e == cudaSuccess) e = cached_tensor_map_2d(w + (size_t)bpr * 192, 1, (uint64_t)bpr * 16, p.n_rows[i], p.w_row_bytes, 16, kTileRows, &maps.m[i][2]);
         } else {
-            const uint32_t unit = g.type == YULE_DTYPE_Q8_0 ? 272 : g.type == YULE_DTYPE_Q4_0 ? 144 : 176;
+            const uint32_t unit = g.type == YULE_DTYPE_Q8_0 ? 272 : g.type == YULE_DTYPE_Q5_K ? 176 : 144;
             e = cached_tensor_map_2d(p.w[i], 8, (uint64_t)bpr * unit / 8, p.n_rows[i], (uint64_t)bpr * unit, unit / 8, kTileRows, &maps.m[i][0]);
         }
         if (e != cudaSuccess) return e;
@@ -699,11 +743,12 @@ cudaError_t launch_qgemm_int(const QGemm &g, const void *params, uint32_t grid, 
     // What the adder's truncation takes of a result on average, measured on products of either sign (bias against 64 bits); two additions a drain
     // cost less than four, and beside hi | lo as one operand less still.
     const bool merged = p.bn <= 64;
-    p.truncation = g.type == YULE_DTYPE_Q6_K ? 0.82e-7f : g.type == YULE_DTYPE_Q5_K ? 0.56e-7f : merged ? 0.15e-7f : 0.45e-7f;
+    p.truncation = g.type == YULE_DTYPE_Q6_K ? 0.82e-7f : g.type == YULE_DTYPE_Q4_K ? 0.8e-7f : g.type == YULE_DTYPE_Q5_K ? 0.56e-7f : merged ? 0.15e-7f : 0.45e-7f;
     switch (g.type) {
         case YULE_DTYPE_Q8_0: return launch_bn<kQ8>(p, maps, grid, g.pdl, s);
         case YULE_DTYPE_Q4_0: return launch_bn<kQ4>(p, maps, grid, g.pdl, s);
         case YULE_DTYPE_Q5_K: return launch_bn<kQ5K>(p, maps, grid, g.pdl, s);
+        case YULE_DTYPE_Q4_K: return launch_int<kQ4K, 128>(p, maps, grid, g.pdl, s);
         default: return launch_bn<kQ6K>(p, maps, grid, g.pdl, s);
     }
 }

@@ -1056,7 +1056,7 @@ cudaError_t encode_tensor_map_2d(const void *base, uint32_t elem_bytes, uint64_t
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// Q4_K runs on the exact-integer kernel, Q8_0, Q4_0, Q5_K and Q6_K on that of qgemm_int.cu, the others on the generic one (YULE_GEMM_GENERIC=1
+// Q4_K runs on the exact-integer kernel here up to 64 activation rows, beyond and for Q8_0, Q4_0, Q5_K and Q6_K on that of qgemm_int.cu, the others on the generic one (YULE_GEMM_GENERIC=1
 // sends all of them there, for comparison).  The activation tiles are laid out per 256 columns.
 bool qgemm_supported(uint32_t type, uint32_t n_cols, uint32_t n_tokens) {
     return is_quantized(type) && n_cols % 256 == 0 && n_cols > 0 && n_cols <= 65536 && n_tokens >= 1;
@@ -1177,7 +1177,7 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     if (generic)
         e = bn == 32 ? launch_gemm<32, true>(p, w_maps, grid, smem, g.pdl, s) : (bn == 64 ? launch_gemm<64, true>(p, w_maps, grid, smem, g.pdl, s) : launch_gemm<128, true>(p, w_maps, grid, smem, g.pdl, s));
     else
-        e = bn == 32 ? launch_gemm<32, false>(p, w_maps, grid, smem, g.pdl, s) : (bn == 64 ? launch_gemm<64, false>(p, w_maps, grid, smem, g.pdl, s) : launch_gemm<128, false>(p, w_maps, grid, smem, g.pdl, s));
+        e = bn == 32 ? launch_gemm<32, false>(p, w_maps, grid, smem, g.pdl, s) : launch_gemm<64, false>(p, w_maps, grid, smem, g.pdl, s);
     if (e != cudaSuccess) return e;
     *launches += 1;
     return cudaSuccess;
