@@ -99,7 +99,7 @@ bool yule_cuda_ctx::find(yule_buffer h, Buffer *out, const char *what) {
     return true;
 }
 
-// Also ends the chain of programmatic dependent launches: only qmv_common re-arms it, after a matvec.
+// Also ends the chain of programmatic dependent launches: a matvec re-arms it (qmv_common), and the ops of a forward pass (CHAINED).
 #define CTX_GUARD(ctx)                                                        \
     if (!(ctx)) return fail(YULE_ERR_INVALID_ARGUMENT, "null context");       \
     const bool _pdl_chain = (ctx)->pdl_chain;                                 \
@@ -125,6 +125,33 @@ bool yule_cuda_ctx::find(yule_buffer h, Buffer *out, const char *what) {
         cudaError_t _e = (call);                              \
         (ctx)->launches.fetch_add(_n);                        \
         if (_e != cudaSuccess) return fail_cuda(_e, #call);   \
+    } while (0)
+
+// An output of a launch that belongs to the chain: listed until the chain ends, since any of its launches may still be running when a matvec that reads its
+// weights (or, late, its input) before it waits is started.
+static void chain_output(yule_cuda_ctx *ctx, const void *at, size_t bytes) {
+    const char *lo = (const char *)at, *hi = lo + bytes;
+    for (int i = 0; i < ctx->chain_n; i++)
+        if (ctx->chain_lo[i] <= lo && hi <= ctx->chain_hi[i]) return;
+    ctx->chain_lo[ctx->chain_n] = lo;
+    ctx->chain_hi[ctx->chain_n] = hi;
+    ctx->chain_n++;
+}
+// Whether a kernel that waits for everything before it, before it reads or writes anything, is launched as a dependent of the launch before: where that was
+// one of the chain and the list still has room for its (at most two) outputs; else it begins a new chain.  Such a launch costs the host 1.9 us instead of 2.4,
+// and the kernel is there when the one before it ends.
+static bool chain_goes_on(yule_cuda_ctx *ctx, bool armed, int n) {
+    const bool on = armed && n + 2 <= yule_cuda_ctx::kChainRanges;
+    ctx->chain_n = on ? n : 0;
+    return on;
+}
+// `call` launches with `pdl`, which it may use, and writes `bytes` bytes at `out`.
+#define CHAINED(ctx, out, bytes, call)                                       \
+    do {                                                                     \
+        const bool pdl = chain_goes_on(ctx, _pdl_chain, _chain_n);           \
+        LAUNCHED(ctx, call);                                                 \
+        chain_output(ctx, out, bytes);                                       \
+        (ctx)->pdl_chain = true;                                             \
     } while (0)
 
 extern "C" {
@@ -318,8 +345,16 @@ int32_t yule_cuda_copy_buffer_offset(yule_cuda_ctx *ctx, yule_buffer src, yule_b
         int32_t rc = drop_planar(ctx, dst);
         if (rc) return rc;
     }
-    YULE_CUDA_TRY(cudaMemcpyAsync((char *)d.ptr + dst_offset, (const char *)s.ptr + src_offset, size,
-                                  cudaMemcpyDeviceToDevice, ctx->stream));
+    char *to = (char *)d.ptr + dst_offset;
+    const char *from = (const char *)s.ptr + src_offset;
+    // Small pieces (a K or V row into its cache) by a kernel, which stays in the chain of launches: a copy costs the host 2.6 us and the launches on either
+    // side of it their overlap.  Pieces that overlap are left to the copy, whatever it makes of them.
+    const bool apart = to + size <= from || from + size <= to;
+    if (apart && size <= kCopyKernelBytes && ((reinterpret_cast<uintptr_t>(to) | reinterpret_cast<uintptr_t>(from) | size) & 15) == 0) {
+        CHAINED(ctx, to, size, launch_copy(from, to, (uint32_t)size, ctx->stream, &_n, pdl));
+        return YULE_OK;
+    }
+    YULE_CUDA_TRY(cudaMemcpyAsync(to, from, size, cudaMemcpyDeviceToDevice, ctx->stream));
     return YULE_OK;
 }
 
@@ -386,8 +421,8 @@ int32_t yule_cuda_rms_norm(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer we
     NEED_BYTES(W, (size_t)size * 4, "rms_norm weight");
     NEED_BYTES(O, (size_t)size * 4, "rms_norm output");
     if (size == 0) return YULE_OK;
-    LAUNCHED(ctx, launch_rms_norm((const float *)I.ptr, (const float *)W.ptr, (float *)O.ptr, size, eps,
-                                  ctx->stream, &_n));
+    CHAINED(ctx, O.ptr, (size_t)size * 4,
+            launch_rms_norm((const float *)I.ptr, (const float *)W.ptr, (float *)O.ptr, size, eps, ctx->stream, &_n, pdl));
     return YULE_OK;
 }
 
@@ -411,8 +446,10 @@ int32_t yule_cuda_rope(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k, uint32_
         ang.cos[i] = cosf(theta);
         ang.sin[i] = sinf(theta);
     }
-    LAUNCHED(ctx, launch_rope_angles((float *)Q.ptr, (float *)K.ptr, head_dim, n_heads_q, n_heads_k, ang,
-                                     ctx->stream, &_n));
+    if (n_heads_q + n_heads_k == 0) return YULE_OK;
+    CHAINED(ctx, Q.ptr, (size_t)n_heads_q * head_dim * 4,
+            launch_rope_angles((float *)Q.ptr, (float *)K.ptr, head_dim, n_heads_q, n_heads_k, ang, ctx->stream, &_n, pdl));
+    chain_output(ctx, K.ptr, (size_t)n_heads_k * head_dim * 4);
     return YULE_OK;
 }
 
@@ -423,8 +460,7 @@ int32_t yule_cuda_silu(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer output
     NEED_BYTES(I, (size_t)size * 4, "silu input");
     NEED_BYTES(O, (size_t)size * 4, "silu output");
     if (size == 0) return YULE_OK;
-    LAUNCHED(ctx, launch_silu_mul((const float *)I.ptr, (const float *)O.ptr, (float *)O.ptr, size,
-                                  ctx->stream, &_n));
+    CHAINED(ctx, O.ptr, (size_t)size * 4, launch_silu_mul((const float *)I.ptr, (const float *)O.ptr, (float *)O.ptr, size, ctx->stream, &_n, pdl));
     return YULE_OK;
 }
 
@@ -438,8 +474,7 @@ int32_t yule_cuda_element_mul(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, 
     NEED_BYTES(B, (size_t)size * 4, "element_mul b");
     NEED_BYTES(O, (size_t)size * 4, "element_mul output");
     if (size == 0) return YULE_OK;
-    LAUNCHED(ctx, launch_silu_mul((const float *)A.ptr, (const float *)B.ptr, (float *)O.ptr, size,
-                                  ctx->stream, &_n));
+    CHAINED(ctx, O.ptr, (size_t)size * 4, launch_silu_mul((const float *)A.ptr, (const float *)B.ptr, (float *)O.ptr, size, ctx->stream, &_n, pdl));
     return YULE_OK;
 }
 
@@ -452,8 +487,7 @@ int32_t yule_cuda_add(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, yule_buf
     NEED_BYTES(B, (size_t)size * 4, "add b");
     NEED_BYTES(O, (size_t)size * 4, "add output");
     if (size == 0) return YULE_OK;
-    LAUNCHED(ctx, launch_add((const float *)A.ptr, (const float *)B.ptr, (float *)O.ptr, size, ctx->stream,
-                             &_n));
+    CHAINED(ctx, O.ptr, (size_t)size * 4, launch_add((const float *)A.ptr, (const float *)B.ptr, (float *)O.ptr, size, ctx->stream, &_n, pdl));
     return YULE_OK;
 }
 
@@ -755,6 +789,7 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
             uint32_t ranks;
             attn_cluster_shape(n_kv_heads, head_dim, seq_len, true, ctx->prop.multiProcessorCount, &ranks, &a.n_splits);
         }
+        bool grown = false;  // scratch is set to zero on the stream, which is no launch of the chain
         {
             std::lock_guard<std::mutex> lock(ctx->mu);
             // (more than 256 positions need the scratch of this entry point, whatever the clusters make of it: a capture that cannot have it is refused)
@@ -768,7 +803,10 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
                 // What either route takes at this length: a host that takes turns between long and short contexts allocates once, and after one
                 // call outside it a capture has what both need.
                 const uint32_t n = splits > a.n_splits ? splits : a.n_splits;
+                const float *had = ctx->attn_scratch;
+                const uint32_t *had_tickets = ctx->attn_tickets;
                 if (int32_t rc = grow_attn_scratch(ctx, attn_scratch_floats(n_heads, n, head_dim), n_heads > cluster_tickets ? n_heads : cluster_tickets)) return rc;
+                grown = ctx->attn_scratch != had || ctx->attn_tickets != had_tickets;
             } else if (!holds(a.n_splits, clustered ? cluster_tickets : n_heads)) {
                 if (longer && !(clustered && holds(splits, n_heads)))
                     return fail(YULE_ERR_INVALID_ARGUMENT, "the attention scratch cannot grow during graph capture: run the call once outside the capture first");
@@ -787,10 +825,13 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
         a.n_kv_heads = n_kv_heads;
         a.kv_stride = kv_stride;
         a.max_seq_len = seq_len;
+        a.pdl = chain_goes_on(ctx, _pdl_chain && !grown, _chain_n);
         if (clustered)
             LAUNCHED(ctx, launch_attn_cluster(a, ctx->prop.multiProcessorCount, ctx->stream, &_n));
         else
             LAUNCHED(ctx, launch_attn_decode(a, ctx->stream, &_n));
+        chain_output(ctx, O.ptr, (size_t)n_heads * head_dim * 4);
+        ctx->pdl_chain = true;
         return YULE_OK;
     }
     LAUNCHED(ctx, launch_multihead_attention((const float *)Q.ptr, (const float *)K.ptr, (const float *)V.ptr,

@@ -137,6 +137,8 @@ __global__ void rms_norm_kernel(const float *__restrict__ in, const float *__res
 // kernels/cuda/rope.cu:3-49 with the angles supplied by the host.
 __global__ void rope_angles_kernel(float *__restrict__ q, float *__restrict__ k, uint32_t head_dim, uint32_t n_heads_q,
                                    uint32_t n_heads_k, RopeAngles ang) {
+    yule_pdl_launch_dependents();
+    yule_pdl_wait();
     const uint32_t half = head_dim / 2;
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t total_q = n_heads_q * half, total_k = n_heads_k * half;
@@ -273,8 +275,17 @@ __global__ void elementwise_kernel(const float *__restrict__ a, const float *__r
 
 // kernels/cuda/add.cu:2-11.
 __global__ void add_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ out, uint32_t n) {
+    yule_pdl_launch_dependents();
+    yule_pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = a[i] + b[i];
+}
+
+__global__ void copy_kernel(const uint4 *__restrict__ from, uint4 *__restrict__ to, uint32_t n) {
+    yule_pdl_launch_dependents();
+    yule_pdl_wait();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) to[i] = from[i];
 }
 
 // kernels/cuda/attn_score.cu:3-33 — one warp per position.
@@ -529,12 +540,11 @@ cudaError_t launch_rms_norm_rows(const float *in, const float *w, float *out, ui
     return launch_kernel(rms_norm_kernel, dim3(rows), dim3(1024), 0, s, true, in, w, out, n, eps);
 }
 cudaError_t launch_rope_angles(float *q, float *k, uint32_t head_dim, uint32_t n_heads_q, uint32_t n_heads_k,
-                               const RopeAngles &ang, cudaStream_t s, uint64_t *launches) {
+                               const RopeAngles &ang, cudaStream_t s, uint64_t *launches, bool pdl) {
     uint32_t total = (n_heads_q + n_heads_k) * (head_dim / 2);
     if (total == 0) return cudaSuccess;
-    rope_angles_kernel<<<(total + 255) / 256, 256, 0, s>>>(q, k, head_dim, n_heads_q, n_heads_k, ang);
     *launches += 1;
-    return cudaGetLastError();
+    return launch_kernel(rope_angles_kernel, dim3((total + 255) / 256), dim3(256), 0, s, pdl, q, k, head_dim, n_heads_q, n_heads_k, ang);
 }
 cudaError_t launch_rope_kv_write(float *q, const float *k_tmp, const float *v_tmp, float *k_cache, float *v_cache,
                                  const float *cos_table, const float *sin_table, const uint32_t *pos_ptr,
@@ -561,10 +571,13 @@ cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint
     *launches += 1;
     return launch_kernel(silu_mul_kernel, dim3((n + 255) / 256), dim3(256), 0, s, pdl, gate, up, out, n);
 }
-cudaError_t launch_add(const float *a, const float *b, float *out, uint32_t n, cudaStream_t s, uint64_t *launches) {
-    add_kernel<<<(n + 255) / 256, 256, 0, s>>>(a, b, out, n);
+cudaError_t launch_add(const float *a, const float *b, float *out, uint32_t n, cudaStream_t s, uint64_t *launches, bool pdl) {
     *launches += 1;
-    return cudaGetLastError();
+    return launch_kernel(add_kernel, dim3((n + 255) / 256), dim3(256), 0, s, pdl, a, b, out, n);
+}
+cudaError_t launch_copy(const void *from, void *to, uint32_t bytes, cudaStream_t s, uint64_t *launches, bool pdl) {
+    *launches += 1;
+    return launch_kernel(copy_kernel, dim3((bytes / 16 + 255) / 256), dim3(256), 0, s, pdl, (const uint4 *)from, (uint4 *)to, bytes / 16);
 }
 cudaError_t launch_attn_score(const float *q, const float *k_cache, float *scores, uint32_t hd, uint32_t seq_len,
                               uint32_t head_offset, uint32_t kv_offset, uint32_t kv_stride, cudaStream_t s,

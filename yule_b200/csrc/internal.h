@@ -105,13 +105,13 @@ struct yule_cuda_ctx {
     // Word the kernels with bounded waits write when they give up; read by synchronize.
     int *device_status = nullptr;
     long long wait_cycles = yule::kDefaultWaitCycles;  // budget of every bounded device-side wait
-    // Programmatic dependent launch between consecutive matvec calls of the trait API: allowed only when the
+    // Programmatic dependent launch between consecutive calls of the trait API (matvecs and the other ops of a forward pass): allowed only when the
     // previous operation enqueued on the stream was one of this library's kernels, and its output does not
     // overlap the weights of the call being launched (weights are read before the dependency wait).
     bool pdl_chain = false;
-    // Outputs of the matvec calls of the current chain, any of which may still be running when the next one starts (a kernel
+    // Outputs of the calls of the current chain, any of which may still be running when the next one starts (a kernel
     // lets its successor start before it waits itself).
-    static constexpr int kChainRanges = 8;
+    static constexpr int kChainRanges = 24;  // (a layer's ops write some eleven vectors, which the next layer's write again, and two cache rows)
     const char *chain_lo[kChainRanges] = {}, *chain_hi[kChainRanges] = {};
     int chain_n = 0;
 
@@ -347,10 +347,16 @@ cudaError_t tp_exchange(yule_cuda_ctx *ctx, size_t buf_offset_floats, uint32_t p
                         const uint32_t *tick, uint32_t epochs_per_tick, uint32_t epoch_index, bool pdl, uint64_t *launches,
                         uint32_t n_rows = 1, size_t row_stride = 0);
 
+// Arguments as they lie, converted where they are not of the parameter's type: some kernels take more than a kilobyte of them.
+template <typename... KArgs>
+inline cudaError_t launch_config(const cudaLaunchConfig_t &cfg, void (*kernel)(KArgs...), const KArgs &...args) {
+    void *at[] = {const_cast<void *>(static_cast<const void *>(&args))...};
+    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void *>(kernel), at);
+}
 // Launch helper shared by every kernel: optional programmatic-dependent-launch attribute.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                 bool pdl, Args... args) {
+                                 bool pdl, const Args &...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -361,7 +367,7 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+    return launch_config<KArgs...>(cfg, kernel, args...);
 }
 
 cudaError_t launch_dequantize(const uint8_t *w, uint32_t type, uint64_t n_blocks, float *out,
@@ -403,11 +409,14 @@ struct RopeAngles {
 };
 cudaError_t launch_rope_angles(float *q, float *k, uint32_t head_dim, uint32_t n_heads_q,
                                uint32_t n_heads_k, const RopeAngles &ang, cudaStream_t s,
-                               uint64_t *launches);
+                               uint64_t *launches, bool pdl = false);
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint32_t n, cudaStream_t s,
                             uint64_t *launches, bool pdl = false);
 cudaError_t launch_add(const float *a, const float *b, float *out, uint32_t n, cudaStream_t s,
-                       uint64_t *launches);
+                       uint64_t *launches, bool pdl = false);
+// `bytes` and both addresses multiples of 16.
+constexpr size_t kCopyKernelBytes = 256 * 1024;
+cudaError_t launch_copy(const void *from, void *to, uint32_t bytes, cudaStream_t s, uint64_t *launches, bool pdl);
 cudaError_t launch_attn_score(const float *q, const float *k_cache, float *scores, uint32_t hd,
                               uint32_t seq_len, uint32_t head_offset, uint32_t kv_offset,
                               uint32_t kv_stride, cudaStream_t s, uint64_t *launches);

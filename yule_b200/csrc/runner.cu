@@ -648,6 +648,7 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches, bool 
 }
 
 int32_t finalize(yule_cuda_runner *r) {
+    r->ctx->pdl_chain = false;  // the runner's launches are not in the list of the ops' chain
     if (r->finalized) return YULE_OK;
     const yule_runner_config &c = r->cfg;
     const uint32_t N = r->ctx->tp_world ? r->ctx->tp_world : 1;
