@@ -111,3 +111,19 @@ def test_copies_of_every_alignment(backend, src, dst, size):
     assert np.array_equal(got, want)
     for h in (ha, hb):
         backend.free(h)
+
+
+@pytest.mark.parametrize("n", [1, 4096, 65536, 65537, 1 << 20])
+def test_a_pinned_source_may_be_overwritten_when_the_call_returns(backend, n):
+    """Up to 64 KB it goes the way of a pageable one, beyond that the call waits."""
+    import torch
+    host = torch.empty(n, dtype=torch.uint8, pin_memory=True).numpy()
+    h, got = backend.allocate(n), np.empty(n, np.uint8)
+    for value in range(1, 20):
+        host[:] = value
+        backend.copy_to_device(host, h)
+        host[:] = 200
+        if value % 6 == 0:
+            backend.copy_from_device(h, got)
+            assert np.all(got == value)
+    backend.free(h)

@@ -11,6 +11,7 @@ SYNTH_SO = os.path.join(HERE, "libyule_synth.so")
 
 _cuda = None
 _synth = None
+_calls = None
 
 u64, u32, i32, f32, size_t = C.c_uint64, C.c_uint32, C.c_int32, C.c_float, C.c_size_t
 vp = C.c_void_p
@@ -132,6 +133,16 @@ def cuda_lib() -> C.CDLL:
         lib.yule_cuda_sampling_random_value.restype = f32
         _cuda = lib
     return _cuda
+
+
+def calls():
+    """The per-op entry points as an extension module (csrc/calls.c): the same functions, names and arguments, a context being its address."""
+    global _calls
+    if _calls is None:
+        cuda_lib()  # says what to do where nothing has been built
+        from . import _calls as module
+        _calls = module
+    return _calls
 
 
 def synth_lib() -> C.CDLL:

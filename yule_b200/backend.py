@@ -71,6 +71,7 @@ class CudaB200Backend:
         ctx = C.c_void_p()
         _check(self._lib.yule_cuda_create(device, C.byref(ctx)))
         self._ctx = ctx
+        self._calls, self._at = _lib.calls(), ctx.value  # the ops of a forward pass go past ctypes
         self._runners = weakref.WeakSet()  # runners created on this context: destroyed before it
 
     def close(self) -> None:
@@ -80,7 +81,7 @@ class CudaB200Backend:
             for run in list(self._runners):
                 run.close()
             self._lib.yule_cuda_destroy(self._ctx)
-            self._ctx = None
+            self._ctx = self._at = None
 
     def __del__(self):
         try:
@@ -113,20 +114,30 @@ class CudaB200Backend:
         _check(self._lib.yule_cuda_softmax(self._ctx, input.id, output.id, size))
 
     def rms_norm(self, input: BufferHandle, weight: BufferHandle, output: BufferHandle, size: int, eps: float) -> None:
-        _check(self._lib.yule_cuda_rms_norm(self._ctx, input.id, weight.id, output.id, size, eps))
+        rc = self._calls.yule_cuda_rms_norm(self._at, input.id, weight.id, output.id, size, eps)
+        if rc:
+            _check(rc)
 
     def rope(self, q: BufferHandle, k: BufferHandle, pos: int, head_dim: int, freq_base: float, n_heads_q: int,
              n_heads_k: int) -> None:
-        _check(self._lib.yule_cuda_rope(self._ctx, q.id, k.id, pos, head_dim, freq_base, n_heads_q, n_heads_k))
+        rc = self._calls.yule_cuda_rope(self._at, q.id, k.id, pos, head_dim, freq_base, n_heads_q, n_heads_k)
+        if rc:
+            _check(rc)
 
     def silu(self, input: BufferHandle, output: BufferHandle, size: int) -> None:
-        _check(self._lib.yule_cuda_silu(self._ctx, input.id, output.id, size))
+        rc = self._calls.yule_cuda_silu(self._at, input.id, output.id, size)
+        if rc:
+            _check(rc)
 
     def element_mul(self, a: BufferHandle, b: BufferHandle, output: BufferHandle, size: int) -> None:
-        _check(self._lib.yule_cuda_element_mul(self._ctx, a.id, b.id, output.id, size))
+        rc = self._calls.yule_cuda_element_mul(self._at, a.id, b.id, output.id, size)
+        if rc:
+            _check(rc)
 
     def add(self, a: BufferHandle, b: BufferHandle, output: BufferHandle, size: int) -> None:
-        _check(self._lib.yule_cuda_add(self._ctx, a.id, b.id, output.id, size))
+        rc = self._calls.yule_cuda_add(self._at, a.id, b.id, output.id, size)
+        if rc:
+            _check(rc)
 
     def copy_to_device(self, data, handle: BufferHandle) -> None:
         ptr, n, keep = _host_ptr(data)
@@ -137,18 +148,24 @@ class CudaB200Backend:
         """Fills ``data`` (a writable bytes-like object or numpy array) from the buffer."""
         if isinstance(data, np.ndarray):
             assert data.flags["C_CONTIGUOUS"] and data.flags["WRITEABLE"]
-            ptr, n = C.c_void_p(data.ctypes.data), data.nbytes
+            ptr, n = data.ctypes.data, data.nbytes
         else:
             arr = np.frombuffer(memoryview(data), dtype=np.uint8)
-            ptr, n = C.c_void_p(arr.ctypes.data), arr.nbytes
-        _check(self._lib.yule_cuda_copy_from_device(self._ctx, handle.id, ptr, n))
+            ptr, n = arr.ctypes.data, arr.nbytes
+        rc = self._calls.yule_cuda_copy_from_device(self._at, handle.id, ptr, n)
+        if rc:
+            _check(rc)
 
     def copy_buffer(self, src: BufferHandle, dst: BufferHandle, size: int) -> None:
-        _check(self._lib.yule_cuda_copy_buffer(self._ctx, src.id, dst.id, size))
+        rc = self._calls.yule_cuda_copy_buffer(self._at, src.id, dst.id, size)
+        if rc:
+            _check(rc)
 
     def copy_buffer_offset(self, src: BufferHandle, dst: BufferHandle, src_offset: int, dst_offset: int,
                            size: int) -> None:
-        _check(self._lib.yule_cuda_copy_buffer_offset(self._ctx, src.id, dst.id, src_offset, dst_offset, size))
+        rc = self._calls.yule_cuda_copy_buffer_offset(self._at, src.id, dst.id, src_offset, dst_offset, size)
+        if rc:
+            _check(rc)
 
     def synchronize(self) -> None:
         _check(self._lib.yule_cuda_synchronize(self._ctx))
@@ -185,16 +202,19 @@ class CudaB200Backend:
 
     def quantized_matmul(self, weights: BufferHandle, input: BufferHandle, output: BufferHandle, n_rows: int,
                          n_cols: int, dtype: DType) -> None:
-        _check(self._lib.yule_cuda_quantized_matmul(self._ctx, weights.id, input.id, output.id, n_rows, n_cols,
-                                                    int(dtype)))
+        rc = self._calls.yule_cuda_quantized_matmul(self._at, weights.id, input.id, output.id, n_rows, n_cols,
+                                                    int(dtype))
+        if rc:
+            _check(rc)
 
     # ── additive entry points ──────────────────────────────────────────────────────────────
     def quantized_matmul_batched(self, weights: BufferHandle, input: BufferHandle, output: BufferHandle,
                                  n_rows: int, n_cols: int, dtype: DType, batch: int, x_stride: int | None = None,
                                  out_stride: int | None = None) -> None:
-        _check(self._lib.yule_cuda_quantized_matmul_batched(
-            self._ctx, weights.id, input.id, output.id, n_rows, n_cols, int(dtype), batch,
-            n_cols if x_stride is None else x_stride, n_rows if out_stride is None else out_stride))
+        rc = self._calls.yule_cuda_quantized_matmul_batched(self._at, weights.id, input.id, output.id, n_rows, n_cols, int(dtype), batch,
+            n_cols if x_stride is None else x_stride, n_rows if out_stride is None else out_stride)
+        if rc:
+            _check(rc)
 
     def quantized_matmul_at(self, weights: BufferHandle, weight_offset: int, input: BufferHandle,
                             output: BufferHandle, n_rows: int, n_cols: int, dtype: DType) -> None:
@@ -210,8 +230,10 @@ class CudaB200Backend:
 
     def multihead_attention(self, q: BufferHandle, k_cache: BufferHandle, v_cache: BufferHandle, out: BufferHandle,
                             head_dim: int, seq_len: int, n_heads: int, n_kv_heads: int, kv_stride: int) -> None:
-        _check(self._lib.yule_cuda_multihead_attention(self._ctx, q.id, k_cache.id, v_cache.id, out.id, head_dim,
-                                                       seq_len, n_heads, n_kv_heads, kv_stride))
+        rc = self._calls.yule_cuda_multihead_attention(self._at, q.id, k_cache.id, v_cache.id, out.id, head_dim,
+                                                       seq_len, n_heads, n_kv_heads, kv_stride)
+        if rc:
+            _check(rc)
 
     def multihead_attention_static(self, q: BufferHandle, k_cache: BufferHandle, v_cache: BufferHandle,
                                    out: BufferHandle, head_dim: int, seq_len: int, n_heads: int, n_kv_heads: int,

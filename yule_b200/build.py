@@ -1,9 +1,10 @@
 """In-tree build of the package's native libraries.
 
 * ``libyule_cuda.so``  — the CUDA backend (``csrc/*.cu``), nvcc, sm_100a only.
+* ``_calls*.so``        — the per-op entry points as a CPython extension module (``csrc/calls.c``) over ``libyule_cuda.so``, gcc.
 * ``libyule_synth.so`` — the host-side synthetic tensor generator / quantiser (``csrc/synth.cpp``), g++.
 
-``python -m yule_b200.build`` builds both (``--force`` rebuilds; ``--verbose`` adds ``-Xptxas -v``).
+``python -m yule_b200.build`` builds all (``--force`` rebuilds; ``--verbose`` adds ``-Xptxas -v``).
 nvcc cross-compiles without a GPU present.
 """
 
@@ -15,11 +16,13 @@ import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 CUDA_SO = os.path.join(HERE, "libyule_cuda.so")
 SYNTH_SO = os.path.join(HERE, "libyule_synth.so")
+CALLS_SO = os.path.join(HERE, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -101,7 +104,17 @@ def build_cuda(force: bool = False, verbose: bool = False) -> str:
     if force or jobs or _stale(CUDA_SO, objs):
         subprocess.check_call([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC"] + objs +
                               ["-ldl", "-o", CUDA_SO])
+    build_calls(force)
     return CUDA_SO
+
+
+def build_calls(force: bool = False) -> str:
+    """The extension module finds ``libyule_cuda.so`` beside itself."""
+    src, include = os.path.join(CSRC, "calls.c"), os.path.join(os.path.dirname(HERE), "include")
+    if force or _stale(CALLS_SO, [src, os.path.join(include, "yule_cuda.h"), os.path.abspath(__file__)]):
+        subprocess.check_call(["gcc", "-O2", "-std=c11", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], "-I", include, src,
+                               "-L", HERE, "-l:libyule_cuda.so", "-Wl,-rpath,$ORIGIN", "-o", CALLS_SO])
+    return CALLS_SO
 
 
 def build_synth(force: bool = False) -> str:
