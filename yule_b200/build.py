@@ -47,7 +47,8 @@ def _stale(target: str, sources: list[str]) -> bool:
 # The 128-row kernels of the GEMMs move registers between its warps (setmaxnreg) out of what their launch brings, and would wait for ever if the compiler had
 # given it fewer than the split adds up to: that is a matter of the compiler, so it is checked where the compiler runs.
 REGISTER_FLOORS = {"qgemm_tc.cu": (r"qgemm_tc_kernelILi128E", r"kLaunchRegs = (\d+);"),
-                   "qgemm_int.cu": (r"qgemm_int_kernelI", r"kLaunchRegs = (\d+);")}
+                   "qgemm_int.cu": (r"qgemm_int_kernelI", r"kLaunchRegs = (\d+);"),
+                   "attn_prefill.cu": (r"attn_prefill_kernelI", r"kLaunchRegs = (\d+);")}
 
 
 def check_registers(report: str, kernel: str, at_least: int) -> None:

@@ -472,8 +472,14 @@ struct AttnPrefill {
     uint32_t n_tokens = 0, n_seq = 1, pos0 = 0, hd = 0, n_heads = 0, n_kv_heads = 0, kv_stride = 0, q_stride = 0, out_stride = 0;
     size_t kv_batch_stride = 0;
     bool pdl = false;
+    // K and V as the tensor core reads them, at least of one KV head of one sequence (attn_prefill_scratch_bytes; of more at a time where there is room);
+    // 16-byte aligned, written before it is read
+    void *scratch = nullptr;
+    size_t scratch_bytes = 0;
+    int *status = nullptr;    // device status word for the kernel's bounded waits
 };
 bool attn_prefill_preferred(uint32_t hd, uint32_t n_heads, uint32_t n_kv_heads, uint32_t n_tokens, uint32_t n_seq, uint32_t pos0, int sm_count);
+size_t attn_prefill_scratch_bytes(uint32_t hd, uint32_t positions);
 cudaError_t launch_attn_prefill(const AttnPrefill &a, cudaStream_t s, uint64_t *launches);
 bool attn_gqa_supported(uint32_t hd, uint32_t n_heads, uint32_t n_kv_heads);
 uint32_t attn_gqa_pick_splits(uint32_t n_kv_heads, uint32_t max_seq_len, int sm_count);

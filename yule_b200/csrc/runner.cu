@@ -1276,6 +1276,10 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
                 ap.out_stride = qdim;
                 ap.kv_batch_stride = cache_stride;
                 ap.pdl = true;
+                // (the GEMM's scratch but for its tickets, which nothing uses between two GEMMs)
+                ap.scratch = static_cast<unsigned char *>(ctx->gemm_scratch) + kGemmTicketBytes;
+                ap.scratch_bytes = ctx->gemm_scratch_bytes - kGemmTicketBytes;
+                ap.status = ctx->device_status;
                 ok(launch_attn_prefill(ap, s, launches));
                 tiled = true;
             }
@@ -1345,6 +1349,7 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
     cudaStream_t s = ctx->stream;
     int32_t rc;
     if ((rc = ensure_chunk_buffers(r, n < prefill_max_rows() ? n : prefill_max_rows()))) return rc;
+    if ((rc = ensure_gemm_scratch(ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(r->cfg.head_dim, r->pos + n)))) return rc;  // (from some 30000 positions on)
     YULE_CUDA_TRY(cudaStreamSynchronize(s));  // staging words may still be in flight
     if ((rc = ensure_pinned(r, n))) return rc;
     const uint32_t C = r->pf_chunk;
@@ -2024,6 +2029,7 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
     uint32_t per_seq = (r->xchg || !prefill_max_rows() ? r->pf_chunk : prefill_max_rows()) / batch;  // prompt tokens of each sequence per pass
     per_seq = per_seq < 1 ? 1 : (per_seq > fed ? fed : per_seq);
     if (fed && (rc = ensure_chunk_buffers(r, per_seq * batch))) return rc;
+    if (fed && (rc = ensure_gemm_scratch(r->ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(c.head_dim, fed)))) return rc;
     if (fed && per_seq * batch > r->pf_chunk) per_seq = r->pf_chunk / batch;  // (a batch is no larger than the basic chunk)
     if ((rc = ensure_batch_graph(r))) return rc;
     // prompts to the device, pass by pass, the rows of a pass in the order of the sequences
