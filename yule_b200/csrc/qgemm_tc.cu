@@ -673,8 +673,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qgemm_tc_kernel(const __grid_
         RingPos ring;
         bool ok = true;
         ItemWalk items(p);
-            for (Item wi; ok && items.next(p, bpr, wi);) {
-            const uint32_t mt = wi.mt, nt = wi.nt;
+        for (Item wi; ok && items.next(p, bpr, wi);) {
+            const uint32_t mt = wi.mt;
             const uint32_t row = mt * kBM + lane_base + lane;
             const uint8_t *rowp = p.w[wi.seg] + (size_t)(row < p.n_rows[wi.seg] ? row : p.n_rows[wi.seg] - 1) * bpr * 144;
             uint64_t acc2[CW / 2];  // pairs of sums: columns 2j, 2j + 1
@@ -790,21 +790,24 @@ struct XprepParams {
     float *oscale;
 };
 
-// ROWS rows per CTA, as many threads (up to 1024) as have columns to work on; a thread keeps its 8·CHUNKS columns of a row in registers from
-// the single read to the stores, so rows of up to 8192·CHUNKS / ROWS columns cost one round trip to memory and two block reductions
-// whatever their length.  A thread's 16 bytes of a term lie alone in their 8-column step, the next row's 16 bytes behind them: with two rows in
-// neighbouring lanes a warp writes whole 32-byte sectors, with one it writes halves.  2048 rows of 14336 columns with SwiGLU 137 -> 102 us,
-// of 4096 columns with RMSNorm 29 -> 24.  Where there are not rows enough to give every SM
-// two, one per CTA keeps more SMs at work.
-constexpr int kXprepThreads = 1024;
-template <int CHUNKS, int ROWS>
-__global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepParams p) {
-    yule_pdl_launch_dependents();
-    yule_pdl_wait();
-    __shared__ float red[32 * ROWS];
-    const uint32_t lane_row = threadIdx.x % ROWS, tc = threadIdx.x / ROWS, row_threads = blockDim.x / ROWS;
-    const uint32_t n = blockIdx.x * ROWS + lane_row, nt = n / p.bn, r = n % p.bn;
-    const bool live = n < p.n_tokens;  // else a padding row of the last tile: all zeros
+__device__ __forceinline__ void load8(const float *from, float (&to)[8]) {  // (the host has checked the alignment)
+    const float4 a = *reinterpret_cast<const float4 *>(from), b = *reinterpret_cast<const float4 *>(from + 4);
+    to[0] = a.x, to[1] = a.y, to[2] = a.z, to[3] = a.w, to[4] = b.x, to[5] = b.y, to[6] = b.z, to[7] = b.w;
+}
+// Power of two that puts a row's largest element in [2^13, 2^14) (a rounding above at the most).
+__device__ __forceinline__ float row_scale(float amax) {
+    float scale = 1.f;
+    if (amax > 1e-30f && amax < 1e30f) {
+        int ex;
+        frexpf(amax, &ex);  // amax = m · 2^ex, m in [0.5, 1)
+        scale = ldexpf(1.f, 14 - ex);
+    }
+    return scale;
+}
+// Eight columns from k0 on of (padded) activation row n, scaled, to the operand tiles; the four threads of a 32-column sub-block, `step` lanes apart, add up its
+// sum, which `first` of them stores.
+__device__ __forceinline__ void put_columns(const XprepParams &p, uint32_t n, uint32_t k0, float (&v)[8], float scale, uint32_t step, bool first) {
+    const uint32_t nt = n / p.bn, r = n % p.bn;
     const uint32_t bpr = p.n_cols / 256;
     const uint32_t x_half_bytes = p.bn * kBK * 2, bm_bytes = p.bn * 32, super_bytes = 8 * x_half_bytes + bm_bytes;
     const uint32_t core = ((r >> 3) * 64 + (r & 7u) * 8) * 2;  // byte offset of this row inside an 8-column step
@@ -820,6 +823,51 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         return reinterpret_cast<__half *>(p.xb + ((size_t)nt * bpr + sb) * super_bytes + 8 * (size_t)x_half_bytes +
                                           term * (p.bn * 16) + core) + s;
     };
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v[i] *= scale;
+        sum += v[i];
+    }
+    // positions 0..7 of the 16 bytes hold columns 0,2,1,3,4,6,5,7
+    const float o[8] = {v[0], v[2], v[1], v[3], v[4], v[6], v[5], v[7]};
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __half2 hh = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
+        const float2 back = __half22float2(hh);
+        h[i] = as_u32(hh);
+        l[i] = as_u32(__floats2half2_rn(o[2 * i] - back.x, o[2 * i + 1] - back.y));
+    }
+    *reinterpret_cast<uint4 *>(slab16(k0, 0)) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(slab16(k0, 1)) = make_uint4(l[0], l[1], l[2], l[3]);
+    // four consecutive threads of a row cover one 32-column sub-block
+    sum += __shfl_xor_sync(0xffffffffu, sum, step);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2 * step);
+    if (first) {
+        sum *= kSumScale;  // 32 elements of up to 2^14 each: keep the sum inside fp16's range
+        const __half sh = __float2half_rn(sum);
+        *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 0) = sh;
+        *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 1) = __float2half_rn(sum - __half2float(sh));
+    }
+}
+
+// ROWS rows per CTA, as many threads (up to 1024) as have columns to work on; a thread keeps its 8·CHUNKS columns of a row in registers from
+// the single read to the stores, so rows of up to 8192·CHUNKS / ROWS columns cost one round trip to memory and two block reductions
+// whatever their length.  A thread's 16 bytes of a term lie alone in their 8-column step, the next row's 16 bytes behind them: with two rows in
+// neighbouring lanes a warp writes whole 32-byte sectors, with one it writes halves.  2048 rows of 14336 columns with SwiGLU 137 -> 102 us,
+// of 4096 columns with RMSNorm 29 -> 24.  Where there are not rows enough to give every SM
+// two, one per CTA keeps more SMs at work.
+constexpr int kXprepThreads = 1024;
+constexpr uint32_t kXprepMaxRanks = 4;  // CTAs that share a row
+template <int CHUNKS, int ROWS>
+__global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepParams p) {
+    yule_pdl_launch_dependents();
+    yule_pdl_wait();
+    __shared__ float red[32 * ROWS];
+    const uint32_t lane_row = threadIdx.x % ROWS, tc = threadIdx.x / ROWS, row_threads = blockDim.x / ROWS;
+    const uint32_t n = blockIdx.x * ROWS + lane_row;
+    const bool live = n < p.n_tokens;  // else a padding row of the last tile: all zeros
     const float *x = p.x + (size_t)n * p.x_stride;
     const float *gate = p.gate ? p.gate + (size_t)n * p.x_stride : nullptr;
     // over the threads of a row, which are every ROWS-th lane
@@ -834,10 +882,6 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
         for (uint32_t w = first; w < n_warps; w += 32 / ROWS) v = both(v, red[w * ROWS + lane_row]);
         for (int o = 16; o >= ROWS; o >>= 1) v = both(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
-    };
-    auto load8 = [&](const float *from, float (&to)[8]) {  // (the host has checked the alignment)
-        const float4 a = *reinterpret_cast<const float4 *>(from), b = *reinterpret_cast<const float4 *>(from + 4);
-        to[0] = a.x, to[1] = a.y, to[2] = a.z, to[3] = a.w, to[4] = b.x, to[5] = b.y, to[6] = b.z, to[7] = b.w;
     };
     float v[CHUNKS][8];
 #pragma unroll
@@ -887,46 +931,91 @@ __global__ void __launch_bounds__(kXprepThreads) gemm_xprep_kernel(const XprepPa
 #pragma unroll
         for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[c][i]));
     amax = row_reduce(amax, true);
-    // power of two that puts the largest element in [2^13, 2^14)
-    float scale = 1.f;
-    if (amax > 1e-30f && amax < 1e30f) {
-        int ex;
-        frexpf(amax, &ex);  // amax = m · 2^ex, m in [0.5, 1)
-        scale = ldexpf(1.f, 14 - ex);
-    }
+    const float scale = row_scale(amax);
     if (tc == 0) p.oscale[n] = live ? 1.0f / scale : 0.f;
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
         const uint32_t k0 = ((uint32_t)c * row_threads + tc) * 8;
         if (k0 >= p.n_cols) break;  // whole warps leave together (256 columns are 32 threads of a row)
-        float sum = 0.f;
+        put_columns(p, n, k0, v[c], scale, ROWS, (tc & 3u) == 0);
+    }
+}
+
+// The same for few rows: a cluster of CTAs has each row (or pair of rows), a CTA an equal share of the 256-column blocks, a thread eight columns.  What bounds one
+// CTA per row is the one SM behind it: a row of 28672 columns with SwiGLU is 230 KB to read and 115 KB to write.  Sum of squares and largest element
+// meet in every CTA's shared memory behind one cluster barrier: under a norm the largest is that of x · w, times the norm's factor (its roundings may
+// put the scaled row's largest element at 2^14 itself, far inside the operands' range).  32 rows, us between the launches around it, one CTA per row and
+// this: 4096 columns with RMSNorm 5.2 -> 3.6, 8192 6.6 -> 4.1; with SwiGLU 14336 columns 8.1 -> 5.3, 28672 15.6 -> 6.5.  128 rows of 4096
+// columns 7.7 -> 5.0, 256 7.5 -> 4.8.
+template <int ROWS>
+__global__ void __launch_bounds__(kXprepThreads) gemm_xprep_cluster_kernel(const XprepParams p) {
+    yule_pdl_launch_dependents();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (every CTA of the cluster runs before another stores to it)
+    __shared__ float2 red[32 * ROWS], shares[kXprepMaxRanks * ROWS];  // (sum of squares, largest)
+    uint32_t rank, ranks;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(ranks));
+    const uint32_t lane_row = threadIdx.x % ROWS, tc = threadIdx.x / ROWS, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t n = blockIdx.x / ranks * ROWS + lane_row, blocks = p.n_cols / 256, b0 = blocks * rank / ranks, b1 = blocks * (rank + 1) / ranks;
+    const uint32_t k0 = b0 * 256 + tc * 8;
+    const bool live = n < p.n_tokens, mine = k0 < b1 * 256;  // (`mine`: whole warps)
+    float v[8] = {}, w[8] = {}, ss = 0.f, most = 0.f;
+    auto reduce = [&]() {  // over the lanes of a row
+#pragma unroll
+        for (int o = 16; o >= ROWS; o >>= 1) {
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        }
+    };
+    if (live && mine && p.norm_w) load8(p.norm_w + k0, w);  // (weights: nothing before this launch writes them)
+    yule_pdl_wait();
+    if (live && mine) {
+        load8(p.x + (size_t)n * p.x_stride + k0, v);
+        if (p.gate) {
+            float gt[8];
+            load8(p.gate + (size_t)n * p.x_stride + k0, gt);
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = (gt[i] / (1.0f + expf(-gt[i]))) * v[i];
+        }
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            v[c][i] *= scale;
-            sum += v[c][i];
-        }
-        // positions 0..7 of the 16 bytes hold columns 0,2,1,3,4,6,5,7
-        const float o[8] = {v[c][0], v[c][2], v[c][1], v[c][3], v[c][4], v[c][6], v[c][5], v[c][7]};
-        uint32_t h[4], l[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const __half2 hh = __floats2half2_rn(o[2 * i], o[2 * i + 1]);
-            const float2 back = __half22float2(hh);
-            h[i] = as_u32(hh);
-            l[i] = as_u32(__floats2half2_rn(o[2 * i] - back.x, o[2 * i + 1] - back.y));
-        }
-        *reinterpret_cast<uint4 *>(slab16(k0, 0)) = make_uint4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<uint4 *>(slab16(k0, 1)) = make_uint4(l[0], l[1], l[2], l[3]);
-        // four consecutive threads of a row cover one 32-column sub-block
-        sum += __shfl_xor_sync(0xffffffffu, sum, ROWS);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2 * ROWS);
-        if ((tc & 3u) == 0) {
-            sum *= kSumScale;  // 32 elements of up to 2^14 each: keep the sum inside fp16's range
-            const __half sh = __float2half_rn(sum);
-            *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 0) = sh;
-            *sum_slot(k0 >> 8, (k0 >> 5) & 7u, 1) = __float2half_rn(sum - __half2float(sh));
+            ss = fmaf(v[i], v[i], ss);
+            most = fmaxf(most, fabsf(p.norm_w ? v[i] * w[i] : v[i]));
         }
     }
+    reduce();
+    if (lane < ROWS) red[warp * ROWS + lane] = make_float2(ss, most);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        ss = 0.f, most = 0.f;
+        for (uint32_t i = lane / ROWS; i < (blockDim.x >> 5); i += 32 / ROWS) {
+            const float2 r = red[i * ROWS + lane_row];
+            ss += r.x, most = fmaxf(most, r.y);
+        }
+        reduce();
+        for (uint32_t to_rank = lane / ROWS; to_rank < ranks; to_rank += 32 / ROWS) {  // this CTA's share to slot `rank` of every CTA
+            uint32_t to;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(&shares[rank * ROWS + lane_row])), "r"(to_rank));
+            asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(ss), "f"(most) : "memory");
+        }
+        __syncwarp();
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    ss = 0.f, most = 0.f;
+    for (uint32_t i = 0; i < ranks; i++) {
+        const float2 r = shares[i * ROWS + lane_row];
+        ss += r.x, most = fmaxf(most, r.y);
+    }
+    if (p.norm_w) {
+        const float inv = 1.0f / sqrtf(ss / (float)p.n_cols + p.eps);
+        most *= inv;
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = v[i] * inv * w[i];
+    }
+    const float scale = row_scale(most);
+    if (rank == 0 && tc == 0) p.oscale[n] = live ? 1.0f / scale : 0.f;
+    if (mine) put_columns(p, n, k0, v, scale, ROWS, (tc & 3u) == 0);
 }
 
 // 2-D view of a Q4_K matrix for the TMA engine: bytes along a row, rows; box = one super-block
@@ -1093,7 +1182,26 @@ cudaError_t launch_qgemm_xprep(const QGemm &g, int sm_count, cudaStream_t s, uin
     auto launch = [&](auto kern, uint32_t chunks, uint32_t rows) {
         return launch_kernel(kern, dim3(padded / rows), dim3(rows * (((g.n_cols / 8 + chunks - 1) / chunks + 31) / 32 * 32)), 0, s, g.pdl, xp);
     };
-    if (padded >= 2 * (uint32_t)sm_count && g.n_cols <= 16384)  // (padded is a multiple of 32)
+    // A row on a cluster where it is read at once: all rows together are a CTA of 1024 threads per SM at the most (beyond: 128 rows of 14336 columns 8.7 us with one
+    // CTA per row, 9.8 on clusters of four; 28672: 16.9 and 22.9), and there are not rows enough for two per SM.  Clusters of four up to 64 rows, two beyond (8192
+    // columns: 32 rows 4.5 us with two, 4.1 with four, 4.2 with eight; 128 rows 5.4 and 5.3 with two and four); two rows per CTA where they fit.
+    const uint32_t blocks = g.n_cols / 256, ranks = 2 * padded <= (uint32_t)sm_count ? 4 : 2, share = (blocks + ranks - 1) / ranks, most_warps = kXprepThreads / 32;
+    if (padded < 2 * (uint32_t)sm_count && (uint64_t)padded * g.n_cols <= (uint64_t)kXprepThreads * 8 * sm_count && blocks >= ranks && share <= most_warps && !(g.gate && g.norm_w)) {
+        const uint32_t rows = 2 * share <= most_warps ? 2 : 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(padded / rows * ranks);
+        cfg.blockDim = dim3(share * 32 * rows);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ranks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = g.pdl ? 2 : 1;
+        e = rows == 2 ? launch_config<XprepParams>(cfg, gemm_xprep_cluster_kernel<2>, xp) : launch_config<XprepParams>(cfg, gemm_xprep_cluster_kernel<1>, xp);
+    } else if (padded >= 2 * (uint32_t)sm_count && g.n_cols <= 16384)  // (padded is a multiple of 32)
         e = g.n_cols <= 4096 ? launch(gemm_xprep_kernel<1, 2>, 1, 2) : (g.n_cols <= 8192 ? launch(gemm_xprep_kernel<2, 2>, 2, 2) : launch(gemm_xprep_kernel<4, 2>, 4, 2));
     else if (g.n_cols <= 8192)
         e = launch(gemm_xprep_kernel<1, 1>, 1, 1);
