@@ -181,13 +181,13 @@ int32_t yule_cuda_sample(yule_cuda_ctx *ctx, yule_buffer logits, uint32_t n, con
  * [batch][x_stride] floats, output [batch][out_stride] floats.  Same per-row
  * arithmetic as quantized_matmul.  Small batches go through the matvec kernels,
  * up to sixteen vectors per pass over the weights (Q4_K, Q5_K, Q6_K, Q8_0,
- * Q4_0); from 13 vectors of Q4_K (17 on matrices of up to 17 Mi weights) or 33 to
- * 49 of the other block formats (n_cols a multiple of 256), the tcgen05 GEMM
- * takes one pass over the weights.
+ * Q4_0); from 13 vectors of Q4_K (17 on matrices of up to 17 Mi weights) or 17 to
+ * 33 of the other block formats (n_cols a multiple of 256; fewest on the large
+ * matrices), the tcgen05 GEMM takes one pass over the weights.
  * The GEMM keeps its activation tiles in a scratch owned by the context, grown
  * on demand; growing is not possible while a graph is being captured, so run
  * one call of the largest batch before yule_cuda_graph_begin.  (Up to 15 vectors
- * of Q4_K, 31 on matrices of up to 8M weights, 63 of Q5_K and 31 of the other
+ * of Q4_K, 31 on matrices of up to 8M weights, 63 of Q5_K and 32 of the other
  * formats need no such call: the matvec kernels take them then.) */
 int32_t yule_cuda_quantized_matmul_batched(yule_cuda_ctx *ctx, yule_buffer weights,
                                            yule_buffer input, yule_buffer output, uint32_t n_rows,
@@ -353,8 +353,8 @@ int32_t yule_cuda_tp_exchange_layout(const yule_runner_config *cfg, uint64_t out
 /* Batched decode: `batch` independent sequences, one new token each per call, every sequence with its own
  * KV caches and position (all start at 0; reset_batch rewinds them).  Per sequence the result is that of
  * decode_step on a runner of its own (the reference serves one sequence per ModelRunner,
- * yule-infer/src/lib.rs:169-216); across the batch every linear is one GEMM, so the weights are read once
- * per step.  Single GPU, fused = 1, Llama op sequence, n_cols in multiples of 256; the first call fixes the
+ * yule-infer/src/lib.rs:169-216); across the batch every linear is a pass of the matvec kernels per sixteen
+ * sequences or one GEMM, whichever is faster.  Single GPU, fused = 1, Llama op sequence, n_cols in multiples of 256; the first call fixes the
  * batch size of the runner.  logits_out: [batch][vocab_size] floats or null. */
 int32_t yule_cuda_runner_decode_batch(yule_cuda_runner *runner, const uint32_t *tokens, uint32_t batch, float *logits_out);
 int32_t yule_cuda_runner_reset_batch(yule_cuda_runner *runner);

@@ -1,9 +1,11 @@
 // Quantised GEMM on the 5th-generation tensor cores (tcgen05, accumulators in TMEM):
 //
-//     out[n][r] = Σ_k W[r][k] · x[n][k]        W: Q4_K blocks, x: N ≥ 8 fp32 activation rows
+//     out[n][r] = Σ_k W[r][k] · x[n][k]        W: Q4_K blocks, x: 8 to 64 fp32 activation rows
+//
+// (With more rows Q4_K goes through qgemm_int.cu, and so do Q8_0, Q4_0, Q5_K and Q6_K at any number; the generic form of this kernel takes the other formats and what those kernels refuse.)
 //
 // This is the prefill / batched-decode counterpart of the matvec kernels: the weights cross HBM
-// once per pass over up to 128 activation rows instead of once per four.  The reference runs
+// once per pass over up to 64 (generic: 128) activation rows instead of once per four.  The reference runs
 // prefill as one matvec chain per token (yule-infer/src/gpu_runner.rs:146-160); the arithmetic
 // contract is the same fp32 dot product.
 //
@@ -33,13 +35,12 @@
 //   warps 9, 11 tcgen05.mma issue, even stages from one, odd stages from the other; warp 9 also owns
 //               the TMEM allocation
 //   warp  10    one thread: tiled TMA loads (cp.async.bulk.tensor.2d) of the raw Q4_K bytes, one
-//               128-row × 144-byte box per super-block, three boxes in flight at 128 activation rows, six
-//               below; rows past the end of the matrix arrive as zeros
+//               128-row × 144-byte box per super-block, six boxes in flight; rows past the end of the matrix arrive as zeros
 //   warps 12-19 unpack Q4_K from that shared-memory copy → fp16 sc·q in tensor memory, where the MMA takes its
 //               W operand from: a row is a lane, a column two weights, and 64 weights of a row are 32 columns
 // A stage is a 128-row × 64-column slab of W plus the matching hi and lo slabs of x in shared memory; the last
 // stage of a super-block also carries the 4 KB m slab (shared memory) and the sub-block sums of x.  At 32 activation rows
-// a stage is two such column groups (a chain of eight MMAs, as at 128 rows, and half the hand-offs per column).  Tensor memory holds
+// a stage is two such column groups (a chain of eight MMAs and half the hand-offs per column).  Tensor memory holds
 // four stages of W and behind them a ring of accumulators, three of 128 columns (four of 64 at 32 rows), in which the min term of a
 // super-block takes its turn like a stage.
 // One launch can run over up to three matrices that read the same activations (Q/K/V; gate/up): their row
@@ -48,10 +49,8 @@
 // core matrices of one 8-column step contiguous along the rows.  Of eight columns the order is
 // 0,2,1,3,4,6,5,7 (the order in which nibble pairs fall out of a 32-bit word) in both operands, so the products pair up correctly.
 //
-// What bounds it, at 128 activation rows, clocks per stage of an SM: the tensor pipe 512 (+ 16 for the min term).  With W in shared memory a
-// stage moved 121 KB through it (970 clocks) and took 1400.  Measured with one role's work taken out at a time, no role alone bounds it
-// now: hand-offs and issue slots do (a stage takes some 850 clocks, the tensor pipe is busy for 60 % of them, the issue slots for 59 %).  8192x8192 by 256 rows 113 -> 78 us (re-layout included);
-// 32 rows 32.6 -> 26.4; the 8B model's 2048-token prompt 115.7 -> 94.2 ms.
+// What bounds it: the hand-offs of a stage between the roles, and issue slots; no role's work alone (measured with one taken out at a time).  32 rows, W in
+// shared memory and in tensor memory: 8192x8192 32.6, 26.4 us (re-layout included); tiles that did not fill a round dealt by super-blocks: gate / up of the 70B shape 121, 103.
 //
 // Every wait is bounded: a pipeline that stops making progress sets the context's status word,
 // raises the CTA's abort flag, lets all roles fall through to the common exit and frees its TMEM.
