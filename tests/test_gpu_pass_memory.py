@@ -80,3 +80,34 @@ def test_long_prompts_without_memory_for_long_passes(backend, weights):
     assert guarded_rel_err(run.prefill(prompt), want) <= REL_TOL
     run.close()
     batch.close()
+
+
+def test_long_prompt_without_memory_for_the_tiled_attention(backend):
+    """The tiled prompt attention writes its operands to the GEMM's scratch, which has to grow for a prompt of 30000 positions.  Without memory for that the prompt
+    goes through the attention of short prompts."""
+    cfg = ModelConfig(dim=512, n_layers=1, n_heads=2, n_kv_heads=1, head_dim=128, vocab_size=512, ff_dim=512, max_seq_len=30016)
+    weights = synth.synthetic_model(cfg, seed=102, std=0.05, linear=DType.Q4_K)
+    prompt = synth.tokens(4, 30000, cfg.vocab_size)
+    own = CudaB200Backend(0)  # (a context whose scratch has not grown)
+    run = CudaTransformerRunner(own, cfg, weights, fused=1)
+    run.prefill(prompt[:3000])
+    run.reset()
+    taken = []
+    for size in (1 << 34, 1 << 30, 1 << 26, 1 << 22):
+        while free_bytes() > size + (16 << 20):
+            try:
+                taken.append(backend.allocate(size))
+            except YuleGpuError:
+                break
+    try:
+        got = run.prefill(prompt)
+    finally:
+        for h in taken:
+            backend.free(h)
+    run.reset()
+    before = free_bytes()
+    want = run.prefill(prompt)
+    assert before - free_bytes() >= 36 << 20  # it grew only now
+    assert guarded_rel_err(got, want) <= REL_TOL
+    run.close()
+    own.close()

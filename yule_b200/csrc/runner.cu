@@ -1017,6 +1017,7 @@ struct RowsPass {
     // otherwise: prompt tokens at positions pos0, pos0 + 1, … of the runner's caches, or (n_seq > 0) of the caches of n_seq
     // sequences of the decode batch, n_live / n_seq rows each
     uint32_t pos0 = 0, n_seq = 0;
+    bool tiles = true;         // false: no scratch for the tiled prompt attention at these positions (at most kPrefillChunk rows then)
 };
 
 cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t *launches) {
@@ -1259,7 +1260,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
             const uint32_t n_seq = ps.n_seq ? ps.n_seq : 1, n_tok = ps.n_live / n_seq;
             ok(launch_rope_kv_write_batch(r->pf_q, r->pf_k, r->pf_v, kc, vc, r->rope_cos, r->rope_sin, ps.pos0, ps.n_live, hd,
                                           c.n_heads / N, c.n_kv_heads / N, s, launches, nullptr, cache_stride, n_tok));
-            if (ps.n_seq || ps.n_live > kPrefillChunk || attn_prefill_preferred(hd, c.n_heads / N, c.n_kv_heads / N, n_tok, n_seq, ps.pos0, sms)) {
+            if (ps.tiles && (ps.n_seq || ps.n_live > kPrefillChunk || attn_prefill_preferred(hd, c.n_heads / N, c.n_kv_heads / N, n_tok, n_seq, ps.pos0, sms))) {
                 AttnPrefill ap;
                 ap.q = r->pf_q;
                 ap.k_cache = kc;
@@ -1349,10 +1350,11 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
     cudaStream_t s = ctx->stream;
     int32_t rc;
     if ((rc = ensure_chunk_buffers(r, n < prefill_max_rows() ? n : prefill_max_rows()))) return rc;
-    if ((rc = ensure_gemm_scratch(ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(r->cfg.head_dim, r->pos + n)))) return rc;  // (from some 30000 positions on)
+    // More scratch from some 30000 positions on.  Without memory for it the prompt goes through the attention that needs none, in passes of the rows that has its buffers for.
+    const bool tiles = ensure_gemm_scratch(ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(r->cfg.head_dim, r->pos + n)) == YULE_OK;
     YULE_CUDA_TRY(cudaStreamSynchronize(s));  // staging words may still be in flight
     if ((rc = ensure_pinned(r, n))) return rc;
-    const uint32_t C = r->pf_chunk;
+    const uint32_t C = tiles || r->pf_chunk < kPrefillChunk ? r->pf_chunk : kPrefillChunk;
     uint64_t launches = 0;
     struct Guard {
         yule_cuda_ctx *ctx;
@@ -1368,6 +1370,7 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
         ps.n_live = m;
         ps.tokens = r->pf_tokens + c0;
         ps.pos0 = r->pos + c0;
+        ps.tiles = tiles;
         cudaError_t e = enqueue_rows_pass(r, ps, &launches);
         if (e != cudaSuccess) return fail_cuda(e, "batched prefill");
         // tensor parallelism: a peer that stopped answering is noticed per chunk
