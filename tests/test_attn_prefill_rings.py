@@ -1,7 +1,10 @@
 """The hand-offs of the prompt attention (csrc/attn_prefill.cu) under random interleavings, on the CPU: two buffers of K, of scores and of
-probabilities by tile parity, one of V and one of output, waits that know a phase's parity only, MMAs that run in the order of their issue some time after it."""
+probabilities by tile parity, one of V and one of output, waits that know a phase's parity only, MMAs that run in the order of their issue some time after it; and,
+byte by byte, the shared memory through which the two soft-max warps of a row exchange its largest score, and hand on its sum at the end."""
 
+import os
 import random
+import re
 
 import pytest
 
@@ -9,9 +12,47 @@ from test_gemm_rings import Barrier
 
 WARPS, SOFT = 4, 8  # warps that read the output; that make probabilities
 
+with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "yule_b200", "csrc", "attn_prefill.cu")) as f:
+    SOURCE = f.read()
 
-def simulate(seed, n, o_waits=True, alpha_waits=True):
+
+def exchange_of_the_source():
+    """Bytes of a row's largest score, where it lies (b: tile parity), and how many threads meet before the sums are stored over them."""
+    kind, = re.findall(r"unsigned short \*most_row = reinterpret_cast<(unsigned short) \*>\(sum_row\)", SOURCE)
+    index, = re.findall(r"most_row\[([^\]]*)\] = ", SOURCE)
+    meet = re.findall(r"bar\.sync (?:%0|\d+), (\d+);", SOURCE[:SOURCE.index("sum_row[half * kRows + r] = l;")])[-1]
+    return {"unsigned short": 2}[kind], index, int(meet)
+
+
+class Meeting:
+    """bar.sync of so many warps."""
+
+    def __init__(self, warps):
+        self.warps, self.here, self.over = warps, 0, 0
+
+    def meet(self):
+        mine = self.over
+        self.here += 1
+        if self.here == self.warps:
+            self.here, self.over = 0, self.over + 1
+        return lambda: self.over > mine
+
+
+def simulate(seed, n, o_waits=True, alpha_waits=True, exchange=exchange_of_the_source()):
     rng = random.Random(seed)
+    size, index, last_meeting = exchange
+    place = lambda b, half, r: size * eval(index, {"b": b, "half": half, "kRows": 128, "r": r})  # noqa: E731
+    memory = [None] * 1024
+    pairs = [Meeting(2) for _ in range(4)]
+    last = [Meeting(8)] * 4 if last_meeting == 256 else pairs
+    assert last_meeting in (64, 256)
+
+    def store(at, width, what):
+        memory[at:at + width] = [what] * width
+
+    def check(at, width, what):
+        assert memory[at:at + width] == [what] * width, f"{what} read, there is {memory[at:at + width]}"
+
     pair = lambda c: [Barrier(c), Barrier(c)]  # noqa: E731
     k_full, k_empty, s_full, s_empty, v_full, v_empty = pair(1), pair(1), pair(1), pair(SOFT), [Barrier(1)], [Barrier(1)]
     p_full, p_empty, a_empty, o_full, o_empty, l_full = pair(SOFT), pair(1), pair(WARPS), Barrier(2), Barrier(WARPS), Barrier(SOFT)
@@ -68,10 +109,18 @@ def simulate(seed, n, o_waits=True, alpha_waits=True):
                 o_full.arrive()
 
     def softmax(w):
+        quarter, half = w & 3, w >> 2
+        rows = (quarter * 32, quarter * 32 + 17, quarter * 32 + 31)
         for j in range(n):
             b = j & 1
             yield lambda: s_full[b].over(j >> 1 & 1)
             assert scores[b] == j
+            for r in rows:
+                store(place(b, half, r), size, ("largest", j, half, r))
+            yield pairs[quarter].meet()
+            yield lambda: True
+            for r in rows:
+                check(place(b, half ^ 1, r), size, ("largest", j, half ^ 1, r))
             yield lambda: p_empty[b].over(j >> 1 & 1 ^ 1)
             if alpha_waits:
                 yield lambda: a_empty[b].over(j >> 1 & 1 ^ 1)
@@ -84,6 +133,9 @@ def simulate(seed, n, o_waits=True, alpha_waits=True):
             yield lambda: True
             probs[b][w] = j
             p_full[b].arrive()
+        yield last[quarter].meet()
+        for r in rows:
+            store(4 * (half * 128 + r), 4, ("sum", half, r))
         l_full.arrive()
 
     def sums(w):
@@ -98,6 +150,9 @@ def simulate(seed, n, o_waits=True, alpha_waits=True):
             out_readers += 1
             o_empty.arrive()
         yield lambda: l_full.over(0)
+        for r in (w * 32, w * 32 + 17, w * 32 + 31):
+            for half in (0, 1):
+                check(4 * (half * 128 + r), 4, ("sum", half, r))
 
     roles = [issue()] + [softmax(w) for w in range(SOFT)] + [sums(w) for w in range(WARPS)] + [load(x) for x in "kv"]
     waits = {r: next(r, None) for r in roles}
@@ -126,3 +181,10 @@ def test_the_model_catches_a_missing_wait(missing):
     with pytest.raises(AssertionError):
         for seed in range(300):
             simulate(seed, 8, **{missing: False})
+
+
+def test_the_model_catches_sums_over_the_largest_scores_of_other_rows():
+    """Scores in 16 bits under sums in 32, and only the two warps of a row meet in between."""
+    with pytest.raises(AssertionError, match="read, there is"):
+        for seed in range(300):
+            simulate(seed, 4, exchange=(2, "(b * 2 + half) * kRows + r", 64))

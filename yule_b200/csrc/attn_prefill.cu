@@ -525,8 +525,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full + 8 * b);
         }
-        // (the last tile's largest scores are not needed any more once both warps are past its barrier: those of the other parity never again)
-        asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
+        // The sums lie over the largest scores, and a row's over those of other rows: not before all eight warps have read the last tile's.
+        asm volatile("bar.sync 5, 256;" ::: "memory");
         sum_row[half * kRows + r] = l;
         __syncwarp();
         if (lane == 0) mbar_arrive(l_full);
