@@ -17,11 +17,12 @@ with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__)
 
 
 def exchange_of_the_source():
-    """Bytes of a row's largest score, where it lies (b: tile parity), and how many threads meet before the sums are stored over them."""
-    kind, = re.findall(r"unsigned short \*most_row = reinterpret_cast<(unsigned short) \*>\(sum_row\)", SOURCE)
+    """Bytes of a row's largest score, where it lies (b: tile parity), whether the two warps meet again after reading, and how many threads meet before the sums are stored over them."""
+    kind, = re.findall(r"(unsigned short|float) \*most_row = ", SOURCE)
     index, = re.findall(r"most_row\[([^\]]*)\] = ", SOURCE)
-    meet = re.findall(r"bar\.sync (?:%0|\d+), (\d+);", SOURCE[:SOURCE.index("sum_row[half * kRows + r] = l;")])[-1]
-    return {"unsigned short": 2}[kind], index, int(meet)
+    read, end, sums = SOURCE.index("const float mx = "), SOURCE.index("mbar_arrive(p_full"), SOURCE.index("sum_row[half * kRows + r] = l;")
+    meet = re.findall(r"bar\.sync (?:%0|\d+), (\d+);", SOURCE[end:sums])
+    return {"unsigned short": 2, "float": 4}[kind], index, "bar.sync" in SOURCE[read:end], int(meet[-1]) if meet else 0
 
 
 class Meeting:
@@ -40,12 +41,12 @@ class Meeting:
 
 def simulate(seed, n, o_waits=True, alpha_waits=True, exchange=exchange_of_the_source()):
     rng = random.Random(seed)
-    size, index, last_meeting = exchange
+    size, index, again, last_meeting = exchange
     place = lambda b, half, r: size * eval(index, {"b": b, "half": half, "kRows": 128, "r": r})  # noqa: E731
     memory = [None] * 1024
     pairs = [Meeting(2) for _ in range(4)]
     last = [Meeting(8)] * 4 if last_meeting == 256 else pairs
-    assert last_meeting in (64, 256)
+    assert last_meeting in (0, 64, 256)
 
     def store(at, width, what):
         memory[at:at + width] = [what] * width
@@ -121,6 +122,8 @@ def simulate(seed, n, o_waits=True, alpha_waits=True, exchange=exchange_of_the_s
             yield lambda: True
             for r in rows:
                 check(place(b, half ^ 1, r), size, ("largest", j, half ^ 1, r))
+            if again:
+                yield pairs[quarter].meet()
             yield lambda: p_empty[b].over(j >> 1 & 1 ^ 1)
             if alpha_waits:
                 yield lambda: a_empty[b].over(j >> 1 & 1 ^ 1)
@@ -133,7 +136,8 @@ def simulate(seed, n, o_waits=True, alpha_waits=True, exchange=exchange_of_the_s
             yield lambda: True
             probs[b][w] = j
             p_full[b].arrive()
-        yield last[quarter].meet()
+        if last_meeting:
+            yield last[quarter].meet()
         for r in rows:
             store(4 * (half * 128 + r), 4, ("sum", half, r))
         l_full.arrive()
@@ -183,8 +187,11 @@ def test_the_model_catches_a_missing_wait(missing):
             simulate(seed, 8, **{missing: False})
 
 
-def test_the_model_catches_sums_over_the_largest_scores_of_other_rows():
-    """Scores in 16 bits under sums in 32, and only the two warps of a row meet in between."""
+@pytest.mark.parametrize("exchange", [
+    (2, "(b * 2 + half) * kRows + r", False, 64),  # scores in 16 bits under sums in 32, and only the two warps of a row meet in between
+    (4, "half * kRows + r", False, 64),            # a row's own words, stored again before they are read
+])
+def test_the_model_catches_stores_over_what_is_still_to_be_read(exchange):
     with pytest.raises(AssertionError, match="read, there is"):
         for seed in range(300):
-            simulate(seed, 4, exchange=(2, "(b * 2 + half) * kRows + r", 64))
+            simulate(seed, 4, exchange=exchange)

@@ -94,6 +94,55 @@ def test_prompt_attention_error(backend, heads, kv_heads, head_dim):
     assert error <= 8 * 2.0 ** -24, error
 
 
+@pytest.mark.parametrize("offset", [1000, -1000, 2100, 4200, -4200, 8000])
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (4, 1, 128)])
+def test_prompt_attention_with_large_scores(backend, heads, kv_heads, head_dim, offset):
+    """Scores of N(0, 1) beside a constant in the thousands, the same for all positions, which cancels in the soft-max.  As in test_prompt_attention_error, but the
+    hidden states are +1 and -1, so that their norm is the same for all tokens, and one channel of a head is +1 in all of them, has a large weight in the norm and belongs
+    to the pair that RoPE all but leaves alone.  The bound: a score rounded to 24 bits moves its probability by up to |offset| units of 2^-24, once where it is added up and
+    once where it is scaled; 8 units as without the constant.  (2 to 6 units where every position prefers itself, 26 to 104 where it prefers all others.)"""
+    n, dim, kv = 700, 512, kv_heads * head_dim
+    cfg = ModelConfig(dim=dim, n_layers=2, n_heads=heads, n_kv_heads=kv_heads, head_dim=head_dim, vocab_size=800, ff_dim=512, max_seq_len=768, rope_freq_base=1e30)
+    weights = synth.synthetic_model(cfg, seed=94, std=0.06, linear=DType.Q8_0, token_embd=DType.Q8_0)
+    channels = np.arange(kv_heads) * head_dim + head_dim - 1
+    x = np.where(np.random.default_rng(95).random((cfg.vocab_size, dim)) < 0.5, -1, 1).astype(np.int8)
+    x[:, channels] = 1
+    embd = np.zeros((cfg.vocab_size, dim // 32, 34), np.uint8)
+    embd[:, :, :2] = np.array([1.0], np.float16).view(np.uint8)
+    embd[:, :, 2:] = x.view(np.uint8).reshape(cfg.vocab_size, dim // 32, 32)
+    weights["token_embd.weight"] = (embd.reshape(-1), DType.Q8_0)
+    group, sign = heads // kv_heads, np.sign(offset)
+    for layer in range(2):
+        name = f"blk.{layer}."
+        weights[name + "attn_q.weight"] = unit_rows([r // (group * head_dim) * head_dim + r % head_dim for r in range(dim)], dim, sign)
+        weights[name + "attn_k.weight"] = unit_rows(range(kv), dim)
+        weights[name + "attn_v.weight"] = unit_rows(range(dim - kv, dim) if layer == 0 else [r // head_dim * group * head_dim + r % head_dim for r in range(kv)], dim)
+        weights[name + "attn_output.weight"] = unit_rows(range(dim), dim, 32.0)
+        weights[name + "ffn_down.weight"] = (np.zeros(dim * cfg.ff_dim // 32 * 34, np.uint8), DType.Q8_0)
+        for norm in ("attn_norm", "ffn_norm"):
+            w = np.ones(dim, np.float32)
+            if norm == "attn_norm" and layer == 0:
+                w[channels] = np.sqrt(abs(offset) * np.sqrt(head_dim))
+            weights[name + norm + ".weight"] = (w.view(np.uint8), DType.F32)
+    run = CudaTransformerRunner(backend, cfg, weights, fused=1)
+    prompt = synth.tokens(96, n, cfg.vocab_size)
+    run.prefill(prompt)
+    m = n - 1  # the last token goes through the token step
+    k, v, out = (backend.download(run.buffer(which, layer), n * kv).astype(np.float64).reshape(n, kv_heads, head_dim)[:m]
+                 for which, layer in (("k_cache", 0), ("v_cache", 0), ("v_cache", 1)))
+    run.close()
+    s = np.einsum("ihd,jhd->hij", sign * k, k) / np.sqrt(head_dim)
+    assert abs(s - offset).max() < 0.02 * abs(offset)
+    s[:, np.arange(m)[:, None] < np.arange(m)] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    att = np.einsum("hij,jhd->ihd", p / p.sum(-1, keepdims=True), v)
+    hidden = x[prompt[:m]].astype(np.float64) + 32 * np.repeat(att, group, axis=1).reshape(m, dim)
+    normed = hidden / np.sqrt((hidden ** 2).mean(-1, keepdims=True) + cfg.norm_eps)
+    want = normed.reshape(m, kv_heads, group, head_dim)[:, :, 0]
+    error = np.linalg.norm(out - want) / np.linalg.norm(want)
+    assert error <= (8 + 2 * abs(offset)) * 2.0 ** -24, error
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (8, 2, 128)])
 @pytest.mark.parametrize("size", ["infinite", "huge"])
 def test_later_tokens_do_not_reach_earlier_ones(backend, oracle, heads, kv_heads, head_dim, size):

@@ -135,7 +135,7 @@ struct Layout {
     static constexpr uint32_t kVPlane = kKeys * HD * 2;   // two
     static constexpr uint32_t kTile = 3 * kKPlane + 2 * kVPlane;  // in memory
     static constexpr uint32_t kOffK = 3 * kQPlane, kOffV = kOffK + 2 * 3 * kKPlane, kOffRows = kOffV + 2 * kVPlane;  // two buffers of K, one of V
-    // per row: alpha (two tiles), soft-max sums of both halves (before them, in 16 bits, their largest scores: two tiles), score factor; then barriers
+    // per row: alpha (two tiles), soft-max sums of both halves (before them, in the same words, their largest scores), score factor; then barriers
     static constexpr uint32_t kOffBars = kOffRows + 5 * kRows * 4;
     static constexpr uint32_t kSmem = kOffBars + 24 * 8 + 16;
     // tensor memory columns: two buffers of scores (product of the first terms | all others), output, two buffers of probabilities (hi, lo)
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
     yule_pdl_launch_dependents();
 
     float *alpha_row = reinterpret_cast<float *>(smem + L::kOffRows), *sum_row = alpha_row + 2 * kRows, *factor_row = sum_row + 2 * kRows;
-    unsigned short *most_row = reinterpret_cast<unsigned short *>(sum_row);
+    float *most_row = sum_row;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kOffBars);
     const uint32_t bar0 = smem_u32(bars);
     // pairs by tile parity: K there, free; scores there, free; probabilities there, free; alpha free; else one: V there, free; output there, free; sums there
@@ -445,12 +445,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
                     mx4[(i & 2) + 1] = fmaxf(mx4[(i & 2) + 1], s.y);
                 }
             }
-            // What is subtracted need not be the largest score itself, only the same for both halves and no smaller: the upper sixteen bits, rounded up.
-            const uint32_t bits = __float_as_uint(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])));
-            const uint32_t up = (bits + ((bits >> 31) ? 0u : 0xFFFFu)) >> 16;
-            most_row[(b * 2 + half) * kRows + r] = (unsigned short)up;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");  // the warps of both halves of these rows
-            const float mx = fmaxf(__uint_as_float(up << 16), __uint_as_float((uint32_t)most_row[(b * 2 + (half ^ 1u)) * kRows + r] << 16));
+            // The largest score itself, in all its bits: sixteen of them, rounded up, are 2^-7 of a score too much, and with scores in the thousands nothing of a
+            // probability is left in fp16.  One word per half and row has to do (there is no room for those of two tiles), so the warps of both halves meet twice.
+            const float most = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            most_row[half * kRows + r] = most;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
+            const float mx = fmaxf(most, most_row[(half ^ 1u) * kRows + r]);
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
             const float mn = mx < -3e38f ? m : fmaxf(m, mx * f);  // (no position of the tile that the row sees)
             const float alpha = expf(m - mn);
             m = mn;
@@ -525,8 +526,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_kernel(const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full + 8 * b);
         }
-        // The sums lie over the largest scores, and a row's over those of other rows: not before all eight warps have read the last tile's.
-        asm volatile("bar.sync 5, 256;" ::: "memory");
+        // (over the largest scores of this row and half, which the other half's warp has read)
         sum_row[half * kRows + r] = l;
         __syncwarp();
         if (lane == 0) mbar_arrive(l_full);
