@@ -44,6 +44,42 @@ def test_arguments_as_ctypes_takes_them(name):
             assert got[0] == got[1], (at, value, got)
 
 
+class Parameter:
+    def __init__(self, value):
+        self._as_parameter_ = value
+
+
+class Odd:
+    def __index__(self):
+        raise ValueError("no number")
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_arguments_that_only_ctypes_knows(name):
+    """Numbers of ctypes' types and objects that stand for another one, in every place, the context's and the host pointer's among them."""
+    fast, slow = getattr(_lib.calls(), name), getattr(_lib.cuda_lib(), name)
+    types = _lib._SIGNATURES[name]
+    zeros = [None] + [0.0 if t is _lib.f32 else 0 for t in types[1:]]
+    assert fast(*[t(0) for t in types]) == slow(*zeros) != 0
+    taken = 0
+    for at in range(len(types)):
+        for value in (ctypes.c_uint32(5), ctypes.c_uint64(5), ctypes.c_int32(5), ctypes.c_size_t(5), ctypes.c_float(2), ctypes.c_void_p(0), Parameter(0), Parameter(types[at](0)), Parameter(Parameter(0)),
+                      Parameter("x"), Odd()):
+            args = list(zeros)
+            args[at] = value
+            if at == 0 and isinstance(value, ctypes.c_void_p) is False and not isinstance(value, Parameter):
+                continue  # (an address that is none)
+            got = []
+            for f in (fast, slow):
+                try:
+                    got.append(f(*args))
+                except ctypes.ArgumentError:
+                    got.append("refused")
+            assert got[0] == got[1], (at, value, got)
+            taken += got[0] != "refused"
+    assert taken >= 2 * len(types)
+
+
 @pytest.mark.parametrize("name", NAMES)
 def test_the_number_of_arguments(name):
     with pytest.raises(TypeError):

@@ -2,8 +2,8 @@
  *
  * Through ctypes such a call spends 0.9 us on its way to the library (finding the function, converting six to nine arguments one object at a time), as
  * long as half a kernel launch; here 0.2.  Arguments are taken as ctypes takes them for the declared types: integers modulo 2^32 or 2^64 from anything
- * that is an index; floats from anything that converts; None is a null pointer; what ctypes refuses raises ctypes.ArgumentError.  The interpreter
- * lock is released during the call, as ctypes does. */
+ * that is an index; floats from anything that converts; None is a null context.  A call with any other argument (ctypes' own numbers, objects with an
+ * _as_parameter_, what nothing takes) goes through ctypes, which takes or refuses it.  The interpreter lock is released during the call, as ctypes does. */
 
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -11,16 +11,18 @@
 
 #include "yule_cuda.h"
 
-static PyObject *argument_error;
-
-static int refuse(Py_ssize_t at, const char *what, PyObject *v) {
+static PyObject *through_ctypes(const char *name, PyObject *const *args, Py_ssize_t n) {
     PyErr_Clear();
-    PyErr_Format(argument_error, "argument %zd: TypeError: %s instead of %s instance", at + 1, what, Py_TYPE(v)->tp_name);
-    return 0;
+    PyObject *module = PyImport_ImportModule("yule_b200._lib"), *lib = module ? PyObject_CallMethod(module, "cuda_lib", NULL) : NULL;
+    PyObject *function = lib ? PyObject_GetAttrString(lib, name) : NULL, *rc = function ? PyObject_Vectorcall(function, args, (size_t)n, NULL) : NULL;
+    Py_XDECREF(function);
+    Py_XDECREF(lib);
+    Py_XDECREF(module);
+    return rc;
 }
 static int whole(PyObject *const *args, Py_ssize_t at, uint64_t *to) {
     PyObject *v = args[at], *index = PyLong_Check(v) ? Py_NewRef(v) : PyNumber_Index(v);
-    if (!index) return refuse(at, "int expected", v);
+    if (!index) return 0;
     *to = PyLong_AsUnsignedLongLongMask(index);
     Py_DECREF(index);
     return 1;
@@ -33,7 +35,7 @@ static int context(PyObject *const *args, yule_cuda_ctx **to) {
 }
 static int real(PyObject *const *args, Py_ssize_t at, float *to) {
     const double v = PyFloat_AsDouble(args[at]);
-    if (v == -1.0 && PyErr_Occurred()) return refuse(at, "float expected", args[at]);
+    if (v == -1.0 && PyErr_Occurred()) return 0;
     *to = (float)v;
     return 1;
 }
@@ -51,9 +53,11 @@ static int count(Py_ssize_t got, Py_ssize_t want) {
         float f = 0;                                                              \
         int32_t rc;                                                               \
         (void)self;                                                               \
-        if (!count(n, N) || !context(args, &ctx)) return NULL;                    \
-        for (Py_ssize_t i = 1; i < N; i++)                                        \
-            if (!(i == FLOAT_AT ? real(args, i, &f) : whole(args, i, &v[i]))) return NULL; \
+        if (!count(n, N)) return NULL;                                            \
+        int ok = context(args, &ctx);                                             \
+        for (Py_ssize_t i = 1; ok && i < N; i++)                                  \
+            ok = i == FLOAT_AT ? real(args, i, &f) : whole(args, i, &v[i]);       \
+        if (!ok) return through_ctypes("yule_cuda_" #NAME, args, n);              \
         (void)f;                                                                  \
         Py_BEGIN_ALLOW_THREADS rc = CALL;                                         \
         Py_END_ALLOW_THREADS return PyLong_FromLong(rc);                          \
@@ -78,10 +82,4 @@ static PyMethodDef methods[] = {METHOD(rms_norm), METHOD(rope), METHOD(silu), ME
                                 {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", "Entry points of libyule_cuda.so without ctypes on the way.", -1, methods, NULL, NULL, NULL, NULL};
 
-PyMODINIT_FUNC PyInit__calls(void) {
-    PyObject *ctypes = PyImport_ImportModule("ctypes");
-    if (!ctypes) return NULL;
-    argument_error = PyObject_GetAttrString(ctypes, "ArgumentError");
-    Py_DECREF(ctypes);
-    return argument_error ? PyModule_Create(&module) : NULL;
-}
+PyMODINIT_FUNC PyInit__calls(void) { return PyModule_Create(&module); }
