@@ -44,6 +44,13 @@ int32_t ensure_gemm_scratch(yule_cuda_ctx *ctx, size_t bytes) {
     if (ctx->gemm_scratch_bytes >= bytes) return YULE_OK;
     if (ctx->capturing)
         return fail(YULE_ERR_INVALID_ARGUMENT, "the GEMM scratch (%zu bytes) cannot grow during graph capture", bytes);
+    // Another stream of the process may be in a capture that forbids everybody to allocate or wait.  What is done here is no part of it: allowed to this thread meanwhile, or
+    // the call would fail and end that capture.
+    struct Allowed {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        Allowed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        ~Allowed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    } allowed;
     YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     // At least twice the block before, so that all the outgrown ones together are no larger than this one.
     void *block = nullptr;
@@ -58,10 +65,10 @@ int32_t ensure_gemm_scratch(yule_cuda_ctx *ctx, size_t bytes) {
         return fail(YULE_ERR_OUT_OF_MEMORY, "cuda allocation of %zu bytes of GEMM scratch failed", bytes);
     }
     // the scratch opens with the split-column tickets of the GEMM, which the kernels expect (and leave) at zero
-    e = cudaMemset(block, 0, got < kGemmTicketBytes ? got : kGemmTicketBytes);
+    e = cudaMemsetAsync(block, 0, got < kGemmTicketBytes ? got : kGemmTicketBytes, ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(block);
-        return fail_cuda(e, "cudaMemset of the GEMM tickets");
+        return fail_cuda(e, "cudaMemsetAsync of the GEMM tickets");
     }
     if (ctx->gemm_scratch) ctx->retired_scratch.push_back(ctx->gemm_scratch);  // graphs captured earlier may still use it
     ctx->gemm_scratch = block;
