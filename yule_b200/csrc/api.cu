@@ -62,6 +62,7 @@ int32_t ensure_gemm_scratch(yule_cuda_ctx *ctx, size_t bytes) {
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation) return fail_cuda(e, "cudaMalloc of the GEMM scratch");  // (callers get by without memory, not with what else may be wrong)
         return fail(YULE_ERR_OUT_OF_MEMORY, "cuda allocation of %zu bytes of GEMM scratch failed", bytes);
     }
     // the scratch opens with the split-column tickets of the GEMM, which the kernels expect (and leave) at zero
@@ -609,7 +610,7 @@ static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight
     bool gemm = takes_gemm(ctx, a);
     if (gemm) {
         const int32_t rc = ensure_gemm_scratch(ctx, qgemm_scratch_bytes(batch, n_cols));
-        if (rc && !rows_can(a)) return rc;
+        if (rc && (rc != YULE_ERR_OUT_OF_MEMORY || !rows_can(a))) return rc;
         gemm = rc == YULE_OK;  // (no memory for its scratch: the matvec needs none)
     }
     if (gemm) {

@@ -1351,7 +1351,8 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
     int32_t rc;
     if ((rc = ensure_chunk_buffers(r, n < prefill_max_rows() ? n : prefill_max_rows()))) return rc;
     // More scratch from some 30000 positions on.  Without memory for it the prompt goes through the attention that needs none, in passes of the rows that has its buffers for.
-    const bool tiles = ensure_gemm_scratch(ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(r->cfg.head_dim, r->pos + n)) == YULE_OK;
+    if ((rc = ensure_gemm_scratch(ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(r->cfg.head_dim, r->pos + n))) && rc != YULE_ERR_OUT_OF_MEMORY) return rc;
+    const bool tiles = rc == YULE_OK;
     YULE_CUDA_TRY(cudaStreamSynchronize(s));  // staging words may still be in flight
     if ((rc = ensure_pinned(r, n))) return rc;
     const uint32_t C = tiles || r->pf_chunk < kPrefillChunk ? r->pf_chunk : kPrefillChunk;
