@@ -111,3 +111,34 @@ def test_long_prompt_without_memory_for_the_tiled_attention(backend):
     assert guarded_rel_err(got, want) <= REL_TOL
     run.close()
     own.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,n", [(2, 1, 128, 56000), (4, 4, 64, 112000)])
+def test_long_prompts_of_a_batch_without_memory_for_the_tiled_attention(backend, heads, kv_heads, head_dim, n):
+    """The same for a batch: sequence by sequence through the attention of short prompts, the same picks."""
+    cfg = ModelConfig(dim=512, n_layers=2, n_heads=heads, n_kv_heads=kv_heads, head_dim=head_dim, vocab_size=512, ff_dim=512, max_seq_len=n + 16)
+    weights = synth.synthetic_model(cfg, seed=103, std=0.05, linear=DType.Q4_K)
+    prompts = synth.tokens(5, 2 * n, cfg.vocab_size).reshape(2, n)
+    own = CudaB200Backend(0)  # (a context whose scratch has not grown)
+    run = CudaTransformerRunner(own, cfg, weights, fused=1)
+    run.generate_greedy_batch(prompts[:, :3000], 1)
+    taken = []
+    for size in (1 << 34, 1 << 30, 1 << 26, 1 << 22):
+        while free_bytes() > size + (16 << 20):
+            try:
+                taken.append(backend.allocate(size))
+            except YuleGpuError:
+                break
+    try:
+        run.reset_batch()
+        got = run.generate_greedy_batch(prompts, 8)
+        odd = run.generate_greedy_batch(prompts[:, :n // 512 * 512 - 510], 8)  # (the last pass has one token of each sequence)
+    finally:
+        for h in taken:
+            backend.free(h)
+    before = free_bytes()
+    assert np.array_equal(run.generate_greedy_batch(prompts, 8), got)
+    assert before - free_bytes() >= 36 << 20  # it grew only now
+    assert np.array_equal(run.generate_greedy_batch(prompts[:, :n // 512 * 512 - 510], 8), odd)
+    run.close()
+    own.close()

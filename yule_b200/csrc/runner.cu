@@ -1017,7 +1017,7 @@ struct RowsPass {
     // otherwise: prompt tokens at positions pos0, pos0 + 1, … of the runner's caches, or (n_seq > 0) of the caches of n_seq
     // sequences of the decode batch, n_live / n_seq rows each
     uint32_t pos0 = 0, n_seq = 0;
-    bool tiles = true;         // false: no scratch for the tiled prompt attention at these positions (at most kPrefillChunk rows then)
+    bool tiles = true;         // false: no scratch for the tiled prompt attention at these positions (at most kPrefillChunk rows of a sequence then)
 };
 
 cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t *launches) {
@@ -1243,6 +1243,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         flush();
         AttnDecode a;
         bool tiled = false;  // the queries share K / V tiles
+        uint32_t launches_of = 1;  // sequences, where a prompt's rows go sequence by sequence
         if (ps.batch) {
             // rotation, KV append and attention in one launch, each sequence at its own position
             a.k_new = r->pf_k;
@@ -1260,6 +1261,7 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
             const uint32_t n_seq = ps.n_seq ? ps.n_seq : 1, n_tok = ps.n_live / n_seq;
             ok(launch_rope_kv_write_batch(r->pf_q, r->pf_k, r->pf_v, kc, vc, r->rope_cos, r->rope_sin, ps.pos0, ps.n_live, hd,
                                           c.n_heads / N, c.n_kv_heads / N, s, launches, nullptr, cache_stride, n_tok));
+            // (Prompts of a batch take the tiles whatever their length: the other kernels know one sequence's prompt, and take a launch for each.)
             if (ps.tiles && (ps.n_seq || ps.n_live > kPrefillChunk || attn_prefill_preferred(hd, c.n_heads / N, c.n_kv_heads / N, n_tok, n_seq, ps.pos0, sms))) {
                 AttnPrefill ap;
                 ap.q = r->pf_q;
@@ -1284,9 +1286,10 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
                 ok(launch_attn_prefill(ap, s, launches));
                 tiled = true;
             }
-            a.k_cache = L.k_cache;
-            a.v_cache = L.v_cache;
+            a.k_cache = kc;
+            a.v_cache = vc;
             a.seq_len = ps.pos0 + 1;  // query z attends to positions [0, pos0 + z]
+            launches_of = n_seq;
         }
         a.q = r->pf_q;
         a.out = r->pf_att + (size_t)R * qdim_l;
@@ -1299,19 +1302,25 @@ cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t 
         a.n_splits = r->pf_splits;
         a.max_seq_len = c.max_seq_len;
         a.gqa = true;
-        a.n_tokens = ps.n_live;
+        a.n_tokens = ps.n_live / launches_of;
         a.q_stride = qdim_l;
         a.out_stride = qdim;
         a.settled = ps.batch;
         // Queries of a prompt share no tiles but are many, and then it is not latency that counts: the splits take fewer instructions per position.  us a pass
         // after so many positions, clusters, splits, 30 / 90 tokens: 11 layers of the 1.1B shape after 0 813, 818 / 1354, 1362 (60 tokens 1066, 1096), after 100 895, 872 / 1503,
         // 1452, after 1900 1417, 1268 / 3007, 2328; 6 layers of the 8B shape after 0 574, 582 / 980, 947, after 1900 1238, 992 / 2622, 1918, after 3800 1829, 1285 / 4194, 2642.
-        const bool splits = knob("YULE_CUDA_ROWS_SPLITS") ? atoi(knob("YULE_CUDA_ROWS_SPLITS")) != 0 : (uint64_t)(ps.pos0 + ps.n_live) * hd > 96 * 64;
-        if (!tiled && !ps.batch && splits) {
-            a.min_chunk = kPrefillMinChunk;
-            ok(launch_attn_decode(a, s, launches));
-        } else if (!tiled) {
-            ok(launch_attn_cluster(a, sms, s, launches));
+        const bool splits = knob("YULE_CUDA_ROWS_SPLITS") ? atoi(knob("YULE_CUDA_ROWS_SPLITS")) != 0 : (uint64_t)(ps.pos0 + a.n_tokens) * hd > 96 * 64;
+        for (uint32_t i = 0; !tiled && i < launches_of; i++) {
+            if (!ps.batch && splits) {
+                a.min_chunk = kPrefillMinChunk;
+                ok(launch_attn_decode(a, s, launches));
+            } else {
+                ok(launch_attn_cluster(a, sms, s, launches));
+            }
+            a.q += (size_t)a.n_tokens * qdim_l;
+            a.out += (size_t)a.n_tokens * qdim;
+            a.k_cache += cache_stride;
+            a.v_cache += cache_stride;
         }
         exchange(r->xb_att, qdim_l, qdim);
         prep(r->pf_att, qdim, nullptr, nullptr);
@@ -2033,7 +2042,10 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
     uint32_t per_seq = (r->xchg || !prefill_max_rows() ? r->pf_chunk : prefill_max_rows()) / batch;  // prompt tokens of each sequence per pass
     per_seq = per_seq < 1 ? 1 : (per_seq > fed ? fed : per_seq);
     if (fed && (rc = ensure_chunk_buffers(r, per_seq * batch))) return rc;
-    if (fed && (rc = ensure_gemm_scratch(r->ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(c.head_dim, fed)))) return rc;
+    // (as for a single prompt: without memory for more scratch, the attention that needs none)
+    if (fed && (rc = ensure_gemm_scratch(r->ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(c.head_dim, fed))) && rc != YULE_ERR_OUT_OF_MEMORY) return rc;
+    const bool tiles = rc == YULE_OK;
+    if (!tiles && per_seq > kPrefillChunk) per_seq = kPrefillChunk;
     if (fed && per_seq * batch > r->pf_chunk) per_seq = r->pf_chunk / batch;  // (a batch is no larger than the basic chunk)
     if ((rc = ensure_batch_graph(r))) return rc;
     // prompts to the device, pass by pass, the rows of a pass in the order of the sequences
@@ -2063,6 +2075,7 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
         ps.n_live = ps.m = (fed - p0 < per_seq ? fed - p0 : per_seq) * batch;
         ps.tokens = r->bd_prompts + (size_t)p0 * batch;
         ps.pos0 = p0;
+        ps.tiles = tiles;
         if (ps.m < 8) ps.m = 8;  // the GEMM works on at least eight rows; the extra ones stay unused
         const cudaError_t e = enqueue_rows_pass(r, ps, &launches);
         if (e != cudaSuccess) {
