@@ -70,6 +70,27 @@ def test_same_bits_as_with_a_wait_after_every_call(backend, seed):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
 
 
+def test_attention_on_the_built_in_scratch(backend):
+    """It ends the chain: the matvec of what it has written waits for it.  (Some 20 us of attention, of which the matvec's start is 2.)"""
+    seq = 6000
+    q, x, y = backend.upload(synth.normal(1, DIM)), backend.upload(synth.normal(2, DIM)), backend.allocate(DIM * 4)
+    k, v = (backend.upload(synth.normal(3 + i, seq * KV * HD)) for i in range(2))
+    w = backend.upload(synth.random_quantized(DType.Q4_K, 5, DIM * DIM))
+    got = []
+    for wait in (False, True) * 20:
+        backend.copy_to_device(synth.normal(100 + len(got) // 2, DIM), q)
+        backend.rope(q, x, 7, HD, 10000.0, HEADS, HEADS)
+        backend.multihead_attention_static(q, k, v, x, HD, seq, HEADS, KV, KV * HD)
+        if wait:
+            backend.synchronize()
+        backend.quantized_matmul(w, x, y, DIM, DIM, DType.Q4_K)
+        got.append(backend.download(y, DIM))
+    for a, b in zip(got[::2], got[1::2]):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    for h in (q, x, y, k, v, w):
+        backend.free(h)
+
+
 def test_captured(backend):
     todo = steps(np.random.default_rng(77), 120)
     h, other = build(backend), build(backend)
