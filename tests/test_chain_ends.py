@@ -26,7 +26,7 @@ BODIES = dict(entry_points())
 
 
 def ends(body):
-    if re.search(r"CTX_GUARD\(ctx\)|pdl_chain = false", body):
+    if re.search(r"CTX_(GUARD|ENQUEUE)\(ctx\)|ctx->take_chain\(\)", body):
         return True
     called = set(re.findall(r"\b(\w+)\((?:ctx|r)\b", body)) & set(BODIES)
     return any(ends(BODIES[c]) for c in called)

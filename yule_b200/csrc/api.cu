@@ -40,6 +40,7 @@ int32_t fail_cuda(cudaError_t e, const char *what) {
 // Grows the context's GEMM scratch.  Not while a graph is being captured: allocation is not a
 // stream operation, so the caller must have run one call of this size before capturing.
 int32_t ensure_gemm_scratch(yule_cuda_ctx *ctx, size_t bytes) {
+    std::lock_guard<std::recursive_mutex> order(ctx->enqueue_mu);  // (not between the launches of a GEMM)
     std::lock_guard<std::mutex> lock(ctx->mu);
     if (ctx->gemm_scratch_bytes >= bytes) return YULE_OK;
     if (ctx->capturing)
@@ -110,13 +111,14 @@ bool yule_cuda_ctx::find(yule_buffer h, Buffer *out, const char *what) {
 // Also ends the chain of programmatic dependent launches: a matvec re-arms it (qmv_common), and the ops of a forward pass (CHAINED).
 #define CTX_GUARD(ctx)                                                        \
     if (!(ctx)) return fail(YULE_ERR_INVALID_ARGUMENT, "null context");       \
-    const bool _pdl_chain = (ctx)->pdl_chain;                                 \
-    (void)_pdl_chain;                                                         \
-    (ctx)->pdl_chain = false;                                                 \
-    const int _chain_n = (ctx)->chain_n;                                      \
-    (void)_chain_n;                                                           \
-    (ctx)->chain_n = 0;                                                       \
+    const yule_cuda_ctx::Chain _chain = (ctx)->take_chain();                  \
+    (void)_chain;                                                             \
     YULE_CUDA_TRY(cudaSetDevice((ctx)->device))
+// The same for entry points that launch kernels: other threads' launches come before or after all of this one's.
+#define CTX_ENQUEUE(ctx)                                                      \
+    if (!(ctx)) return fail(YULE_ERR_INVALID_ARGUMENT, "null context");       \
+    std::lock_guard<std::recursive_mutex> _order((ctx)->enqueue_mu);          \
+    CTX_GUARD(ctx)
 
 #define FIND(ctx, handle, var)  \
     Buffer var;                 \
@@ -156,7 +158,7 @@ static bool chain_goes_on(yule_cuda_ctx *ctx, bool armed, int n) {
 // `call` launches with `pdl`, which it may use, and writes `bytes` bytes at `out`.
 #define CHAINED(ctx, out, bytes, call)                                       \
     do {                                                                     \
-        const bool pdl = chain_goes_on(ctx, _pdl_chain, _chain_n);           \
+        const bool pdl = chain_goes_on(ctx, _chain.armed, _chain.n);           \
         LAUNCHED(ctx, call);                                                 \
         chain_output(ctx, out, bytes);                                       \
         (ctx)->pdl_chain = true;                                             \
@@ -341,13 +343,13 @@ int32_t yule_cuda_copy_from_device(yule_cuda_ctx *ctx, yule_buffer src, void *da
     FIND(ctx, src, s);
     if (len && !data) return fail(YULE_ERR_INVALID_ARGUMENT, "null data");
     size_t n = len < s.size ? len : s.size;
-    YULE_CUDA_TRY(read_back(ctx, s.ptr, data, n, _pdl_chain));
+    YULE_CUDA_TRY(read_back(ctx, s.ptr, data, n, _chain.armed));
     return YULE_OK;
 }
 
 int32_t yule_cuda_copy_buffer_offset(yule_cuda_ctx *ctx, yule_buffer src, yule_buffer dst, size_t src_offset,
                                      size_t dst_offset, size_t size) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, src, s);
     FIND(ctx, dst, d);
     if (src_offset > s.size || size > s.size - src_offset)
@@ -403,7 +405,7 @@ int32_t yule_cuda_set_wait_budget(yule_cuda_ctx *ctx, uint64_t cycles) {
 int32_t yule_cuda_matmul(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, yule_buffer out, uint32_t m,
                          uint32_t n, uint32_t k) {
     (void)n;
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, a, A);
     FIND(ctx, b, B);
     FIND(ctx, out, O);
@@ -417,7 +419,7 @@ int32_t yule_cuda_matmul(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, yule_
 }
 
 int32_t yule_cuda_softmax(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer output, uint32_t size) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, input, I);
     FIND(ctx, output, O);
     NEED_BYTES(I, (size_t)size * 4, "softmax input");
@@ -429,7 +431,7 @@ int32_t yule_cuda_softmax(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer out
 
 int32_t yule_cuda_rms_norm(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer weight, yule_buffer output,
                            uint32_t size, float eps) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, input, I);
     FIND(ctx, weight, W);
     FIND(ctx, output, O);
@@ -444,7 +446,7 @@ int32_t yule_cuda_rms_norm(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer we
 
 int32_t yule_cuda_rope(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k, uint32_t pos, uint32_t head_dim,
                        float freq_base, uint32_t n_heads_q, uint32_t n_heads_k) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, q, Q);
     FIND(ctx, k, K);
     if (head_dim == 0 || head_dim % 2 || head_dim > 256)
@@ -470,7 +472,7 @@ int32_t yule_cuda_rope(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k, uint32_
 }
 
 int32_t yule_cuda_silu(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer output, uint32_t size) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, input, I);
     FIND(ctx, output, O);
     NEED_BYTES(I, (size_t)size * 4, "silu input");
@@ -482,7 +484,7 @@ int32_t yule_cuda_silu(yule_cuda_ctx *ctx, yule_buffer input, yule_buffer output
 
 int32_t yule_cuda_element_mul(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, yule_buffer output,
                               uint32_t size) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, a, A);
     FIND(ctx, b, B);
     FIND(ctx, output, O);
@@ -495,7 +497,7 @@ int32_t yule_cuda_element_mul(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, 
 }
 
 int32_t yule_cuda_add(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, yule_buffer output, uint32_t size) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, a, A);
     FIND(ctx, b, B);
     FIND(ctx, output, O);
@@ -510,7 +512,7 @@ int32_t yule_cuda_add(yule_cuda_ctx *ctx, yule_buffer a, yule_buffer b, yule_buf
 int32_t yule_cuda_attn_score(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k_cache, yule_buffer scores,
                              uint32_t head_dim, uint32_t seq_len, uint32_t head_offset, uint32_t kv_offset,
                              uint32_t kv_stride) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, q, Q);
     FIND(ctx, k_cache, K);
     FIND(ctx, scores, S);
@@ -526,7 +528,7 @@ int32_t yule_cuda_attn_score(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k_ca
 int32_t yule_cuda_attn_value(yule_cuda_ctx *ctx, yule_buffer weights, yule_buffer v_cache, yule_buffer output,
                              uint32_t head_dim, uint32_t seq_len, uint32_t kv_offset, uint32_t kv_stride,
                              uint32_t out_offset) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     FIND(ctx, weights, W);
     FIND(ctx, v_cache, V);
     FIND(ctx, output, O);
@@ -572,7 +574,7 @@ static bool takes_gemm(const yule_cuda_ctx *ctx, const QmvArgs &a) {
 static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight_offset, yule_buffer input,
                           yule_buffer output, uint32_t n_rows, uint32_t n_cols, uint32_t type, uint32_t batch,
                           uint32_t x_stride, uint32_t out_stride) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     if (!is_quantized(type))
         return fail(YULE_ERR_UNSUPPORTED_DTYPE, "unsupported dtype for CUDA qmv: GGUF type %u", type);
     uint32_t bs = block_size(type);
@@ -643,14 +645,14 @@ static int32_t qmv_common(yule_cuda_ctx *ctx, yule_buffer weights, size_t weight
     const char *x_lo = (const char *)X.ptr, *x_hi = x_lo + ((size_t)(batch - 1) * x_stride + n_cols) * 4;
     const char *o_lo = (const char *)O.ptr, *o_hi = o_lo + ((size_t)(batch - 1) * out_stride + n_rows) * 4;
     bool w_hazard = false, x_hazard = false;
-    ctx->chain_n = _chain_n;  // (the guard above ended the chain for every other entry point)
+    ctx->chain_n = _chain.n;  // (the guard above ended the chain for every other entry point)
     for (int i = 0; i < ctx->chain_n; i++) {
         w_hazard = w_hazard || (w_lo < ctx->chain_hi[i] && ctx->chain_lo[i] < w_hi);
         x_hazard = x_hazard || (x_lo < ctx->chain_hi[i] && ctx->chain_lo[i] < x_hi);
     }
     bool listed = false;
     for (int i = 0; i < ctx->chain_n; i++) listed = listed || (ctx->chain_lo[i] <= o_lo && o_hi <= ctx->chain_hi[i]);
-    a.pdl = _pdl_chain && !w_hazard && (listed || ctx->chain_n < yule_cuda_ctx::kChainRanges);
+    a.pdl = _chain.armed && !w_hazard && (listed || ctx->chain_n < yule_cuda_ctx::kChainRanges);
     a.late_wait = a.pdl && !x_hazard;
     a.status = ctx->device_status;
     a.wait_cycles = ctx->wait_cycles;
@@ -688,7 +690,7 @@ int32_t yule_cuda_quantized_matmul_batched(yule_cuda_ctx *ctx, yule_buffer weigh
 
 int32_t yule_cuda_prepare_weights(yule_cuda_ctx *ctx, yule_buffer weights, uint32_t gguf_type, uint32_t n_rows,
                                   uint32_t n_cols) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     if (!is_quantized(gguf_type))
         return fail(YULE_ERR_UNSUPPORTED_DTYPE, "unsupported dtype for CUDA qmv: GGUF type %u", gguf_type);
     if (n_cols == 0 || n_cols % block_size(gguf_type))
@@ -732,7 +734,7 @@ int32_t yule_cuda_prepare_weights(yule_cuda_ctx *ctx, yule_buffer weights, uint3
 
 int32_t yule_cuda_dequantize(yule_cuda_ctx *ctx, yule_buffer weights, uint32_t gguf_type, uint64_t n_blocks,
                              yule_buffer out_f32) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     if (!is_quantized(gguf_type) && gguf_type != YULE_DTYPE_F16 && gguf_type != YULE_DTYPE_F32)
         return fail(YULE_ERR_UNSUPPORTED_DTYPE, "dequant not implemented for GGUF type %u", gguf_type);
     FIND(ctx, weights, W);
@@ -774,7 +776,7 @@ static int32_t grow_attn_scratch(yule_cuda_ctx *ctx, size_t floats, uint32_t tic
 int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_buffer k_cache, yule_buffer v_cache,
                                       yule_buffer out, uint32_t head_dim, uint32_t seq_len, uint32_t n_heads,
                                       uint32_t n_kv_heads, uint32_t kv_stride) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     if (n_kv_heads == 0 || n_heads == 0 || n_heads % n_kv_heads || head_dim == 0 || seq_len == 0)
         return fail(YULE_ERR_INVALID_ARGUMENT, "bad attention shape (heads %u, kv heads %u, head_dim %u, seq %u)",
                     n_heads, n_kv_heads, head_dim, seq_len);
@@ -841,7 +843,7 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
         a.n_kv_heads = n_kv_heads;
         a.kv_stride = kv_stride;
         a.max_seq_len = seq_len;
-        a.pdl = chain_goes_on(ctx, _pdl_chain && !grown, _chain_n);
+        a.pdl = chain_goes_on(ctx, _chain.armed && !grown, _chain.n);
         if (clustered)
             LAUNCHED(ctx, launch_attn_cluster(a, ctx->prop.multiProcessorCount, ctx->stream, &_n));
         else
@@ -858,7 +860,7 @@ int32_t yule_cuda_multihead_attention(yule_cuda_ctx *ctx, yule_buffer q, yule_bu
 
 int32_t yule_cuda_embed_gather(yule_cuda_ctx *ctx, yule_buffer table, uint32_t gguf_type, uint32_t dim,
                                uint32_t token, yule_buffer out) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     uint32_t bs = block_size(gguf_type);
     if (bs == 0) return fail(YULE_ERR_UNSUPPORTED_DTYPE, "embedding dtype %u not supported", gguf_type);
     if (dim == 0 || dim % bs) return fail(YULE_ERR_INVALID_ARGUMENT, "dim %u not a multiple of block size %u", dim, bs);
@@ -912,7 +914,7 @@ int32_t yule_cuda_graph_end(yule_cuda_ctx *ctx, uint32_t *out_graph_id) {
 }
 
 int32_t yule_cuda_graph_launch(yule_cuda_ctx *ctx, uint32_t graph_id) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     yule_cuda_ctx::Graph g;
     {
         std::lock_guard<std::mutex> lock(ctx->mu);
@@ -939,7 +941,7 @@ int32_t yule_cuda_graph_destroy(yule_cuda_ctx *ctx, uint32_t graph_id) {
 // Sampler::sample_with_history (yule-infer/src/sampler.rs:17-136) on the device.
 int32_t yule_cuda_sample(yule_cuda_ctx *ctx, yule_buffer logits, uint32_t n, const yule_sampling_params *params,
                          yule_buffer previous_tokens, uint32_t n_previous, float random_value, uint32_t *out_token) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     if (!params || !out_token) return fail(YULE_ERR_INVALID_ARGUMENT, "null argument");
     if (n == 0) return fail(YULE_ERR_INVALID_ARGUMENT, "empty logits");  // sampler.rs:19-21
     if (!(random_value >= 0.0f && random_value < 1.0f)) return fail(YULE_ERR_INVALID_ARGUMENT, "the random value must lie in [0, 1)");
@@ -967,6 +969,7 @@ int32_t yule_cuda_sample(yule_cuda_ctx *ctx, yule_buffer logits, uint32_t n, con
     a.scratch = ctx->sampler_scratch;
     a.out_token = reinterpret_cast<uint32_t *>(ctx->sampler_scratch + 2 * (size_t)n);
     LAUNCHED(ctx, launch_sample(a, ctx->stream, &_n));
+    // (the word is one for all callers: read before the next one samples)
     YULE_CUDA_TRY(cudaMemcpyAsync(out_token, a.out_token, 4, cudaMemcpyDeviceToHost, ctx->stream));
     YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return YULE_OK;
@@ -1011,7 +1014,7 @@ int32_t yule_cuda_event_reset(yule_cuda_ctx *ctx) {
 }
 
 int32_t yule_cuda_flush_l2(yule_cuda_ctx *ctx) {
-    CTX_GUARD(ctx);
+    CTX_ENQUEUE(ctx);
     if (!ctx->flush_buf) {
         // Twice the L2 size, so that nothing of an earlier kernel's inputs survives.
         size_t bytes = (size_t)ctx->prop.l2CacheSize * 2;

@@ -370,7 +370,8 @@ extern "C" int32_t yule_cuda_multihead_attention_static(yule_cuda_ctx *ctx, yule
                                                         uint32_t kv_stride) {
     using namespace yule;
     if (!ctx) return fail(YULE_ERR_INVALID_ARGUMENT, "null context");
-    ctx->pdl_chain = false;  // not a launch of the ops' chain: a matvec of what it writes must not read before it waits
+    std::lock_guard<std::recursive_mutex> order(ctx->enqueue_mu);  // (tickets, then the launch that counts on them)
+    ctx->take_chain();  // not a launch of the ops' chain: a matvec of what it writes must not read before it waits
     YULE_CUDA_TRY(cudaSetDevice(ctx->device));
     if (n_kv_heads == 0 || n_heads == 0 || n_heads % n_kv_heads || head_dim == 0 || seq_len == 0)
         return fail(YULE_ERR_INVALID_ARGUMENT, "bad attention shape (heads %u, kv heads %u, head_dim %u, seq %u)", n_heads,

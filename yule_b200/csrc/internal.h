@@ -114,6 +114,21 @@ struct yule_cuda_ctx {
     static constexpr int kChainRanges = 24;  // (a layer's ops write some eleven vectors, which the next layer's write again, and two cache rows)
     const char *chain_lo[kChainRanges] = {}, *chain_hi[kChainRanges] = {};
     int chain_n = 0;
+    // Held while an entry point puts on the stream what belongs together: the launches that share the context's scratch (a GEMM is two, a pass of prompt rows
+    // some hundred), and a launch with the change of the chain above that goes with it.  Not while one waits for results or copies host memory.
+    std::recursive_mutex enqueue_mu;
+    struct Chain {
+        bool armed;
+        int n;
+    };
+    // Ends the chain; what it was, for those that go on with it (they hold enqueue_mu until they have).
+    Chain take_chain() {
+        std::lock_guard<std::recursive_mutex> lock(enqueue_mu);
+        const Chain was{pdl_chain, chain_n};
+        pdl_chain = false;
+        chain_n = 0;
+        return was;
+    }
 
     // Looks a handle up under the lock; returns false (and sets the error) when unknown.
     bool find(yule_buffer h, yule::Buffer *out, const char *what);

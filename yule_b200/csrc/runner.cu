@@ -648,7 +648,7 @@ cudaError_t enqueue_forward_graph(yule_cuda_runner *r, uint64_t *launches, bool 
 }
 
 int32_t finalize(yule_cuda_runner *r) {
-    r->ctx->pdl_chain = false;  // the runner's launches are not in the list of the ops' chain
+    r->ctx->take_chain();  // the runner's launches are not in the list of the ops' chain
     if (r->finalized) return YULE_OK;
     const yule_runner_config &c = r->cfg;
     const uint32_t N = r->ctx->tp_world ? r->ctx->tp_world : 1;
@@ -1023,6 +1023,7 @@ struct RowsPass {
 cudaError_t enqueue_rows_pass(yule_cuda_runner *r, const RowsPass &ps, uint64_t *launches) {
     const yule_runner_config &c = r->cfg;
     yule_cuda_ctx *ctx = r->ctx;
+    std::lock_guard<std::recursive_mutex> order(ctx->enqueue_mu);  // its launches hand the context's scratch on to one another
     cudaStream_t s = ctx->stream;
     const uint32_t N = ctx->tp_world > 1 ? ctx->tp_world : 1, R = N > 1 ? ctx->tp_rank : 0;
     const uint32_t dim = c.dim, hd = c.head_dim, qdim = c.n_heads * hd, kvdim = c.n_kv_heads * hd, ff = c.ff_dim;

@@ -309,8 +309,8 @@ int32_t yule_cuda_tp_init(yule_cuda_ctx *ctx, uint32_t rank, uint32_t world, con
 }
 
 int32_t yule_cuda_tp_all_gather(yule_cuda_ctx *ctx, yule_buffer buffer, size_t count_per_rank) {
-    if (ctx) ctx->pdl_chain = false;  // not a launch of the ops' chain
     if (!ctx) return fail(YULE_ERR_INVALID_ARGUMENT, "null context");
+    ctx->take_chain();  // not a launch of the ops' chain
     YULE_CUDA_TRY(cudaSetDevice(ctx->device));
     Buffer b;
     if (!ctx->find(buffer, &b, "tp_all_gather")) return YULE_ERR_UNKNOWN_BUFFER;
