@@ -32,6 +32,7 @@ struct GemmParams {
     // The first split_tiles tiles are dealt by super-blocks: their split_units = split_tiles · n_cols / 256 in equal runs to split_ctas CTAs; whole
     // tiles follow, one per CTA and round.
     uint32_t split_tiles, split_ctas, split_units;
+    uint64_t by_ctas, by_units, by_bpr, by_ntiles;  // what divides by split_ctas, split_units, n_cols / 256 and n_ntiles (see quotient)
     float *split_part;        // blocks of [bn][128] partial results: two per CTA (its runs touch at most two tiles), then one per CTA
     uint32_t *split_tickets;  // per (split tile, drain warp) the number of its parts that are stored; left at zero
     uint32_t type;         // GGUF type id of the weights (generic kernel)
@@ -252,6 +253,12 @@ struct RingPos {
     }
 };
 
+// n / d for any 32-bit n, with by = divide_by(d): ceil(2^64 / d), which is too large by less than 2^-32 of it, so that what n times it has too much never reaches
+// the next whole number; 0 stands for d = 1.  (A division by a number that is not known takes some hundred clocks, and an item has seven, some of them one after the other and
+// between its last sums and their stores: 1024x4096 by 65 rows 16.5 us with multiplications, 17.1 with divisions.)
+inline uint64_t divide_by(uint32_t d) { return d > 1 ? ~0ull / d + 1 : 0ull; }
+__device__ __forceinline__ uint32_t quotient(uint32_t n, uint64_t by) { return by ? (uint32_t)__umul64hi(by, n) : n; }
+
 // A work item: tile (row tile x activation tile) and the range of super-blocks [sb0, sb1) of its columns.
 struct Item {
     uint32_t tile, mt, nt, sb0, sb1, seg;  // mt: row tile inside matrix `seg`
@@ -268,16 +275,15 @@ struct ItemWalk {
     uint32_t step;
     __device__ __forceinline__ explicit ItemWalk(const GemmParams &p) : step((uint32_t)(blockIdx.x >= p.split_ctas) << 1) {}
     __device__ __forceinline__ bool next(const GemmParams &p, uint32_t bpr, Item &r) {
-        const uint32_t ctas = p.split_ctas > 1 ? p.split_ctas : 1;
-        const uint32_t lo = blockIdx.x * p.split_units / ctas, hi = (blockIdx.x + 1) * p.split_units / ctas;  // this CTA's run
-        const uint32_t first = lo / bpr, mid = (first + 1) * bpr;                                                // and where its first tile ends
+        const uint32_t lo = quotient(blockIdx.x * p.split_units, p.by_ctas), hi = quotient((blockIdx.x + 1) * p.split_units, p.by_ctas);  // this CTA's run
+        const uint32_t first = quotient(lo, p.by_bpr), mid = (first + 1) * bpr;                                                       // and where its first tile ends
         const bool run = step < 2, second = step == 1;
         r.tile = run ? first + step : p.split_tiles + (step - 2) * gridDim.x + blockIdx.x;
         r.sb0 = run && !second ? lo + bpr - mid : 0;
         r.sb1 = !run ? bpr : second ? hi - mid : (hi < mid ? hi : mid) + bpr - mid;
         r.part = run ? step : 0;
         step = run && hi <= mid ? 2 : step + 1;
-        r.mt = r.tile / p.n_ntiles;
+        r.mt = quotient(r.tile, p.by_ntiles);
         r.nt = r.tile - r.mt * p.n_ntiles;
         r.seg = 0;
         while (r.seg + 1 < p.n_seg && r.mt >= p.mt0[r.seg + 1]) r.seg++;
@@ -311,8 +317,30 @@ __device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi,
                                             float (&acc)[CW]) {
     const uint32_t row = wi.mt * kTileRows + lane_base + lane;
     const uint32_t n0 = wi.nt * BN + col_base;
-    float truncation = p.truncation, scale = p.out_scale;
-    bool summed = false;
+    // Four residuals are asked for before the first of their stores (which may be to the same matrix, so nothing but
+    // this order lets them overlap): one by one they took 24 us per tile, so they take 7.
+    auto store = [&](auto scaledc) {
+        constexpr bool scaled = decltype(scaledc)::value;
+#pragma unroll
+        for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
+            const float osc = !scaled && lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;  // padded to whole tiles
+#pragma unroll
+            for (uint32_t j0 = 0; j0 < 16; j0 += 4) {
+                const size_t o0 = (size_t)(n0 + c0 + j0) * p.out_stride[wi.seg] + row;
+                const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 + j0 < p.n_tokens ? p.n_tokens - (n0 + c0 + j0) : 0u;
+                float res[4];
+                if (p.residual) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < 4; j++) {
+                    const float a = acc[c0 + j0 + j], val = scaled ? a : fmaf(a, p.truncation, a) * __shfl_sync(0xffffffffu, osc, j0 + j) * p.out_scale;
+                    if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? val + res[j] : val;
+                }
+            }
+        }
+    };
     if (wi.sb1 - wi.sb0 < bpr) {
         // This item covers a part of the columns.  Every drain warp stores its block of scaled partial sums, then
         // takes a ticket of its (tile, warp); the warp that finds all the other parts stored adds them in the
@@ -321,15 +349,15 @@ __device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi,
         float *mine = part_block(p, own_part(wi), BN) + in_block;
 #pragma unroll
         for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-            const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;  // padded to whole tiles
+            const float osc = lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;
 #pragma unroll
             for (uint32_t j = 0; j < 16; j++)
-                __stcg(mine + (size_t)(c0 + j) * kTileRows, fmaf(acc[c0 + j], truncation, acc[c0 + j]) * __shfl_sync(0xffffffffu, osc, j) * scale);
+                __stcg(mine + (size_t)(c0 + j) * kTileRows, fmaf(acc[c0 + j], p.truncation, acc[c0 + j]) * __shfl_sync(0xffffffffu, osc, j) * p.out_scale);
         }
         __syncwarp();
         // the CTAs whose runs hold the tile's first and its last super-block; the first of them may have begun with the tile before
         const uint32_t u0 = wi.tile * bpr;
-        const uint32_t cta0 = ((u0 + 1) * p.split_ctas - 1) / p.split_units, n_parts = ((u0 + bpr) * p.split_ctas - 1) / p.split_units - cta0 + 1;
+        const uint32_t cta0 = quotient((u0 + 1) * p.split_ctas - 1, p.by_units), n_parts = quotient((u0 + bpr) * p.split_ctas - 1, p.by_units) - cta0 + 1;
         uint32_t ticket = 0;
         uint32_t *tk = p.split_tickets + (size_t)wi.tile * kEpiWarps + warp;
         if (lane == 0) {
@@ -340,7 +368,7 @@ __device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi,
         ticket = __shfl_sync(0xffffffffu, ticket, 0);
         if (ticket != n_parts - 1) return;
         __syncwarp();
-        const uint32_t first = 2 * cta0 + (cta0 * p.split_units / p.split_ctas < u0 ? 1u : 0u);
+        const uint32_t first = 2 * cta0 + (quotient(cta0 * p.split_units, p.by_ctas) < u0 ? 1u : 0u);
 #pragma unroll
         for (uint32_t j = 0; j < CW; j++) acc[j] = 0.f;
         // the loads of up to KS parts are in flight together; the additions keep the order of the parts
@@ -360,29 +388,10 @@ __device__ __forceinline__ void finish_item(const GemmParams &p, const Item &wi,
 #pragma unroll
                 for (uint32_t j = 0; j < CW; j++) acc[j] += v[q][j];
         }
-        summed = true, truncation = 0.f, scale = 1.f;  // the parts were scaled
+        store(std::true_type{});  // the parts were scaled
+        return;
     }
-    // Four residuals are asked for before the first of their stores (which may be to the same matrix, so nothing but
-    // this order lets them overlap): one by one they took 24 us per tile, so they take 7.
-#pragma unroll
-    for (uint32_t c0 = 0; c0 < CW; c0 += 16) {
-        const float osc = summed ? 1.f : lane < 16 ? p.oscale[n0 + c0 + lane] : 0.f;
-#pragma unroll
-        for (uint32_t j0 = 0; j0 < 16; j0 += 4) {
-            const size_t o0 = (size_t)(n0 + c0 + j0) * p.out_stride[wi.seg] + row;
-            const uint32_t live = row < p.n_rows[wi.seg] && n0 + c0 + j0 < p.n_tokens ? p.n_tokens - (n0 + c0 + j0) : 0u;
-            float res[4];
-            if (p.residual) {
-#pragma unroll
-                for (uint32_t j = 0; j < 4; j++) res[j] = j < live ? p.residual[o0 + j * p.out_stride[wi.seg]] : 0.f;
-            }
-#pragma unroll
-            for (uint32_t j = 0; j < 4; j++) {
-                const float val = fmaf(acc[c0 + j0 + j], truncation, acc[c0 + j0 + j]) * __shfl_sync(0xffffffffu, osc, j0 + j) * scale;
-                if (j < live) p.out[wi.seg][o0 + j * p.out_stride[wi.seg]] = p.residual ? val + res[j] : val;
-            }
-        }
-    }
+    store(std::false_type{});
 }
 
 }  // namespace

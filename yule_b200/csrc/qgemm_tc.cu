@@ -1247,6 +1247,10 @@ cudaError_t launch_qgemm_mm(const QGemm &g, int sm_count, cudaStream_t s, uint64
     p.n_ntiles = n_ntiles;
     const uint32_t ctas = (uint32_t)sm_count < kGemmMaxCtas ? (uint32_t)sm_count : kGemmMaxCtas, tiles = p.n_mtiles * p.n_ntiles;
     split_tiles(p, tiles, g.n_cols / 256, ctas);
+    p.by_ctas = divide_by(p.split_ctas);
+    p.by_units = divide_by(p.split_units);
+    p.by_bpr = divide_by(g.n_cols / 256);
+    p.by_ntiles = divide_by(n_ntiles);
     p.split_tickets = reinterpret_cast<uint32_t *>(g.scratch);
     p.split_part = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(g.scratch) + kGemmTicketBytes);
     p.status = g.status;
