@@ -13,9 +13,9 @@ pytestmark = pytest.mark.gpu
     (1024, 20),     # a block per CTA
     (1280, 17),     # shares of one and two blocks, padding rows
     (2304, 64),
-    (4096, 100),    # clusters of two
+    (4096, 100),    # 65 rows and more, laid out and no more: one CTA per row (the prompts below have the clusters of two)
     (4608, 250),
-    (9472, 128),    # the last size and the first that are (not) read at once on 148 SMs
+    (9472, 128),
     (9728, 128),
     (16384, 40),    # 32 warps of two rows
     (16640, 40),    # one row per CTA

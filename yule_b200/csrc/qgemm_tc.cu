@@ -1184,8 +1184,11 @@ cudaError_t launch_qgemm_xprep(const QGemm &g, int sm_count, cudaStream_t s, uin
     // A row on a cluster where it is read at once: all rows together are a CTA of 1024 threads per SM at the most (beyond: 128 rows of 14336 columns 8.7 us with one
     // CTA per row, 9.8 on clusters of four; 28672: 16.9 and 22.9), and there are not rows enough for two per SM.  Clusters of four up to 64 rows, two beyond (8192
     // columns: 32 rows 4.5 us with two, 4.1 with four, 4.2 with eight; 128 rows 5.4 and 5.3 with two and four); two rows per CTA where they fit.
+    // Not rows that are only laid out, on clusters of two, by a launch that nothing hides: its start costs more than a half row saves (a call of 128 rows and 128 rows of W,
+    // re-layout and GEMM: 1024 columns 22.3 us, 21.4 with one CTA per row, 2048 25.3, 23.5, 4096 27.1, 25.8; in a prompt's chain of launches the same or 1 % for the clusters).
     const uint32_t blocks = g.n_cols / 256, ranks = 2 * padded <= (uint32_t)sm_count ? 4 : 2, share = (blocks + ranks - 1) / ranks, most_warps = kXprepThreads / 32;
-    if (padded < 2 * (uint32_t)sm_count && (uint64_t)padded * g.n_cols <= (uint64_t)kXprepThreads * 8 * sm_count && blocks >= ranks && share <= most_warps && !(g.gate && g.norm_w)) {
+    const bool plain = !g.gate && !g.norm_w && !g.pdl && ranks == 2;
+    if (!plain && padded < 2 * (uint32_t)sm_count && (uint64_t)padded * g.n_cols <= (uint64_t)kXprepThreads * 8 * sm_count && blocks >= ranks && share <= most_warps && !(g.gate && g.norm_w)) {
         const uint32_t rows = 2 * share <= most_warps ? 2 : 1;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(padded / rows * ranks);
