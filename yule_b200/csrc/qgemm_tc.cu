@@ -1051,6 +1051,8 @@ cudaError_t launch_gemm(const GemmParams &p, const GemmMaps &w_maps, uint32_t gr
 // super-blocks of 1.8 us at 128 activation rows and 1.1 at 32.  So not where that would shorten the round by fewer than three super-blocks, and runs that
 // end inside a tile, with two parts for most CTAs, only where they shorten it by four more (128 rows) or eight (32 rows: 64 tiles of 32 super-blocks in halves
 // 21 us, in 148 equal runs 23.5; 80 tiles 31 us whole, 25 in equal runs; 448 tiles 119.5 us as four rounds, 104 as three and the rest in parts).
+// Nor runs in place of a round of whole tiles of which they spare no more than an eighth: their CTAs are at different columns, and share nothing in the caches that they
+// do not hold whole (8192x28672 by 2016 rows, 136 tiles beyond six rounds: 2291 us whole, 2354 in 148 runs; 128 tiles of 32 super-blocks 75.2, 76.3; 120 of 56 127.9, 120.6).
 void split_tiles(GemmParams &p, uint32_t tiles, uint32_t bpr, uint32_t ctas) {
     p.split_tiles = p.split_ctas = p.split_units = 0;
     const uint32_t rest = tiles % ctas, units = rest * bpr;
@@ -1063,7 +1065,7 @@ void split_tiles(GemmParams &p, uint32_t tiles, uint32_t bpr, uint32_t ctas) {
     const uint32_t equal = least(ctas, rest * most, units / run);                                         // runs that may end inside a tile
     auto longest = [&](uint32_t to) { return (units + to - 1) / to; };
     uint32_t to = even;
-    if (equal > even && longest(even) >= longest(equal) + (p.bn >= 128 ? 4u : 8u)) to = equal;
+    if (equal > even && longest(even) >= longest(equal) + (p.bn >= 128 ? 4u : 8u) && (even > rest || longest(even) > longest(equal) + bpr / 8)) to = equal;
     if (to <= rest || (run > 1 && bpr < longest(to) + 3)) return;
     p.split_tiles = rest;
     p.split_ctas = to;
