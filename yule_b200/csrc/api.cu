@@ -325,15 +325,16 @@ int32_t yule_cuda_copy_to_device(yule_cuda_ctx *ctx, const void *data, size_t le
     }
     // A pageable source has been staged when cudaMemcpyAsync returns; a pinned one has not, and the caller's slice is only borrowed for the duration of this
     // call.  Waiting for the copy takes 10 us (8 KB), so a small pinned source takes the way of a pageable one.
-    const bool pinned = is_pinned_host(data);
     constexpr size_t kStagedBytes = 64 * 1024;
-    if (pinned && n <= kStagedBytes && !ctx->capturing) {
+    bool pinned = n <= kStagedBytes && is_pinned_host(data);
+    if (pinned && !ctx->capturing) {
         alignas(64) static thread_local unsigned char pageable[kStagedBytes];
         memcpy(pageable, data, n);
         YULE_CUDA_TRY(cudaMemcpyAsync(d.ptr, pageable, n, cudaMemcpyHostToDevice, ctx->stream));
         return YULE_OK;
     }
     YULE_CUDA_TRY(cudaMemcpyAsync(d.ptr, data, n, cudaMemcpyHostToDevice, ctx->stream));
+    if (n > kStagedBytes) pinned = is_pinned_host(data);  // (asked while the copy runs)
     if (pinned) YULE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return YULE_OK;
 }
