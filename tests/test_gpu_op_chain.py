@@ -134,6 +134,19 @@ def test_copies_of_every_alignment(backend, src, dst, size):
         backend.free(h)
 
 
+@pytest.mark.parametrize("n", [1, 255, 257, 148 * 8 * 256, 148 * 8 * 256 + 1, 304127, 304128, 304129, 1 << 20, (1 << 20) + 769])
+def test_add(backend, n):
+    """One element a thread and four; into a buffer of its own and into an operand's; what lies behind stays."""
+    a, b = (synth.normal(seed, n + 40) for seed in (7, 8))
+    ha, hb, ho = backend.upload(a), backend.upload(b), backend.upload(np.full(n + 40, 3.0, np.float32))
+    backend.add(ha, hb, ho, n)
+    backend.add(ha, hb, hb, n)
+    assert np.array_equal(backend.download(ho, n + 40), np.concatenate([a[:n] + b[:n], np.full(40, 3.0, np.float32)]))
+    assert np.array_equal(backend.download(hb, n + 40), np.concatenate([a[:n] + b[:n], b[n:]]))
+    for h in (ha, hb, ho):
+        backend.free(h)
+
+
 @pytest.mark.parametrize("n", [1, 4096, 65536, 65537, 1 << 20])
 def test_a_pinned_source_may_be_overwritten_when_the_call_returns(backend, n):
     """Up to 64 KB it goes the way of a pageable one, beyond that the call waits."""
