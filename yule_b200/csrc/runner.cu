@@ -1365,7 +1365,8 @@ int32_t prefill_batched(yule_cuda_runner *r, const uint32_t *tokens, uint32_t n)
     const bool tiles = rc == YULE_OK;
     YULE_CUDA_TRY(cudaStreamSynchronize(s));  // staging words may still be in flight
     if ((rc = ensure_pinned(r, n))) return rc;
-    const uint32_t C = tiles || r->pf_chunk < kPrefillChunk ? r->pf_chunk : kPrefillChunk;
+    // (Under tensor parallelism whether it has memory or not: all ranks have to make the same passes.)
+    const uint32_t C = (tiles && !r->xchg) || r->pf_chunk < kPrefillChunk ? r->pf_chunk : kPrefillChunk;
     uint64_t launches = 0;
     struct Guard {
         yule_cuda_ctx *ctx;
@@ -2046,7 +2047,7 @@ int32_t yule_cuda_runner_generate_greedy_batch(yule_cuda_runner *r, const uint32
     // (as for a single prompt: without memory for more scratch, the attention that needs none)
     if (fed && (rc = ensure_gemm_scratch(r->ctx, kGemmTicketBytes + attn_prefill_scratch_bytes(c.head_dim, fed))) && rc != YULE_ERR_OUT_OF_MEMORY) return rc;
     const bool tiles = rc == YULE_OK;
-    if (!tiles && per_seq > kPrefillChunk) per_seq = kPrefillChunk;
+    if ((!tiles || r->xchg) && per_seq > kPrefillChunk) per_seq = kPrefillChunk;
     if (fed && per_seq * batch > r->pf_chunk) per_seq = r->pf_chunk / batch;  // (a batch is no larger than the basic chunk)
     if ((rc = ensure_batch_graph(r))) return rc;
     // prompts to the device, pass by pass, the rows of a pass in the order of the sequences
