@@ -118,7 +118,9 @@ bool yule_cuda_ctx::find(yule_buffer h, Buffer *out, const char *what) {
 #define CTX_ENQUEUE(ctx)                                                      \
     if (!(ctx)) return fail(YULE_ERR_INVALID_ARGUMENT, "null context");       \
     std::lock_guard<std::recursive_mutex> _order((ctx)->enqueue_mu);          \
-    CTX_GUARD(ctx)
+    const yule_cuda_ctx::Chain _chain = (ctx)->take_held_chain();             \
+    (void)_chain;                                                             \
+    YULE_CUDA_TRY(cudaSetDevice((ctx)->device))
 
 #define FIND(ctx, handle, var)  \
     Buffer var;                 \

@@ -122,12 +122,15 @@ struct yule_cuda_ctx {
         int n;
     };
     // Ends the chain; what it was, for those that go on with it (they hold enqueue_mu until they have).
-    Chain take_chain() {
-        std::lock_guard<std::recursive_mutex> lock(enqueue_mu);
+    Chain take_held_chain() {
         const Chain was{pdl_chain, chain_n};
         pdl_chain = false;
         chain_n = 0;
         return was;
+    }
+    Chain take_chain() {
+        std::lock_guard<std::recursive_mutex> lock(enqueue_mu);
+        return take_held_chain();
     }
 
     // Looks a handle up under the lock; returns false (and sets the error) when unknown.
