@@ -8,7 +8,7 @@ import re
 
 import pytest
 
-from test_gemm_rings import Barrier
+from interleavings import Barrier, interleave
 
 WARPS, SOFT = 4, 8  # warps that read the output; that make probabilities
 
@@ -159,19 +159,7 @@ def simulate(seed, n, o_waits=True, alpha_waits=True, exchange=exchange_of_the_s
                 check(4 * (half * 128 + r), 4, ("sum", half, r))
 
     roles = [issue()] + [softmax(w) for w in range(SOFT)] + [sums(w) for w in range(WARPS)] + [load(x) for x in "kv"]
-    waits = {r: next(r, None) for r in roles}
-    speed = {r: rng.choice([1, 1, 3, 20]) for r in roles}
-    waits = {r: c for r, c in waits.items() if c is not None}
-    while waits or queue:
-        ready = [r for r, c in waits.items() if c()]
-        assert ready or queue, "nothing can go on"
-        if queue and (not ready or rng.random() < 0.3):
-            queue.pop(0)()
-            continue
-        r = rng.choices(ready, [1 / speed[x] for x in ready])[0]
-        waits[r] = next(r, None)
-        if waits[r] is None:
-            del waits[r]
+    interleave(rng, roles, [queue])
 
 
 @pytest.mark.parametrize("n", [1, 2, 3, 8, 13])

@@ -7,7 +7,7 @@ import re
 
 import pytest
 
-from test_gemm_rings import Barrier
+from interleavings import Barrier, interleave
 
 with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "yule_b200", "csrc", "qgemm_int.cu")) as f:
     SOURCE = f.read()
@@ -88,20 +88,7 @@ def simulate(seed, nbuf, name, blocks, scale_ring=SCALES):
                 a += 1
 
     roles = [producer(p) for p in range(WARPS + 1)] + [issuer(0), issuer(1)] + [drain() for _ in range(WARPS)]
-    waits = {r: next(r, None) for r in roles}
-    speed = {r: rng.choice([1, 1, 3, 20]) for r in roles}
-    waits = {r: c for r, c in waits.items() if c is not None}
-    while waits or queues[0] or queues[1]:
-        ready = [r for r, c in waits.items() if c()]
-        pipe = [q for q in queues if q]
-        assert ready or pipe, "nothing can go on"
-        if pipe and (not ready or rng.random() < 0.3):
-            rng.choice(pipe).pop(0)()
-            continue
-        r = rng.choices(ready, [1 / speed[x] for x in ready])[0]
-        waits[r] = next(r, None)
-        if waits[r] is None:
-            del waits[r]
+    interleave(rng, roles, queues)
 
 
 @pytest.mark.parametrize("bn,name,nbuf", CASES)

@@ -5,23 +5,10 @@ import random
 
 import pytest
 
+from interleavings import Barrier, interleave
 from test_gemm_pipeline_model import RINGS
 
 STAGES, WARPS = RINGS["q4k-128"].stages, 8
-
-
-class Barrier:
-    def __init__(self, count):
-        self.count, self.pending, self.done = count, count, 0
-
-    def arrive(self):
-        self.pending -= 1
-        assert self.pending >= 0, "more arrivals than a phase has"
-        if self.pending == 0:
-            self.pending, self.done = self.count, self.done + 1
-
-    def over(self, parity):  # what mbarrier.try_wait.parity can tell
-        return (self.done - 1) & 1 == parity
 
 
 def simulate(seed, nbuf, per_block, with_min, blocks):
@@ -77,25 +64,7 @@ def simulate(seed, nbuf, per_block, with_min, blocks):
             acc_empty[slot].arrive()
 
     roles = [producer(p) for p in range(WARPS + 1)] + [issuer(0), issuer(1)] + [drain() for _ in range(WARPS)]
-    waits = {}
-    speed = {}
-    for r in roles:
-        waits[r] = next(r, None)
-        speed[r] = rng.choice([1, 1, 3, 20])
-    while waits or queues[0] or queues[1]:
-        ready = [r for r, c in waits.items() if c is None or c()]
-        pipe = [q for q in queues if q]
-        assert ready or pipe, "nothing can go on"
-        if pipe and (not ready or rng.random() < 0.3):
-            rng.choice(pipe).pop(0)()
-            continue
-        r = rng.choices(ready, [1 / speed[x] for x in ready])[0]
-        if waits[r] is None:
-            del waits[r]
-            continue
-        waits[r] = next(r, None)
-        if waits[r] is None:
-            del waits[r]
+    interleave(rng, roles, queues)
 
 
 # accumulators, stages per super-block, min term of every instantiation, as the source has them
