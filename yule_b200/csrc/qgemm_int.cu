@@ -13,7 +13,7 @@
 //   Q6_K        sc·(q − 32) has up to 13 bits: hi (rounded to 11) and lo (the rest, exact), three MMAs per 16 columns, drained with d.
 //
 // An accumulator of Q4_K holds two stages, which halves the drains: gate / up of the 8B shape against 2047 rows 894 us in qgemm_tc.cu, 831 here (1160 TFLOP/s of MMAs; cuBLAS
-// sustains 1397), error against 64 bits 2.8e-7 and 1.3e-7.  The others hold one: two would take 7 to 12 % less time, but the adder truncates, and at 2048
+// sustains 1397; both as first measured), error against 64 bits 2.8e-7 and 1.3e-7.  The others hold one: two would take 7 to 12 % less time, but the adder truncates, and at 2048
 // columns the error would be 1.3e-7 where the kernel that these formats had before gave 1.25e-7.
 //
 // The weights arrive as tiled TMA boxes of one super-block (256 columns) of 128 rows: Q8_0 272 bytes a row, Q4_K and Q4_0 144, Q5_K 176 (odd multiples of 16: eight

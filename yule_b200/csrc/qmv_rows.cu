@@ -862,8 +862,8 @@ bool qmv_rows_over_matvecs(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint
 // 14336x4096 26.7, 24.0, 28672x4096 42.3, 42.4, 28672x8192 71.8, 83.5, 8192x28672 67.8, 84.4; 16 vectors 4096x4096 17.7, 13.7, 14336x4096 27.2, 29.2,
 // 8192x8192 28.8, 33.4.  (Up to twelve vectors it is this one also where the GEMM is faster: its accumulators truncate, and the error against
 // 64 bits would go from 1.6e-7 to 3.2e-7 to 4.0e-7, 4608x28672.)
-// The other formats' GEMM (qgemm_int.cu) has the error of this kernel (Q8_0 4096 columns and 24 vectors 0.9e-7 both, Q5_K 1.1e-7 against 1.4e-7), so time
-// decides; a seventeenth vector is a second pass here.  17, 24, 32 vectors, GEMM against this: Q5_K 2048x2048 17, 17, 17 against 15, 17, 20 us, 2048x5632 20, 20, 20
+// The other formats' GEMM (qgemm_int.cu) has the error of this kernel up to 4096 columns (Q8_0 by 24 vectors 1.0e-7 both, Q5_K 1.1e-7 both) and up to 6 % more beyond (14336 columns:
+// Q8_0 1.07e-7, 1.12e-7, Q5_K 1.17, 1.19, Q6_K 1.14, 1.20; 65536: Q6_K 1.25, 1.35), so time decides; a seventeenth vector is a second pass here.  17, 24, 32 vectors, GEMM against this: Q5_K 2048x2048 17, 17, 17 against 15, 17, 20 us, 2048x5632 20, 20, 20
 // against 22, 24, 33, 8192x28672 112, 113, 114 against 170, 188, 232; Q6_K 2048x2048 18, 18, 18 against 15, 17, 19, 4096x4096 18, 19, 19 against 23, 24, 27; Q8_0 2048x2048 20, 21, 21
 // against 14, 15, 16, 2048x5632 23, 23, 24 against 21, 24, 27, 8192x8192 47, 47, 47 against 44, 50, 61, 4096x14336 40, 40, 41 against 47, 52, 81; Q4_0 the same within 10 %.
 bool qmv_rows_preferred(uint32_t type, uint64_t n_rows, uint32_t n_cols, uint32_t batch) {
